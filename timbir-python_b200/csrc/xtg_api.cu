@@ -1812,12 +1812,11 @@ static int run_columns(xtg_ctx *c, int iter, const int4 *items, int lo, int n, c
     CK(launch_magmap_zero(c->G, A, c->sm_count * 4, c->st));
     c->launches++;
   }
-  int grid;
+  int grid, nt = XTG_THREADS;
+  A.grab = 1;
   if (seq) {
     grid = 1;
   } else {
-    const int occ = icd_occupancy(vec, amode, 0, as, vcap, zmax, g.zovl);
-    grid = c->sm_count * occ;
     // Columns updated at the same time read each other's stale error
     // sinogram; near neighbours share most of their footprint, so too many
     // of them at once overshoot (Jacobi-like) and the cost stops falling.
@@ -1825,12 +1824,21 @@ static int run_columns(xtg_ctx *c, int iter, const int4 *items, int lo, int n, c
     // 32^2-column grid 64 and more at once left the cost oscillating 20-50 %
     // above the converged value, 32 did not; grids of 256^2 columns and up
     // keep every resident CTA busy.
-    grid = std::min(grid, std::max(8, (int)(((long long)g.N_time * c->n_masked) / XTG_CONC_DIV)));
-    if (c->max_columns > 0) grid = std::min(grid, c->max_columns);
-    if (!n_dev) grid = std::min(grid, std::max(n * nsub, 1));
+    int cols = std::max(8, (int)(((long long)g.N_time * c->n_masked) / XTG_CONC_DIV));
+    if (c->max_columns > 0) cols = std::min(cols, c->max_columns);
+    // items of this launch; a selection keeps about one column in
+    // XT_NHICD_CHUNKS, half of them in each half-pass
+    const long long nexp = (n_dev ? (long long)g.N_time * g.nzb * (c->n_masked / XT_NHICD_CHUNKS) / 2 : n) * (long long)nsub;
+    if (!n_dev) cols = std::min(cols, (int)std::max(nexp, 1ll));
+    nt = icd_threads(vec, amode, 0, zmax, g.zovl, vcap, cols, c->sm_count);
+    grid = std::min(cols, c->sm_count * icd_occupancy(vec, amode, 0, as, vcap, zmax, g.zovl, nt));
+    // a batch per atomic only where every CTA gets several of them: eight at a
+    // time left 205 of 512 CTAs with all of a 128^2 x 4 launch's items (69 us
+    // a launch against 38)
+    if (nt < XTG_THREADS) A.grab = (int)std::max(1ll, std::min(8ll, nexp / (4ll * grid)));
   }
   CK(cudaMemsetAsync(c->d_counter, 0, 4, c->st));
-  CK(launch_icd(c->G, A, vec, amode, seq, as, vcap, zmax, grid, c->st));
+  CK(launch_icd(c->G, A, vec, amode, seq, as, vcap, zmax, grid, nt, c->st));
   c->icd_launches++;
   c->launches++;
   return 0;

@@ -21,26 +21,26 @@
 
 namespace xtg {
 
-// Work items of at most XTG_SMALL_ROWS detector rows run in CTAs of
-// XTG_SMALL_NT threads (table modes, parallel schedule).
-#ifndef XTG_SMALL_ROWS
-#define XTG_SMALL_ROWS 16
-#endif
-#ifndef XTG_SMALL_NT
-#define XTG_SMALL_NT 64
-#endif
-// Longer items whose column runs hold at most XTG_MEDIUM_ENTRIES A entries
-// run in CTAs of XTG_MEDIUM_NT threads (table modes, parallel schedule): the
-// per-item fixed work weighs more when the footprint is short, and twice as
-// many CTAs per SM overlap it better.  The largest 4D volume (352 entries
-// per column and frame): 745 -> 888 M voxel updates/s; 64 threads: equal;
-// plain 3D (2195 entries) in 128-thread CTAs: 221 against 241 M.
-#ifndef XTG_MEDIUM_ENTRIES
-#define XTG_MEDIUM_ENTRIES 1024
-#endif
-#ifndef XTG_MEDIUM_NT
-#define XTG_MEDIUM_NT 128
-#endif
+// Threads per CTA.  An item's row groups (16 bytes of e and of w of one
+// footprint entry) are dealt to the CTA's threads, so small items want small
+// CTAs (the fixed work of an item -- neighbourhood, A staging, barriers, the
+// surrogate step -- then overlaps over more items at once) and long items, or
+// few columns in flight, want large ones.  icd_threads picks the size per
+// launch from these three, all measured:
+// XTG_GROUPS_LONG: row groups per thread above which an item counts as long.
+// 24 / 48 / 96: 256^2 x 32, 512 views, a scan step 12.6 / 11.6 / 11.3 ms (17.8
+// with 64 threads for every item of at most 16 rows); 108^2 x 85 x 8 frames
+// 9.8 / 8.5 / 8.5 ms; 260^2 x 4, 602 views 6.75 / 6.75 / 6.94 ms.
+#define XTG_GROUPS_LONG 48
+// XTG_GROUPS_PER_THREAD: below it a larger CTA no longer helps to fill the
+// SMs.  2 / 4 / 8: 128^2 x 4, 180 views 3.15 / 2.69 / 2.61 ms an iteration.
+#define XTG_GROUPS_PER_THREAD 8
+// XTG_FILL4: quarters of the SMs' threads that the columns in flight must
+// leave idle before larger CTAs are taken.  2 / 3 / 4: the 128^2 x 16 coarse
+// stage of a 256^2 x 32 start 166 / 166 / 180 ms (319 with 64 threads).
+#define XTG_FILL4 3
+#define XTG_NT_MIN 64
+#define XTG_NT_MAX 1024
 
 // Footprint loads with L2 cache hints: e (re-read and updated through L2 by
 // other columns' reductions) is kept (evict_last), w (read once per visit) is
@@ -82,7 +82,7 @@ __device__ __forceinline__ void cp_async4(void *s, const void *g) {
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Where a work item's column run lies in the A column table, fetched for the
-// next item while the current one is processed (small CTAs).
+// next item while the current one is processed.
 struct ItemMeta {
   int4 item;           // frame, row, column, z-block
   long long s0, s1;    // tstart[ti], tstart[ti + 1]
@@ -145,25 +145,10 @@ __device__ __forceinline__ Nbr nbr_term(const DevGeo &G, const float *sNb, const
   return o;
 }
 
-// Next-item prefetch in the 256-thread CTAs too (the small ones always):
-// measured equal on plain 3D (237.6-238.5 against 236.5-237.1 M voxel
-// updates/s), so off
-#ifndef XTG_PF_ALL
-#define XTG_PF_ALL 0
-#endif
-
-// resident 256-thread CTAs per SM the register budget is cut for (5: 48
-// registers with spills, 8 % slower on plain 3D)
-#ifndef XTG_CTAS_256
-#define XTG_CTAS_256 4
-#endif
-
-// NT threads per CTA: 256 for long z-lines; 64 where a work item is short
-// (few detector rows), so the per-item fixed work (neighbourhood, A staging,
-// barriers, the surrogate step) runs in four times as many CTAs at once.
+// Every CTA size keeps 1024 threads resident per SM (64 registers a thread;
+// 1280, 48 registers with spills, measured 8 % slower on plain 3D).
 template <int VEC, int AMODE, int SEQ, int AS, int NT = XTG_THREADS>
-__global__ void __launch_bounds__(NT, NT == XTG_THREADS ? XTG_CTAS_256 : 1024 / NT) k_icd_columns(DevGeo G, IcdArgs A, int vmax,
-                                                                                 int zmax) {
+__global__ void __launch_bounds__(NT, 1024 / NT) k_icd_columns(DevGeo G, IcdArgs A, int vmax, int zmax) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int NW = NT / 32;
   unsigned char *smem = smem_raw;
@@ -188,25 +173,24 @@ __global__ void __launch_bounds__(NT, NT == XTG_THREADS ? XTG_CTAS_256 : 1024 / 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nitems = A.n_items_dev ? *A.n_items_dev : A.n_items;
   const bool hlo = A.halo_lo != nullptr, hhi = A.halo_hi != nullptr;
-  // Short items (small CTAs) are taken GRAB at a time and the CTA's
-  // statistics are added up in thread 0 and flushed once at the end: with
-  // tens of thousands of items per launch, per-item atomics on the same few
-  // addresses would queue at L2.
+  // Items are taken A.grab at a time and the CTA's statistics are added up in
+  // thread 0 and flushed once at the end: with tens of thousands of items per
+  // launch, per-item atomics on the same few addresses would queue at L2.
   // (kept in shared memory: registers are the kernel's occupancy limit)
-  constexpr int GRAB = NT < XTG_THREADS ? 8 : 1;
   __shared__ int sGrab[2];                 // base, next of the batch
   __shared__ double sCtaAbs;
   __shared__ unsigned long long sCta[3];   // voxel updates, zero skipped, items
-  // Small CTAs fetch the next item's record and table run asynchronously in
-  // three dependent steps (record; column rank; run bounds), one per phase of
-  // the current item, so that the chain's round trips overlap its work.
-  constexpr bool PF = (NT < XTG_THREADS || XTG_PF_ALL) && AMODE != 0 && !SEQ;
+  // The next item's record and table run are fetched asynchronously in three
+  // dependent steps (record; column rank; run bounds), one per phase of the
+  // current item, so that the chain's round trips overlap its work (in the
+  // 256-thread CTAs 118.5 -> 117.2 ms per plain-3D iteration).
+  constexpr bool PF = AMODE != 0 && !SEQ;
   __shared__ __align__(16) ItemMeta sMeta[2];
   int mb = 0;  // sMeta[mb]: the current item; sMeta[mb ^ 1]: the next
   const int total = nitems * A.nsub;
   auto grab = [&]() -> int {  // thread 0 only
-    if (sGrab[1] == GRAB) {
-      sGrab[0] = atomicAdd(A.counter, GRAB);
+    if (sGrab[1] == A.grab) {
+      sGrab[0] = atomicAdd(A.counter, A.grab);
       sGrab[1] = 0;
     }
     return sGrab[0] + sGrab[1]++;
@@ -239,7 +223,7 @@ __global__ void __launch_bounds__(NT, NT == XTG_THREADS ? XTG_CTAS_256 : 1024 / 
   };
   if (tid == 0) {
     sGrab[0] = 0;
-    sGrab[1] = GRAB;
+    sGrab[1] = A.grab;
     sCtaAbs = 0.0;
     sCta[0] = sCta[1] = sCta[2] = 0;
     if (PF) {
@@ -294,7 +278,7 @@ __global__ void __launch_bounds__(NT, NT == XTG_THREADS ? XTG_CTAS_256 : 1024 / 
     //    as the reference's ranks read Object[i][0] / [N_z+1],
     //    XT_VoxUpdate.c:94-99)
     const size_t plane = (size_t)G.N_y * G.N_x;
-    // (small CTAs, FP32 table) the column's table run goes to shared memory
+    // (FP32 table) the column's table run goes to shared memory
     // asynchronously first, so that its round trip overlaps the
     // neighbourhood's; a quiet line (below) has fetched it for nothing
     constexpr bool PFE = PF && AMODE == 2;
@@ -526,7 +510,27 @@ __global__ void __launch_bounds__(NT, NT == XTG_THREADS ? XTG_CTAS_256 : 1024 / 
           accumulate(en.x, __int_as_float(en.y));
         }
       } else {
-        for (int e = vg; e < ne; e += vgs) {
+        // single rows: four entries' loads in flight (one at a time left the
+        // loop waiting on each round trip)
+        int e = vg;
+        constexpr int UNR = 4;
+        for (; e + (UNR - 1) * vgs < ne; e += UNR * vgs) {
+          int2 en[UNR];
+          float ev[UNR], wv[UNR];
+#pragma unroll
+          for (int u = 0; u < UNR; u++) en[u] = sEnt[e + u * vgs];
+#pragma unroll
+          for (int u = 0; u < UNR; u++) {
+            ev[u] = __ldcg(eb + en[u].x);
+            wv[u] = __ldg(wb + en[u].x);
+          }
+#pragma unroll
+          for (int u = 0; u < UNR; u++) {
+            const float e1[VEC] = {ev[u]}, w1[VEC] = {wv[u]};
+            accumulate_arr(e1, w1, __int_as_float(en[u].y));
+          }
+        }
+        for (; e < ne; e += vgs) {
           const int2 en = sEnt[e];
           accumulate(en.x, __int_as_float(en.y));
         }
@@ -789,17 +793,27 @@ typedef void (*IcdKernel)(DevGeo, IcdArgs, int, int);
 static IcdKernel icd_kernel(int vec, int amode, int seq, int as, int nt) {
 #define XTG_K(V, S) (as == 3 ? k_icd_columns<V, 0, S, 3> : as == 4 ? k_icd_columns<V, 0, S, 4> : k_icd_columns<V, 0, S, 12>)
 #define XTG_T(V, M, S) k_icd_columns<V, M, S, 3>
-  if (nt != XTG_THREADS && vec == 4 && amode != 0 && !seq)  // short items, table modes
-    return nt == XTG_SMALL_NT ? (amode == 1 ? k_icd_columns<4, 1, 0, 3, XTG_SMALL_NT> : k_icd_columns<4, 2, 0, 3, XTG_SMALL_NT>)
-                              : (amode == 1 ? k_icd_columns<4, 1, 0, 3, XTG_MEDIUM_NT> : k_icd_columns<4, 2, 0, 3, XTG_MEDIUM_NT>);
+  if (amode != 0 && !seq) {
+#define XTG_N(V, M)                                                                                                 \
+  switch (nt) {                                                                                                     \
+    case 64: return k_icd_columns<V, M, 0, 3, 64>;                                                                  \
+    case 128: return k_icd_columns<V, M, 0, 3, 128>;                                                                \
+    case 256: return k_icd_columns<V, M, 0, 3, 256>;                                                                \
+    case 512: return k_icd_columns<V, M, 0, 3, 512>;                                                                \
+    default: return k_icd_columns<V, M, 0, 3, 1024>;                                                                \
+  }
+    if (vec == 4 && amode == 1) XTG_N(4, 1)
+    if (vec == 4) XTG_N(4, 2)
+    if (amode == 1) XTG_N(1, 1)
+    XTG_N(1, 2)
+#undef XTG_N
+  }
   if (vec == 4) {
     if (amode == 0) return seq ? XTG_K(4, 1) : XTG_K(4, 0);
-    if (amode == 1) return seq ? XTG_T(4, 1, 1) : XTG_T(4, 1, 0);
-    return seq ? XTG_T(4, 2, 1) : XTG_T(4, 2, 0);
+    return amode == 1 ? XTG_T(4, 1, 1) : XTG_T(4, 2, 1);
   }
   if (amode == 0) return seq ? XTG_K(1, 1) : XTG_K(1, 0);
-  if (amode == 1) return seq ? XTG_T(1, 1, 1) : XTG_T(1, 1, 0);
-  return seq ? XTG_T(1, 2, 1) : XTG_T(1, 2, 0);
+  return amode == 1 ? XTG_T(1, 1, 1) : XTG_T(1, 2, 1);
 #undef XTG_K
 #undef XTG_T
 }
@@ -823,16 +837,24 @@ cudaError_t launch_magmap_zero(const DevGeo &G, const IcdArgs &A, int grid, cuda
   return cudaGetLastError();
 }
 
-// threads per CTA for items of zmax slices: XTG_SMALL_NT for short table-mode items
-int icd_threads(int vec, int amode, int seq, int zmax, int zovl, int vmax) {
-  if (vec == 4 && amode != 0 && !seq && zmax * zovl <= XTG_SMALL_ROWS) return XTG_SMALL_NT;
-  if (vec == 4 && amode != 0 && !seq && vmax <= XTG_MEDIUM_ENTRIES) return XTG_MEDIUM_NT;
-  return XTG_THREADS;
+// Threads per CTA for items of zmax slices, at most `cols` of them in flight
+// on `sms` SMs.  Table modes, parallel schedule; otherwise XTG_THREADS.
+int icd_threads(int vec, int amode, int seq, int zmax, int zovl, int vmax, int cols, int sms) {
+  if (amode == 0 || seq) return XTG_THREADS;
+  int tlp = 1;
+  while (tlp * vec < zmax * zovl) tlp *= 2;
+  const long long groups = (long long)tlp * vmax;
+  int nt = XTG_NT_MIN;
+  // long items
+  while (nt < XTG_THREADS && groups > (long long)nt * XTG_GROUPS_LONG) nt *= 2;
+  // too few columns in flight to fill the SMs' 1024 threads each
+  while (nt < XTG_NT_MAX && (long long)cols * nt * 4 < (long long)sms * 1024 * XTG_FILL4 && groups > (long long)nt * XTG_GROUPS_PER_THREAD)
+    nt *= 2;
+  return nt;
 }
 
 cudaError_t launch_icd(const DevGeo &G, const IcdArgs &A, int vec, int amode, int seq, int as, int vmax, int zmax,
-                       int grid, cudaStream_t st) {
-  const int nt = icd_threads(vec, amode, seq, zmax, G.zovl, vmax);
+                       int grid, int nt, cudaStream_t st) {
   const size_t smem = icd_smem_bytes(vmax, zmax, G.zovl, as, amode, vec, nt);
   IcdKernel k = icd_kernel(vec, amode, seq, as, nt);
   cudaError_t e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -846,8 +868,7 @@ cudaError_t launch_icd(const DevGeo &G, const IcdArgs &A, int vec, int amode, in
   return cudaGetLastError();
 }
 
-int icd_occupancy(int vec, int amode, int seq, int as, int vmax, int zmax, int zovl) {
-  const int nt = icd_threads(vec, amode, seq, zmax, zovl, vmax);
+int icd_occupancy(int vec, int amode, int seq, int as, int vmax, int zmax, int zovl, int nt) {
   const size_t smem = icd_smem_bytes(vmax, zmax, zovl, as, amode, vec, nt);
   IcdKernel k = icd_kernel(vec, amode, seq, as, nt);
   int nb = 0;

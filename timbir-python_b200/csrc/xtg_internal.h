@@ -16,6 +16,7 @@ struct IcdArgs {
   int n_items;             // host item count when n_items_dev is null
   int item_lo;             // first item index of this launch
   int *counter;
+  int grab;                // items a CTA takes per atomic on the counter
   int use_perm;
   unsigned long long perm_key;
   // z-slab split: base item i is processed as nsub pieces of at most zslab
@@ -90,7 +91,8 @@ cudaError_t launch_fbp(const DevGeo &G, const float *y, const float *d, float *q
                        const int *col_rank, float *x, cudaStream_t st);
 cudaError_t launch_magmap_zero(const DevGeo &G, const IcdArgs &A, int grid, cudaStream_t st);
 cudaError_t launch_icd(const DevGeo &G, const IcdArgs &A, int vec, int amode, int seq, int as, int vmax, int zmax,
-                       int grid, cudaStream_t st);
-int icd_occupancy(int vec, int amode, int seq, int as, int vmax, int zmax, int zovl);
+                       int grid, int nt, cudaStream_t st);
+int icd_threads(int vec, int amode, int seq, int zmax, int zovl, int vmax, int cols, int sms);
+int icd_occupancy(int vec, int amode, int seq, int as, int vmax, int zmax, int zovl, int nt);
 
 }  // namespace xtg
