@@ -1806,6 +1806,9 @@ static int run_columns(xtg_ctx *c, int iter, const int4 *items, int lo, int n, c
   A.tstart = c->d_tstart; A.toff = c->d_toff; A.tval32 = c->d_tval32; A.tval16 = c->d_tval16; A.tscale = c->d_tscale;
   A.T2 = g.T * g.T; A.Tdelta = g.T * g.delta; A.st_absx = c->d_absx; A.st_cnt = c->d_cnt; A.err = c->d_err;
   A.zslab = hz; A.nsub = nsub;
+  A.e2p = 2.0f - g.MRF_P;
+  A.l_sqp = (float)log2((double)g.Sigma_S_Q_P); A.l_tqp = (float)log2((double)g.Sigma_T_Q_P);
+  A.inv_sq = (float)(1.0 / g.Sigma_S_Q); A.inv_tq = (float)(1.0 / g.Sigma_T_Q);
   A.halo_lo = c->halo_lo; A.halo_hi = c->halo_hi;
   A.w_keep = XTG_W_KEEP && 2 * c->ns * 4 <= (size_t)XTG_W_KEEP_BYTES;
   if (nsub > 1) {

@@ -7,11 +7,22 @@
 // registers, or read from the FP16 table), then streams the column's
 // footprint e[p][bin][t0..t0+T) and w[...] (contiguous in t) with 16-byte
 // loads, thread (view group, t lane) accumulating theta1/theta2 for its rows;
-// shuffles and one shared-memory pass reduce them over view groups.  The
-// slices' qGGMRF surrogate steps run in red/black z order with 8 lanes per
-// voxel (or strictly in increasing z on one thread, the reference's order, in
-// sequential mode), and the e update goes back with vector red.global.add,
-// so columns in flight that share sinogram entries never lose an update.
+// shuffles reduce them over view groups inside a warp.  The qGGMRF surrogate
+// sums over the neighbours that the visit does not change are formed by all
+// threads before the footprint is read; then one warp adds the theta partials
+// and takes the slices' steps in red/black z order, a lane per voxel (or
+// strictly in increasing z on one thread, the reference's order, in
+// sequential mode), while another fetches the next item's record, and the e
+// update goes back with vector red.global.add, so columns in flight that
+// share sinogram entries never lose an update.
+//
+// What bounds it.  Short items: the fixed chain of an item.  With the whole
+// surrogate step between two barriers, per-phase barriers and block-wide
+// statistics a 16-row item of 137 entries took 35,000 cycles, 11,000 of them
+// in that step; with four barriers and the split above 19,000 (4D 256^2 x 16 x
+// 16: 24.8 -> 19.4 ms an iteration, 128^2 x 4: 2.67 -> 2.40 ms).  Long ones:
+// the L2, which serves 9 TB/s of e and w plus the reductions in the footprint
+// loop of plain 3D (117.5 -> 115.6 ms).
 //
 // Reference: updateVoxels_Aditya + compute_voxel_update_Aditya
 // (Source_Code_4D_Fast/XT_VoxUpdate.c:11-254), CE_FunctionalSubstitution
@@ -81,15 +92,13 @@ __device__ __forceinline__ void cp_async4(void *s, const void *g) {
 }
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Where a work item's column run lies in the A column table, fetched for the
-// next item while the current one is processed.
+// A work item and where its column run lies in the A column table, fetched
+// for the next item while the current one is processed.
 struct ItemMeta {
   int4 item;           // frame, row, column, z-block
   long long s0, s1;    // tstart[ti], tstart[ti + 1]
   float sc;            // tscale[ti] (FP16 table)
-  int rank;            // col_rank[row][column]
   int it;              // launch-wide item index (>= the launch's total: none)
-  int pad;
 };
 
 // Packed FP32 (two lanes per instruction, sm_100) for the footprint
@@ -106,43 +115,19 @@ struct ItemMeta {
 #define XTG_UNROLL 2
 #endif
 
-// surrogate coefficient with fast intrinsics: the step size only needs a few
-// digits, the fixed point of the iteration is unchanged
-__device__ __forceinline__ float qcoef_fast(float d, float sq, float sqp, float c, float p) {
-  if (d == 0.f) return __fdividef(2.0f, sq * c);
-  const float t1 = __fdividef(__powf(fabsf(d), 2.0f - p), sqp);
-  const float t3 = c + t1;
-  return __fdividef(2.0f - __fdividef((2.0f - p) * t1, t3), t3 * sq);
-}
-
-// the 29 neighbour slots of a voxel: 0..26 the 3x3x3 block in [dz][dy][dx]
-// order (13 = the voxel itself, skipped), 27 = frame - 1, 28 = frame + 1
-struct Nbr {
-  float v;
-  float b;  // filter weight * surrogate coefficient, 0 when the slot is absent
-};
-
-// hlo / hhi: the slices below slice 0 and above slice N_z - 1 belong to a
-// neighbouring slab (their values are staged in sNb like any other)
-__device__ __forceinline__ Nbr nbr_term(const DevGeo &G, const float *sNb, const float *sTn, int zmax, int z, int zb,
-                                        int fr, int row, int col, float Vv, int n, bool hlo, bool hhi) {
-  Nbr o{0.f, 0.f};
-  if (n < 27) {
-    if (n == 13) return o;
-    const int dz = n / 9, c = n % 9;
-    const int za = zb + z + dz - 1;
-    if ((za < 0 && !hlo) || (za >= G.N_z && !hhi)) return o;
-    const int jj = row + c / 3 - 1, kk = col + c % 3 - 1;
-    if (jj < 0 || jj >= G.N_y || kk < 0 || kk >= G.N_x) return o;
-    o.v = sNb[c * (zmax + 2) + z + dz];
-    o.b = G.SF[n] * qcoef_fast(Vv - o.v, G.Sigma_S_Q, G.Sigma_S_Q_P, G.C_S, G.MRF_P);
-  } else {
-    const int f2 = fr + (n == 27 ? -1 : 1);
-    if (f2 < 0 || f2 >= G.N_time) return o;
-    o.v = sTn[(n - 27) * zmax + z];
-    o.b = G.TF * qcoef_fast(Vv - o.v, G.Sigma_T_Q, G.Sigma_T_Q_P, G.C_T, G.MRF_P);
-  }
-  return o;
+// sigma_q times the surrogate coefficient rho'(d) / d of the qGGMRF prior with
+// q = 2 (CE_QGGMRF, XT_ICD_update.c:79-125): with t = |d|^(2-p) / sigma_qp it is
+// (2 - (2-p) t / (c+t)) / (c+t) = (2c + p t) / (c+t)^2, one reciprocal; t comes
+// from the special-function unit's log2 and 2^x (lq = log2 sigma_qp).  The step
+// size only needs a few digits, the fixed point of the iteration is unchanged.
+__device__ __forceinline__ float qcoef(float d, float c, float lq, float e2p, float p) {
+  const float ad = fabsf(d);
+  float l, t;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(ad));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(e2p, l, -lq)));
+  t = ad == 0.f ? 0.f : t;
+  const float r = __fdividef(1.0f, c + t);
+  return fmaf(p, t, 2.0f * c) * r * r;
 }
 
 // Every CTA size keeps 1024 threads resident per SM (64 registers a thread;
@@ -159,99 +144,72 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_icd_columns(DevGeo G, IcdArgs
   // AMODE 1/2 (column table): the column's entry run, vmax = longest run,
   // {(p*N_r + bin)*N_t, bits of A * delta_t} per entry (one 8-byte load)
   int2 *sEnt = reinterpret_cast<int2 *>(smem);           // [vmax]
-  float *sRed = (AMODE == 0) ? sVal + (size_t)vmax * AS : reinterpret_cast<float *>(sEnt + vmax);  // [2][NW][128]
-  float *sTh = sRed + 2 * NW * 128;                       // [2][zmax*zovl]
-  const int rowsmax = zmax * G.zovl;
-  float *sNb = sTh + 2 * rowsmax;                         // [9][zmax+2]
+  const int rowsmax = zmax * G.zovl, rp = (rowsmax + 3) & ~3;
+  float *sRed = (AMODE == 0) ? sVal + (size_t)vmax * AS : reinterpret_cast<float *>(sEnt + vmax);  // [2][NW][rp]
+  float *sNb = sRed + 2 * NW * rp;                        // [9][zmax+2]
   float *sTn = sNb + 9 * (zmax + 2);                      // [2][zmax]
   float *sDelta = sTn + 2 * zmax;                         // [zmax]
+  float *sNum = sDelta + zmax;                            // [zmax] sum of b * neighbour, then
+  float *sDen = sNum + zmax;                              // [zmax] sum of b, over the slots outside the column
+  int *sPos = reinterpret_cast<int *>(sDen + zmax);       // [zmax] one of those neighbours is positive
 
-  __shared__ int sItem;
-  __shared__ double sAbs[NT / 32];
-  __shared__ unsigned sUpd, sZero;
+  __shared__ float sW[28];                  // filter weight / sigma_q: 27 spatial slots, temporal
+  __shared__ double sAbs[32];               // statistics of warp 0's lanes over the CTA's items
+  __shared__ unsigned sUpd[32], sZero[32];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nitems = A.n_items_dev ? *A.n_items_dev : A.n_items;
   const bool hlo = A.halo_lo != nullptr, hhi = A.halo_hi != nullptr;
-  // Items are taken A.grab at a time and the CTA's statistics are added up in
-  // thread 0 and flushed once at the end: with tens of thousands of items per
-  // launch, per-item atomics on the same few addresses would queue at L2.
-  // (kept in shared memory: registers are the kernel's occupancy limit)
-  __shared__ int sGrab[2];                 // base, next of the batch
-  __shared__ double sCtaAbs;
-  __shared__ unsigned long long sCta[3];   // voxel updates, zero skipped, items
-  // The next item's record and table run are fetched asynchronously in three
-  // dependent steps (record; column rank; run bounds), one per phase of the
-  // current item, so that the chain's round trips overlap its work (in the
-  // 256-thread CTAs 118.5 -> 117.2 ms per plain-3D iteration).
-  constexpr bool PF = AMODE != 0 && !SEQ;
+  const int total = nitems * A.nsub;
+  // The first lane of the last warp fetches the next item's record and table
+  // run (a chain of four dependent reads) while warp 0 does the current
+  // item's surrogate step.  Items are taken A.grab at a time and the CTA's
+  // statistics are flushed once at the end: with tens of thousands of items
+  // per launch, per-item atomics on the same few addresses would queue at L2.
+  constexpr int META = NT - 32;
   __shared__ __align__(16) ItemMeta sMeta[2];
   int mb = 0;  // sMeta[mb]: the current item; sMeta[mb ^ 1]: the next
-  const int total = nitems * A.nsub;
-  auto grab = [&]() -> int {  // thread 0 only
-    if (sGrab[1] == A.grab) {
-      sGrab[0] = atomicAdd(A.counter, A.grab);
-      sGrab[1] = 0;
-    }
-    return sGrab[0] + sGrab[1]++;
-  };
+  __shared__ int sGrab[2];  // the batch taken last: next item, items left
   auto item_index = [&](int i) -> int {
     const int ii = A.nsub == 1 ? i : i % nitems;
     return A.item_lo + (A.use_perm ? (int)xt_perm((uint32_t)ii, (uint32_t)nitems, A.perm_key) : ii);
   };
-  auto fetch_rank = [&]() {  // thread 0, the next item's record in place
-    ItemMeta &N = sMeta[mb ^ 1];
-    if (N.it < total) cp_async4(&N.rank, A.col_rank + N.item.y * G.N_x + N.item.z);
-  };
-  auto fetch_bounds = [&]() {  // thread 0, the next item's rank in place
-    ItemMeta &N = sMeta[mb ^ 1];
-    if (N.it < total) {
-      const long long ti = (long long)N.item.x * A.n_masked + N.rank;
-      cp_async8(&N.s0, A.tstart + ti);
-      cp_async8(&N.s1, A.tstart + ti + 1);
-      if (AMODE == 1) cp_async4(&N.sc, A.tscale + ti);
+  auto fetch_meta = [&](ItemMeta &N) {  // thread META only
+    if (sGrab[1] == 0) {
+      sGrab[0] = atomicAdd(A.counter, A.grab);
+      sGrab[1] = A.grab;
     }
-  };
-  // the rank and run-bound steps with plain loads (prologue, skipped pieces)
-  auto meta_finish = [&](ItemMeta &N) {
+    N.it = sGrab[0]++;
+    sGrab[1]--;
     if (N.it >= total) return;
-    N.rank = A.col_rank[N.item.y * G.N_x + N.item.z];
-    const long long ti = (long long)N.item.x * A.n_masked + N.rank;
-    N.s0 = A.tstart[ti];
-    N.s1 = A.tstart[ti + 1];
-    N.sc = (AMODE == 1) ? A.tscale[ti] : 1.f;
+    const int4 q = A.items[item_index(N.it)];
+    N.item = q;
+    if (AMODE != 0) {
+      const long long ti = (long long)q.x * A.n_masked + A.col_rank[q.y * G.N_x + q.z];
+      N.s0 = A.tstart[ti];
+      N.s1 = A.tstart[ti + 1];
+      N.sc = (AMODE == 1) ? A.tscale[ti] : 1.f;
+    }
   };
-  if (tid == 0) {
-    sGrab[0] = 0;
-    sGrab[1] = A.grab;
-    sCtaAbs = 0.0;
-    sCta[0] = sCta[1] = sCta[2] = 0;
-    if (PF) {
-      sMeta[0].it = grab();
-      if (sMeta[0].it < total) {
-        sMeta[0].item = A.items[item_index(sMeta[0].it)];
-        meta_finish(sMeta[0]);
-      }
-    }
+  if (tid == META) {
+    sGrab[1] = 0;
+    fetch_meta(sMeta[0]);
   }
+  if (warp == 0) {
+    sAbs[lane] = 0.0;
+    sUpd[lane] = 0u;
+    sZero[lane] = 0u;
+    if (lane < 27) sW[lane] = G.SF[lane] * A.inv_sq;
+    if (lane == 27) sW[27] = G.TF * A.inv_tq;
+  }
+  unsigned ncol = 0;  // items whose first piece this CTA took
 
-  for (;;) {
-    if (tid == 0) {
-      if (PF) {
-        ItemMeta &N = sMeta[mb ^ 1];
-        N.it = grab();
-        if (N.it < total) cp_async16(&N.item, A.items + item_index(N.it));
-      } else {
-        sItem = grab();
-      }
-      sUpd = 0;
-      sZero = 0;
-    }
-    __syncthreads();
-    const int it = PF ? sMeta[mb].it : sItem;
+  for (;; mb ^= 1) {
+    __syncthreads();  // the item's record is in place, the previous item is done with shared memory
+    const int it = sMeta[mb].it;
     if (it >= total) break;
     const int piece = A.nsub == 1 ? 0 : it / nitems;
-    const int4 item = PF ? sMeta[mb].item : A.items[item_index(it)];
+    const int4 item = sMeta[mb].item;
     const int fr = item.x, row = item.y, col = item.z, blk = item.w;
     int zb = 0, ze = G.N_z - 1;
     if (blk >= 0) {
@@ -260,42 +218,34 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_icd_columns(DevGeo G, IcdArgs
     }
     zb += piece * A.zslab;
     if (zb > ze) {  // this item has fewer pieces (uniform over the CTA)
-      if (PF && tid == 0) {
-        cp_wait_all();
-        meta_finish(sMeta[mb ^ 1]);
-      }
-      __syncthreads();
-      mb ^= 1;
+      if (tid == META) fetch_meta(sMeta[mb ^ 1]);
       continue;
     }
+    if (piece == 0) ncol++;
     ze = min(ze, zb + A.zslab - 1);
     const int Z = ze - zb + 1, T = Z * G.zovl, t0 = zb * G.zovl;
-    const int V = A.view_num[fr], vs = A.view_start[fr];
 
-    // 1. neighbourhood: the 3x3 columns' z-lines over [zb-1, ze+1], and the
-    //    same column in frames fr-1 and fr+1 (0 outside the volume; slices
-    //    -1 and N_z from the neighbouring slabs' halo planes when present,
-    //    as the reference's ranks read Object[i][0] / [N_z+1],
-    //    XT_VoxUpdate.c:94-99)
-    const size_t plane = (size_t)G.N_y * G.N_x;
-    // (FP32 table) the column's table run goes to shared memory
-    // asynchronously first, so that its round trip overlaps the
-    // neighbourhood's; a quiet line (below) has fetched it for nothing
-    constexpr bool PFE = PF && AMODE == 2;
-    if (PFE) {
-      const long long s0 = sMeta[mb].s0;
-      const int n = (int)(sMeta[mb].s1 - s0);
-      for (int e = tid; e < n; e += NT) {
+    // 1. the column's table run (times delta_t, XT_VoxUpdate.c:27) goes to
+    //    shared memory asynchronously, so that its round trip overlaps the
+    //    neighbourhood's; a quiet line (below) has fetched it for nothing
+    const long long s0 = AMODE != 0 ? sMeta[mb].s0 : 0;
+    const int ne = AMODE != 0 ? (int)(sMeta[mb].s1 - s0) : 0;
+    if (AMODE != 0) {
+      for (int e = tid; e < ne; e += NT) {
         cp_async4(&sEnt[e].x, A.toff + s0 + e);
-        cp_async4(&sEnt[e].y, A.tval32 + s0 + e);
+        if (AMODE == 2) cp_async4(&sEnt[e].y, A.tval32 + s0 + e);
       }
     }
+    // the neighbourhood: the 3x3 columns' z-lines over [zb-1, ze+1], and the
+    // same column in frames fr-1 and fr+1 (0 outside the volume; slices -1
+    // and N_z from the neighbouring slabs' halo planes when present, as the
+    // reference's ranks read Object[i][0] / [N_z+1], XT_VoxUpdate.c:94-99)
+    const size_t plane = (size_t)G.N_y * G.N_x;
     // Zero skipping (XT_VoxUpdate.c:208-232) decided for the whole z-line
     // before any footprint work: from the second iteration a voxel equal to 0
     // with no positive spatial or temporal neighbour is not updated.  When
-    // that holds for every voxel of the item, theta is never used, so neither
-    // A nor the footprint is read (the update step below skips each voxel by
-    // the same test and the e update has nothing to add).  Each thread tests
+    // that holds for every voxel of the item, theta is never used, so the
+    // footprint is not read.  Each thread tests
     // the values it stages.
     bool quiet = A.iter > 1;
     // k / (Z + 2) as (k * mz2) >> 20: exact while k (Z + 2) < 2^20, and here
@@ -325,9 +275,39 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_icd_columns(DevGeo G, IcdArgs
       sTn[s * zmax + z] = v;
       if (v > 0.f) quiet = false;
     }
+    if (AMODE == 1) {
+      const float sc = sMeta[mb].sc;
+      for (int e = tid; e < ne; e += NT) sEnt[e].y = __float_as_int(__half2float(A.tval16[s0 + e]) * sc);
+    }
+    if (AMODE != 0) cp_wait_all();
     const bool skip_all = __syncthreads_and(quiet) != 0;
-    // 2. the column's A entries (times delta_t, XT_VoxUpdate.c:27) -> smem
-    if (AMODE == 0 && !skip_all) {
+    // MagUpdateMap[frame][block][row][col] = sum |delta| over the block's
+    // slices of this visit (XT_VoxUpdate.c:128, 236), lanes of one warp over blocks
+    auto write_magmap = [&]() {
+      for (int b = lane; b < G.nzb; b += 32) {
+        const int bz0 = b * G.zstep, bz1 = (b >= G.nzb - 1) ? G.N_z - 1 : (b + 1) * G.zstep - 1;
+        const int lo = max(bz0, zb), hi = min(bz1, ze);
+        if (lo > hi) continue;
+        float m = 0.f;
+        if (!skip_all)
+          for (int z = lo; z <= hi; z++) m += fabsf(sDelta[z - zb]);
+        float *mp = A.magmap + (((size_t)fr * G.nzb + b) * G.N_y + row) * G.N_x + col;
+        if (A.nsub > 1)
+          atomicAdd(mp, m);  // pieces of one block add into the entry zeroed before the launch
+        else if (bz0 >= zb && bz1 <= ze)
+          *mp = m;
+      }
+    };
+    if (skip_all) {  // uniform over the CTA
+      if (tid == 0) sZero[0] += (unsigned)Z;
+      if (tid == META) fetch_meta(sMeta[mb ^ 1]);
+      if (warp == NW - 1) write_magmap();
+      continue;
+    }
+    int V = 0;
+    if (AMODE == 0) {
+      const int vs = A.view_start[fr];
+      V = A.view_num[fr];
       for (int v = tid; v < V; v += NT) {
         const int p = A.view_idx[vs + v];
         float vals[AS];
@@ -339,37 +319,62 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_icd_columns(DevGeo G, IcdArgs
 #pragma unroll
         for (int s = 0; s < AS; s++) sVal[s * vmax + v] = __fmul_rn(vals[s], G.delta_t);
       }
+      __syncthreads();
     }
-    int ne = 0;
-    if (AMODE != 0 && !skip_all) {
-      long long s0;
-      float sc;
-      if (PF) {
-        s0 = sMeta[mb].s0;
-        ne = (int)(sMeta[mb].s1 - s0);
-        sc = sMeta[mb].sc;
-      } else {
-        const long long ti = (long long)fr * A.n_masked + A.col_rank[row * G.N_x + col];
-        s0 = A.tstart[ti];
-        ne = (int)(A.tstart[ti + 1] - s0);
-        sc = (AMODE == 1) ? A.tscale[ti] : 1.f;
-      }
-      if (!PFE) {
-        for (int e = tid; e < ne; e += NT) {
-          const float a = (AMODE == 2) ? __ldg(A.tval32 + s0 + e) : __half2float(A.tval16[s0 + e]) * sc;
-          sEnt[e] = make_int2(__ldg(A.toff + s0 + e), __float_as_int(a));
+
+    // 2. the surrogate sums over the slots that this visit does not change:
+    //    8 neighbouring columns x 3 slices and the two frames, 1 << lv lanes
+    //    per voxel (as many as the CTA's threads give).  Out of the update
+    //    step below, whose two passes every other warp waits for, they took it
+    //    from a third of a short item's time to a tenth.
+    const uint32_t cm = (col > 0 ? 0111u : 0u) | 0222u | (col + 1 < G.N_x ? 0444u : 0u);
+    const uint32_t colmask = ((row > 0 ? 0007u : 0u) | 0070u | (row + 1 < G.N_y ? 0700u : 0u)) & cm;
+    if (!SEQ) {
+      int lv = 0;
+      while (lv < 5 && (Z << (lv + 1)) <= NT) lv++;
+      const int sub = tid & ((1 << lv) - 1);
+      for (int z0 = 0; z0 < Z; z0 += NT >> lv) {
+        const int z = z0 + (tid >> lv);
+        float num = 0.f, den = 0.f;
+        int pos = 0;
+        if (z < Z) {
+          const float Vv = sNb[4 * (zmax + 2) + z + 1];
+          const int za = zb + z;
+          const uint32_t zm = (za > 0 || hlo ? 1u : 0u) | 2u | (za + 1 < G.N_z || hhi ? 4u : 0u);
+          for (int n = sub; n < 26; n += 1 << lv) {
+            float v, w, c, lq;
+            bool in;
+            if (n < 24) {
+              const int dz = n >> 3, cc = (n & 7) + ((n & 4) >> 2);
+              v = sNb[cc * (zmax + 2) + z + dz];
+              w = sW[dz * 9 + cc];
+              in = ((colmask >> cc) & (zm >> dz) & 1u) != 0u;
+              c = G.C_S;
+              lq = A.l_sqp;
+            } else {
+              v = sTn[(n - 24) * zmax + z];
+              w = sW[27];
+              in = n == 24 ? fr > 0 : fr + 1 < G.N_time;
+              c = G.C_T;
+              lq = A.l_tqp;
+            }
+            const float b = in ? w * qcoef(Vv - v, c, lq, A.e2p, G.MRF_P) : 0.f;
+            num = fmaf(b, v, num);
+            den += b;
+            pos |= v > 0.f;  // absent slots read 0
+          }
+        }
+        for (int off = 1; off < (1 << lv); off <<= 1) {
+          num += __shfl_xor_sync(0xffffffffu, num, off);
+          den += __shfl_xor_sync(0xffffffffu, den, off);
+          pos |= __shfl_xor_sync(0xffffffffu, pos, off);
+        }
+        if (sub == 0 && z < Z) {
+          sNum[z] = num;
+          sDen[z] = den;
+          sPos[z] = pos;
         }
       }
-    }
-    if (PFE) cp_wait_all();
-    __syncthreads();
-    // The next item's chain steps are issued by thread 0 where a phase of
-    // this item follows that needs none of its own asynchronous copies (its
-    // waits complete every copy it has in flight): the rank during the
-    // footprint loop, the run bounds during the surrogate step.
-    if (PF && tid == 0) {
-      cp_wait_all();  // the next item's record
-      fetch_rank();
     }
 
     // 3. theta1 / theta2 over the column's footprint (XT_VoxUpdate.c:20-51)
@@ -480,7 +485,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_icd_columns(DevGeo G, IcdArgs
       }
       accumulate_arr(ev, wv, a);
     };
-    if (tl < tln && !skip_all) {
+    if (tl < tln) {
       if (AMODE == 0) {
         for (int v = vg; v < V; v += vgs) {
           const int pk = sPack[v], first = pk & 0xffffff, n = pk >> 24;
@@ -547,176 +552,108 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_icd_columns(DevGeo G, IcdArgs
     if (lane < tlp && tl < tln) {
 #pragma unroll
       for (int c = 0; c < VEC; c++) {
-        sRed[warp * 128 + tl * VEC + c] = th1[c];
-        sRed[NW * 128 + warp * 128 + tl * VEC + c] = th2[c];
+        sRed[warp * rp + tl * VEC + c] = th1[c];
+        sRed[(NW + warp) * rp + tl * VEC + c] = th2[c];
       }
-    }
-    __syncthreads();
-    if (PF && tid == 0) {
-      cp_wait_all();
-      fetch_bounds();
-    }
-    for (int t = tid; t < T; t += NT) {
-      float s1 = 0.f, s2 = 0.f;
-#pragma unroll
-      for (int wq = 0; wq < NW; wq++) {  // every warp wrote its partial (zeros if idle)
-        s1 += sRed[wq * 128 + t];
-        s2 += sRed[NW * 128 + wq * 128 + t];
-      }
-      sTh[t] = s1;
-      sTh[rowsmax + t] = s2;
     }
     __syncthreads();
 
     // 4. qGGMRF surrogate step per slice (CE_FunctionalSubstitution,
-    //    XT_ICD_update.c:130-179) with zero skipping (XT_VoxUpdate.c:208-232)
-    double absx = 0.0;
+    //    XT_ICD_update.c:130-179) with zero skipping (XT_VoxUpdate.c:208-232).
+    //    theta of a slice: its rows' partials over warps (every warp wrote its
+    //    own, zeros if idle)
+    auto theta = [&](int z, float &t1, float &t2) {
+      t1 = t2 = 0.f;
+      for (int r = z * G.zovl; r < (z + 1) * G.zovl; r++) {
+        float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+        for (int wq = 0; wq < NW; wq++) {
+          s1 += sRed[wq * rp + r];
+          s2 += sRed[(NW + wq) * rp + r];
+        }
+        t1 += s1;
+        t2 += s2;
+      }
+    };
+    // the new value of slice z; returns false where the voxel is skipped
+    auto update = [&](int z, float Vv, float num, float den) {
+      float t1, t2;
+      theta(z, t1, t2);
+      const float u = (num + t2 * Vv - t1) / (den + t2);
+      float nvx = Vv + G.alpha * (u - Vv);
+      if (G.positivity && nvx <= 0.f) nvx = 0.f;
+      if (!isfinite(nvx)) {
+        atomicExch(A.err, 1);
+        nvx = Vv;
+      }
+      sNb[4 * (zmax + 2) + z + 1] = nvx;
+      A.x[(((size_t)fr * plane) + (size_t)row * G.N_x + col) * G.N_z + zb + z] = nvx;
+      sDelta[z] = nvx - Vv;
+      sAbs[lane] += (double)fabsf(nvx);
+      sUpd[lane]++;
+    };
+    // the slots of the column itself, slices z - 1 and z + 1
+    auto own_terms = [&](int z, float Vv, float &num, float &den, bool &pos) {
+      const float vl = sNb[4 * (zmax + 2) + z], vh = sNb[4 * (zmax + 2) + z + 2];
+      const float bl = zb + z > 0 || hlo ? sW[4] * qcoef(Vv - vl, G.C_S, A.l_sqp, A.e2p, G.MRF_P) : 0.f;
+      const float bh = zb + z + 1 < G.N_z || hhi ? sW[22] * qcoef(Vv - vh, G.C_S, A.l_sqp, A.e2p, G.MRF_P) : 0.f;
+      num = fmaf(bl, vl, fmaf(bh, vh, num));
+      den += bl + bh;
+      pos = pos || vl > 0.f || vh > 0.f;
+    };
     if (SEQ) {
+      // slices in increasing z on one thread, the reference's order
       if (tid == 0) {
         for (int z = 0; z < Z; z++) {
           const float Vv = sNb[4 * (zmax + 2) + z + 1];
-          float t1 = 0.f, t2 = 0.f;
-          for (int r = 0; r < G.zovl; r++) {
-            t1 += sTh[z * G.zovl + r];
-            t2 += sTh[rowsmax + z * G.zovl + r];
-          }
-          bool skip = false;
-          if (Vv == 0.f && A.iter > 1) {
-            skip = !(sTn[z] > 0.f || sTn[zmax + z] > 0.f);
-            for (int c = 0; c < 9 && skip; c++)
-              for (int dz = 0; dz < 3; dz++)
-                if (sNb[c * (zmax + 2) + z + dz] > 0.f) skip = false;
-          }
-          if (skip) {
-            sDelta[z] = 0.f;
-            sZero++;
-            continue;
-          }
+          const uint32_t zm = (zb + z > 0 || hlo ? 1u : 0u) | 2u | (zb + z + 1 < G.N_z || hhi ? 4u : 0u);
           float num = 0.f, den = 0.f;
+          bool pos = false;
           for (int n = 0; n < 29; n++) {
-            const Nbr o = nbr_term(G, sNb, sTn, zmax, z, zb, fr, row, col, Vv, n, hlo, hhi);
-            num += o.b * o.v;
-            den += o.b;
+            if (n == 13) continue;
+            const int dz = n / 9, cc = n % 9;
+            const float v = n < 27 ? sNb[cc * (zmax + 2) + z + dz] : sTn[(n - 27) * zmax + z];
+            const bool in = n < 27 ? ((colmask >> cc) & (zm >> dz) & 1u) != 0u : n == 27 ? fr > 0 : fr + 1 < G.N_time;
+            const float b = !in      ? 0.f
+                            : n < 27 ? sW[n] * qcoef(Vv - v, G.C_S, A.l_sqp, A.e2p, G.MRF_P)
+                                     : sW[27] * qcoef(Vv - v, G.C_T, A.l_tqp, A.e2p, G.MRF_P);
+            num += b * v;
+            den += b;
+            pos = pos || v > 0.f;
           }
-          const float u = (num + t2 * Vv - t1) / (den + t2);
-          float nvx = Vv + G.alpha * (u - Vv);
-          if (G.positivity && nvx <= 0.f) nvx = 0.f;
-          if (!isfinite(nvx)) {
-            atomicExch(A.err, 1);
-            nvx = Vv;
+          if (Vv == 0.f && A.iter > 1 && !pos) {
+            sDelta[z] = 0.f;
+            sZero[0]++;
+          } else {
+            update(z, Vv, num, den);
           }
-          sNb[4 * (zmax + 2) + z + 1] = nvx;
-          A.x[(((size_t)fr * plane) + (size_t)row * G.N_x + col) * G.N_z + zb + z] = nvx;
-          sDelta[z] = nvx - Vv;
-          absx += (double)fabsf(nvx);
-          sUpd++;
         }
       }
-    } else {
-      // red/black in z, 8 lanes per voxel, each lane a subset of the 29
-      // neighbour slots; the lane group reduces with shuffles
-      const int sub = tid & 7, slot = tid >> 3;
+    } else if (warp == 0) {
+      // red/black in z: the even slices from the old values, the odd ones from
+      // the new; one lane per voxel, so one warp does both passes
       for (int par = 0; par < 2; par++) {
         const int zfirst = ((zb & 1) == par) ? 0 : 1;  // first z (relative) with absolute parity par
-        const int nvox = (Z - zfirst + 1) / 2;
-        for (int s0 = 0; s0 < nvox; s0 += NT / 8) {
-          const int vi = s0 + slot;
-          const bool act = vi < nvox;
-          const int z = zfirst + 2 * (act ? vi : 0);
+        for (int z = zfirst + 2 * lane; z < Z; z += 64) {
           const float Vv = sNb[4 * (zmax + 2) + z + 1];
-          // zero skipping: V == 0 from the second iteration and no positive neighbour
-          bool pos = false;
-          float num = 0.f, den = 0.f;
-#pragma unroll
-          for (int k = 0; k < 4; k++) {
-            const int n = sub + 8 * k;
-            if (n < 29) {
-              const Nbr o = nbr_term(G, sNb, sTn, zmax, z, zb, fr, row, col, Vv, n, hlo, hhi);
-              num += o.b * o.v;
-              den += o.b;
-            }
-          }
-          // positive-neighbour test over the raw values (absent slots read 0)
-          if (Vv == 0.f && A.iter > 1) {
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-              const int n = sub + 8 * k;
-              if (n < 27) {
-                if (sNb[(n % 9) * (zmax + 2) + z + n / 9] > 0.f) pos = true;
-              } else if (n < 29) {
-                if (sTn[(n - 27) * zmax + z] > 0.f) pos = true;
-              }
-            }
-          }
-#pragma unroll
-          for (int off = 1; off < 8; off <<= 1) {
-            num += __shfl_xor_sync(0xffffffffu, num, off);
-            den += __shfl_xor_sync(0xffffffffu, den, off);
-            pos |= __shfl_xor_sync(0xffffffffu, (int)pos, off) != 0;
-          }
-          if (act && sub == 0) {
-            const int zr = z;
-            if (Vv == 0.f && A.iter > 1 && !pos) {
-              sDelta[zr] = 0.f;
-              atomicAdd(&sZero, 1u);
-            } else {
-              float t1 = 0.f, t2 = 0.f;
-              for (int r = 0; r < G.zovl; r++) {
-                t1 += sTh[zr * G.zovl + r];
-                t2 += sTh[rowsmax + zr * G.zovl + r];
-              }
-              const float u = (num + t2 * Vv - t1) / (den + t2);
-              float nvx = Vv + G.alpha * (u - Vv);
-              if (G.positivity && nvx <= 0.f) nvx = 0.f;
-              if (!isfinite(nvx)) {
-                atomicExch(A.err, 1);
-                nvx = Vv;
-              }
-              sNb[4 * (zmax + 2) + zr + 1] = nvx;
-              A.x[(((size_t)fr * plane) + (size_t)row * G.N_x + col) * G.N_z + zb + zr] = nvx;
-              sDelta[zr] = nvx - Vv;
-              absx += (double)fabsf(nvx);
-              atomicAdd(&sUpd, 1u);
-            }
+          float num = sNum[z], den = sDen[z];
+          bool pos = sPos[z] != 0;
+          own_terms(z, Vv, num, den, pos);
+          if (Vv == 0.f && A.iter > 1 && !pos) {
+            sDelta[z] = 0.f;
+            sZero[lane]++;
+          } else {
+            update(z, Vv, num, den);
           }
         }
-        __syncthreads();
+        __syncwarp();
       }
     }
+    if (tid == META) fetch_meta(sMeta[mb ^ 1]);
     __syncthreads();
+    if (warp == NW - 1) write_magmap();
 
-    // 5. MagUpdateMap[frame][block][row][col] = sum |delta| over the block's
-    //    slices of this visit (XT_VoxUpdate.c:128, 236); sum |x| and counters
-    for (int b = tid; b < G.nzb; b += NT) {
-      const int bz0 = b * G.zstep, bz1 = (b >= G.nzb - 1) ? G.N_z - 1 : (b + 1) * G.zstep - 1;
-      const int lo = max(bz0, zb), hi = min(bz1, ze);
-      float *mp = A.magmap + (((size_t)fr * G.nzb + b) * G.N_y + row) * G.N_x + col;
-      if (A.nsub > 1) {
-        // pieces of one block add into the entry zeroed before the launch
-        if (lo <= hi) {
-          float m = 0.f;
-          for (int z = lo; z <= hi; z++) m += fabsf(sDelta[z - zb]);
-          atomicAdd(mp, m);
-        }
-      } else if (bz0 >= zb && bz1 <= ze) {
-        float m = 0.f;
-        for (int z = bz0; z <= bz1; z++) m += fabsf(sDelta[z - zb]);
-        *mp = m;
-      }
-    }
-    for (int off = 16; off > 0; off >>= 1) absx += __shfl_xor_sync(0xffffffffu, absx, off);
-    if (lane == 0) sAbs[warp] = absx;
-    __syncthreads();
-    if (tid == 0) {
-      double s = 0.0;
-      for (int wq = 0; wq < NT / 32; wq++) s += sAbs[wq];
-      sCtaAbs += s;
-      sCta[0] += sUpd;
-      sCta[1] += sZero;
-      if (piece == 0) sCta[2]++;
-    }
-
-    // 6. e -= (A delta_t) * delta_x on the footprint (XT_VoxUpdate.c:62-82)
+    // 5. e -= (A delta_t) * delta_x on the footprint (XT_VoxUpdate.c:62-82)
     if (tl < tln) {
       float dv[VEC];
       bool any = false;
@@ -758,15 +695,21 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_icd_columns(DevGeo G, IcdArgs
         }
       }
     }
-    if (PF && tid == 0) cp_wait_all();  // the next item's meta is complete
-    __syncthreads();
-    mb ^= 1;
   }
-  if (tid == 0 && (sCta[0] || sCta[1] || sCta[2] || sCtaAbs != 0.0)) {  // pieces past the first count no item
-    atomicAdd(&A.st_absx[blockIdx.x & 63], sCtaAbs);
-    atomicAdd(&A.st_cnt[0], sCta[0]);
-    atomicAdd(&A.st_cnt[1], sCta[1]);
-    atomicAdd(&A.st_cnt[2], sCta[2]);
+  if (warp == 0) {
+    double ab = sAbs[lane];
+    unsigned long long up = sUpd[lane], zr = sZero[lane];
+    for (int off = 16; off > 0; off >>= 1) {
+      ab += __shfl_xor_sync(0xffffffffu, ab, off);
+      up += __shfl_xor_sync(0xffffffffu, up, off);
+      zr += __shfl_xor_sync(0xffffffffu, zr, off);
+    }
+    if (lane == 0 && (up || zr || ncol)) {
+      atomicAdd(&A.st_absx[blockIdx.x & 63], ab);
+      atomicAdd(&A.st_cnt[0], up);
+      atomicAdd(&A.st_cnt[1], zr);
+      atomicAdd(&A.st_cnt[2], (unsigned long long)ncol);
+    }
   }
 }
 
@@ -776,11 +719,10 @@ size_t icd_smem_bytes(int vmax, int zmax, int zovl, int as, int amode, int vec, 
     b += (size_t)vmax * (4 * 2 + 4 * (size_t)as);  // sPack, sView, sVal
   else
     b += (size_t)vmax * 8;                         // sEnt
-  b += 2 * (size_t)(nt / 32) * 128 * 4;            // sRed
-  b += 2 * (size_t)zmax * zovl * 4;                // sTh
+  b += 2 * (size_t)(nt / 32) * (((size_t)zmax * zovl + 3) / 4 * 4) * 4;  // sRed
   b += 9 * (size_t)(zmax + 2) * 4;                 // sNb
   b += 2 * (size_t)zmax * 4;                       // sTn
-  b += (size_t)zmax * 4;                           // sDelta
+  b += 4 * (size_t)zmax * 4;                       // sDelta, sNum, sDen, sPos
   return b;
 }
 

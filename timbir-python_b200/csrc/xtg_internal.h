@@ -35,6 +35,8 @@ struct IcdArgs {
   int w_keep;  // e and w fit in L2 together: w loads keep their lines (evict_last)
   int iter;
   float T2, Tdelta;
+  // qGGMRF constants: 2 - p, log2 of sigma_qp and 1 / sigma_q (spatial, temporal)
+  float e2p, l_sqp, l_tqp, inv_sq, inv_tq;
   // z slab of a larger volume: the neighbouring slabs' boundary slices,
   // [N_time][N_y][N_x] (null where this slab ends the volume)
   const float *halo_lo, *halo_hi;
