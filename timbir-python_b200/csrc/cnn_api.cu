@@ -1,5 +1,6 @@
 // cnn_api.cu -- C ABI of the warm-start network (include/xtg_cnn.h).
 #include <cstdio>
+#include <mutex>
 
 #include "../../include/xtg.h"
 #include "../../include/xtg_cnn.h"
@@ -70,12 +71,17 @@ int xtc_conv3d_path(const void *in, const void *w, const float *bias, void *out,
     xtg_set_error_text("xtc_conv3d: shape not supported by the tile kernel");
     return XTG_E_ARG;
   }
+  const bool box = path == XTC_CONV_AUTO && !tile && kpad % 64 == 0 && kpad >= 27 * cin && xtc::conv_box_supported(s);
   cudaError_t e;
-  if (tile) {
-    // the weights packed per 16-channel chunk, in a buffer kept for later calls
+  static std::mutex mu;
+  std::unique_lock<std::mutex> lk(mu, std::defer_lock);
+  if (tile || box) {
+    // the packed weights, in a buffer kept for later calls: one call at a time
+    // (each ends synchronised)
+    lk.lock();
     static void *wp = nullptr;
     static size_t wp_bytes = 0;
-    const size_t need = xtc::conv_tile_wp_elems(cin, cout) * 2;
+    const size_t need = (tile ? xtc::conv_tile_wp_elems(cin, cout) : xtc::conv_box_wp_elems(cin, cout)) * 2;
     if (need > wp_bytes) {
       if (wp) cudaFree(wp);
       wp = nullptr;
@@ -83,11 +89,18 @@ int xtc_conv3d_path(const void *in, const void *w, const float *bias, void *out,
       if ((e = cudaMalloc(&wp, need)) != cudaSuccess) return fail(e, "xtc_conv3d");
       wp_bytes = need;
     }
-    e = xtc::conv_tile_pack(cin, cout, kpad, sign, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)wp, 0);
-    if (e == cudaSuccess)
+    e = tile ? xtc::conv_tile_pack(cin, cout, kpad, sign, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)wp, 0)
+             : xtc::conv_box_pack(cin, cout, kpad, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)wp, 0);
+    if (e == cudaSuccess && box)
+      e = xtc::conv_forward_box(s, (const __nv_bfloat16 *)in, (const __nv_bfloat16 *)wp, bias, out, epi, sign, g_err, 0);
+    else if (e == cudaSuccess)
       e = xtc::conv_forward_tile(s, (const __nv_bfloat16 *)in, (const __nv_bfloat16 *)wp, bias, out, epi, sign,
                                  g_err, 0);
   } else {
+    e = cudaErrorNotSupported;
+  }
+  if (e == cudaErrorNotSupported && !tile) {
+    cudaGetLastError();
     e = xtc::conv_forward(s, (const __nv_bfloat16 *)in, (const __nv_bfloat16 *)w, bias, out, epi, sign, g_err, 0);
   }
   if (e != cudaSuccess) return fail(e, "xtc_conv3d");

@@ -460,6 +460,10 @@ cudaError_t conv_wgrad(const ConvShape &s, const __nv_bfloat16 *in, const __nv_b
   } else if (path == 2) {
     return cudaErrorNotSupported;
   }
+  if (path == 0 && wgrad_box_supported(s)) {
+    const cudaError_t e = conv_wgrad_box(s, in, dout, dw, err, st);
+    if (e != cudaErrorNotSupported) return e;
+  }
   const long long M = (long long)s.nb * s.Y * s.X * s.Z;
   const int mt = (27 * s.cin + 127) / 128;
   // enough K splits to fill the GPU twice over, each a multiple of KT voxels

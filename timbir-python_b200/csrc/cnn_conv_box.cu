@@ -1,0 +1,578 @@
+// cnn_conv_box.cu -- 3x3x3 convolutions and weight gradients of the warm-start
+// network for any volume size, operands staged by TMA (BF16 in, FP32
+// accumulation in TMEM).
+//
+// The gather kernels (cnn_conv.cu) build every operand row with per-thread
+// loads; the tile kernels (cnn_conv_tile.cu) need rows of 128 x-voxels.  Here a
+// tile is a box of 128 voxels, z x x x y x batch with power-of-two sides chosen
+// to cover the volume with the fewest boxes, and the operand of a tap is the
+// same box read at the tap's offset: one TMA load of 128 voxels x CH channels,
+// zero filled outside the volume (the padding) and past the last channel.
+// Each input voxel is fetched 27 times, from L2: what bounds both kernels is
+// the rate at which an SM's TMA unit takes rows (about four cycles each, 64- or
+// 128-byte ones alike), not the MMAs.
+//
+// CH is 64 (128-byte rows, the 128-byte swizzle) or 32 (64-byte rows, 64-byte
+// swizzle), whichever pads the channels less.
+#include <cuda.h>
+#include <cudaTypedefs.h>
+#include <cuda_bf16.h>
+
+#include <algorithm>
+#include <mutex>
+
+#include "cnn_tc.cuh"
+#include "xtg_cnn_internal.h"
+
+namespace xtc {
+
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encode() {
+  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+  });
+  return fn;
+}
+
+namespace {
+
+constexpr long long kLim = 1ll << 24;  // polls of a bounded wait
+
+// the 128-voxel box: sides (powers of two) and the boxes along each dimension
+struct Box {
+  int z, x, y, b;
+  int nz, nx, ny, nbx;
+  __host__ __device__ int count() const { return nz * nx * ny * nbx; }
+};
+
+// fewest boxes; among equals the longest runs in memory (z, then x)
+bool choose_box(const ConvShape &s, Box *out) {
+  long long best = -1;
+  for (int z = 1; z <= 128; z *= 2)
+    for (int x = 1; z * x <= 128; x *= 2)
+      for (int y = 1; z * x * y <= 128; y *= 2) {
+        const int b = 128 / (z * x * y);
+        auto up = [](int n, int d) { return (n + d - 1) / d; };
+        const long long n = (long long)up(s.Z, z) * up(s.X, x) * up(s.Y, y) * up(s.nb, b);
+        if (best < 0 || n < best || (n == best && (z > out->z || (z == out->z && x > out->x)))) {
+          best = n;
+          *out = Box{z, x, y, b, up(s.Z, z), up(s.X, x), up(s.Y, y), up(s.nb, b)};
+        }
+      }
+  return best > 0 && best < (1ll << 30);
+}
+
+__device__ __forceinline__ void box_origin(const Box &B, int t, int &z0, int &x0, int &y0, int &b0) {
+  z0 = (t % B.nz) * B.z;
+  t /= B.nz;
+  x0 = (t % B.nx) * B.x;
+  t /= B.nx;
+  y0 = (t % B.ny) * B.y;
+  b0 = (t / B.ny) * B.b;
+}
+
+// channels per TMA row
+int box_ch(int cin) { return (cin + 63) / 64 * 64 <= (cin + 31) / 32 * 32 ? 64 : 32; }
+
+// 16-byte unit u of row r in the swizzle of CH-channel rows (as TMA writes it)
+template <int CH>
+__host__ __device__ constexpr int swz(int r, int u) {
+  return CH == 64 ? u ^ (r & 7) : u ^ ((r >> 1) & 3);
+}
+
+// K-major operand: rows of CH channels, 8-row groups CH * 16 bytes apart
+template <int CH>
+__device__ __forceinline__ uint64_t desc_k(uint32_t saddr) {
+  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)1 << 16) | ((uint64_t)CH << 32) | ((uint64_t)1 << 46) |
+         ((uint64_t)(CH == 64 ? 2 : 4) << 61);
+}
+// MN-major operand: a row per K index, 8-row groups CH * 16 bytes apart (SBO),
+// atoms of CH channels `lbo` bytes apart
+template <int CH>
+__device__ __forceinline__ uint64_t desc_mn(uint32_t saddr, uint32_t lbo) {
+  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) | ((uint64_t)CH << 32) |
+         ((uint64_t)1 << 46) | ((uint64_t)(CH == 64 ? 2 : 4) << 61);
+}
+
+__host__ __device__ constexpr uint32_t pow2_cols(int n) {
+  uint32_t c = 32;
+  while (c < (uint32_t)n) c *= 2;
+  return c;
+}
+
+__device__ __forceinline__ void tap_of(int t, int &dy, int &dx, int &dz) {
+  dy = t / 9 - 1;
+  dx = t / 3 % 3 - 1;
+  dz = t % 3 - 1;
+}
+
+// ---------------------------------------------------------------------------
+// Forward and input gradient.  Persistent CTAs of 192 threads: warp 4 (one
+// thread) issues a stage's copies -- the tap's box and the matching weight
+// rows, packed and swizzled beforehand, in one bulk copy -- warp 5 (one
+// thread) the MMAs, M = the box's voxels, N = cout, K = CH; warps 0-3 drain
+// the finished accumulator while the other TMEM buffer fills.  The K order
+// (tap, then channel) is the gather kernel's, so the results are its bits.
+//
+// Training step, 8 patches of 32 x 128 x 32, gather -> box:
+//   level 1 48 -> 48 (131072 voxels)       195 -> 57 us
+//   level 1 112 -> 48                      595 -> 100 us
+//   level 2 160 -> 64 (16384 voxels)       215 -> 56 us
+//   level 3 96 -> 96 (2048 voxels)         147 -> 38 us
+//   level 0 32 -> 80 input gradient        1047 -> 429 us
+template <int CH, int EPI>
+__global__ void __launch_bounds__(192) k_conv_box(const __grid_constant__ CUtensorMap tin, ConvShape s, Box B, int sign,
+                                                  const __nv_bfloat16 *__restrict__ wp, const float *__restrict__ bias,
+                                                  void *out, int nstage, int *err) {
+  extern __shared__ __align__(1024) uint8_t sm_raw[];
+  // stages start on the 1024 bytes the swizzle repeats over
+  uint8_t *sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);
+  constexpr uint32_t ABYTES = 128 * CH * 2;
+  constexpr int MAXST = 8;
+  const int N = s.n;
+  const uint32_t BBYTES = (uint32_t)N * CH * 2, STAGE = ABYTES + BBYTES;
+  __shared__ uint64_t full[MAXST], empty[MAXST], acc_full[2], acc_empty[2], done;
+  __shared__ uint32_t tbase;
+  __shared__ volatile int bad;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nchunk = (s.cin + CH - 1) / CH, nk = 27 * nchunk;
+  const int ntiles = B.count();
+  const int mine = ntiles > (int)blockIdx.x ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  const uint32_t cols = pow2_cols(2 * N);
+  if (tid == 0) {
+    for (int i = 0; i < nstage; i++) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    for (int i = 0; i < 2; i++) {
+      mbar_init(&acc_full[i], 1);
+      mbar_init(&acc_empty[i], 4);
+    }
+    mbar_init(&done, 1);
+    mbar_init_fence();
+    bad = 0;
+  }
+  if (warp == 0) tmem_alloc(&tbase, cols);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tbase;
+  if (warp == 4) {
+    if (lane == 0) {
+      int q = 0;
+      bool ok = true;
+      for (int tl = 0; tl < mine && ok; tl++) {
+        int z0, x0, y0, b0;
+        box_origin(B, (int)blockIdx.x + tl * (int)gridDim.x, z0, x0, y0, b0);
+        for (int t = 0; t < 27 && ok; t++) {
+          int dy, dx, dz;
+          tap_of(t, dy, dx, dz);
+          for (int c = 0; c < nchunk; c++, q++) {
+            const int st = q % nstage;
+            if (q >= nstage && (!mbar_wait(&empty[st], (uint32_t)(q / nstage - 1) & 1u, kLim) || bad)) {
+              ok = false;
+              break;
+            }
+            uint8_t *a = sm + (size_t)st * STAGE;
+            mbar_expect_tx(&full[st], STAGE);
+            tma_load_5d(a, &tin, c * CH, z0 + sign * dz, x0 + sign * dx, y0 + sign * dy, b0, &full[st]);
+            bulk_load(a + ABYTES, wp + (size_t)(t * nchunk + c) * N * CH, BBYTES, &full[st]);
+          }
+        }
+      }
+      if (!ok) {
+        atomicExch(err, 1);
+        bad = 1;
+      }
+      // the copies issued last land before the shared memory is released
+      for (int i = q > nstage ? q - nstage : 0; i < q; i++) mbar_wait(&full[i % nstage], (uint32_t)(i / nstage) & 1u, kLim);
+    }
+    __syncwarp();
+  } else if (warp == 5) {
+    if (lane == 0) {
+      const uint32_t idesc = idesc_bf16(N, 0, 0);
+      bool ok = true;
+      int q = 0;
+      for (int tl = 0; tl < mine && ok; tl++) {
+        const int ab = tl & 1;
+        if (tl >= 2 && !mbar_wait(&acc_empty[ab], (uint32_t)((tl >> 1) - 1) & 1u, kLim)) {
+          ok = false;
+          break;
+        }
+        const uint32_t acc = tmem + (uint32_t)(ab * N);
+        for (int k = 0; k < nk; k++, q++) {
+          const int st = q % nstage;
+          if (!mbar_wait(&full[st], (uint32_t)(q / nstage) & 1u, kLim) || bad) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t a0 = smem_u32(sm + (size_t)st * STAGE);
+          const uint64_t da = desc_k<CH>(a0), db = desc_k<CH>(a0 + ABYTES);
+#pragma unroll
+          for (int ks = 0; ks < CH / 16; ks++)
+            mma_bf16(acc, da + (uint64_t)(2 * ks), db + (uint64_t)(2 * ks), idesc, (k > 0 || ks > 0) ? 1u : 0u);
+          mma_commit(&empty[st]);
+        }
+        if (ok) mma_commit(&acc_full[ab]);
+      }
+      if (!ok) {
+        atomicExch(err, 1);
+        bad = 1;
+      }
+      mma_commit(&done);
+      mbar_wait(&done, 0, kLim);  // every MMA issued above has completed
+    }
+    __syncwarp();
+  } else {
+    // row r of a box: z fastest, then x, y, batch
+    const int r = warp * 32 + lane;
+    const int rz = r % B.z, rx = r / B.z % B.x, ry = r / (B.z * B.x) % B.y, rb = r / (B.z * B.x * B.y);
+    for (int tl = 0; tl < mine; tl++) {
+      const int ab = tl & 1;
+      const bool gone = !mbar_wait(&acc_full[ab], (uint32_t)(tl >> 1) & 1u, kLim) || bad;
+      if (__any_sync(0xffffffffu, gone)) {
+        if (lane == 0) atomicExch(err, 1);
+        bad = 1;
+        break;
+      }
+      tc_fence_after();
+      int z, x, y, b;
+      box_origin(B, (int)blockIdx.x + tl * (int)gridDim.x, z, x, y, b);
+      z += rz;
+      x += rx;
+      y += ry;
+      b += rb;
+      const bool in = z < s.Z && x < s.X && y < s.Y && b < s.nb;
+      const size_t vox = (((size_t)b * s.Y + y) * s.X + x) * s.Z + z;
+      for (int n0 = 0; n0 < N; n0 += 16) {
+        float v[16];
+        tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(ab * N + n0), v);
+        if (!in) continue;
+        if (EPI == 2) {
+          float *o = reinterpret_cast<float *>(out) + vox * N + n0;
+#pragma unroll
+          for (int i = 0; i < 16; i += 4)
+            *reinterpret_cast<float4 *>(o + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+        } else {
+          __align__(16) __nv_bfloat16 h[16];
+#pragma unroll
+          for (int i = 0; i < 16; i++) {
+            float f = v[i];
+            if (EPI == 0) f = fmaxf(f + bias[n0 + i], 0.f);
+            h[i] = __float2bfloat16_rn(f);
+          }
+          __nv_bfloat16 *o = reinterpret_cast<__nv_bfloat16 *>(out) + vox * N + n0;
+          *reinterpret_cast<int4 *>(o) = *reinterpret_cast<const int4 *>(h);
+          *reinterpret_cast<int4 *>(o + 8) = *reinterpret_cast<const int4 *>(h + 8);
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[ab]);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_free(tmem, cols);
+  }
+}
+
+// K-major W[n][kpad] (k = tap * cin + ci) -> rows of CH channels per (tap,
+// chunk, n), 16-byte units swizzled, zero past cin
+template <int CH>
+__global__ void k_pack_box_w(int cin, int n, int kpad, const __nv_bfloat16 *__restrict__ w, __nv_bfloat16 *__restrict__ wp) {
+  const int nchunk = (cin + CH - 1) / CH;
+  const long long total = 27ll * nchunk * n * CH;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const int e = (int)(i % 8), u = (int)(i / 8 % (CH / 8));
+    const long long row = i / CH;  // (tap * nchunk + c) * n + nn
+    const int nn = (int)(row % n), tc = (int)(row / n), c = tc % nchunk, t = tc / nchunk;
+    const int ci = c * CH + swz<CH>(nn, u) * 8 + e;
+    wp[i] = ci < cin ? w[(size_t)nn * kpad + (size_t)t * cin + ci] : __float2bfloat16_rn(0.f);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Weight gradient: dW[tap][ci][co] += sum_v in[v + d(tap)][ci] dout[v][co].  A CTA owns
+// the nine taps of one dy and one chunk of CH input channels over a slice of
+// the boxes.  K is the box's 128 voxels, so both operands are MN-major as they
+// lie in memory: A stacks 128 / CH taps along M (one TMA box each), B is the
+// box of dout, kept for the nine taps.  The accumulators of the ceil(9 CH / 128)
+// M tiles stay in TMEM over the slice and are added into dw at the end.
+//
+// Training step, 8 patches of 32 x 128 x 32, gather -> box: level 1 48 x 48
+// 320 -> 63 us, 112 x 48 813 -> 117 us, level 2 160 x 64 165 -> 31 us.
+constexpr int WB_SLOTS = 4;                    // A slots (one M tile each)
+constexpr uint32_t WB_A = 128 * 128 * 2;       // bytes of a slot
+template <int CH>
+__host__ __device__ constexpr int wb_mtiles() {
+  return (9 * CH + 127) / 128;
+}
+
+template <int CH, int CHB>
+__global__ void __launch_bounds__(192, 1) k_wgrad_box(const __grid_constant__ CUtensorMap tin,
+                                                      const __grid_constant__ CUtensorMap tdy, ConvShape s, Box B,
+                                                      float *dw, int slices, int *err) {
+  extern __shared__ __align__(1024) uint8_t sm_raw[];
+  // stages start on the 1024 bytes the swizzle repeats over
+  uint8_t *sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);
+  constexpr int MT = wb_mtiles<CH>(), TPM = 128 / CH;  // M tiles, taps per M tile
+  constexpr uint32_t ABOX = 128 * CH * 2, BBOX = 128 * CHB * 2;
+  const int N = s.n, nbc = (N + CHB - 1) / CHB;
+  const uint32_t BSLOT = (uint32_t)nbc * BBOX;
+  uint8_t *sA = sm, *sB = sm + WB_SLOTS * WB_A;
+  __shared__ uint64_t fullA[WB_SLOTS], emptyA[WB_SLOTS], fullB[2], emptyB[2], acc_full;
+  __shared__ uint32_t tbase;
+  __shared__ volatile int bad;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nchunk = (s.cin + CH - 1) / CH;
+  const int grp = (int)blockIdx.x / slices, slice = (int)blockIdx.x % slices;
+  const int dyi = grp / nchunk, ck = grp % nchunk;
+  const int ntiles = B.count();
+  const int mine = ntiles > slice ? (ntiles - 1 - slice) / slices + 1 : 0;
+  const uint32_t cols = pow2_cols(MT * N);
+  if (tid == 0) {
+    for (int i = 0; i < WB_SLOTS; i++) {
+      mbar_init(&fullA[i], 1);
+      mbar_init(&emptyA[i], 1);
+    }
+    for (int i = 0; i < 2; i++) {
+      mbar_init(&fullB[i], 1);
+      mbar_init(&emptyB[i], 1);
+    }
+    mbar_init(&acc_full, 1);
+    mbar_init_fence();
+    bad = 0;
+  }
+  if (warp == 0) tmem_alloc(&tbase, cols);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tbase;
+  if (warp == 4) {
+    if (lane == 0) {
+      bool ok = true;
+      int q = 0, nb = 0;  // A slots, B slots filled so far
+      for (int tl = 0; tl < mine && ok; tl++) {
+        int z0, x0, y0, b0;
+        box_origin(B, slice + tl * slices, z0, x0, y0, b0);
+        if (tl >= 2 && (!mbar_wait(&emptyB[tl & 1], (uint32_t)((tl >> 1) - 1) & 1u, kLim) || bad)) {
+          ok = false;
+          break;
+        }
+        mbar_expect_tx(&fullB[tl & 1], BSLOT);
+        for (int c = 0; c < nbc; c++)
+          tma_load_5d(sB + (tl & 1) * BSLOT + c * BBOX, &tdy, c * CHB, z0, x0, y0, b0, &fullB[tl & 1]);
+        nb++;
+        for (int m = 0; m < MT; m++, q++) {
+          const int st = q % WB_SLOTS;
+          if (q >= WB_SLOTS && (!mbar_wait(&emptyA[st], (uint32_t)(q / WB_SLOTS - 1) & 1u, kLim) || bad)) {
+            ok = false;
+            break;
+          }
+          const int nt = m * TPM + TPM <= 9 ? TPM : 9 - m * TPM;  // taps of this M tile
+          mbar_expect_tx(&fullA[st], (uint32_t)nt * ABOX);
+          for (int u = 0; u < nt; u++) {
+            const int t9 = m * TPM + u;
+            tma_load_5d(sA + st * WB_A + u * ABOX, &tin, ck * CH, z0 + t9 % 3 - 1, x0 + t9 / 3 - 1, y0 + dyi - 1, b0,
+                        &fullA[st]);
+          }
+        }
+      }
+      if (!ok) {
+        atomicExch(err, 1);
+        bad = 1;
+      }
+      // the copies issued last land before the shared memory is released
+      for (int i = q > WB_SLOTS ? q - WB_SLOTS : 0; i < q; i++)
+        mbar_wait(&fullA[i % WB_SLOTS], (uint32_t)(i / WB_SLOTS) & 1u, kLim);
+      for (int i = nb > 2 ? nb - 2 : 0; i < nb; i++) mbar_wait(&fullB[i & 1], (uint32_t)(i >> 1) & 1u, kLim);
+    }
+    __syncwarp();
+  } else if (warp == 5) {
+    if (lane == 0) {
+      const uint32_t idesc = idesc_bf16(N, 1, 1);
+      bool ok = true;
+      int q = 0;
+      for (int tl = 0; tl < mine && ok; tl++) {
+        if (!mbar_wait(&fullB[tl & 1], (uint32_t)(tl >> 1) & 1u, kLim) || bad) {
+          ok = false;
+          break;
+        }
+        const uint32_t b0 = smem_u32(sB + (tl & 1) * BSLOT);
+        for (int m = 0; m < MT; m++, q++) {
+          const int st = q % WB_SLOTS;
+          if (!mbar_wait(&fullA[st], (uint32_t)(q / WB_SLOTS) & 1u, kLim) || bad) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t a0 = smem_u32(sA + st * WB_A);
+#pragma unroll
+          for (int ks = 0; ks < 8; ks++)  // 16 voxels each
+            mma_bf16(tmem + (uint32_t)(m * N), desc_mn<CH>(a0 + ks * 16 * CH * 2, ABOX),
+                     desc_mn<CHB>(b0 + ks * 16 * CHB * 2, BBOX), idesc, (tl > 0 || ks > 0) ? 1u : 0u);
+          mma_commit(&emptyA[st]);
+        }
+        if (ok) mma_commit(&emptyB[tl & 1]);
+      }
+      if (!ok) {
+        atomicExch(err, 1);
+        bad = 1;
+      }
+      mma_commit(&acc_full);  // arrives once every MMA issued above has completed
+      mbar_wait(&acc_full, 0, kLim);
+    }
+    __syncwarp();
+  } else {
+    bool ready = mbar_wait(&acc_full, 0, kLim);
+    if (!ready) {
+      if (lane == 0) atomicExch(err, 1);
+      bad = 1;
+    }
+    ready = !__any_sync(0xffffffffu, !ready || bad);
+    tc_fence_after();
+    if (ready && mine > 0) {
+      const int r = warp * 32 + lane;  // accumulator row: tap u of the M tile, channel
+      const int u = r / CH, ci = ck * CH + r % CH;
+      const bool al = (reinterpret_cast<uintptr_t>(dw) & 15) == 0;
+      for (int m = 0; m < MT; m++) {
+        const int t9 = m * TPM + u;
+        const bool in = t9 < 9 && ci < s.cin;
+        // tap (dy, dx, dz): t9 = 3 (dx + 1) + (dz + 1)
+        float *o = dw + ((size_t)(dyi * 9 + t9) * s.cin + ci) * N;
+        for (int n0 = 0; n0 < N; n0 += 16) {
+          float v[16];
+          tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(m * N + n0), v);
+          if (!in) continue;
+          if (al) {
+#pragma unroll
+            for (int i = 0; i < 16; i += 4)
+              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(o + n0 + i), "f"(v[i]), "f"(v[i + 1]),
+                           "f"(v[i + 2]), "f"(v[i + 3])
+                           : "memory");
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; i++) atomicAdd(o + n0 + i, v[i]);
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_free(tmem, cols);
+  }
+}
+
+// activations [nb][Y][X][Z][c] seen as (c, z, x, y, b), boxes of ch channels x 128 voxels
+bool encode_box(CUtensorMap *m, const __nv_bfloat16 *p, const ConvShape &s, int c, int ch, const Box &B) {
+  const cuuint64_t C2 = (cuuint64_t)c * 2;
+  const cuuint64_t dims[5] = {(cuuint64_t)c, (cuuint64_t)s.Z, (cuuint64_t)s.X, (cuuint64_t)s.Y, (cuuint64_t)s.nb};
+  const cuuint64_t strides[4] = {C2, (cuuint64_t)s.Z * C2, (cuuint64_t)s.X * s.Z * C2, (cuuint64_t)s.Y * s.X * s.Z * C2};
+  const cuuint32_t box[5] = {(cuuint32_t)ch, (cuuint32_t)B.z, (cuuint32_t)B.x, (cuuint32_t)B.y, (cuuint32_t)B.b};
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  return tensor_map_encode()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<__nv_bfloat16 *>(p), dims, strides, box,
+                             estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                             ch == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+cudaError_t sm_count(int *n) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  return e == cudaSuccess ? cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, dev) : e;
+}
+
+bool shape_ok(const ConvShape &s) {
+  return s.nb >= 1 && s.Y >= 1 && s.X >= 1 && s.Z >= 1 && s.cin >= 16 && s.cin % 16 == 0 && s.n >= 16 && s.n % 16 == 0 &&
+         tensor_map_encode() != nullptr;
+}
+
+}  // namespace
+
+bool conv_box_supported(const ConvShape &s) {
+  Box B;
+  return shape_ok(s) && s.n <= 256 && choose_box(s, &B);
+}
+
+size_t conv_box_wp_elems(int cin, int n) {
+  const int ch = box_ch(cin);
+  return (size_t)27 * ((cin + ch - 1) / ch) * n * ch;
+}
+
+cudaError_t conv_box_pack(int cin, int n, int kpad, const __nv_bfloat16 *w, __nv_bfloat16 *wp, cudaStream_t st) {
+  const unsigned grid = (unsigned)std::min<size_t>((conv_box_wp_elems(cin, n) + 255) / 256, 4096);
+  if (box_ch(cin) == 64)
+    k_pack_box_w<64><<<grid, 256, 0, st>>>(cin, n, kpad, w, wp);
+  else
+    k_pack_box_w<32><<<grid, 256, 0, st>>>(cin, n, kpad, w, wp);
+  return cudaGetLastError();
+}
+
+cudaError_t conv_forward_box(const ConvShape &s, const __nv_bfloat16 *in, const __nv_bfloat16 *wp, const float *bias,
+                             void *out, int epi, int sign, int *err, cudaStream_t st) {
+  Box B;
+  if (!conv_box_supported(s) || !choose_box(s, &B) || (epi == 0 && !bias) || epi < 0 || epi > 2 || (sign != 1 && sign != -1))
+    return cudaErrorNotSupported;
+  const int ch = box_ch(s.cin);
+  CUtensorMap m;
+  if (!encode_box(&m, in, s, s.cin, ch, B)) return cudaErrorNotSupported;
+  typedef void (*K)(const CUtensorMap, ConvShape, Box, int, const __nv_bfloat16 *, const float *, void *, int, int *);
+  K k = ch == 64 ? (epi == 0 ? k_conv_box<64, 0> : epi == 1 ? k_conv_box<64, 1> : k_conv_box<64, 2>)
+                 : (epi == 0 ? k_conv_box<32, 0> : epi == 1 ? k_conv_box<32, 1> : k_conv_box<32, 2>);
+  int sms = 0;
+  cudaError_t e = sm_count(&sms);
+  if (e != cudaSuccess) return e;
+  // two CTAs per SM where their accumulators fit the SM's 512 TMEM columns
+  const int per_sm = pow2_cols(2 * s.n) <= 256 ? 2 : 1;
+  const size_t stage = (size_t)(128 + s.n) * ch * 2, room = per_sm == 2 ? 110 * 1024 : 200 * 1024;
+  const int nstage = (int)std::min<size_t>(8, room / stage);
+  // (one per SM: more shared memory than two would leave)
+  const size_t smem = 1024 + std::max(nstage * stage, per_sm == 2 ? (size_t)78 * 1024 : (size_t)116 * 1024);
+  e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const int grid = std::min(B.count(), sms * per_sm);
+  k<<<(unsigned)grid, 192, smem, st>>>(m, s, B, sign, wp, bias, out, nstage, err);
+  return cudaGetLastError();
+}
+
+bool wgrad_box_supported(const ConvShape &s) {
+  Box B;
+  if (!shape_ok(s) || !choose_box(s, &B)) return false;
+  return (box_ch(s.cin) == 64 ? wb_mtiles<64>() : wb_mtiles<32>()) * s.n <= 512 && s.n <= 128;
+}
+
+cudaError_t conv_wgrad_box(const ConvShape &s, const __nv_bfloat16 *in, const __nv_bfloat16 *dout, float *dw, int *err,
+                           cudaStream_t st) {
+  Box B;
+  if (!wgrad_box_supported(s) || !choose_box(s, &B)) return cudaErrorNotSupported;
+  const int ch = box_ch(s.cin), chb = box_ch(s.n);
+  CUtensorMap mi, md;
+  if (!encode_box(&mi, in, s, s.cin, ch, B) || !encode_box(&md, dout, s, s.n, chb, B)) return cudaErrorNotSupported;
+  typedef void (*K)(const CUtensorMap, const CUtensorMap, ConvShape, Box, float *, int, int *);
+  K k = ch == 64 ? (chb == 64 ? k_wgrad_box<64, 64> : k_wgrad_box<64, 32>)
+                 : (chb == 64 ? k_wgrad_box<32, 64> : k_wgrad_box<32, 32>);
+  int sms = 0;
+  cudaError_t e = sm_count(&sms);
+  if (e != cudaSuccess) return e;
+  const int groups = 3 * ((s.cin + ch - 1) / ch);
+  const int slices = std::max(1, std::min(B.count(), sms / groups));
+  const size_t smem = 1024 + (size_t)WB_SLOTS * WB_A + 2 * (size_t)((s.n + chb - 1) / chb) * 128 * chb * 2;
+  e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k<<<(unsigned)(groups * slices), 192, smem, st>>>(mi, md, s, B, dw, slices, err);
+  return cudaGetLastError();
+}
+
+}  // namespace xtc

@@ -37,12 +37,13 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
-#include <mutex>
 
 #include "cnn_tc.cuh"
 #include "xtg_cnn_internal.h"
 
 namespace xtc {
+
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encode();  // cnn_conv_box.cu
 
 namespace {
 
@@ -465,19 +466,6 @@ __global__ void __launch_bounds__(160, 1)
   }
 }
 
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-  });
-  return fn;
-}
-
 }  // namespace
 
 // tile height for a shape: 4 z-lines when cout <= 32 and Z allows, else 2
@@ -486,7 +474,7 @@ static int tile_tz(const ConvShape &s) { return (s.n <= 32 && s.Z % 4 == 0) ? 4 
 bool wgrad_tile_supported(const ConvShape &s) {
   return s.nb >= 1 && s.Y >= 1 && s.X >= TX && s.X % TX == 0 && s.Z >= WG_TZ && s.Z % WG_TZ == 0 && s.cin >= 16 &&
          s.cin % 16 == 0 && s.n == 32 && (long long)(s.X / TX) * (s.Z / WG_TZ) * s.nb * s.Y < (1ll << 31) &&
-         encode_fn() != nullptr;
+         tensor_map_encode() != nullptr;
 }
 
 // activations [nb][Y][X][Z][c] seen as (c, x, z, y, b), boxes of 16 channels
@@ -496,7 +484,7 @@ static bool encode_act(CUtensorMap *m, const __nv_bfloat16 *p, const ConvShape &
   const cuuint64_t strides[4] = {(cuuint64_t)s.Z * C2, C2, (cuuint64_t)s.X * s.Z * C2, (cuuint64_t)s.Y * s.X * s.Z * C2};
   const cuuint32_t box[5] = {16, (cuuint32_t)bx, (cuuint32_t)bz, 1, 1};
   const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-  return encode_fn()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<__nv_bfloat16 *>(p), dims, strides, box, estr,
+  return tensor_map_encode()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<__nv_bfloat16 *>(p), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -528,7 +516,7 @@ cudaError_t conv_wgrad_tile(const ConvShape &s, const __nv_bfloat16 *in, const _
 bool conv_tile_supported(const ConvShape &s) {
   return s.nb >= 1 && s.Y >= 1 && s.X >= TX && s.X % TX == 0 && s.Z >= 2 && s.Z % 2 == 0 && s.cin >= 8 &&
          s.cin % 8 == 0 && s.n >= 16 && s.n % 16 == 0 && s.n <= TN_MAX &&
-         (long long)(s.X / TX) * (s.Z / 2) * s.nb * s.Y < (1ll << 31) && encode_fn() != nullptr;
+         (long long)(s.X / TX) * (s.Z / 2) * s.nb * s.Y < (1ll << 31) && tensor_map_encode() != nullptr;
 }
 
 size_t conv_tile_wp_elems(int cin, int n) { return (size_t)((cin + 15) / 16) * 27 * 2 * n * 8; }
@@ -555,7 +543,7 @@ cudaError_t conv_forward_tile(const ConvShape &s, const __nv_bfloat16 *in, const
   const int tz = tile_tz(s);
   const cuuint32_t box[5] = {16, TXS, (cuuint32_t)tz + 2, 3, 1};
   const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-  if (encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<__nv_bfloat16 *>(in), dims, strides, box, estr,
+  if (tensor_map_encode()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<__nv_bfloat16 *>(in), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return cudaErrorNotSupported;

@@ -28,6 +28,17 @@ cudaError_t conv_tile_pack(int cin, int n, int kpad, int sign, const __nv_bfloat
                            cudaStream_t st);
 cudaError_t conv_forward_tile(const ConvShape &s, const __nv_bfloat16 *in, const __nv_bfloat16 *wp, const float *bias,
                               void *out, int epi, int sign, int *err, cudaStream_t st);
+// TMA boxes of 128 voxels per tap (cnn_conv_box.cu): any volume, cin and n
+// multiples of 16; weights pre-packed by conv_box_pack into
+// conv_box_wp_elems values (the sign stays an argument)
+bool conv_box_supported(const ConvShape &s);
+size_t conv_box_wp_elems(int cin, int n);
+cudaError_t conv_box_pack(int cin, int n, int kpad, const __nv_bfloat16 *w, __nv_bfloat16 *wp, cudaStream_t st);
+cudaError_t conv_forward_box(const ConvShape &s, const __nv_bfloat16 *in, const __nv_bfloat16 *wp, const float *bias,
+                             void *out, int epi, int sign, int *err, cudaStream_t st);
+bool wgrad_box_supported(const ConvShape &s);
+cudaError_t conv_wgrad_box(const ConvShape &s, const __nv_bfloat16 *in, const __nv_bfloat16 *dout, float *dw, int *err,
+                           cudaStream_t st);
 // weight gradient: the TMA tile kernel where wgrad_tile_supported (cout 32,
 // cin a multiple of 16, X a multiple of 128, Z even), else the gather kernel;
 // path 1 forces the gather kernel, 2 the tile kernel (cudaErrorNotSupported
