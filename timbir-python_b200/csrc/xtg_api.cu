@@ -10,13 +10,13 @@
 //   k_prior_cost64    qGGMRF prior over forward neighbour pairs, FP64
 //   k_running_cost64  data term from the running e, FP64
 //   k_zinger_refresh  ProjSelect = |e sqrt(w)| < T
-//   k_vsc_filter / k_rs_hist + k_rs_pick / k_nhicd_compact   NHICD selection
-//   k_radix_select    the same order statistic in one CTA (allocation-free path)
+//   k_vsc_filter / k_nhicd_pick   NHICD selection
 //   k_offset_* / k_var_*   offset d and variance re-estimation
 //   k_build_items / k_magsum / k_build_a16 / k_counts / object transposes
 #include <algorithm>
 #include <numeric>
 #include <cmath>
+#include <cstddef>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -52,6 +52,20 @@ void xtg_set_error_text(const char *msg) { snprintf(g_err, sizeof g_err, "%s", m
   } while (0)
 
 #define NSLOT 64
+// What an iteration's kernels count, in one block: cleared by one memset when
+// the iteration starts and read by one copy to pinned memory when it ends (with
+// the error flag, which outlives it).  Statistics have three phases, since the
+// reference's vox_mag covers the last chunk's random pass alone
+// (XT_ICD_update.c:798): launches before it, it, launches after it.
+struct IterBlock {
+  double absx[3][NSLOT];            // sum |x| over updated voxels
+  unsigned long long cnt[3][4];     // voxel updates, zero skipped, items
+  double mag[NSLOT];                // sum of MagUpdateMap
+  int counter[3 * XT_NHICD_CHUNKS]; // item counters of the ICD launches (three per chunk)
+  int nhcnt[2 * XT_NHICD_CHUNKS];   // list lengths of each chunk's selection
+  int err;                          // not cleared with the rest
+};
+#define ITER_CLEAR offsetof(IterBlock, err)
 // parallel ICD: at most 1 in XTG_CONC_DIV of the columns updated at once
 #define XTG_CONC_DIV 32
 // ICD footprint loads keep w in L2 (like e) when e and w together take at
@@ -62,8 +76,6 @@ void xtg_set_error_text(const char *msg) { snprintf(g_err, sizeof g_err, "%s", m
 #ifndef XTG_W_KEEP_BYTES
 #define XTG_W_KEEP_BYTES (48u << 20)
 #endif
-
-struct RsState;  // radix-select state per segment (defined with its kernels)
 
 struct xtg_ctx {
   xt_params prm;
@@ -80,15 +92,14 @@ struct xtg_ctx {
   float *d_hr = nullptr, *d_cos = nullptr, *d_sin = nullptr, *d_ax = nullptr, *d_filt = nullptr, *d_tmp = nullptr;
   float *d_num = nullptr, *d_den = nullptr, *d_thr = nullptr, *d_var = nullptr;
   int *d_view_idx = nullptr, *d_view_start = nullptr, *d_view_num = nullptr, *d_fov = nullptr;
-  int *d_mcols = nullptr, *d_rank = nullptr, *d_counter = nullptr, *d_nhcnt = nullptr, *d_err = nullptr;
+  int *d_mcols = nullptr, *d_rank = nullptr;
+  IterBlock *d_it = nullptr, *h_it = nullptr;  // device, pinned host copy
+  int phase = 0;  // whose statistics the ICD launches add to
   int *d_kth = nullptr;
-  unsigned *d_rs_hist = nullptr;  // [segments][256] radix-select histograms
-  RsState *d_rs_st = nullptr;     // [segments]
   int4 *d_items = nullptr, *d_nh = nullptr;
   size_t items_cap = 0, nh_cap = 0;
   double *d_red = nullptr;       // [8][NSLOT] reduction slots
-  double *d_absx = nullptr;      // [NSLOT]
-  unsigned long long *d_cnt = nullptr;  // [4]
+  unsigned long long *d_cnt = nullptr;  // zinger count
   // A column table (CSC): entry runs per (frame, masked column)
   long long *d_tstart = nullptr;
   int *d_toff = nullptr;
@@ -129,7 +140,9 @@ struct xtg_ctx {
   cudaEvent_t ev_dx = nullptr, ev_dl = nullptr;
   int dl_pending = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ek0 = nullptr, ek1 = nullptr;
-  std::vector<cudaEvent_t> tev;  // start/stop pairs of the ICD launches of one iteration
+  std::vector<cudaEvent_t> tev;            // marks around the ICD launches of one iteration
+  std::vector<std::pair<int, int>> runs;   // first and last mark of each run of them
+  int nmark = 0;
   int have_sino = 0;
   long long launches = 0;
   float last_kms = 0.f;
@@ -337,154 +350,300 @@ __constant__ float c_vsc[25] = {0.0064f, 0.0432f, 0.0800f, 0.0432f, 0.0064f, 0.0
                                 0.0432f, 0.0800f, 0.5400f, 1.0000f, 0.5400f, 0.0800f, 0.0432f, 0.2916f, 0.5400f,
                                 0.2916f, 0.0432f, 0.0064f, 0.0432f, 0.0800f, 0.0432f, 0.0064f};
 
+__device__ __forceinline__ float vsc_value(const float *m, int ny, int nx, int j, int k) {
+  float f = 0.f;
+  if (j >= 2 && j + 2 < ny && k >= 2 && k + 2 < nx) {
+    const float *c = m + (size_t)(j - 2) * nx + k - 2;
+#pragma unroll
+    for (int p = 0; p < 5; p++)
+#pragma unroll
+      for (int s = 0; s < 5; s++) f = __fadd_rn(f, __fmul_rn(c_vsc[p * 5 + s], __ldg(c + (size_t)p * nx + s)));
+    return f;
+  }
+  for (int p = -2; p <= 2; p++)
+    for (int s = -2; s <= 2; s++)
+      if (j + p >= 0 && j + p < ny && k + s >= 0 && k + s < nx)
+        f = __fadd_rn(f, __fmul_rn(c_vsc[(p + 2) * 5 + s + 2], m[(size_t)(j + p) * nx + (k + s)]));
+  return f;
+}
+
 __global__ void k_vsc_filter(int nseg, int ny, int nx, const float *map, float *out) {
   const size_t n = (size_t)nseg * ny * nx;
   for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
     const int k = (int)(q % nx);
     const int j = (int)((q / nx) % ny);
     const size_t seg = q / ((size_t)nx * ny);
-    const float *m = map + seg * (size_t)nx * ny;
-    float f = 0.f;
-    for (int p = -2; p <= 2; p++)
-      for (int s = -2; s <= 2; s++)
-        if (j + p >= 0 && j + p < ny && k + s >= 0 && k + s < nx)
-          f = __fadd_rn(f, __fmul_rn(c_vsc[(p + 2) * 5 + s + 2], m[(size_t)(j + p) * nx + (k + s)]));
-    out[q] = f;
+    out[q] = vsc_value(map + seg * (size_t)nx * ny, ny, nx, j, k);
   }
 }
 
-// k-th smallest (1-based) of each segment by 4 passes of 8-bit radix
-// histograms; the exact order statistic RandomizedSelect returns
-// (XT_NHICD.c:63-126).
-__global__ void __launch_bounds__(1024) k_radix_select(const float *vals, int seglen, const int *kth, float *out) {
-  __shared__ unsigned hist[256];
-  __shared__ unsigned s_prefix, s_mask, s_k;
-  const float *v = vals + (size_t)blockIdx.x * seglen;
-  if (threadIdx.x == 0) {
-    s_prefix = 0;
-    s_mask = 0;
-    s_k = (unsigned)kth[blockIdx.x];
-  }
-  for (int shift = 24; shift >= 0; shift -= 8) {
-    for (int b = threadIdx.x; b < 256; b += blockDim.x) hist[b] = 0;
-    __syncthreads();
-    const unsigned pre = s_prefix, msk = s_mask;
-    for (int i = threadIdx.x; i < seglen; i += blockDim.x) {
-      const unsigned key = xt_f2key(v[i]);
-      if ((key & msk) == pre) atomicAdd(&hist[(key >> shift) & 255u], 1u);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned k = s_k, cum = 0;
-      int b = 0;
-      for (; b < 255; b++) {
-        if (cum + hist[b] >= k) break;
-        cum += hist[b];
-      }
-      s_k = k - cum;
-      s_prefix = pre | ((unsigned)b << shift);
-      s_mask = msk | (255u << shift);
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[blockIdx.x] = xt_key2f(s_prefix);
-}
-
-// The same order statistic spread over many CTAs per segment: per 8-bit pass,
-// k_rs_hist counts the keys that match the prefix found so far into a global
-// 256-bin histogram of the segment (a warp whose lanes share one bin adds 32
-// with a single atomic), and k_rs_pick finds the bin that holds the k-th key,
-// narrows the prefix and clears the histogram for the next pass.
-struct RsState {
-  unsigned prefix, mask, k, pad;
+// NHICD selection of one segment (a frame's z-block, or one map) by a cluster
+// of CTAs: the k-th smallest filtered value -- the order statistic
+// RandomizedSelect returns (XT_NHICD.c:63-126) -- and the columns above it.
+//
+// The segment is dealt to the cluster's CTAs, which keep their keys in shared
+// memory; four 8-bit radix passes count the keys under the prefix found so far
+// into shared histograms, every CTA adds the cluster's through distributed
+// shared memory (16 bytes a thread) and picks the bin that holds the k-th key,
+// so a pass costs one cluster barrier and no launch.  Bound by launch and barrier
+// latency: per chunk of an iteration the filter, eight histogram and pick
+// launches, the compaction (an atomic per selected column on two addresses)
+// and the copies between them took 96 us at 128^2 x 4 and 270 us for the 4D
+// volume of 16 frames of 256^2; this kernel 17 and 53 us (512^2: 126 -> 67).
+//
+// FILL 0: filtered values stay in global memory (segments too long for the
+// cluster's shared memory); 1: read from there; 2: filtered here from the maps.
+struct SelArgs {
+  const float *map;       // [segments][ny][nx] (FILL 2)
+  const float *filt;      // filtered maps (FILL 0, 1)
+  int ny, nx, chunk;      // chunk: values per CTA
+  const int *kth_dev;     // rank per segment, or null: kth for all
+  int kth;
+  float *thr;             // threshold per segment, or null
+  unsigned char *sel;     // 1 above the threshold, or null
+  // work items of the columns above the threshold (list0 null: none)
+  int nzb;
+  const int *col_rank;
+  float *mag;
+  int4 *list0, *list1;
+  int *cnt;
+  int cap0, cap1;
 };
+struct SelRanks {
+  int k[XTG_NOALLOC_MAX_MAPS];
+};
+#define SEL_THREADS 512
+#define SEL_BINS 256
 
-__global__ void k_rs_init(const int *kth, RsState *st, unsigned *hist) {
-  if (threadIdx.x == 0) st[blockIdx.x] = RsState{0u, 0u, (unsigned)kth[blockIdx.x], 0u};
-  for (int b = threadIdx.x; b < 256; b += blockDim.x) hist[(size_t)blockIdx.x * 256 + b] = 0u;
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned cluster_size() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// 16 bytes of another cluster CTA's shared memory
+__device__ __forceinline__ uint4 cluster_ld4(const unsigned *p, unsigned rank) {
+  unsigned a;
+  uint4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(a)
+               : "memory");
+  return v;
 }
 
-__global__ void __launch_bounds__(256) k_rs_hist(const float *vals, int seglen, int shift, const RsState *st,
-                                                 unsigned *hist) {
-  __shared__ unsigned h[256];
-  const int seg = blockIdx.y, lane = threadIdx.x & 31;
-  h[threadIdx.x] = 0u;
-  __syncthreads();
-  const unsigned pre = st[seg].prefix, msk = st[seg].mask;
-  const float *v = vals + (size_t)seg * seglen;
-  const int stride = gridDim.x * blockDim.x;
-  for (int i0 = blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < seglen; i0 += stride) {
-    const int i = i0 + lane;
-    unsigned bin = 256u;  // no key here, or not under the prefix
-    if (i < seglen) {
-      const unsigned key = xt_f2key(v[i]);
-      if ((key & msk) == pre) bin = (key >> shift) & 255u;
-    }
-    const unsigned b0 = __shfl_sync(0xffffffffu, bin, 0);
-    if (__all_sync(0xffffffffu, bin == b0)) {
-      if (lane == 0 && b0 < 256u) atomicAdd(&h[b0], 32u);
-    } else if (bin < 256u) {
-      atomicAdd(&h[bin], 1u);
-    }
+// exclusive prefix sum of v over the CTA's SEL_THREADS threads; total in *sum
+__device__ __forceinline__ unsigned block_scan(unsigned v, unsigned *warps, unsigned *sum) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned inc = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
   }
+  __syncthreads();  // warps may still be read by the previous scan
+  if (lane == 31) warps[warp] = inc;
   __syncthreads();
-  if (h[threadIdx.x]) atomicAdd(&hist[(size_t)seg * 256 + threadIdx.x], h[threadIdx.x]);
-}
-
-__global__ void __launch_bounds__(256) k_rs_pick(int shift, RsState *st, unsigned *hist, float *out) {
-  const int seg = blockIdx.x;
-  unsigned *hs = hist + (size_t)seg * 256;
-  if (threadIdx.x == 0) {
-    const unsigned k = st[seg].k;
-    unsigned cum = 0;
-    int b = 0;
-    for (; b < 255; b++) {
-      if (cum + hs[b] >= k) break;
-      cum += hs[b];
-    }
-    st[seg].k = k - cum;
-    st[seg].prefix |= (unsigned)b << shift;
-    st[seg].mask |= 255u << shift;
-    if (shift == 0) out[seg] = xt_key2f(st[seg].prefix);
+  unsigned base = 0, tot = 0;
+#pragma unroll
+  for (int w = 0; w < SEL_THREADS / 32; w++) {
+    const unsigned u = warps[w];
+    if (w < warp) base += u;
+    tot += u;
   }
-  __syncthreads();
-  hs[threadIdx.x] = 0u;
+  *sum = tot;
+  return base + inc - v;
 }
 
-// columns above the threshold -> NHICD work items.  List 0 holds the
-// (frame, block) pairs the reference updates in its first half-pass (block
-// parity = frame parity, XT_ICD_update.c:846-857), list 1 the others.
-// A selected column outside the object-support disk has no voxel to update;
-// the reference still visits it, which only zeroes its MagUpdateMap entry
-// (XT_VoxUpdate.c:128, 138), so that is all done for it here.
-__global__ void k_nhicd_compact(int ntime, int nzb, int ny, int nx, const float *filt, const float *thr,
-                                const int *col_rank, float *mag, int4 *list0, int4 *list1, int *cnt, int cap0,
-                                int cap1) {
-  const size_t n = (size_t)ntime * nzb * ny * nx;
-  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-    const size_t seg = q / ((size_t)nx * ny);
-    if (!(filt[q] > thr[seg])) continue;
-    const int k = (int)(q % nx), j = (int)((q / nx) % ny);
-    if (col_rank[(size_t)j * nx + k] < 0) {
-      mag[q] = 0.f;
-      continue;
+template <int FILL>
+__global__ void __launch_bounds__(SEL_THREADS) k_nhicd_pick(SelArgs S, SelRanks R) {
+  extern __shared__ __align__(16) unsigned sel_keys[];  // [chunk rounded up to 4] (FILL 1, 2)
+  __shared__ __align__(16) unsigned hist[2][SEL_BINS];
+  __shared__ unsigned total[SEL_BINS], warps[SEL_THREADS / 32];
+  __shared__ unsigned s_bin, s_k, s_base;
+  const int seg = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
+  const unsigned rank = cluster_rank(), nc = cluster_size();
+  const size_t seglen = (size_t)S.ny * S.nx;
+  const size_t lo = (size_t)rank * S.chunk;
+  const int n = lo < seglen ? (int)min((size_t)S.chunk, seglen - lo) : 0;
+  const float *filt = FILL < 2 ? S.filt + seg * seglen + lo : nullptr;
+  if (FILL == 1)
+    for (int i = tid; i < n; i += SEL_THREADS) sel_keys[i] = xt_f2key(filt[i]);
+  if (FILL == 2)
+    for (int i = tid; i < n; i += SEL_THREADS) {
+      const int q = (int)lo + i, j = q / S.nx;
+      sel_keys[i] = xt_f2key(vsc_value(S.map + seg * seglen, S.ny, S.nx, j, q - j * S.nx));
     }
-    const int b = (int)(seg % nzb), f = (int)(seg / nzb);
-    const int h = ((f & 1) == (b & 1)) ? 0 : 1;
-    const int slot = atomicAdd(&cnt[h], 1);
-    if (h == 0) {
-      if (slot < cap0) list0[slot] = make_int4(f, j, k, b);
+  auto key_at = [&](int i) { return FILL ? sel_keys[i] : xt_f2key(filt[i]); };
+  unsigned prefix = 0, mask = 0, k = (unsigned)(S.kth_dev ? S.kth_dev[seg] : S.kth ? S.kth : R.k[seg]);
+  for (int shift = 24; shift >= 0; shift -= 8) {
+    unsigned *h = hist[(shift >> 3) & 1];  // the other one may still be read by the cluster
+    for (int b = tid; b < SEL_BINS; b += SEL_THREADS) h[b] = total[b] = 0u;
+    __syncthreads();  // (and the keys are in place)
+    // a thread adds up runs of one bin in registers: neighbouring values (and
+    // zeros) share their leading bits, and in the later passes few keys match
+    // (warp votes on every key instead took ten times as long)
+    unsigned cur = 0u, run = 0u;
+    auto count = [&](unsigned key, bool valid) {
+      if (valid && (key & mask) == prefix) {
+        const unsigned bin = (key >> shift) & 255u;
+        if (bin != cur) {
+          if (run) atomicAdd(&h[cur], run);
+          cur = bin;
+          run = 0u;
+        }
+        run++;
+      }
+    };
+    if (FILL) {
+      for (int i = tid * 4; i < n; i += SEL_THREADS * 4) {
+        const uint4 q = *reinterpret_cast<const uint4 *>(sel_keys + i);
+        count(q.x, true);
+        count(q.y, i + 1 < n);
+        count(q.z, i + 2 < n);
+        count(q.w, i + 3 < n);
+      }
     } else {
-      if (slot < cap1) list1[slot] = make_int4(f, j, k, b);
+      for (int i = tid * 4; i < n; i += SEL_THREADS * 4)
+        for (int u = 0; u < 4 && i + u < n; u++) count(key_at(i + u), true);
+    }
+    if (run) atomicAdd(&h[cur], run);
+    cluster_barrier();
+    for (int u = tid; u < (int)nc * (SEL_BINS / 4); u += SEL_THREADS) {
+      const int b = (u % (SEL_BINS / 4)) * 4;
+      const uint4 v = cluster_ld4(h + b, (unsigned)u / (SEL_BINS / 4));
+      if (v.x) atomicAdd(&total[b], v.x);
+      if (v.y) atomicAdd(&total[b + 1], v.y);
+      if (v.z) atomicAdd(&total[b + 2], v.z);
+      if (v.w) atomicAdd(&total[b + 3], v.w);
+    }
+    __syncthreads();
+    if (tid < 32) {
+      unsigned c[8], mine = 0;
+#pragma unroll
+      for (int u = 0; u < 8; u++) mine += c[u] = total[lane * 8 + u];
+      unsigned inc = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
+      }
+      unsigned cum = inc - mine;
+      if (cum < k && k <= inc) {
+        int u = 0;
+        while (u < 7 && cum + c[u] < k) cum += c[u++];
+        s_bin = (unsigned)(lane * 8 + u);
+        s_k = k - cum;
+      }
+    }
+    __syncthreads();
+    prefix |= s_bin << shift;
+    mask |= 255u << shift;
+    k = s_k;
+  }
+  const float thr = xt_key2f(prefix);
+  if (S.thr && rank == 0 && tid == 0) S.thr[seg] = thr;
+  if (S.sel)
+    for (int i = tid; i < n; i += SEL_THREADS) S.sel[seg * seglen + lo + i] = xt_key2f(key_at(i)) > thr ? 1 : 0;
+  if (S.list0) {
+    // Columns above the threshold -> work items.  List 0 holds the (frame,
+    // block) pairs the reference updates in its first half-pass (block parity
+    // = frame parity, XT_ICD_update.c:846-857), list 1 the others.  A selected
+    // column outside the object-support disk has no voxel to update; the
+    // reference still visits it, which only zeroes its MagUpdateMap entry
+    // (XT_VoxUpdate.c:128, 138), so that is all done for it here.  (Every CTA
+    // of the cluster has read the map by now.)
+    const int b = seg % S.nzb, f = seg / S.nzb, half = ((f & 1) == (b & 1)) ? 0 : 1;
+    // four columns a thread at a time, their ranks loaded ahead of the test:
+    // looked up one by one for the selected columns they were half the kernel
+    const bool al = (seglen & 3) == 0;  // (lo is a multiple of 4)
+    auto picked = [&](int i) {
+      int r[4];
+      if (al && i + 3 < n) {
+        const int4 v = __ldg(reinterpret_cast<const int4 *>(S.col_rank + lo + i));
+        r[0] = v.x; r[1] = v.y; r[2] = v.z; r[3] = v.w;
+      } else {
+#pragma unroll
+        for (int u = 0; u < 4; u++) r[u] = i + u < n ? __ldg(S.col_rank + lo + i + u) : -1;
+      }
+      unsigned m = 0;  // bits 0-3: to update; bits 4-7: outside the disk
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (i + u < n && xt_key2f(key_at(i + u)) > thr) m |= (r[u] >= 0 ? 1u : 16u) << u;
+      return m;
+    };
+    unsigned c = 0;
+#pragma unroll 4
+    for (int i = tid * 4; i < n; i += SEL_THREADS * 4) {
+      const unsigned m = picked(i);
+      c += __popc(m & 15u);
+      for (unsigned o = m >> 4; o; o &= o - 1) S.mag[seg * seglen + lo + i + __ffs(o) - 1] = 0.f;
+    }
+    unsigned tot, at = block_scan(c, warps, &tot);
+    if (tid == 0) s_base = tot ? (unsigned)atomicAdd(&S.cnt[half], (int)tot) : 0u;
+    __syncthreads();
+    at += s_base;
+    int4 *list = half ? S.list1 : S.list0;
+    const unsigned cap = (unsigned)(half ? S.cap1 : S.cap0);
+    if (c) {
+#pragma unroll 4
+      for (int i = tid * 4; i < n; i += SEL_THREADS * 4) {
+        for (unsigned m = picked(i) & 15u; m; m &= m - 1, at++) {
+          const int q = (int)lo + i + __ffs(m) - 1, j = q / S.nx;
+          if (at < cap) list[at] = make_int4(f, j, q - j * S.nx, b);
+        }
+      }
     }
   }
+  cluster_barrier();  // no CTA leaves while its histogram may be read
 }
 
-__global__ void k_clamp_count(int *cnt, int cap0, int cap1) {
-  if (threadIdx.x == 0) {
-    cnt[0] = min(cnt[0], cap0);
-    cnt[1] = min(cnt[1], cap1);
+// nseg segments of ny x nx values; returns the launches made through *launches
+static cudaError_t nhicd_pick(SelArgs S, const SelRanks *R, int nseg, int sms, float *filt, cudaStream_t st, int *launches) {
+  const size_t seglen = (size_t)S.ny * S.nx;
+  // CTAs per segment: enough to share the work, no more than the GPU holds
+  // twice, but chunks that fit in shared memory where eight can do that
+  int nc = seglen > 4096 ? 8 : seglen > 1024 ? 4 : 1;
+  while (nc > 1 && nseg * nc > 2 * sms && seglen <= (size_t)nc / 2 * 16384) nc /= 2;
+  S.chunk = (int)(((seglen + nc - 1) / nc + 3) / 4 * 4);
+  // Filtering here spares a launch and a pass; where the clusters leave most of
+  // the GPU idle and chunks are long, all of it filters sooner (16 maps of
+  // 256^2: 57 us here, 47 with the filter kernel; 32 of them: 53 and 61 an
+  // iteration chunk; 4 of 128^2 30 either way)
+  const int fill = S.chunk <= (nseg * nc >= sms ? 8192 : 2048) ? 2 : S.chunk <= 49152 ? 1 : 0;
+  *launches = 1;
+  if (fill < 2) {
+    const size_t n = (size_t)nseg * seglen;
+    k_vsc_filter<<<(unsigned)std::min<size_t>((n + 255) / 256, (size_t)sms * 8), 256, 0, st>>>(nseg, S.ny, S.nx, S.map, filt);
+    S.filt = filt;
+    *launches = 2;
   }
+  const size_t smem = fill ? ((size_t)S.chunk + 3) / 4 * 16 : 0;
+  auto k = fill == 2 ? k_nhicd_pick<2> : fill == 1 ? k_nhicd_pick<1> : k_nhicd_pick<0>;
+  cudaError_t e = full_smem((const void *)k);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)nc, (unsigned)nseg);
+  cfg.blockDim = dim3(SEL_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)nc;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  static const SelRanks none = {};
+  return cudaLaunchKernelEx(&cfg, k, S, R ? *R : none);
 }
 
 // update_Sinogram_Offset (XT_ICD_update.c:666-759), one thread per (r, t),
@@ -762,13 +921,14 @@ void xtg_destroy(xtg_ctx *c) {
   if (c->coarse) xtg_destroy(c->coarse);
   void *ptrs[] = {c->d_y, c->d_w, c->d_e, c->d_d, c->d_x, c->d_mag, c->d_hr, c->d_cos, c->d_sin, c->d_ax,
                   c->d_filt, c->d_tmp, c->d_num, c->d_den, c->d_thr, c->d_var, c->d_view_idx, c->d_view_start,
-                  c->d_view_num, c->d_fov, c->d_mcols, c->d_rank, c->d_counter, c->d_nhcnt, c->d_err, c->d_kth,
-                  c->d_items, c->d_nh, c->d_red, c->d_absx, c->d_cnt, c->d_tstart, c->d_toff, c->d_tval32,
-                  c->d_tscale, c->d_tval16, c->d_rs_hist, c->d_rs_st, c->d_cptr, c->d_cent};
+                  c->d_view_num, c->d_fov, c->d_mcols, c->d_rank, c->d_it, c->d_kth,
+                  c->d_items, c->d_nh, c->d_red, c->d_cnt, c->d_tstart, c->d_toff, c->d_tval32,
+                  c->d_tscale, c->d_tval16, c->d_cptr, c->d_cent};
   if (c->dl_pending && c->ev_dl) cudaEventSynchronize(c->ev_dl);
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (c->d_dl) cudaFree(c->d_dl);
+  if (c->h_it) cudaFreeHost(c->h_it);
   if (c->ev_dx) cudaEventDestroy(c->ev_dx);
   if (c->ev_dl) cudaEventDestroy(c->ev_dl);
   if (c->ev0) cudaEventDestroy(c->ev0);
@@ -863,8 +1023,6 @@ int xtg_create(const xt_params *prm, const double *times, const double *angles, 
   rc |= dalloc(c, &c->d_den, c->nrt);
   rc |= dalloc(c, &c->d_thr, (size_t)g.N_time * g.nzb);
   rc |= dalloc(c, &c->d_kth, (size_t)g.N_time * g.nzb);
-  rc |= dalloc(c, &c->d_rs_hist, (size_t)g.N_time * g.nzb * 256);
-  rc |= dalloc(c, &c->d_rs_st, (size_t)g.N_time * g.nzb);
   rc |= dalloc(c, &c->d_var, 1);
   rc |= dalloc(c, &c->d_view_idx, (size_t)g.N_p);
   rc |= dalloc(c, &c->d_view_start, (size_t)g.N_time);
@@ -872,12 +1030,9 @@ int xtg_create(const xt_params *prm, const double *times, const double *angles, 
   rc |= dalloc(c, &c->d_fov, (size_t)g.N_p);
   rc |= dalloc(c, &c->d_mcols, (size_t)c->n_masked);
   rc |= dalloc(c, &c->d_rank, c->nxy);
-  rc |= dalloc(c, &c->d_counter, 8);
-  rc |= dalloc(c, &c->d_nhcnt, 2);
-  rc |= dalloc(c, &c->d_err, 1);
+  rc |= dalloc(c, &c->d_it, 1);
   rc |= dalloc(c, &c->d_red, 8 * NSLOT);
-  rc |= dalloc(c, &c->d_absx, NSLOT);
-  rc |= dalloc(c, &c->d_cnt, 4);
+  rc |= dalloc(c, &c->d_cnt, 1);
   c->items_cap = (size_t)g.N_time * c->n_masked + 1;
   rc |= dalloc(c, &c->d_items, c->items_cap);
   c->nh_cap = (size_t)g.N_time * g.nzb * (c->n_masked / XT_NHICD_CHUNKS + 1) + 2;
@@ -904,7 +1059,8 @@ int xtg_create(const xt_params *prm, const double *times, const double *angles, 
   CK(cudaMemset(c->d_e, 0, c->ns * 4));
   CK(cudaMemset(c->d_d, 0, c->nrt * 4));
   CK(cudaMemset(c->d_mag, 0, c->nmag * 4));
-  CK(cudaMemset(c->d_err, 0, 4));
+  CK(cudaMemset(c->d_it, 0, sizeof(IterBlock)));
+  CK(cudaMallocHost(&c->h_it, sizeof(IterBlock)));
   const float var = g.var_est;
   CK(cudaMemcpy(c->d_var, &var, 4, cudaMemcpyHostToDevice));
   *out = c;
@@ -994,12 +1150,10 @@ int xtg_set_options(xtg_ctx *c, int32_t a_mode, int32_t order, int32_t max_colum
   return 0;
 }
 
+// the error flag of the iteration block just read to the host
 static int check_err_flag(xtg_ctx *c) {
-  int h = 0;
-  CK(cudaMemcpyAsync(&h, c->d_err, 4, cudaMemcpyDeviceToHost, c->st));
-  CK(cudaStreamSynchronize(c->st));
-  if (h) {
-    CK(cudaMemsetAsync(c->d_err, 0, 4, c->st));
+  if (c->h_it->err) {
+    CK(cudaMemsetAsync(&c->d_it->err, 0, 4, c->st));
     set_err("non-finite voxel value in an update (theta2 + prior weight <= 0)");
     return XTG_E_NUMERIC;
   }
@@ -1572,12 +1726,12 @@ int xtg_zinger_refresh(xtg_ctx *c, uint8_t *sel, int64_t *nsel) {
   if (!c) return XTG_E_ARG;
   unsigned char *ds = nullptr;
   if (sel) CK(cudaMalloc(&ds, c->ns));
-  CK(cudaMemsetAsync(c->d_cnt + 3, 0, 8, c->st));
+  CK(cudaMemsetAsync(c->d_cnt, 0, 8, c->st));
   const unsigned grid = std::min<unsigned>(blocks_for(c->ns, 256), (unsigned)c->sm_count * 8);
-  k_zinger_refresh<<<grid, 256, 0, c->st>>>(c->ns, c->d_e, c->d_w, c->g.T, ds, c->d_cnt + 3);
+  k_zinger_refresh<<<grid, 256, 0, c->st>>>(c->ns, c->d_e, c->d_w, c->g.T, ds, c->d_cnt);
   c->launches++;
   unsigned long long h = 0;
-  cudaMemcpyAsync(&h, c->d_cnt + 3, 8, cudaMemcpyDeviceToHost, c->st);
+  cudaMemcpyAsync(&h, c->d_cnt, 8, cudaMemcpyDeviceToHost, c->st);
   if (sel) cudaMemcpyAsync(sel, ds, c->ns, cudaMemcpyDeviceToHost, c->st);
   cudaError_t e = cudaStreamSynchronize(c->st);
   if (ds) cudaFree(ds);
@@ -1753,7 +1907,7 @@ static int zslab(const xtg_ctx *c) {
 
 // one ICD launch over items[lo, lo+n) (or a device-counted list)
 static int run_columns(xtg_ctx *c, int iter, const int4 *items, int lo, int n, const int *n_dev, int use_perm,
-                       unsigned long long key, int has_whole, int has_blocks, int seq_override) {
+                       unsigned long long key, int has_whole, int has_blocks, int seq_override, int slot = -1) {
   const xt_geom &g = c->g;
   if (c->a_mode != XTG_A_FP32) {
     int rc = ensure_table(c);
@@ -1801,10 +1955,11 @@ static int run_columns(xtg_ctx *c, int iter, const int4 *items, int lo, int n, c
   memset(&A, 0, sizeof(A));
   A.e = c->d_e; A.w = c->d_w; A.x = c->d_x; A.magmap = c->d_mag; A.hr = c->d_hr; A.cosv = c->d_cos;
   A.sinv = c->d_sin; A.view_idx = c->d_view_idx; A.view_start = c->d_view_start; A.view_num = c->d_view_num;
-  A.items = items; A.n_items_dev = n_dev; A.n_items = n; A.item_lo = lo; A.counter = c->d_counter;
+  A.items = items; A.n_items_dev = n_dev; A.n_items = n; A.item_lo = lo; A.counter = &c->d_it->counter[std::max(slot, 0)];
   A.use_perm = use_perm; A.perm_key = key; A.col_rank = c->d_rank; A.n_masked = c->n_masked; A.iter = iter;
   A.tstart = c->d_tstart; A.toff = c->d_toff; A.tval32 = c->d_tval32; A.tval16 = c->d_tval16; A.tscale = c->d_tscale;
-  A.T2 = g.T * g.T; A.Tdelta = g.T * g.delta; A.st_absx = c->d_absx; A.st_cnt = c->d_cnt; A.err = c->d_err;
+  A.T2 = g.T * g.T; A.Tdelta = g.T * g.delta; A.st_absx = c->d_it->absx[c->phase]; A.st_cnt = c->d_it->cnt[c->phase];
+  A.err = &c->d_it->err;
   A.zslab = hz; A.nsub = nsub;
   A.e2p = 2.0f - g.MRF_P;
   A.l_sqp = (float)log2((double)g.Sigma_S_Q_P); A.l_tqp = (float)log2((double)g.Sigma_T_Q_P);
@@ -1840,7 +1995,7 @@ static int run_columns(xtg_ctx *c, int iter, const int4 *items, int lo, int n, c
     // a launch against 38)
     if (nt < XTG_THREADS) A.grab = (int)std::max(1ll, std::min(8ll, nexp / (4ll * grid)));
   }
-  CK(cudaMemsetAsync(c->d_counter, 0, 4, c->st));
+  if (slot < 0) CK(cudaMemsetAsync(A.counter, 0, 4, c->st));  // an iteration clears its launches' counters together
   CK(launch_icd(c->G, A, vec, amode, seq, as, vcap, zmax, grid, nt, c->st));
   c->icd_launches++;
   c->launches++;
@@ -1850,65 +2005,53 @@ static int run_columns(xtg_ctx *c, int iter, const int4 *items, int lo, int n, c
 static void magsum_launch(xtg_ctx *c) {
   const size_t n = (size_t)c->g.N_time * c->g.nzb * c->n_masked;
   const unsigned grid = std::min<unsigned>(blocks_for(n, 256), (unsigned)c->sm_count * 4);
-  k_magsum<<<std::max(grid, 1u), 256, 0, c->st>>>(c->G, c->n_masked, c->d_mcols, c->d_mag, c->d_red + 4 * NSLOT);
+  k_magsum<<<std::max(grid, 1u), 256, 0, c->st>>>(c->G, c->n_masked, c->d_mcols, c->d_mag, c->d_it->mag);
   c->launches++;
 }
 
-// k-th smallest of each of nseg segments of c->d_filt (k from c->d_kth) into
-// c->d_thr: four 8-bit passes, each a histogram over many CTAs and a pick
-static void radix_select_multi(xtg_ctx *c, int nseg) {
-  const int seglen = (int)c->nxy;
-  const int parts = std::max(1, std::min(64, (seglen + 8191) / 8192));
-  k_rs_init<<<nseg, 256, 0, c->st>>>(c->d_kth, c->d_rs_st, c->d_rs_hist);
-  for (int shift = 24; shift >= 0; shift -= 8) {
-    k_rs_hist<<<dim3((unsigned)parts, (unsigned)nseg), 256, 0, c->st>>>(c->d_filt, seglen, shift, c->d_rs_st,
-                                                                       c->d_rs_hist);
-    k_rs_pick<<<nseg, 256, 0, c->st>>>(shift, c->d_rs_st, c->d_rs_hist, c->d_thr);
-  }
-  c->launches += 9;
-}
-
-// NHICD selection on the device: filter, per-(frame, block) order statistic,
-// compaction into the two half-pass lists.
-static int nhicd_select_device(xtg_ctx *c) {
+// NHICD selection on the device: filter, per-(frame, block) order statistic
+// and the two half-pass lists, whose lengths go to cnt[0..1] (zero before; the
+// ICD kernel stops at the lists' capacity).
+static int nhicd_select_device(xtg_ctx *c, int *cnt) {
   const xt_geom &g = c->g;
-  const int nseg = g.N_time * g.nzb;
-  const int nsel = c->n_masked / XT_NHICD_CHUNKS;
-  std::vector<int> kth(nseg, (int)c->nxy - nsel);
-  CK(cudaMemcpyAsync(c->d_kth, kth.data(), nseg * 4, cudaMemcpyHostToDevice, c->st));
-  const unsigned grid = std::min<unsigned>(blocks_for(c->nmag, 256), (unsigned)c->sm_count * 8);
-  k_vsc_filter<<<grid, 256, 0, c->st>>>(nseg, g.N_y, g.N_x, c->d_mag, c->d_filt);
-  radix_select_multi(c, nseg);
-  CK(cudaMemsetAsync(c->d_nhcnt, 0, 8, c->st));
-  const int cap0 = (int)(c->nh_cap / 2), cap1 = (int)(c->nh_cap - c->nh_cap / 2);
-  k_nhicd_compact<<<grid, 256, 0, c->st>>>(g.N_time, g.nzb, g.N_y, g.N_x, c->d_filt, c->d_thr, c->d_rank,
-                                           c->d_mag, c->d_nh, c->d_nh + cap0, c->d_nhcnt, cap0, cap1);
-  k_clamp_count<<<1, 32, 0, c->st>>>(c->d_nhcnt, cap0, cap1);
-  c->launches += 3;
-  CK(cudaGetLastError());
+  SelArgs S;
+  memset(&S, 0, sizeof(S));
+  S.map = c->d_mag;
+  S.ny = g.N_y;
+  S.nx = g.N_x;
+  S.kth = (int)c->nxy - c->n_masked / XT_NHICD_CHUNKS;
+  S.nzb = g.nzb;
+  S.col_rank = c->d_rank;
+  S.mag = c->d_mag;
+  S.cap0 = (int)(c->nh_cap / 2);
+  S.cap1 = (int)(c->nh_cap - c->nh_cap / 2);
+  S.list0 = c->d_nh;
+  S.list1 = c->d_nh + S.cap0;
+  S.cnt = cnt;
+  int nl = 0;
+  CK(nhicd_pick(S, nullptr, g.N_time * g.nzb, c->sm_count, c->d_filt, c->st, &nl));
+  c->launches += nl;
   return 0;
 }
 
-static int read_stats(xtg_ctx *c, xtg_stats *st, double *absx_out) {
-  double ab[NSLOT];
-  unsigned long long cnt[3];
-  CK(cudaMemcpyAsync(ab, c->d_absx, sizeof(ab), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaMemcpyAsync(cnt, c->d_cnt, sizeof(cnt), cudaMemcpyDeviceToHost, c->st));
+// the iteration block to the host; adds a phase's counts to st
+static int fetch_block(xtg_ctx *c) {
+  CK(cudaMemcpyAsync(c->h_it, c->d_it, sizeof(IterBlock), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
-  double s = 0;
-  for (int i = 0; i < NSLOT; i++) s += ab[i];
-  if (absx_out) *absx_out = s;
-  if (st) {
-    st->voxel_updates += (int64_t)cnt[0];
-    st->zero_skipped += (int64_t)cnt[1];
-    st->columns += (int64_t)cnt[2];
-  }
   return 0;
 }
+static double add_phase(const IterBlock *h, int phase, xtg_stats *st) {
+  double s = 0;
+  for (int i = 0; i < NSLOT; i++) s += h->absx[phase][i];
+  st->voxel_updates += (int64_t)h->cnt[phase][0];
+  st->zero_skipped += (int64_t)h->cnt[phase][1];
+  st->columns += (int64_t)h->cnt[phase][2];
+  return s;
+}
 
-static int reset_stats(xtg_ctx *c) {
-  CK(cudaMemsetAsync(c->d_absx, 0, NSLOT * 8, c->st));
-  CK(cudaMemsetAsync(c->d_cnt, 0, 3 * 8, c->st));
+static int clear_block(xtg_ctx *c) {
+  CK(cudaMemsetAsync(c->d_it, 0, ITER_CLEAR, c->st));
+  c->phase = 0;
   return 0;
 }
 
@@ -2001,54 +2144,59 @@ static int icd_iteration_parallel(xtg_ctx *c, int iter, xtg_stats *st) {
   c->launches++;
   CK(cudaGetLastError());
   const int K = XT_NHICD_CHUNKS, chunk = n / K;
-  const int cap0 = (int)(c->nh_cap / 2);
-  float kms_total = 0.f;
+  const int cap0 = (int)(c->nh_cap / 2), cap1 = (int)(c->nh_cap - c->nh_cap / 2);
   long long items_total = 0;
-  double vox_mag = 0;
-  // ICD launches are timed with event pairs read once at the end of the
-  // iteration, so the host never waits between launches
-  const size_t npair = (size_t)3 * K;
-  while (c->tev.size() < 2 * npair) {
-    cudaEvent_t e;
-    CK(cudaEventCreate(&e));
-    c->tev.push_back(e);
-  }
-  size_t ntimed = 0;
+  // ICD launches are timed with events read once at the end of the iteration,
+  // so the host never waits between launches.  A timing event costs the stream
+  // about 3 us, so launches that follow each other directly share one: the
+  // list holds runs of marks, each run's last - first added up.
+  c->nmark = 0;
+  std::vector<std::pair<int, int>> runs;  // first, last mark of each run
+  auto mark = [&]() -> cudaError_t {
+    if (c->nmark == (int)c->tev.size()) {
+      cudaEvent_t e;
+      const cudaError_t r = cudaEventCreate(&e);
+      if (r != cudaSuccess) return r;
+      c->tev.push_back(e);
+    }
+    return cudaEventRecord(c->tev[c->nmark++], c->st);
+  };
+  auto launch_begins = [&](bool follows) -> cudaError_t {  // follows: directly after the launch marked last
+    if (follows && !runs.empty()) return cudaSuccess;
+    runs.emplace_back(c->nmark, c->nmark);
+    return mark();
+  };
+  auto launch_ends = [&]() -> cudaError_t {
+    const cudaError_t r = mark();
+    runs.back().second = c->nmark - 1;
+    return r;
+  };
+  // whether nothing is queued between a launch and the next one
+  const bool direct = !c->xfn && c->prm.updateProjOffset <= 1;
+  const bool nhicd = iter > 1 && !c->prm.no_NHICD;
   for (int j = 0; j < K; j++) {
     const int lo = j * chunk, hi = (j == K - 1) ? n : (j + 1) * chunk;
-    if (j == K - 1) {  // the reference's vox_mag covers the last chunk only (XT_ICD_update.c:798)
-      double tmp;
-      int rc = read_stats(c, st, &tmp);
-      if (rc) return rc;
-      rc = reset_stats(c);
-      if (rc) return rc;
-    }
-    CK(cudaEventRecord(c->tev[2 * ntimed], c->st));
-    int rc = run_columns(c, iter, c->d_items, lo, hi - lo, nullptr, 0, 0, 1, 0, -1);
+    if (j == K - 1) c->phase = 1;
+    CK(launch_begins(direct && nhicd && j > 0));
+    int rc = run_columns(c, iter, c->d_items, lo, hi - lo, nullptr, 0, 0, 1, 0, -1, 3 * j);
     if (rc) return rc;
-    CK(cudaEventRecord(c->tev[2 * ntimed + 1], c->st));
-    ntimed++;
+    CK(launch_ends());
+    if (j == K - 1) c->phase = 2;
     if ((rc = slab_exchange(c))) return rc;
-    if (j == K - 1) {
-      rc = read_stats(c, st, &vox_mag);
-      if (rc) return rc;
-      rc = reset_stats(c);
-      if (rc) return rc;
-    }
     items_total += hi - lo;
     if (c->prm.updateProjOffset > 1) {
       rc = xtg_update_offset(c);
       if (rc) return rc;
     }
-    rc = nhicd_select_device(c);
+    rc = nhicd_select_device(c, c->d_it->nhcnt + 2 * j);
     if (rc) return rc;
-    if (iter > 1 && !c->prm.no_NHICD) {
+    if (nhicd) {
       for (int h = 0; h < 2; h++) {
-        CK(cudaEventRecord(c->tev[2 * ntimed], c->st));
-        rc = run_columns(c, iter, c->d_nh, h ? cap0 : 0, 0, c->d_nhcnt + h, 1, key + 17 * (j * 2 + h + 1), 0, 1, -1);
+        CK(launch_begins(direct && h == 1));
+        rc = run_columns(c, iter, c->d_nh, h ? cap0 : 0, h ? cap1 : cap0, c->d_it->nhcnt + 2 * j + h, 1,
+                         key + 17 * (j * 2 + h + 1), 0, 1, -1, 3 * j + 1 + h);
         if (rc) return rc;
-        CK(cudaEventRecord(c->tev[2 * ntimed + 1], c->st));
-        ntimed++;
+        if (!direct || (h == 1 && j == K - 1)) CK(launch_ends());
         if ((rc = slab_exchange(c))) return rc;
         if (c->prm.updateProjOffset > 1) {
           rc = xtg_update_offset(c);
@@ -2057,19 +2205,9 @@ static int icd_iteration_parallel(xtg_ctx *c, int iter, xtg_stats *st) {
       }
     }
   }
-  if (ntimed) CK(cudaEventSynchronize(c->tev[2 * ntimed - 1]));
-  for (size_t i = 0; i < ntimed; i++) {
-    float ms = 0;
-    CK(cudaEventElapsedTime(&ms, c->tev[2 * i], c->tev[2 * i + 1]));
-    kms_total += ms;
-  }
-  double tmp;
-  int rc = read_stats(c, st, &tmp);
-  if (rc) return rc;
-  c->last_kms = kms_total;
+  c->runs = runs;
   c->last_items = items_total;
   c->last_icd = c->icd_launches - icd0;
-  st->vox_mag = vox_mag;
   return 0;
 }
 
@@ -2080,7 +2218,6 @@ static int icd_iteration_sequential(xtg_ctx *c, int iter, xtg_stats *st) {
   std::vector<int> usn, xs, ys;
   host_random_lists(c, usn, xs, ys);
   std::vector<int4> items;
-  double vox_mag = 0;
   float kms_total = 0;
   long long items_total = 0;
   auto run_list = [&](std::vector<int4> &L) -> int {
@@ -2105,13 +2242,7 @@ static int icd_iteration_sequential(xtg_ctx *c, int iter, xtg_stats *st) {
   std::vector<int> nsn((size_t)g.N_time * g.nzb);
   std::vector<int> xn((size_t)g.N_time * g.nzb * nxy), yn((size_t)g.N_time * g.nzb * nxy);
   for (int j = 0; j < K; j++) {
-    if (j == K - 1) {
-      double tmp;
-      int rc = read_stats(c, st, &tmp);
-      if (rc) return rc;
-      rc = reset_stats(c);
-      if (rc) return rc;
-    }
+    if (j == K - 1) c->phase = 1;  // the reference's vox_mag covers the last chunk only (XT_ICD_update.c:798)
     for (int half = 0; half < 2; half++) {
       items.clear();
       for (int i = 0; i < g.N_time; i++)
@@ -2130,12 +2261,7 @@ static int icd_iteration_sequential(xtg_ctx *c, int iter, xtg_stats *st) {
         if (rc) return rc;
       }
     }
-    if (j == K - 1) {
-      int rc = read_stats(c, st, &vox_mag);
-      if (rc) return rc;
-      rc = reset_stats(c);
-      if (rc) return rc;
-    }
+    if (j == K - 1) c->phase = 2;
     // NHICD selection with the reference's RandomizedSelect on the device-filtered map
     const int nseg = g.N_time * g.nzb;
     const unsigned grid = std::min<unsigned>(blocks_for(c->nmag, 256), (unsigned)c->sm_count * 8);
@@ -2181,13 +2307,9 @@ static int icd_iteration_sequential(xtg_ctx *c, int iter, xtg_stats *st) {
       }
     }
   }
-  double tmp;
-  int rc = read_stats(c, st, &tmp);
-  if (rc) return rc;
   c->last_kms = kms_total;
   c->last_items = items_total;
   c->last_icd = c->icd_launches - icd0;
-  st->vox_mag = vox_mag;
   return 0;
 }
 
@@ -2199,7 +2321,7 @@ int xtg_icd_iteration(xtg_ctx *c, int32_t iter, xtg_stats *st_out) {
   }
   xtg_stats st;
   memset(&st, 0, sizeof(st));
-  int rc = reset_stats(c);
+  int rc = clear_block(c);
   if (rc) return rc;
   // a slab starts every iteration from its neighbours' current boundary slices
   c->xphase = 0;
@@ -2212,16 +2334,25 @@ int xtg_icd_iteration(xtg_ctx *c, int32_t iter, xtg_stats *st_out) {
     if (rc) return rc;
   }
   // stop statistic (XT_ICD_update.c:884-925)
-  CK(cudaMemsetAsync(c->d_red + 4 * NSLOT, 0, NSLOT * 8, c->st));
   magsum_launch(c);
   CK(cudaGetLastError());
-  double h[NSLOT];
-  CK(cudaMemcpyAsync(h, c->d_red + 4 * NSLOT, sizeof(h), cudaMemcpyDeviceToHost, c->st));
+  CK(cudaMemcpyAsync(c->h_it, c->d_it, sizeof(IterBlock), cudaMemcpyDeviceToHost, c->st));
   CK(cudaEventRecord(c->ev1, c->st));
   CK(cudaEventSynchronize(c->ev1));
   CK(cudaEventElapsedTime(&st.ms, c->ev0, c->ev1));
+  if (c->order != XTG_ORDER_SEQUENTIAL) {
+    c->last_kms = 0.f;
+    for (const auto &r : c->runs) {
+      float ms = 0;
+      CK(cudaEventElapsedTime(&ms, c->tev[r.first], c->tev[r.second]));
+      c->last_kms += ms;
+    }
+  }
+  add_phase(c->h_it, 0, &st);
+  st.vox_mag = add_phase(c->h_it, 1, &st);
+  add_phase(c->h_it, 2, &st);
   double ms = 0;
-  for (int i = 0; i < NSLOT; i++) ms += h[i];
+  for (int i = 0; i < NSLOT; i++) ms += c->h_it->mag[i];
   st.mag_sum = ms;
   st.total_pix = (double)c->n_masked * c->g.N_time * c->g.nzb * (double)(c->g.N_z / c->g.nzb);
   st.avg_update_pct = (st.vox_mag > 0) ? 100.0 * ms / st.vox_mag : INFINITY;
@@ -2260,18 +2391,16 @@ int xtg_update_columns(xtg_ctx *c, int32_t iter, int32_t n, const int32_t *items
   }
   xtg_stats st;
   memset(&st, 0, sizeof(st));
-  int rc = reset_stats(c);
+  int rc = clear_block(c);
   if (rc) return rc;
   if (n) CK(cudaMemcpyAsync(c->d_items, items, (size_t)n * sizeof(int4), cudaMemcpyHostToDevice, c->st));
   CK(cudaEventRecord(c->ek0, c->st));
   rc = run_columns(c, iter, c->d_items, 0, n, nullptr, 0, 0, any_whole, any_block, -1);
   if (rc) return rc;
   CK(cudaEventRecord(c->ek1, c->st));
-  double ab = 0;
-  rc = read_stats(c, &st, &ab);
-  if (rc) return rc;
+  if ((rc = fetch_block(c))) return rc;
   CK(cudaEventElapsedTime(&st.ms, c->ek0, c->ek1));
-  st.vox_mag = ab;
+  st.vox_mag = add_phase(c->h_it, 0, &st);
   c->last_kms = st.ms;
   c->last_items = n;
   c->last_icd = c->icd_launches - icd0;
@@ -2295,9 +2424,17 @@ int xtg_nhicd_select(xtg_ctx *c, const int32_t *usn, int32_t *nnum, int32_t *xse
   CK(cudaMemcpyAsync(c->d_kth, kth.data(), nseg * 4, cudaMemcpyHostToDevice, c->st));
   const unsigned grid = std::min<unsigned>(blocks_for(c->nmag, 256), (unsigned)c->sm_count * 8);
   k_vsc_filter<<<grid, 256, 0, c->st>>>(nseg, g.N_y, g.N_x, c->d_mag, c->d_filt);
-  radix_select_multi(c, nseg);
-  c->launches += 1;
   CK(cudaGetLastError());
+  SelArgs S;
+  memset(&S, 0, sizeof(S));
+  S.map = c->d_mag;
+  S.ny = g.N_y;
+  S.nx = g.N_x;
+  S.kth_dev = c->d_kth;
+  S.thr = c->d_thr;
+  int nl = 0;
+  CK(nhicd_pick(S, nullptr, nseg, c->sm_count, c->d_filt, c->st, &nl));
+  c->launches += 1 + nl;
   std::vector<float> th(nseg), f(c->nmag);
   CK(cudaMemcpyAsync(th.data(), c->d_thr, nseg * 4, cudaMemcpyDeviceToHost, c->st));
   CK(cudaMemcpyAsync(f.data(), c->d_filt, c->nmag * 4, cudaMemcpyDeviceToHost, c->st));
@@ -2332,27 +2469,11 @@ int xtg_last_kernel_time(const xtg_ctx *c, float *ms, int64_t *items, int64_t *l
 }  // extern "C"
 
 // ------------------------------------------- allocation-free NHICD threshold --
-// Scratch of xtg_nhicd_threshold_noalloc: the filtered maps, then the per-map
-// ranks.  It lives for the life of the library on every device that loads it.
+// Scratch of xtg_nhicd_threshold_noalloc: the filtered maps.  It lives for the life of the library on every device that loads it.
 // Host code must not use the symbol itself as a device address (it is a host
 // stand-in); the device address comes from cudaGetSymbolAddress, once per
 // device.
-static __device__ __align__(256) float g_noalloc_scratch[XTG_NOALLOC_MAX_ELEMS + XTG_NOALLOC_MAX_MAPS];
-
-struct NoallocRanks {
-  int k[XTG_NOALLOC_MAX_MAPS];
-};
-
-// the ranks travel by value in the launch, so no host-to-device copy (and no
-// staging allocation) is needed
-__global__ void k_noalloc_put_ranks(NoallocRanks r, int n, int *dst) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = r.k[i];
-}
-
-__global__ void k_noalloc_select(size_t n, int plane, const float *filt, const float *thr, unsigned char *sel) {
-  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
-    sel[q] = filt[q] > thr[q / plane] ? 1 : 0;
-}
+static __device__ __align__(256) float g_noalloc_scratch[XTG_NOALLOC_MAX_ELEMS];
 
 static std::mutex g_noalloc_mu;
 static void *g_noalloc_addr[256];
@@ -2370,7 +2491,7 @@ extern "C" int xtg_nhicd_threshold_noalloc(const float *magmap, int32_t nmaps, i
             nmaps, ny, nx, n, XTG_NOALLOC_MAX_ELEMS, XTG_NOALLOC_MAX_MAPS);
     return XTG_E_ARG;
   }
-  NoallocRanks r;
+  SelRanks r;  // travel by value in the launch: no host-to-device copy, no staging allocation
   for (int s = 0; s < nmaps; s++) {
     if (kth[s] < 1 || (size_t)kth[s] > plane) {
       set_err("xtg_nhicd_threshold_noalloc: rank %d of map %d outside 1..%zu", kth[s], s, plane);
@@ -2402,18 +2523,15 @@ extern "C" int xtg_nhicd_threshold_noalloc(const float *magmap, int32_t nmaps, i
   }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   float *filt = reinterpret_cast<float *>(base);
-  int *ranks = reinterpret_cast<int *>(filt + XTG_NOALLOC_MAX_ELEMS);
   // every value read below is written first in this call: no clearing needed
-  k_noalloc_put_ranks<<<1, 256, 0, st>>>(r, nmaps, ranks);
-  CK(cudaGetLastError());
-  const unsigned grid = (unsigned)std::min<size_t>((n + 255) / 256, 4096);
-  k_vsc_filter<<<grid, 256, 0, st>>>(nmaps, ny, nx, magmap, filt);
-  CK(cudaGetLastError());
-  k_radix_select<<<nmaps, 1024, 0, st>>>(filt, (int)plane, ranks, thresholds);
-  CK(cudaGetLastError());
-  if (select) {
-    k_noalloc_select<<<grid, 256, 0, st>>>(n, (int)plane, filt, thresholds, select);
-    CK(cudaGetLastError());
-  }
+  SelArgs S;
+  memset(&S, 0, sizeof(S));
+  S.map = magmap;
+  S.ny = ny;
+  S.nx = nx;
+  S.thr = thresholds;
+  S.sel = select;
+  int nl = 0;
+  CK(nhicd_pick(S, &r, nmaps, 148, filt, st, &nl));
   return 0;
 }

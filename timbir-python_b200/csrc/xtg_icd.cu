@@ -28,6 +28,10 @@
 // (Source_Code_4D_Fast/XT_VoxUpdate.c:11-254), CE_FunctionalSubstitution
 // (XT_ICD_update.c:130-179); the z-line batching follows updateVoxels_AttTomo
 // (XT_VoxUpdate.c:266-586).
+#include <mutex>
+#include <utility>
+#include <vector>
+
 #include "xtg_internal.h"
 
 namespace xtg {
@@ -158,7 +162,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_icd_columns(DevGeo G, IcdArgs
   __shared__ unsigned sUpd[32], sZero[32];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nitems = A.n_items_dev ? *A.n_items_dev : A.n_items;
+  const int nitems = A.n_items_dev ? min(*A.n_items_dev, A.n_items) : A.n_items;
   const bool hlo = A.halo_lo != nullptr, hhi = A.halo_hi != nullptr;
   const int total = nitems * A.nsub;
   // The first lane of the last warp fetches the next item's record and table
@@ -764,7 +768,7 @@ static IcdKernel icd_kernel(int vec, int amode, int seq, int as, int nt) {
 // item covers) of an ICD launch whose items are split into z pieces, which
 // then add their partial sums into it.
 __global__ void k_magmap_zero(DevGeo G, IcdArgs A) {
-  const int nitems = A.n_items_dev ? *A.n_items_dev : A.n_items;
+  const int nitems = A.n_items_dev ? min(*A.n_items_dev, A.n_items) : A.n_items;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nitems; i += gridDim.x * blockDim.x) {
     const int q = A.use_perm ? (int)xt_perm((uint32_t)i, (uint32_t)nitems, A.perm_key) : i;
     const int4 item = A.items[A.item_lo + q];
@@ -799,12 +803,9 @@ cudaError_t launch_icd(const DevGeo &G, const IcdArgs &A, int vec, int amode, in
                        int grid, int nt, cudaStream_t st) {
   const size_t smem = icd_smem_bytes(vmax, zmax, G.zovl, as, amode, vec, nt);
   IcdKernel k = icd_kernel(vec, amode, seq, as, nt);
-  cudaError_t e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
   // e and w stream through L2 (e must, it is updated by other CTAs' atomics),
-  // so give the unified L1/shared space to shared memory: more CTAs per SM
-  e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributePreferredSharedMemoryCarveout,
-                           (int)cudaSharedmemCarveoutMaxShared);
+  // so the unified L1/shared space goes to shared memory: more CTAs per SM
+  cudaError_t e = full_smem((const void *)k);
   if (e != cudaSuccess) return e;
   k<<<grid, nt, smem, st>>>(G, A, vmax, zmax);
   return cudaGetLastError();
@@ -813,12 +814,48 @@ cudaError_t launch_icd(const DevGeo &G, const IcdArgs &A, int vec, int amode, in
 int icd_occupancy(int vec, int amode, int seq, int as, int vmax, int zmax, int zovl, int nt) {
   const size_t smem = icd_smem_bytes(vmax, zmax, zovl, as, amode, vec, nt);
   IcdKernel k = icd_kernel(vec, amode, seq, as, nt);
-  int nb = 0;
-  cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  cudaFuncSetAttribute((const void *)k, cudaFuncAttributePreferredSharedMemoryCarveout,
-                       (int)cudaSharedmemCarveoutMaxShared);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void *)k, nt, smem) != cudaSuccess) return 1;
-  return nb > 0 ? nb : 1;
+  // asked once per kernel, size and device (2 us of host time a launch)
+  struct Entry {
+    const void *fn;
+    size_t smem;
+    int dev, nb;
+  };
+  static std::mutex mu;
+  static std::vector<Entry> seen;
+  int dev = 0, nb = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+  std::lock_guard<std::mutex> lk(mu);
+  for (const Entry &q : seen)
+    if (q.fn == (const void *)k && q.smem == smem && q.dev == dev) return q.nb;
+  if (full_smem((const void *)k) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void *)k, nt, smem) != cudaSuccess)
+    return 1;
+  if (seen.size() >= 1024) seen.clear();
+  seen.push_back(Entry{(const void *)k, smem, dev, nb > 0 ? nb : 1});
+  return seen.back().nb;
+}
+
+// Once per kernel and device: as much dynamic shared memory as the device
+// gives a CTA, and the L1/shared split in favour of shared memory.
+cudaError_t full_smem(const void *fn) {
+  static std::mutex mu;
+  static std::vector<std::pair<const void *, int>> done;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lk(mu);
+  for (const auto &q : done)
+    if (q.first == fn && q.second == dev) return cudaSuccess;
+  int most = 0;
+  cudaFuncAttributes at;
+  if ((e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess ||
+      (e = cudaFuncGetAttributes(&at, fn)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)at.sharedSizeBytes)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared)) !=
+          cudaSuccess)
+    return e;
+  done.emplace_back(fn, dev);
+  return cudaSuccess;
 }
 
 }  // namespace xtg

@@ -13,7 +13,7 @@ struct IcdArgs {
   const int *view_idx, *view_start, *view_num;
   const int4 *items;
   const int *n_items_dev;  // device item count (NHICD lists), or null
-  int n_items;             // host item count when n_items_dev is null
+  int n_items;             // item count, or the most a device count may ask for
   int item_lo;             // first item index of this launch
   int *counter;
   int grab;                // items a CTA takes per atomic on the counter
@@ -94,6 +94,7 @@ cudaError_t launch_fbp(const DevGeo &G, const float *y, const float *d, float *q
 cudaError_t launch_magmap_zero(const DevGeo &G, const IcdArgs &A, int grid, cudaStream_t st);
 cudaError_t launch_icd(const DevGeo &G, const IcdArgs &A, int vec, int amode, int seq, int as, int vmax, int zmax,
                        int grid, int nt, cudaStream_t st);
+cudaError_t full_smem(const void *fn);
 int icd_threads(int vec, int amode, int seq, int zmax, int zovl, int vmax, int cols, int sms);
 int icd_occupancy(int vec, int amode, int seq, int as, int vmax, int zmax, int zovl, int nt);
 
