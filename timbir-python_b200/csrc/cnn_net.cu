@@ -76,7 +76,8 @@ struct xtc_net {
   cudaStream_t st = 0;
   // activations (BF16) and gradients (FP32) for the current batch shape
   int nb = 0, Y = 0, X = 0, Z = 0;
-  Buf in0, a[kLayers], u0, u1, u2, p0, p1, p2, g32, gtmp, gskip[3], gpre;
+  bool grads = false;  // the gradient buffers fit that shape too
+  Buf in0, a[kLayers], u0, u1, u2, p0, p1, p2, g32, gtmp, gcat[3], gpre;  // gcat: gradients of u0, u1, u2
   Buf start;  // the learned start's three images (xtg_warm.cu), kept between calls
 };
 
@@ -133,16 +134,16 @@ int check_err(xtc_net *n) {
   return 0;
 }
 
-// activation and gradient buffers for a batch shape
-int ensure_buffers(xtc_net *n, int nb, int Y, int X, int Z) {
-  if (n->nb == nb && n->Y == Y && n->X == X && n->Z == Z) return 0;
+// activation buffers for a batch shape, and gradient buffers for training
+int ensure_buffers(xtc_net *n, int nb, int Y, int X, int Z, bool training) {
+  if (n->nb == nb && n->Y == Y && n->X == X && n->Z == Z && (n->grads || !training)) return 0;
   const size_t v0 = (size_t)nb * Y * X * Z, v1 = v0 / 8, v2 = v1 / 8, v3 = v2 / 8;
   const size_t lv[kLayers] = {v0, v0, v1, v1, v2, v2, v3, v3, v2, v2, v1, v1, v0, v0};
   NCK(n->in0.ensure(v0 * 8 * sizeof(bf16)));
   size_t gmax = 0;
   for (int i = 0; i < kLayers; i++) {
     NCK(n->a[i].ensure(lv[i] * n->L[i].cout * sizeof(bf16)));
-    gmax = std::max(gmax, lv[i] * (size_t)n->L[i].cin);
+    if (i != 8 && i != 10 && i != 12) gmax = std::max(gmax, lv[i] * (size_t)n->L[i].cin);  // (those go to gcat)
     gmax = std::max(gmax, lv[i] * (size_t)n->L[i].cout);
   }
   NCK(n->p0.ensure(v1 * 32 * sizeof(bf16)));
@@ -151,16 +152,19 @@ int ensure_buffers(xtc_net *n, int nb, int Y, int X, int Z) {
   NCK(n->u2.ensure(v2 * 160 * sizeof(bf16)));
   NCK(n->u1.ensure(v1 * 112 * sizeof(bf16)));
   NCK(n->u0.ensure(v0 * 80 * sizeof(bf16)));
-  NCK(n->g32.ensure(gmax * sizeof(float)));
-  NCK(n->gtmp.ensure(gmax * sizeof(float)));
-  NCK(n->gpre.ensure(gmax * sizeof(bf16)));
-  NCK(n->gskip[0].ensure(v0 * 32 * sizeof(float)));
-  NCK(n->gskip[1].ensure(v1 * 48 * sizeof(float)));
-  NCK(n->gskip[2].ensure(v2 * 64 * sizeof(float)));
+  if (training) {
+    NCK(n->g32.ensure(gmax * sizeof(float)));
+    NCK(n->gtmp.ensure(gmax * sizeof(float)));
+    NCK(n->gpre.ensure(gmax * sizeof(bf16)));
+    NCK(n->gcat[0].ensure(v0 * 80 * sizeof(float)));
+    NCK(n->gcat[1].ensure(v1 * 112 * sizeof(float)));
+    NCK(n->gcat[2].ensure(v2 * 160 * sizeof(float)));
+  }
   n->nb = nb;
   n->Y = Y;
   n->X = X;
   n->Z = Z;
+  n->grads = training;
   return 0;
 }
 
@@ -220,20 +224,27 @@ int forward(xtc_net *n, const float *fbp, const float *icd, float *out, const fl
   xtc::up_concat(nb, Y, X, Z, 48, 32, A[11], A[1], n->u0.as<bf16>(), st);
   if ((rc = conv(n, 12, n->u0.as<bf16>(), 0, A[12]))) return rc;
   if ((rc = conv(n, 13, A[12], 0, A[13]))) return rc;
-  if (target) NCK(cudaMemsetAsync(n->d_loss, 0, sizeof(double), st));
-  xtc::head(v0, kHeadC, A[13], n->P + n->off_hw, n->P + n->off_hb, icd, kScale, out, target, n->d_loss,
-            n->g32.as<float>(), n->G + n->off_hw, n->G + n->off_hb, st);
+  if (target) {
+    NCK(cudaMemsetAsync(n->d_loss, 0, sizeof(double), st));
+    xtc::head_train(v0, A[13], n->P + n->off_hw, n->P + n->off_hb, icd, kScale, target, n->d_loss, n->g32.as<float>(),
+                    n->G + n->off_hw, n->G + n->off_hb, st);
+  } else {
+    xtc::head(v0, kHeadC, A[13], n->P + n->off_hw, n->P + n->off_hb, icd, kScale, out, st);
+  }
   NCK(cudaGetLastError());
   return 0;
 }
 
-// backward of conv li with post-ReLU gradient dpost (FP32) and post-activation
-// `post`; writes the input gradient (FP32) to din when din != nullptr
-int conv_back(xtc_net *n, int li, const float *dpost, const bf16 *post, const bf16 *in, int lvl, float *din) {
+// backward of conv li with post-ReLU gradient dpost (FP32, rows of ld floats,
+// the layer's channels from off on; plus the pooling's, `pooled`, where the
+// layer was pooled too) and post-activation `post`; writes the input gradient
+// (FP32) to din when din != nullptr
+int conv_back(xtc_net *n, int li, const float *dpost, const bf16 *post, const bf16 *in, int lvl, float *din, int ld = 0,
+              int off = 0, const float *pooled = nullptr) {
   const Layer &l = n->L[li];
-  const long long nv = (long long)n->nb * (n->Y >> lvl) * (n->X >> lvl) * (n->Z >> lvl);
   bf16 *dpre = n->gpre.as<bf16>();
-  xtc::relu_back(nv, l.cout, dpost, post, dpre, n->G + l.off_b, n->st);
+  xtc::relu_back(n->nb, n->Y >> lvl, n->X >> lvl, n->Z >> lvl, l.cout, dpost, ld ? ld : l.cout, off, pooled, post, dpre,
+                 n->G + l.off_b, n->st);
   xtc::ConvShape s{n->nb, n->Y >> lvl, n->X >> lvl, n->Z >> lvl, l.cin, l.cout, l.kpad};
   if (l.cin == l.cin_real) {
     NCK(xtc::conv_wgrad(s, in, dpre, n->G + l.off_w, n->d_err, n->st));
@@ -273,34 +284,27 @@ int backward(xtc_net *n) {
   bf16 *A[kLayers];
   for (int i = 0; i < kLayers; i++) A[i] = n->a[i].as<bf16>();
   float *g = n->g32.as<float>(), *t = n->gtmp.as<float>();
-  float *s0 = n->gskip[0].as<float>(), *s1 = n->gskip[1].as<float>(), *s2 = n->gskip[2].as<float>();
-  const size_t v0 = (size_t)nb * Y * X * Z, v1 = v0 / 8, v2 = v1 / 8;
-  NCK(cudaMemsetAsync(s0, 0, v0 * 32 * sizeof(float), st));
-  NCK(cudaMemsetAsync(s1, 0, v1 * 48 * sizeof(float), st));
-  NCK(cudaMemsetAsync(s2, 0, v2 * 64 * sizeof(float), st));
+  float *u0 = n->gcat[0].as<float>(), *u1 = n->gcat[1].as<float>(), *u2 = n->gcat[2].as<float>();
   int rc;
   // decoder, level 0: g = d A13 (from the head)
-  if ((rc = conv_back(n, 13, g, A[13], A[12], 0, t))) return rc;                  // t = d A12
-  if ((rc = conv_back(n, 12, t, A[12], n->u0.as<bf16>(), 0, g))) return rc;        // g = d u0
-  xtc::up_concat_back(nb, Y, X, Z, 48, 32, g, t, s0, st);                          // t = d A11, s0 +=
+  if ((rc = conv_back(n, 13, g, A[13], A[12], 0, t))) return rc;                   // t = d A12
+  if ((rc = conv_back(n, 12, t, A[12], n->u0.as<bf16>(), 0, u0))) return rc;       // u0 = d (up A11, A1)
+  xtc::up_back(nb, Y, X, Z, 48, 32, u0, t, st);                                    // t = d A11
   if ((rc = conv_back(n, 11, t, A[11], A[10], 1, g))) return rc;                   // g = d A10
-  if ((rc = conv_back(n, 10, g, A[10], n->u1.as<bf16>(), 1, t))) return rc;        // t = d u1
-  xtc::up_concat_back(nb, Y / 2, X / 2, Z / 2, 64, 48, t, g, s1, st);              // g = d A9, s1 +=
+  if ((rc = conv_back(n, 10, g, A[10], n->u1.as<bf16>(), 1, u1))) return rc;       // u1 = d (up A9, A3)
+  xtc::up_back(nb, Y / 2, X / 2, Z / 2, 64, 48, u1, g, st);                        // g = d A9
   if ((rc = conv_back(n, 9, g, A[9], A[8], 2, t))) return rc;                      // t = d A8
-  if ((rc = conv_back(n, 8, t, A[8], n->u2.as<bf16>(), 2, g))) return rc;          // g = d u2
-  xtc::up_concat_back(nb, Y / 4, X / 4, Z / 4, 96, 64, g, t, s2, st);              // t = d A7, s2 +=
+  if ((rc = conv_back(n, 8, t, A[8], n->u2.as<bf16>(), 2, u2))) return rc;         // u2 = d (up A7, A5)
+  xtc::up_back(nb, Y / 4, X / 4, Z / 4, 96, 64, u2, t, st);                        // t = d A7
   // bottom
   if ((rc = conv_back(n, 7, t, A[7], A[6], 3, g))) return rc;                      // g = d A6
   if ((rc = conv_back(n, 6, g, A[6], n->p2.as<bf16>(), 3, t))) return rc;          // t = d p2
-  xtc::avgpool_back(nb, Y / 4, X / 4, Z / 4, 64, t, s2, st);                       // s2 += (d A5 complete)
-  // encoder, level 2..0
-  if ((rc = conv_back(n, 5, s2, A[5], A[4], 2, g))) return rc;                     // g = d A4
+  // encoder, level 2..0: an encoder output's gradient is its skip's and its pooling's
+  if ((rc = conv_back(n, 5, u2, A[5], A[4], 2, g, 160, 96, t))) return rc;         // g = d A4
   if ((rc = conv_back(n, 4, g, A[4], n->p1.as<bf16>(), 2, t))) return rc;          // t = d p1
-  xtc::avgpool_back(nb, Y / 2, X / 2, Z / 2, 48, t, s1, st);                       // s1 += (d A3 complete)
-  if ((rc = conv_back(n, 3, s1, A[3], A[2], 1, g))) return rc;                     // g = d A2
+  if ((rc = conv_back(n, 3, u1, A[3], A[2], 1, g, 112, 64, t))) return rc;         // g = d A2
   if ((rc = conv_back(n, 2, g, A[2], n->p0.as<bf16>(), 1, t))) return rc;          // t = d p0
-  xtc::avgpool_back(nb, Y, X, Z, 32, t, s0, st);                                   // s0 += (d A1 complete)
-  if ((rc = conv_back(n, 1, s0, A[1], A[0], 0, g))) return rc;                     // g = d A0
+  if ((rc = conv_back(n, 1, u0, A[1], A[0], 0, g, 80, 48, t))) return rc;          // g = d A0
   if ((rc = conv_back(n, 0, g, A[0], n->in0.as<bf16>(), 0, nullptr))) return rc;
   NCK(cudaGetLastError());
   return 0;
@@ -470,7 +474,7 @@ int xtc_net_forward(xtc_net *n, const float *fbp, const float *icd, float *out, 
   if (!n || !fbp || !icd || !out) return XTG_E_ARG;
   int rc = check_dims(nb, Y, X, Z);
   if (rc) return rc;
-  if ((rc = ensure_buffers(n, nb, Y, X, Z))) return rc;
+  if ((rc = ensure_buffers(n, nb, Y, X, Z, false))) return rc;
   if (!n->packed && (rc = pack_all(n))) return rc;
   if ((rc = forward(n, fbp, icd, out, nullptr))) return rc;
   return check_err(n);
@@ -481,11 +485,10 @@ int xtc_net_backward(xtc_net *n, const float *fbp, const float *icd, const float
   if (!n || !fbp || !icd || !target) return XTG_E_ARG;
   int rc = check_dims(nb, Y, X, Z);
   if (rc) return rc;
-  if ((rc = ensure_buffers(n, nb, Y, X, Z))) return rc;
+  if ((rc = ensure_buffers(n, nb, Y, X, Z, true))) return rc;
   if (!n->packed && (rc = pack_all(n))) return rc;
   NCK(cudaMemsetAsync(n->G, 0, n->n_params * 4, n->st));
-  float *scratch = n->gtmp.as<float>();  // the head's output is not kept in training
-  if ((rc = forward(n, fbp, icd, scratch, target))) return rc;
+  if ((rc = forward(n, fbp, icd, nullptr, target))) return rc;
   if ((rc = backward(n))) return rc;
   if (loss) NCK(cudaMemcpyAsync(loss, n->d_loss, sizeof(double), cudaMemcpyDeviceToHost, n->st));
   return check_err(n);

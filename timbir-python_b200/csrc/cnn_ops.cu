@@ -4,6 +4,8 @@
 // and the Adam update.  Channels-last BF16 volumes [nb][Y][X][Z][C].
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "xtg_cnn_internal.h"
 
 namespace xtc {
@@ -79,23 +81,6 @@ __global__ void k_avgpool8(int nb, int Y, int X, int Z, int G, const int4 *in, i
   }
 }
 
-// gradient of the pooling, added into dIn (FP32 accumulation buffer)
-__global__ void k_avgpool_back(int nb, int Y, int X, int Z, int C, const float *dout, float *din) {
-  const long long n = (long long)nb * Y * X * Z * C;
-  GRID_STRIDE(i, n) {
-    long long r = i;
-    const int c = (int)(r % C);
-    r /= C;
-    const int z = (int)(r % Z);
-    r /= Z;
-    const int x = (int)(r % X);
-    r /= X;
-    const int y = (int)(r % Y);
-    const int b = (int)(r / Y);
-    din[i] += 0.125f * dout[((((size_t)b * (Y / 2) + y / 2) * (X / 2) + x / 2) * (Z / 2) + z / 2) * C + c];
-  }
-}
-
 // out[v] = [up2(a)[v] (Ca channels), skip[v] (Cb channels)] at the fine grid
 __global__ void k_up_concat(int nb, int Y, int X, int Z, int Ca, int Cb, const __nv_bfloat16 *a,
                             const __nv_bfloat16 *skip, __nv_bfloat16 *out) {
@@ -136,52 +121,80 @@ __global__ void k_up_concat8(int nb, int Y, int X, int Z, int ga, int gb, const 
   }
 }
 
-// gradient of k_up_concat: da (coarse, FP32, overwritten) and dskip (added into FP32)
-__global__ void k_up_concat_back(int nb, int Y, int X, int Z, int Ca, int Cb, const float *dout, float *da,
-                                 float *dskip) {
-  const int C = Ca + Cb;
-  const int Yo = Y / 2, Xo = X / 2, Zo = Z / 2;
-  const long long na = (long long)nb * Yo * Xo * Zo * Ca;
-  GRID_STRIDE(i, na) {
-    long long r = i;
-    const int c = (int)(r % Ca);
-    r /= Ca;
-    const int z = (int)(r % Zo);
-    r /= Zo;
-    const int x = (int)(r % Xo);
-    r /= Xo;
-    const int y = (int)(r % Yo);
-    const int b = (int)(r / Yo);
-    float s = 0.f;
+// gradient of k_up_concat with respect to a: da (coarse, FP32) sums the eight
+// fine voxels' first Ca channels of dout (four channels a thread; the skip's
+// channels are read in place by k_relu_back)
+__global__ void k_up_back(int nb, int Yo, int Xo, int Zo, int Ca4, int C4, const float4 *__restrict__ dout,
+                          float4 *__restrict__ da) {
+  const int X = 2 * Xo, Z = 2 * Zo;
+  const long long n = (long long)nb * Yo * Xo * Zo * Ca4;
+  GRID_STRIDE(i, n) {
+    const int c = (int)(i % Ca4);
+    const unsigned v = (unsigned)(i / Ca4);
+    const unsigned z = v % Zo, r1 = v / Zo, x = r1 % Xo, r2 = r1 / Xo;  // r2 = b * Yo + y
+    const float4 *p = dout + (((size_t)r2 * 2 * X + 2 * x) * Z + 2 * z) * C4 + c;
+    float4 q[8];
+#pragma unroll
+    for (int d = 0; d < 8; d++) q[d] = __ldg(p + ((size_t)((d >> 2) * X + ((d >> 1) & 1)) * Z + (d & 1)) * C4);
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
     for (int d = 0; d < 8; d++) {
-      const int yy = 2 * y + (d >> 2), xx = 2 * x + ((d >> 1) & 1), zz = 2 * z + (d & 1);
-      s += dout[((((size_t)b * Y + yy) * X + xx) * Z + zz) * C + c];
+      s.x += q[d].x;
+      s.y += q[d].y;
+      s.z += q[d].z;
+      s.w += q[d].w;
     }
     da[i] = s;
   }
-  const long long nskip = (long long)nb * Y * X * Z * Cb;
-  GRID_STRIDE(i, nskip) {
-    const long long v = i / Cb;
-    const int c = (int)(i - v * Cb);
-    dskip[i] += dout[v * C + Ca + c];
-  }
 }
 
-// dpre = dpost * (post > 0), FP32 in -> BF16 out; the bias gradient summed per channel
-__global__ void k_relu_back(long long nv, int C, const float *dpost, const __nv_bfloat16 *post, __nv_bfloat16 *dpre,
-                            float *dbias) {
+// dpre = dpost * (post > 0), FP32 in -> BF16 out, and the bias gradient summed
+// per channel.  dpost has rows of ld floats, the layer's C channels first
+// at off; with `pooled` the gradient of the 2x pooling that also read the layer
+// (coarse, rows of C floats) is added, an eighth of it per voxel.  Eight
+// channels a thread; the block and the grid stride are multiples of C / 8, so
+// a thread keeps its channels and their bias sums in registers.  Bound by
+// memory: level 0 of a 8 x 32 x 128 x 32 step (8 bytes an element) 190 -> 48 us,
+// and the pooling's and the skip's own passes over FP32 gradients (0.6 ms) go.
+__global__ void __launch_bounds__(192) k_relu_back(unsigned nv, int C8, const float *__restrict__ dpost, int ld, int off,
+                                                   const int4 *__restrict__ post, int4 *__restrict__ dpre, float *dbias,
+                                                   const float *__restrict__ pooled, int Y, int X, int Z) {
   extern __shared__ float sb[];
-  for (int c = threadIdx.x; c < C; c += blockDim.x) sb[c] = 0.f;
+  for (int c = threadIdx.x; c < 8 * C8; c += blockDim.x) sb[c] = 0.f;
   __syncthreads();
-  const long long n = nv * C;
-  GRID_STRIDE(i, n) {
-    const int c = (int)(i % C);
-    const float g = __bfloat162float(post[i]) > 0.f ? dpost[i] : 0.f;
-    dpre[i] = __float2bfloat16_rn(g);
-    if (g != 0.f) atomicAdd(&sb[c], g);
+  const int g = threadIdx.x % C8;
+  float bs[8];
+#pragma unroll
+  for (int c = 0; c < 8; c++) bs[c] = 0.f;
+  const unsigned vpb = blockDim.x / C8;  // voxels a block takes at once
+  for (unsigned v = blockIdx.x * vpb + threadIdx.x / C8; v < nv; v += gridDim.x * vpb) {
+    const float4 *p = reinterpret_cast<const float4 *>(dpost + (size_t)v * ld + off) + 2 * g;
+    const float4 a = __ldcs(p), b = __ldcs(p + 1);
+    float d[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    const int4 q = __ldg(post + (size_t)v * C8 + g);
+    if (pooled) {
+      const unsigned z = v % Z, r1 = v / Z, x = r1 % X, r2 = r1 / X;  // r2 = batch * Y + y, Y even
+      const size_t cv = ((size_t)(r2 >> 1) * (X >> 1) + (x >> 1)) * (Z >> 1) + (z >> 1);
+      const float4 *pp = reinterpret_cast<const float4 *>(pooled) + (cv * C8 + g) * 2;
+      const float4 e = __ldg(pp), f = __ldg(pp + 1);
+      const float pv[8] = {e.x, e.y, e.z, e.w, f.x, f.y, f.z, f.w};
+#pragma unroll
+      for (int c = 0; c < 8; c++) d[c] += 0.125f * pv[c];
+    }
+    const __nv_bfloat16 *h = reinterpret_cast<const __nv_bfloat16 *>(&q);
+    __align__(16) __nv_bfloat16 o[8];
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+      const float t = __bfloat162float(h[c]) > 0.f ? d[c] : 0.f;
+      o[c] = __float2bfloat16_rn(t);
+      bs[c] += t;
+    }
+    dpre[(size_t)v * C8 + g] = *reinterpret_cast<const int4 *>(o);
   }
+#pragma unroll
+  for (int c = 0; c < 8; c++) atomicAdd(&sb[8 * g + c], bs[c]);
   __syncthreads();
-  for (int c = threadIdx.x; c < C; c += blockDim.x) atomicAdd(&dbias[c], sb[c]);
+  for (int c = threadIdx.x; c < 8 * C8; c += blockDim.x) atomicAdd(&dbias[c], sb[c]);
 }
 
 // BF16 -> FP32 conversion (input gradients of the convolutions are produced in FP32 directly)
@@ -189,48 +202,100 @@ __global__ void k_to_f32(long long n, const __nv_bfloat16 *a, float *b) {
   GRID_STRIDE(i, n) b[i] = __bfloat162float(a[i]);
 }
 
-// 1x1 head: y[v] = base[v] + (sum_c h[v][c] w[c] + bias) / scale; optional loss
-// against target and its gradient w.r.t. h (BF16), w (FP32 atomics), bias.
-// loss = mean((y - target)^2 * scale^2), accumulated in FP64.
+// 1x1 head: y[v] = base[v] + (sum_c h[v][c] w[c] + bias) / scale
 __global__ void k_head(long long nv, int C, const __nv_bfloat16 *h, const float *w, const float *bias,
-                       const float *base, float scale, float *y, const float *target, double *loss, float *dh32,
-                       float *dw, float *db, float inv_n) {
-  extern __shared__ float sh[];  // [C] dw partials, [1] db partial
-  for (int c = threadIdx.x; c <= C; c += blockDim.x) sh[c] = 0.f;
-  __syncthreads();
-  double lsum = 0.0;
+                       const float *base, float scale, float *y) {
   GRID_STRIDE(v, nv) {
     float acc = bias[0];
-    if (C % 8 == 0) {
-      for (int c0 = 0; c0 < C; c0 += 8) {
-        const int4 q = __ldg(reinterpret_cast<const int4 *>(h + v * C + c0));
+    for (int c0 = 0; c0 < C; c0 += 8) {
+      const int4 q = __ldg(reinterpret_cast<const int4 *>(h + v * C + c0));
+      const __nv_bfloat16 *hq = reinterpret_cast<const __nv_bfloat16 *>(&q);
+#pragma unroll
+      for (int c = 0; c < 8; c++) acc += __bfloat162float(hq[c]) * w[c0 + c];
+    }
+    y[v] = base[v] + acc / scale;
+  }
+}
+
+// The head in training, 32 channels: loss = mean((y - target)^2 scale^2),
+// accumulated in FP64, and its gradients with respect to h (FP32), w and bias.
+// A warp takes 32 voxels: a lane each for the output (channels added in order,
+// as in k_head), then four lanes a voxel, eight channels each, for the
+// gradients, so that the stores are contiguous over the warp and a lane's
+// weight-gradient sums stay in registers until the end (a shared atomic per
+// voxel and channel before: 662 -> %HT% us for 8 x 32 x 128 x 32 voxels;
+// memory-bound).
+__global__ void __launch_bounds__(256) k_head_train(long long nv, const __nv_bfloat16 *__restrict__ h,
+                                                    const float *__restrict__ w, const float *__restrict__ bias,
+                                                    const float *__restrict__ base, float scale,
+                                                    const float *__restrict__ target, double *loss,
+                                                    float *__restrict__ dh, float *dw, float *db, float inv_n) {
+  __shared__ float sh[33];
+  if (threadIdx.x < 33) sh[threadIdx.x] = 0.f;
+  __syncthreads();
+  const int sub = threadIdx.x & 3, lane = threadIdx.x & 31;
+  float wv[8], dwv[8], dbv = 0.f;
+#pragma unroll
+  for (int c = 0; c < 8; c++) {
+    wv[c] = w[8 * sub + c];
+    dwv[c] = 0.f;
+  }
+  const float b0 = bias[0];
+  double lsum = 0.0;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long v0 = (long long)blockIdx.x * blockDim.x + threadIdx.x - lane; v0 < nv; v0 += stride) {
+    const long long v = v0 + lane;
+    float g = 0.f;  // d loss / d acc
+    if (v < nv) {
+      float acc = b0;
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int4 q = __ldg(reinterpret_cast<const int4 *>(h + v * 32) + u);
         const __nv_bfloat16 *hq = reinterpret_cast<const __nv_bfloat16 *>(&q);
 #pragma unroll
-        for (int c = 0; c < 8; c++) acc += __bfloat162float(hq[c]) * w[c0 + c];
+        for (int c = 0; c < 8; c++) acc += __bfloat162float(hq[c]) * w[8 * u + c];
       }
-    } else {
-      for (int c = 0; c < C; c++) acc += __bfloat162float(h[v * C + c]) * w[c];
-    }
-    const float out = base[v] + acc / scale;
-    if (y) y[v] = out;
-    if (target) {
+      const float out = base[v] + acc / scale;
       const float diff = (out - target[v]) * scale;
       lsum += (double)diff * diff;
-      const float g = 2.f * diff * inv_n;  // d loss / d acc
-      for (int c = 0; c < C; c++) {
-        dh32[v * C + c] = g * w[c];
-        atomicAdd(&sh[c], g * __bfloat162float(h[v * C + c]));
+      g = 2.f * diff * inv_n;
+      dbv += g;
+    }
+#pragma unroll
+    for (int it = 0; it < 4; it++) {
+      const long long vv = v0 + 8 * it + (lane >> 2);
+      const float gg = __shfl_sync(0xffffffffu, g, 8 * it + (lane >> 2));
+      if (vv < nv) {
+        const int4 q = __ldg(reinterpret_cast<const int4 *>(h + vv * 32) + sub);
+        const __nv_bfloat16 *hq = reinterpret_cast<const __nv_bfloat16 *>(&q);
+        float4 *d = reinterpret_cast<float4 *>(dh + vv * 32) + 2 * sub;
+        d[0] = make_float4(gg * wv[0], gg * wv[1], gg * wv[2], gg * wv[3]);
+        d[1] = make_float4(gg * wv[4], gg * wv[5], gg * wv[6], gg * wv[7]);
+#pragma unroll
+        for (int c = 0; c < 8; c++) dwv[c] += gg * __bfloat162float(hq[c]);
       }
-      atomicAdd(&sh[C], g);
     }
   }
-  if (target) {
-    for (int off = 16; off > 0; off >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, off);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, lsum * inv_n);
-    __syncthreads();
-    for (int c = threadIdx.x; c < C; c += blockDim.x) atomicAdd(&dw[c], sh[c]);
-    if (threadIdx.x == 0) atomicAdd(db, sh[C]);
+  __syncwarp();
+  for (int off = 4; off < 32; off <<= 1) {
+#pragma unroll
+    for (int c = 0; c < 8; c++) dwv[c] += __shfl_xor_sync(0xffffffffu, dwv[c], off);
   }
+  for (int off = 1; off < 32; off <<= 1) {
+    dbv += __shfl_xor_sync(0xffffffffu, dbv, off);
+    lsum += __shfl_xor_sync(0xffffffffu, lsum, off);
+  }
+  if (lane < 4) {
+#pragma unroll
+    for (int c = 0; c < 8; c++) atomicAdd(&sh[8 * sub + c], dwv[c]);
+    if (sub == 0) {
+      atomicAdd(&sh[32], dbv);
+      atomicAdd(loss, lsum * inv_n);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) atomicAdd(&dw[threadIdx.x], sh[threadIdx.x]);
+  if (threadIdx.x == 32) atomicAdd(db, sh[32]);
 }
 
 // master weights P[(tap*cin + ci)][cout] (FP32) -> W[cout][kpad] and Wt[ci][kpad_t] (BF16)
@@ -316,9 +381,6 @@ void avgpool(int nb, int Y, int X, int Z, int C, const __nv_bfloat16 *in, __nv_b
   else
     k_avgpool<<<blocks((long long)nb * Y * X * Z * C / 8), 256, 0, st>>>(nb, Y, X, Z, C, in, out);
 }
-void avgpool_back(int nb, int Y, int X, int Z, int C, const float *dout, float *din, cudaStream_t st) {
-  k_avgpool_back<<<blocks((long long)nb * Y * X * Z * C), 256, 0, st>>>(nb, Y, X, Z, C, dout, din);
-}
 void up_concat(int nb, int Y, int X, int Z, int Ca, int Cb, const __nv_bfloat16 *a, const __nv_bfloat16 *skip,
                __nv_bfloat16 *out, cudaStream_t st) {
   const long long n8 = (long long)nb * Y * X * Z * (Ca + Cb) / 8;
@@ -333,21 +395,30 @@ void up_concat(int nb, int Y, int X, int Z, int Ca, int Cb, const __nv_bfloat16 
   } else
     k_up_concat<<<blocks((long long)nb * Y * X * Z * (Ca + Cb)), 256, 0, st>>>(nb, Y, X, Z, Ca, Cb, a, skip, out);
 }
-void up_concat_back(int nb, int Y, int X, int Z, int Ca, int Cb, const float *dout, float *da, float *dskip,
-                    cudaStream_t st) {
-  k_up_concat_back<<<blocks((long long)nb * Y * X * Z * Cb), 256, 0, st>>>(nb, Y, X, Z, Ca, Cb, dout, da, dskip);
+void up_back(int nb, int Y, int X, int Z, int Ca, int Cb, const float *dout, float *da, cudaStream_t st) {
+  k_up_back<<<blocks((long long)nb * Y * X * Z / 8 * Ca / 4), 256, 0, st>>>(
+      nb, Y / 2, X / 2, Z / 2, Ca / 4, (Ca + Cb) / 4, reinterpret_cast<const float4 *>(dout), reinterpret_cast<float4 *>(da));
 }
-void relu_back(long long nv, int C, const float *dpost, const __nv_bfloat16 *post, __nv_bfloat16 *dpre, float *dbias,
-               cudaStream_t st) {
-  k_relu_back<<<blocks(nv * C), 256, C * sizeof(float), st>>>(nv, C, dpost, post, dpre, dbias);
+void relu_back(int nb, int Y, int X, int Z, int C, const float *dpost, int ld, int off, const float *pooled,
+               const __nv_bfloat16 *post, __nv_bfloat16 *dpre, float *dbias, cudaStream_t st) {
+  const unsigned nv = (unsigned)nb * Y * X * Z;
+  const int c8 = C / 8, vpb = 192 / c8;  // C / 8 is 4, 6, 8 or 12
+  const unsigned grid = (unsigned)std::min<long long>(((long long)nv + vpb - 1) / vpb, 148 * 10);
+  k_relu_back<<<grid, (unsigned)(vpb * c8), C * sizeof(float), st>>>(nv, c8, dpost, ld, off,
+                                                                     reinterpret_cast<const int4 *>(post),
+                                                                     reinterpret_cast<int4 *>(dpre), dbias, pooled, Y, X, Z);
 }
 void to_f32(long long n, const __nv_bfloat16 *a, float *b, cudaStream_t st) {
   k_to_f32<<<blocks(n), 256, 0, st>>>(n, a, b);
 }
 void head(long long nv, int C, const __nv_bfloat16 *h, const float *w, const float *bias, const float *base, float scale,
-          float *y, const float *target, double *loss, float *dh32, float *dw, float *db, cudaStream_t st) {
-  k_head<<<blocks(nv), 256, (C + 1) * sizeof(float), st>>>(nv, C, h, w, bias, base, scale, y, target, loss, dh32, dw,
-                                                            db, 1.f / (float)nv);
+          float *y, cudaStream_t st) {
+  k_head<<<blocks(nv), 256, 0, st>>>(nv, C, h, w, bias, base, scale, y);
+}
+void head_train(long long nv, const __nv_bfloat16 *h, const float *w, const float *bias, const float *base, float scale,
+                const float *target, double *loss, float *dh, float *dw, float *db, cudaStream_t st) {
+  const unsigned grid = (unsigned)std::min<long long>((nv + 255) / 256, 148 * 8);
+  k_head_train<<<grid, 256, 0, st>>>(nv, h, w, bias, base, scale, target, loss, dh, dw, db, 1.f / (float)nv);
 }
 void pack_weights(int cin_real, int cin, int cout, int kpad, int kpad_t, const float *P, __nv_bfloat16 *W,
                   __nv_bfloat16 *Wt, cudaStream_t st) {

@@ -51,16 +51,18 @@ cudaError_t conv_wgrad_tile(const ConvShape &s, const __nv_bfloat16 *in, const _
 
 void pack_input(long long nv, const float *a, const float *b, float scale, __nv_bfloat16 *out, cudaStream_t st);
 void avgpool(int nb, int Y, int X, int Z, int C, const __nv_bfloat16 *in, __nv_bfloat16 *out, cudaStream_t st);
-void avgpool_back(int nb, int Y, int X, int Z, int C, const float *dout, float *din, cudaStream_t st);
 void up_concat(int nb, int Y, int X, int Z, int Ca, int Cb, const __nv_bfloat16 *a, const __nv_bfloat16 *skip,
                __nv_bfloat16 *out, cudaStream_t st);
-void up_concat_back(int nb, int Y, int X, int Z, int Ca, int Cb, const float *dout, float *da, float *dskip,
-                    cudaStream_t st);
-void relu_back(long long nv, int C, const float *dpost, const __nv_bfloat16 *post, __nv_bfloat16 *dpre, float *dbias,
-               cudaStream_t st);
+// gradient of up_concat w.r.t. its coarse input; the skip's is dout's channels from Ca on
+void up_back(int nb, int Y, int X, int Z, int Ca, int Cb, const float *dout, float *da, cudaStream_t st);
+// dpost: rows of ld floats, the C channels from off on; pooled (or null): gradient of the 2x pooling of the same layer
+void relu_back(int nb, int Y, int X, int Z, int C, const float *dpost, int ld, int off, const float *pooled,
+               const __nv_bfloat16 *post, __nv_bfloat16 *dpre, float *dbias, cudaStream_t st);
 void to_f32(long long n, const __nv_bfloat16 *a, float *b, cudaStream_t st);
 void head(long long nv, int C, const __nv_bfloat16 *h, const float *w, const float *bias, const float *base, float scale,
-          float *y, const float *target, double *loss, float *dh32, float *dw, float *db, cudaStream_t st);
+          float *y, cudaStream_t st);
+void head_train(long long nv, const __nv_bfloat16 *h, const float *w, const float *bias, const float *base, float scale,
+                const float *target, double *loss, float *dh, float *dw, float *db, cudaStream_t st);
 void pack_weights(int cin_real, int cin, int cout, int kpad, int kpad_t, const float *P, __nv_bfloat16 *W,
                   __nv_bfloat16 *Wt, cudaStream_t st);
 void fold_wgrad(int cin_real, int cin, int cout, const float *g, float *out, cudaStream_t st);
