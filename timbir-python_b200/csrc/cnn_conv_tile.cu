@@ -1,16 +1,16 @@
-// cnn_conv_tile.cu -- 3x3x3 convolutions of the warm-start network on tiles
-// staged once by TMA (BF16 in, FP32 accumulation in TMEM).
+// cnn_conv_tile.cu -- 3x3x3 convolutions of the warm-start network on staged
+// tiles (BF16 in, FP32 accumulation in TMEM).
 //
 // The gather kernel in cnn_conv.cu builds every A row (voxel x 64 K values)
 // with per-thread loads: each input voxel is fetched 27 times.  Here a CTA
-// owns an output tile of 128 x-voxels x TZ z-lines of one y-row; one TMA box
-// per 16-channel chunk stages the tile's input halo (130 x (TZ + 2) x 3
-// voxels, zero filled outside the volume) in shared memory once, one 32-byte
-// row per voxel (16 channels, the 32-byte swizzle), x fastest:
-// row r = (y' * TZS + z') * TXS + x'.  In that layout the A operand of tap
-// (dy, dx, dz) for output line z is the run of 128 rows starting at
-// r0(z) + (dy * TZS + dz) * TXS + dx -- one shared-memory descriptor with a
-// shifted start address.  No im2col gather is ever materialised.
+// owns an output tile of 128 x-voxels x TZ z-lines of one y-row, and a stage
+// holds, for one 16-channel chunk, one of the three y-rows of the tile's input
+// halo (130 x (TZ + 2) voxels, zero filled outside the volume) in shared
+// memory, one 32-byte row per voxel (16 channels, the 32-byte swizzle), x
+// fastest: row r = z' * TXS + x'.  In that layout the A operand of tap (dx, dz)
+// for output line z is the run of 128 rows starting at (z + 1 + dz) * TXS + 1 +
+// dx -- one shared-memory descriptor with a shifted start address.  No im2col
+// gather is ever materialised.
 //
 // One MMA serves up to three output lines: staged z-line L feeds output lines
 // L - 1, L and L + 1 through the taps dz = +1, 0, -1, so with the weights of
@@ -22,16 +22,16 @@
 //
 // Weights come pre-packed per 16-channel chunk as
 // Wp[chunk][dy, dx][half][dz = +1, 0, -1][n][8] (offsets as the kernel applies
-// them, i.e. mirrored for sign -1) and are copied with one bulk copy per stage.  One thread issues the TMA, the bulk copies and all
-// MMAs; stages are double-buffered so the copies for chunk c + 1 overlap the
-// MMAs of chunk c, across tile boundaries too (persistent CTAs), and the
-// accumulators are double-buffered in TMEM so the epilogue of one tile
-// overlaps the next.  Every wait is bounded and reports through *err.
+// them, i.e. mirrored for sign -1) and are copied with one bulk copy per stage.
+// Up to six stages run ahead of the MMAs, across tile boundaries too
+// (persistent CTAs), and the accumulators are double-buffered in TMEM so the
+// epilogue of one tile overlaps the next.  Every wait is bounded and reports
+// through *err.
 //
 // Shapes: X a multiple of 128, Z even, cin a multiple of 8, cout a multiple of
-// 16 up to 64.  Tiles are 4 z-lines high for cout <= 32 (shared memory
-// 2 x (75,776 + 864 cout) bytes), else 2 (2 x (50,176 + 864 cout)).  Other
-// shapes use the gather kernel.
+// 16 up to 64.  Tiles are 4 z-lines high for cout <= 32 (stages of 25,600 +
+// 288 cout bytes), else 2 (17,408 + 288 cout).  Other shapes use the box or the
+// gather kernel.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
@@ -54,9 +54,8 @@ constexpr int TN_MAX = 64;
 template <int TZ>
 struct TileDims {
   static constexpr int TZS = TZ + 2;                   // staged z-lines
-  static constexpr int ROWS = 3 * TZS * TXS;           // staged voxels, one 32-byte row (16 channels) each
-  static constexpr uint32_t BOX = ROWS * 32;           // bytes one TMA box writes
-  static constexpr uint32_t A_STAGE = (BOX + 1023) / 1024 * 1024;  // stages stay aligned to the swizzle atom
+  static constexpr int ROWS = TZS * TXS;               // staged voxels of a y-row, one 32-byte row (16 channels) each
+  static constexpr uint32_t A_STAGE = (ROWS * 32 + 1023) / 1024 * 1024;  // stages stay aligned to the swizzle atom
 };
 
 // K-major operand with 32-byte rows in the 32-byte swizzle (16-byte chunk
@@ -69,25 +68,37 @@ __device__ __forceinline__ uint64_t sdesc_sw32(uint32_t saddr) {
          ((uint64_t)6 << 61);
 }
 
-__host__ __device__ constexpr uint32_t b_stage_bytes(int n) { return 27u * (uint32_t)n * 32u; }
+// a stage's weights: nine taps of 16 channels
+__host__ __device__ constexpr uint32_t b_stage_bytes(int n) { return 9u * (uint32_t)n * 32u; }
+
+constexpr int TILE_LOADERS = 128;  // threads of warps 5-8
+constexpr int TILE_STAGES = 6;     // at most; as many as shared memory holds
+constexpr int TILE_AHEAD = 2;      // stages a loader has in flight before it waits for the oldest
 
 // Persistent: each CTA walks the tiles blockIdx.x, blockIdx.x + gridDim.x, ...
-// Warp 4 (one thread) issues the copies and MMAs of the CTA's whole chunk
-// sequence through two shared-memory stages; the accumulators alternate
-// between two TMEM buffers, so warps 0-3 (TMEM lanes 32w .. 32w + 31) drain
-// tile i while tile i + 1 is computed.
+// A stage is one (16-channel chunk, dy): the staged y-row y + dy and its nine
+// taps' weights.  Warps 5-8 copy it in with 16-byte asynchronous copies (a row
+// is two of them; zero filled outside the volume), several stages ahead, and
+// publish it to the tensor core's proxy once it has landed; warp 4 (one
+// thread) issues the MMAs; the accumulators alternate between two TMEM
+// buffers, so warps 0-3 (TMEM lanes 32w .. 32w + 31) drain tile i while tile
+// i + 1 is computed.
+//
+// What bounds it: the copies and the MMAs about equally (with either left out
+// 1.25 and 1.17 ms of 1.27 at 512^2 x 64 voxels, 32 -> 32 channels).  As one TMA
+// box a chunk (2340 rows of 32 bytes for TZ 4) the copies took 3.4 cycles a
+// row and set the time, 1.86 ms; 80 -> 32 4.21 -> 2.85 ms, 48 -> 48 at half the
+// resolution 496 -> 414 us.
 template <int EPI, int TZ>
-__global__ void __launch_bounds__(160, 1)
-    k_conv_tile(const __grid_constant__ CUtensorMap tin, ConvShape s, const __nv_bfloat16 *__restrict__ wp,
-                const float *__restrict__ bias, void *out, int *err) {
+__global__ void __launch_bounds__(288, 1)
+    k_conv_tile(const __nv_bfloat16 *__restrict__ in, ConvShape s, const __nv_bfloat16 *__restrict__ wp,
+                const float *__restrict__ bias, void *out, int nstage, int *err) {
   using D = TileDims<TZ>;
   constexpr int TZS = D::TZS;
-  constexpr uint32_t TA_STAGE = D::A_STAGE;
   extern __shared__ __align__(1024) uint8_t sm[];
   const int N = s.n;
-  const uint32_t B_STAGE = b_stage_bytes(N);
-  uint8_t *sA = sm, *sB = sm + 2 * TA_STAGE;
-  __shared__ uint64_t full[2], empty[2], acc_full[2], acc_empty[2], done;
+  const uint32_t BB = b_stage_bytes(N), STAGE = D::A_STAGE + (BB + 1023u) / 1024u * 1024u;
+  __shared__ uint64_t full[TILE_STAGES], empty[TILE_STAGES], acc_full[2], acc_empty[2], done;
   __shared__ uint32_t tbase;
   __shared__ volatile int bad;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -98,9 +109,11 @@ __global__ void __launch_bounds__(160, 1)
   const uint32_t acc_cols = tmem_cols(2 * TZ * N);
   const long long lim = 1ll << 24;
   if (tid == 0) {
-    for (int i = 0; i < 2; i++) {
-      mbar_init(&full[i], 1);
+    for (int i = 0; i < nstage; i++) {
+      mbar_init(&full[i], TILE_LOADERS + 1);  // each loader, and the weights' transaction
       mbar_init(&empty[i], 1);
+    }
+    for (int i = 0; i < 2; i++) {
       mbar_init(&acc_full[i], 1);
       mbar_init(&acc_empty[i], 4);
     }
@@ -129,73 +142,145 @@ __global__ void __launch_bounds__(160, 1)
     y = t % s.Y;
     b = t / s.Y;
   };
-  if (warp == 4) {
+  const int nq = 3 * nchunk;  // stages of a tile
+  if (warp >= 5) {
+    const int lt = tid - 160;
+    bool ok = true;
+    int q = 0, st = 0, landed = 0;  // stages issued and published
+    uint32_t ph = 1;                // parity of the stage's last release (none yet: passes)
+    // This thread's copies, the same in every stage: (x, z, half) of the staged
+    // y-row, the halves and z of one x next to each other in memory.  Source
+    // and destination offsets are worked out once (done per stage they were
+    // the kernel's bound), and which copies lie on the tile's edges.
+    constexpr int NE = (TXS * TZS * 2 + TILE_LOADERS - 1) / TILE_LOADERS;
+    int off[NE];
+    uint32_t dst[NE], have = 0, on_x0 = 0, on_x1 = 0, on_z0 = 0, on_z1 = 0, on_h1 = 0;
+#pragma unroll
+    for (int e = 0; e < NE; e++) {
+      const int i = lt + e * TILE_LOADERS;
+      const int xx = i / (TZS * 2), rem = i - xx * (TZS * 2), zz = rem >> 1, h = rem & 1, r = zz * TXS + xx;
+      off[e] = (xx * s.Z + zz) * s.cin + 8 * h;
+      dst[e] = (uint32_t)r * 32u + (uint32_t)((h ^ ((r >> 2) & 1)) << 4);
+      if (xx < TXS) have |= 1u << e;
+      if (xx == 0) on_x0 |= 1u << e;
+      if (xx == TXS - 1) on_x1 |= 1u << e;
+      if (zz == 0) on_z0 |= 1u << e;
+      if (zz == TZS - 1) on_z1 |= 1u << e;
+      if (h) on_h1 |= 1u << e;
+    }
+    // stages up to `upto` have landed for this thread: make them visible to the
+    // async proxy and arrive
+    auto publish = [&](int upto) {
+      fence_async_smem();
+      for (; landed < upto; landed++) mbar_arrive(&full[landed % nstage]);
+    };
+    for (int tl = 0; tl < mine && ok; tl++) {
+      int x0, z0, y, b;
+      tile_of(tl, x0, z0, y, b);
+      // the copies inside the volume in x and z
+      uint32_t inside = have;
+      if (x0 == 0) inside &= ~on_x0;
+      if (x0 + TX == s.X) inside &= ~on_x1;
+      if (z0 == 0) inside &= ~on_z0;
+      if (z0 + TZ == s.Z) inside &= ~on_z1;
+      const __nv_bfloat16 *row = in + (((long long)b * s.Y + y - 1) * s.X + x0 - 1) * s.Z * s.cin + (z0 - 1) * s.cin;
+      const long long ystep = (long long)s.X * s.Z * s.cin;
+      int c = 0, dyi = 0;
+      for (int k = 0; k < nq; k++) {
+        if (!mbar_wait(&empty[st], ph, lim) || bad) {
+          ok = false;
+          break;
+        }
+        uint8_t *a = sm + (size_t)st * STAGE;
+        if (lt == 0) {
+          mbar_expect_tx(&full[st], BB);
+          bulk_load(a + D::A_STAGE, wp + (size_t)k * (BB / 2), BB, &full[st]);
+        }
+        const int y2 = y + dyi - 1;
+        uint32_t m = y2 >= 0 && y2 < s.Y ? inside : 0u;
+        if (16 * c + 8 >= s.cin) m &= ~on_h1;  // a half chunk
+        const __nv_bfloat16 *src = row + dyi * ystep + 16 * c;
+        const uint32_t sa = smem_u32(a);
+#pragma unroll
+        for (int e = 0; e < NE; e++) {
+          const bool v = (m >> e) & 1u;
+          const __nv_bfloat16 *g = v ? src + off[e] : in;
+          if (e + 1 < NE || ((have >> e) & 1u))
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sa + dst[e]), "l"(g), "r"(v ? 16 : 0)
+                         : "memory");
+        }
+        if (++dyi == 3) {
+          dyi = 0;
+          c++;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        q++;
+        if (++st == nstage) {
+          st = 0;
+          ph ^= 1u;
+        }
+        if (q > TILE_AHEAD) {
+          asm volatile("cp.async.wait_group %0;" ::"n"(TILE_AHEAD) : "memory");
+          publish(q - TILE_AHEAD);
+        }
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    publish(q);
+    if (!ok && lane == 0) {
+      atomicExch(err, 1);
+      bad = 1;
+    }
+    // the weights issued last land before the shared memory is released
+    for (int i = q > nstage ? q - nstage : 0; i < q; i++) mbar_wait(&full[i % nstage], (uint32_t)(i / nstage) & 1u, lim);
+  } else if (warp == 4) {
     if (lane == 0 && mine > 0) {
       const uint32_t idesc[3] = {idesc_bf16(N, 0, 0), idesc_bf16(2 * N, 0, 0), idesc_bf16(3 * N, 0, 0)};
-      const int Q = mine * nchunk;
-      int issued[2] = {0, 0}, landed[2] = {0, 0};
-      auto load = [&](int q) {
-        const int st = q & 1, c = q % nchunk;
-        int x0, z0, y, b;
-        tile_of(q / nchunk, x0, z0, y, b);
-        uint8_t *a = sA + st * TA_STAGE;
-        mbar_expect_tx(&full[st], D::BOX + B_STAGE);
-        // channels 16c .. 16c + 15 (past cin: zero fill)
-        tma_load_5d(a, &tin, 16 * c, x0 - 1, z0 - 1, y - 1, b, &full[st]);
-        bulk_load(sB + st * B_STAGE, wp + (size_t)c * (B_STAGE / 2), B_STAGE, &full[st]);
-        issued[st]++;
-      };
       bool ok = true;
-      load(0);
-      if (Q > 1) load(1);
-      for (int q = 0; q < Q && ok; q++) {
-        const int st = q & 1, c = q % nchunk, tl = q / nchunk, ab = tl & 1;
-        if (c == 0 && !mbar_wait(&acc_empty[ab], (uint32_t)(((tl >> 1) & 1) ^ 1), lim)) {
+      int st = 0;
+      uint32_t ph = 0;
+      for (int tl = 0; tl < mine && ok; tl++) {
+        const int ab = tl & 1;
+        if (!mbar_wait(&acc_empty[ab], (uint32_t)(((tl >> 1) & 1) ^ 1), lim)) {
           ok = false;
           break;
         }
-        if (!mbar_wait(&full[st], (uint32_t)(q >> 1) & 1u, lim)) {
-          ok = false;
-          break;
-        }
-        landed[st]++;
-        tc_fence_after();
-        // descriptors advance in 16-byte units: an A row by 2; a (dy, dx)
-        // B block (2 halves x 3 dz x N rows x 16 bytes) by 6N, one dz block by N
         const uint32_t acc = tmem + (uint32_t)(ab * TZ * N);
-        const uint64_t da0 = sdesc_sw32(smem_u32(sA + st * TA_STAGE) + (uint32_t)((TZS + 1) * TXS + 1) * 32);
-        uint64_t db = sdesc(smem_u32(sB + st * B_STAGE), (uint32_t)N * 48, 128);
-#pragma unroll
-        for (int g = 0; g < 9; g++) {
-          const int dy = g / 3 - 1, dx = g % 3 - 1;
-#pragma unroll
-          for (int zl = 0; zl < TZS; zl++) {
-            // staged line zl (z = z0 - 1 + zl) feeds output lines zl - 2 .. zl
-            // (relative to z0) through dz = +1, 0, -1; keep those inside the tile
-            const int zf = zl - 2 < 0 ? 0 : zl - 2, zt = zl > TZ - 1 ? TZ - 1 : zl;
-            const int cnt = zt - zf + 1, blk = zf - (zl - 2);
-            mma_bf16(acc + (uint32_t)(zf * N), da0 + (uint64_t)(int64_t)(2 * ((dy * TZS + zl - 1) * TXS + dx)),
-                     db + (uint64_t)(blk * N), idesc[cnt - 1], 1u);
-          }
-          db += (uint64_t)(6 * N);
-        }
-        mma_commit(&empty[st]);
-        if (c == nchunk - 1) mma_commit(&acc_full[ab]);
-        if (q >= 1 && q + 1 < Q) {
-          // chunk q + 1 reuses the stage of chunk q - 1 once its MMAs are done
-          if (!mbar_wait(&empty[(q - 1) & 1], (uint32_t)((q - 1) >> 1) & 1u, lim)) {
+        for (int k = 0; k < nq; k++) {
+          if (!mbar_wait(&full[st], ph, lim) || bad) {
             ok = false;
             break;
           }
-          load(q + 1);
+          tc_fence_after();
+          // descriptors advance in 16-byte units: an A row by 2; a (dy, dx)
+          // B block (2 halves x 3 dz x N rows x 16 bytes) by 6N, one dz block by N
+          const uint32_t a0 = smem_u32(sm + (size_t)st * STAGE);
+          const uint64_t da0 = sdesc_sw32(a0);
+          uint64_t db = sdesc(a0 + D::A_STAGE, (uint32_t)N * 48, 128);
+#pragma unroll
+          for (int dxi = 0; dxi < 3; dxi++) {
+#pragma unroll
+            for (int zl = 0; zl < TZS; zl++) {
+              // staged line zl (z = z0 - 1 + zl) feeds output lines zl - 2 .. zl
+              // (relative to z0) through dz = +1, 0, -1; keep those inside the tile
+              const int zf = zl - 2 < 0 ? 0 : zl - 2, zt = zl > TZ - 1 ? TZ - 1 : zl;
+              const int cnt = zt - zf + 1, blk = zf - (zl - 2);
+              mma_bf16(acc + (uint32_t)(zf * N), da0 + (uint64_t)(2 * (zl * TXS + dxi)), db + (uint64_t)(blk * N),
+                       idesc[cnt - 1], 1u);
+            }
+            db += (uint64_t)(6 * N);
+          }
+          mma_commit(&empty[st]);
+          if (++st == nstage) {
+            st = 0;
+            ph ^= 1u;
+          }
         }
+        if (ok) mma_commit(&acc_full[ab]);
       }
-      if (!ok || bad) {
+      if (!ok) {
         atomicExch(err, 1);
         bad = 1;
-        // let the copies already issued land before the shared memory is released
-        for (int st = 0; st < 2; st++)
-          for (; landed[st] < issued[st]; landed[st]++) mbar_wait(&full[st], (uint32_t)landed[st] & 1u, lim);
       }
       mma_commit(&done);
       mbar_wait(&done, 0, lim);  // every MMA issued above has completed
@@ -205,7 +290,8 @@ __global__ void __launch_bounds__(160, 1)
     // epilogue: warp w drains accumulator rows (x) 32w .. 32w + 31
     for (int tl = 0; tl < mine; tl++) {
       const int ab = tl & 1;
-      if (!mbar_wait(&acc_full[ab], (uint32_t)(tl >> 1) & 1u, lim) || bad) {
+      const bool gone = !mbar_wait(&acc_full[ab], (uint32_t)(tl >> 1) & 1u, lim) || bad;
+      if (__any_sync(0xffffffffu, gone)) {
         if (lane == 0) atomicExch(err, 1);
         bad = 1;
         break;
@@ -531,31 +617,21 @@ cudaError_t conv_tile_pack(int cin, int n, int kpad, int sign, const __nv_bfloat
 
 cudaError_t conv_forward_tile(const ConvShape &s, const __nv_bfloat16 *in, const __nv_bfloat16 *wp, const float *bias,
                               void *out, int epi, int sign, int *err, cudaStream_t st) {
-  if (!conv_tile_supported(s) || (epi == 0 && !bias) || epi < 0 || epi > 2 || (sign != 1 && sign != -1))
+  if (!conv_tile_supported(s) || (epi == 0 && !bias) || epi < 0 || epi > 2 || (sign != 1 && sign != -1) ||
+      (reinterpret_cast<uintptr_t>(in) & 15))
     return cudaErrorNotSupported;
-  // activations [nb][Y][X][Z][cin] seen as (c, x, z, y, b): the box lands x-fastest
-  CUtensorMap m;
-  const cuuint64_t C2 = (cuuint64_t)s.cin * 2;
-  const cuuint64_t dims[5] = {(cuuint64_t)s.cin, (cuuint64_t)s.X, (cuuint64_t)s.Z, (cuuint64_t)s.Y,
-                              (cuuint64_t)s.nb};
-  const cuuint64_t strides[4] = {(cuuint64_t)s.Z * C2, C2, (cuuint64_t)s.X * s.Z * C2,
-                                 (cuuint64_t)s.Y * s.X * s.Z * C2};
   const int tz = tile_tz(s);
-  const cuuint32_t box[5] = {16, TXS, (cuuint32_t)tz + 2, 3, 1};
-  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-  if (tensor_map_encode()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<__nv_bfloat16 *>(in), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return cudaErrorNotSupported;
-  typedef void (*K)(const CUtensorMap, ConvShape, const __nv_bfloat16 *, const float *, void *, int *);
+  typedef void (*K)(const __nv_bfloat16 *, ConvShape, const __nv_bfloat16 *, const float *, void *, int, int *);
   K k;
   // the sign lives in the packed weights
   if (tz == 4)
     k = epi == 0 ? k_conv_tile<0, 4> : epi == 1 ? k_conv_tile<1, 4> : k_conv_tile<2, 4>;
   else
     k = epi == 0 ? k_conv_tile<0, 2> : epi == 1 ? k_conv_tile<1, 2> : k_conv_tile<2, 2>;
-  const size_t smem =
-      2 * ((size_t)(tz == 4 ? TileDims<4>::A_STAGE : TileDims<2>::A_STAGE) + b_stage_bytes(s.n));
+  const size_t stage =
+      (size_t)(tz == 4 ? TileDims<4>::A_STAGE : TileDims<2>::A_STAGE) + (b_stage_bytes(s.n) + 1023) / 1024 * 1024;
+  const int nstage = (int)std::min<size_t>(TILE_STAGES, (size_t)220 * 1024 / stage);
+  const size_t smem = nstage * stage;
   cudaError_t e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   static int sms = 0;
@@ -566,7 +642,7 @@ cudaError_t conv_forward_tile(const ConvShape &s, const __nv_bfloat16 *in, const
   }
   const long long ntiles = (long long)(s.X / TX) * (s.Z / tz) * s.nb * s.Y;
   const unsigned grid = (unsigned)std::min<long long>(ntiles, sms);  // one CTA per SM (shared memory)
-  k<<<grid, 160, smem, st>>>(m, s, wp, bias, out, err);
+  k<<<grid, 288, smem, st>>>(in, s, wp, bias, out, nstage, err);
   return cudaGetLastError();
 }
 
