@@ -92,6 +92,7 @@ struct xtg_ctx {
   float *d_hr = nullptr, *d_cos = nullptr, *d_sin = nullptr, *d_ax = nullptr, *d_filt = nullptr, *d_tmp = nullptr;
   float *d_num = nullptr, *d_den = nullptr, *d_thr = nullptr, *d_var = nullptr;
   int *d_view_idx = nullptr, *d_view_start = nullptr, *d_view_num = nullptr, *d_fov = nullptr;
+  int *d_vord = nullptr;  // views by frame, then angle
   int *d_mcols = nullptr, *d_rank = nullptr;
   IterBlock *d_it = nullptr, *h_it = nullptr;  // device, pinned host copy
   int phase = 0;  // whose statistics the ICD launches add to
@@ -110,9 +111,10 @@ struct xtg_ctx {
   // tried yet, 1 = built, -1 = not used (does not fit, or the gather projector
   // was requested)
   long long *d_cptr = nullptr;
-  int2 *d_cent = nullptr;
+  int4 *d_cent = nullptr;
   int csr_state = 0, projector = XTG_PROJ_AUTO;
-  long long csr_nnz = 0;
+  long long csr_nnz = 0;   // A entries of the table
+  size_t csr_bytes = 0;
   long long table_nnz = 0;
   int table_max = 0;
   // options
@@ -846,32 +848,37 @@ static cudaError_t ensure_csr(xtg_ctx *c) {
   if (c->projector == XTG_PROJ_GATHER) return cudaSuccess;
   // entries hold a z-line's element offset within its frame as an int32
   if ((size_t)c->g.N_y * c->g.N_x * c->g.N_z >= ((size_t)1 << 31)) return cudaSuccess;
-  const size_t rows = (size_t)c->g.N_p * c->g.N_r;
-  int *d_cnt = nullptr;
-  if (cudaMalloc(&d_cnt, rows * 4) != cudaSuccess) {
+  const size_t rows = (size_t)c->g.N_p * ((c->g.N_r + 1) / 2);
+  int *d_cnt = nullptr;  // records per row, then (8-byte aligned) the entry count
+  const size_t ent_at = (rows + 1) / 2 * 2;
+  if (cudaMalloc(&d_cnt, ent_at * 4 + 8) != cudaSuccess) {
     cudaGetLastError();
     return cudaSuccess;
   }
   CsrBuildArgs B;
   memset(&B, 0, sizeof(B));
   B.hr = c->d_hr; B.cosv = c->d_cos; B.sinv = c->d_sin; B.win_margin = fp_win_margin(c); B.count = d_cnt;
-  cudaError_t e = launch_csr_build(c->G, B, 0, c->span, c->st);
+  B.entries = reinterpret_cast<unsigned long long *>(d_cnt + ent_at);
+  cudaError_t e = cudaMemsetAsync(B.entries, 0, 8, c->st);
+  if (e == cudaSuccess) e = launch_csr_build(c->G, B, 0, c->span, c->st);
   std::vector<int> cnt(rows);
+  unsigned long long entries = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(cnt.data(), d_cnt, rows * 4, cudaMemcpyDeviceToHost, c->st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&entries, B.entries, 8, cudaMemcpyDeviceToHost, c->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
   cudaFree(d_cnt);
   c->launches++;
   if (e != cudaSuccess) return e;
   std::vector<long long> ptr(rows + 1, 0);
   for (size_t i = 0; i < rows; i++) ptr[i + 1] = ptr[i] + cnt[i];
-  const long long nnz = ptr[rows];
+  const long long nrec = ptr[rows];
   size_t fr = 0, tot = 0;
   if ((e = cudaMemGetInfo(&fr, &tot)) != cudaSuccess) return e;
   // the column table, if one is still to be built, has at most as many entries
-  const size_t pending = (c->a_mode != XTG_A_FP32 && c->table_mode == 0) ? (size_t)nnz * 8 : 0;
-  const size_t need = (size_t)nnz * 8 + (rows + 1) * 8;
+  const size_t pending = (c->a_mode != XTG_A_FP32 && c->table_mode == 0) ? (size_t)entries * 8 : 0;
+  const size_t need = (size_t)nrec * 16 + (rows + 1) * 8;
   if (need + pending + ((size_t)2 << 30) > fr) return cudaSuccess;
-  if (cudaMalloc(&c->d_cptr, (rows + 1) * 8) != cudaSuccess || cudaMalloc(&c->d_cent, (size_t)nnz * 8 + 8) != cudaSuccess) {
+  if (cudaMalloc(&c->d_cptr, (rows + 1) * 8) != cudaSuccess || cudaMalloc(&c->d_cent, (size_t)nrec * 16 + 16) != cudaSuccess) {
     cudaGetLastError();
     cudaFree(c->d_cptr);
     cudaFree(c->d_cent);
@@ -879,7 +886,8 @@ static cudaError_t ensure_csr(xtg_ctx *c) {
     c->d_cent = nullptr;
     return cudaSuccess;
   }
-  c->dev_bytes += need + 8;
+  c->csr_bytes = need + 16;
+  c->dev_bytes += c->csr_bytes;
   if ((e = cudaMemcpyAsync(c->d_cptr, ptr.data(), (rows + 1) * 8, cudaMemcpyHostToDevice, c->st)) != cudaSuccess)
     return e;
   B.count = nullptr;
@@ -888,7 +896,7 @@ static cudaError_t ensure_csr(xtg_ctx *c) {
   if ((e = launch_csr_build(c->G, B, 1, c->span, c->st)) != cudaSuccess) return e;
   if ((e = cudaStreamSynchronize(c->st)) != cudaSuccess) return e;
   c->launches++;
-  c->csr_nnz = nnz;
+  c->csr_nnz = (long long)entries;
   c->csr_state = 1;
   return cudaSuccess;
 }
@@ -901,11 +909,13 @@ static cudaError_t launch_fp(xtg_ctx *c, float *out, double *slots) {
   F.x = c->d_x; F.y = c->d_y; F.d = c->d_d; F.w = c->d_w; F.hr = c->d_hr; F.cosv = c->d_cos; F.sinv = c->d_sin;
   F.fov = c->d_fov; F.out = out; F.cost_slots = slots; F.T = c->g.T; F.delta = c->g.delta;
   F.win_margin = fp_win_margin(c);
+  F.neg0 = -0.0f;
   c->launches++;
   if (c->csr_state == 1) {
     CsrView T;
     T.ptr = c->d_cptr;
     T.ent = c->d_cent;
+    T.order = c->d_vord;
     return xtg::launch_fp_csr(c->G, F, T, MODE, c->st);
   }
   return xtg::launch_fp(c->G, F, MODE, c->span, c->st);
@@ -921,7 +931,7 @@ void xtg_destroy(xtg_ctx *c) {
   if (c->coarse) xtg_destroy(c->coarse);
   void *ptrs[] = {c->d_y, c->d_w, c->d_e, c->d_d, c->d_x, c->d_mag, c->d_hr, c->d_cos, c->d_sin, c->d_ax,
                   c->d_filt, c->d_tmp, c->d_num, c->d_den, c->d_thr, c->d_var, c->d_view_idx, c->d_view_start,
-                  c->d_view_num, c->d_fov, c->d_mcols, c->d_rank, c->d_it, c->d_kth,
+                  c->d_view_num, c->d_fov, c->d_vord, c->d_mcols, c->d_rank, c->d_it, c->d_kth,
                   c->d_items, c->d_nh, c->d_red, c->d_cnt, c->d_tstart, c->d_toff, c->d_tval32,
                   c->d_tscale, c->d_tval16, c->d_cptr, c->d_cent};
   if (c->dl_pending && c->ev_dl) cudaEventSynchronize(c->ev_dl);
@@ -1028,6 +1038,7 @@ int xtg_create(const xt_params *prm, const double *times, const double *angles, 
   rc |= dalloc(c, &c->d_view_start, (size_t)g.N_time);
   rc |= dalloc(c, &c->d_view_num, (size_t)g.N_time);
   rc |= dalloc(c, &c->d_fov, (size_t)g.N_p);
+  rc |= dalloc(c, &c->d_vord, (size_t)g.N_p);
   rc |= dalloc(c, &c->d_mcols, (size_t)c->n_masked);
   rc |= dalloc(c, &c->d_rank, c->nxy);
   rc |= dalloc(c, &c->d_it, 1);
@@ -1053,6 +1064,13 @@ int xtg_create(const xt_params *prm, const double *times, const double *angles, 
   CK(cudaMemcpy(c->d_view_start, c->v.view_start, (size_t)g.N_time * 4, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(c->d_view_num, c->v.view_num, (size_t)g.N_time * 4, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(c->d_fov, c->v.frame_of_view, (size_t)g.N_p * 4, cudaMemcpyHostToDevice));
+  std::vector<int> ord((size_t)g.N_p);
+  std::iota(ord.begin(), ord.end(), 0);
+  std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) {
+    if (c->v.frame_of_view[a] != c->v.frame_of_view[b]) return c->v.frame_of_view[a] < c->v.frame_of_view[b];
+    return fmod((double)c->v.angle[a], 2 * M_PI) < fmod((double)c->v.angle[b], 2 * M_PI);
+  });
+  CK(cudaMemcpy(c->d_vord, ord.data(), (size_t)g.N_p * 4, cudaMemcpyHostToDevice));
   if (c->n_masked) CK(cudaMemcpy(c->d_mcols, c->mcols.data(), (size_t)c->n_masked * 4, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(c->d_rank, c->col_rank.data(), c->nxy * 4, cudaMemcpyHostToDevice));
   CK(cudaMemset(c->d_x, 0, c->nvox * 4));
@@ -1809,7 +1827,7 @@ int xtg_set_projector(xtg_ctx *c, int32_t kind) {
   if (kind != c->projector) {
     cudaFree(c->d_cptr);
     cudaFree(c->d_cent);
-    if (c->csr_state == 1) c->dev_bytes -= (size_t)c->csr_nnz * 8 + ((size_t)c->g.N_p * c->g.N_r + 2) * 8;
+    if (c->csr_state == 1) c->dev_bytes -= c->csr_bytes;
     c->d_cptr = nullptr;
     c->d_cent = nullptr;
     c->csr_state = 0;

@@ -55,19 +55,22 @@ struct FpArgs {
   float T;
   float delta;
   double win_margin;
+  float neg0;          // -0
 };
 
-// bin-major A table: row (view p, bin r) = entries [ptr[p N_r + r], ptr[p N_r + r + 1])
+// bin-major A table: row (view p, bins 2 i and 2 i + 1) = records [ptr[p np2 + i], ptr[p np2 + i + 1]), np2 = ceil(N_r / 2)
 struct CsrBuildArgs {
   const float *hr, *cosv, *sinv;
   double win_margin;
-  int *count;           // build pass 0: entries per row
-  const long long *ptr; // build pass 1: row starts
-  int2 *ent;            // {(j * N_x + k) * N_z, bits of its A (without delta_t)} per entry
+  int *count;                   // build pass 0: records per row
+  unsigned long long *entries;  // ... and A entries in all
+  const long long *ptr;         // build pass 1: row starts
+  int4 *ent;                    // {(j * N_x + k) * N_z, bits of its A at either bin (without delta_t), 0} per record
 };
 struct CsrView {
   const long long *ptr;
-  const int2 *ent;
+  const int4 *ent;
+  const int *order;  // views by frame, then angle
 };
 
 struct TableArgs {

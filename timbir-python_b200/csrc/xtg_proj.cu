@@ -204,15 +204,18 @@ cudaError_t launch_fp(const DevGeo &G, const FpArgs &F, int mode, int ns, cudaSt
 }
 
 // ------------------------------------------------ bin-major A table ------
-// The A entries regrouped by sinogram row (view p, detector bin r): row
-// (p, r) lists (column j N_x + k, A) for every column of p's frame that
-// reaches bin r, in increasing (j, k) -- the order in which the reference
-// adds a column's contribution to that entry (initErrorSinogam,
-// XT_ICD_update.c:551-569).  Built once per context by the enumeration of
-// k_fp_bins, so every value is the exact A of calcAMatrixColumnforAngle
-// (XT_AMatrix.c:50-110).  Lane b of a warp owns bin rb + b of the warp's 32
-// bins: for each hit column the lanes test their own bin in parallel, so the
-// appends of a bin stay in column order without atomics.
+// The A entries regrouped by sinogram row pair (view p, detector bins 2 i and
+// 2 i + 1): a row lists {column j N_x + k, its A at each of the two bins} for
+// every column of p's frame that reaches either, in increasing (j, k) -- the
+// order in which the reference adds a column's contribution to those entries
+// (initErrorSinogam, XT_ICD_update.c:551-569).  A column reaches 2.14 bins on
+// average at voxels one bin wide, so 1.57 records stand for 2.14 entries, and
+// the z-line a record names is loaded once for both bins.  Built once per
+// context by the enumeration of k_fp_bins, so every value is the exact A of
+// calcAMatrixColumnforAngle (XT_AMatrix.c:50-110).  Lane b of a warp owns bin
+// rb + b of the warp's 32 bins: for each hit column the lanes test their own
+// bin in parallel, so the appends of a pair (its even lane's) stay in column
+// order without atomics.
 template <int FILL, int NS>
 __global__ void __launch_bounds__(FP_WARPS * 32) k_csr_build(DevGeo G, CsrBuildArgs B) {
   extern __shared__ __align__(16) unsigned char cb_sm[];
@@ -225,11 +228,12 @@ __global__ void __launch_bounds__(FP_WARPS * 32) k_csr_build(DevGeo G, CsrBuildA
   const float *H = B.hr + (size_t)p * XT_HR_STRIDE;
   const double lo = (double)G.R0 + (double)rb * G.delta_r - G.delta_xy - B.win_margin;
   const double hi = (double)G.R0 + (double)(rb + 32) * G.delta_r + G.delta_xy + B.win_margin;
-  const int r = rb + lane;
-  const bool own = r < G.N_r;
+  const int r = rb + lane, np2 = (G.N_r + 1) / 2;
+  const bool own = r < G.N_r, head = own && !(lane & 1);
+  const size_t row = (size_t)p * np2 + r / 2;
   long long cur = 0;
-  int cnt = 0;
-  if (FILL && own) cur = B.ptr[(size_t)p * G.N_r + r];
+  int cnt = 0, ent = 0;
+  if (FILL && head) cur = B.ptr[row];
   for (int j = 0; j < G.N_y; j++) {
     int klo, khi;
     if (!fp_col_range(G, cp, sp, xt_coord(G.y0, j, G.delta_xy), lo, hi, &klo, &khi)) continue;
@@ -254,22 +258,25 @@ __global__ void __launch_bounds__(FP_WARPS * 32) k_csr_build(DevGeo G, CsrBuildA
         const int q = __shfl_sync(0xffffffffu, pk, l);
         const int sl = (q >> 8) & 0xFF, sh = q & 0xFF;
         const int sidx = lane - ((q >> 16) - 64);  // this lane's bin within the column's run
-        if (own && sidx >= sl && sidx < sh) {
-          const float a = vsm[l * NS + sidx];
-          if (a != 0.f) {
-            if (FILL) {
-              B.ent[cur] = make_int2((j * G.N_x + kb + l) * G.N_z, __float_as_int(a));
-              cur++;
-            } else {
-              cnt++;
-            }
-          }
+        float a = 0.f;
+        if (own && sidx >= sl && sidx < sh) a = vsm[l * NS + sidx];
+        const float a1 = __shfl_down_sync(0xffffffffu, a, 1);
+        ent += a != 0.f;
+        if (head && (a != 0.f || a1 != 0.f)) {
+          if (FILL)
+            B.ent[cur++] = make_int4((j * G.N_x + kb + l) * G.N_z, __float_as_int(a), __float_as_int(a1), 0);
+          else
+            cnt++;
         }
       }
       __syncwarp();  // the staged entries are rewritten by the next round
     }
   }
-  if (!FILL && own) B.count[(size_t)p * G.N_r + r] = cnt;
+  if (!FILL) {
+    if (head) B.count[row] = cnt;
+    for (int off = 16; off > 0; off >>= 1) ent += __shfl_xor_sync(0xffffffffu, ent, off);
+    if (lane == 0) atomicAdd(B.entries, (unsigned long long)ent);
+  }
 }
 
 template <int FILL>
@@ -290,137 +297,182 @@ cudaError_t launch_csr_build(const DevGeo &G, const CsrBuildArgs &B, int fill, i
   return fill ? launch_csr_build_t<1>(G, B, ns, st) : launch_csr_build_t<0>(G, B, ns, st);
 }
 
-// Forward projection from the bin-major table: one warp per sinogram row
-// (view, bin) and 64 detector rows.  Every lane reads each entry
-// {z-line offset, A} (a broadcast from L1; two entries per 16-byte load) and
-// its rows of that z-line (PAIR: rows 2 lane, 2 lane + 1 as one 8-byte load
-// when a slice covers one detector row; the warp's loads form one 256-byte
-// run), and accumulates in registers, entries in table order: in FP32
-// (__fadd_rn(__fmul_rn)) that is the reference's summation order, so MODE
-// 0 / 1 are bit-identical to k_fp_bins and to initErrorSinogam; MODE 2 / 3
-// accumulate in FP64 in the same order (a product of two FP32 values is
-// exact in FP64, so the sums equal k_fp_bins' bit for bit).  Eight entries
-// are loaded before any is added.  The eight warps of a CTA take eight
-// consecutive bins of one view, which share most of their columns, so many
-// z-lines are L1 hits.  FULL: every 64-row chunk is complete (N_t a multiple
-// of 64), so no lane needs a bounds test.
-#define CSR_WARPS 8
-template <int MODE, typename ACC, bool PAIR, bool FULL>
-__global__ void __launch_bounds__(CSR_WARPS * 32) k_fp_csr(DevGeo G, FpArgs F, CsrView T) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int p = blockIdx.x;
-  const int r = blockIdx.y * CSR_WARPS + warp;
-  if (r >= G.N_r) return;  // whole warp; no block-wide barrier follows
-  const int t0 = blockIdx.z * 64, nt = FULL ? 64 : min(64, G.N_t - t0);
-  // rows of this lane: PAIR (zovl == 1, N_t even): 2 lane, 2 lane + 1, one
-  // float2 at slice t0 + 2 lane; otherwise lane and lane + 32
-  const int ta = PAIR ? 2 * lane : lane, tb = PAIR ? 2 * lane + 1 : lane + 32;
-  const bool va = FULL || ta < nt, vb = FULL || tb < nt;
+// Forward projection from the bin-major table.  LT lanes, four detector rows
+// each, take one (view, bin pair) and 4 LT rows, and accumulate both bins in
+// registers, records in table order: in FP32 (__fadd_rn(__fmul_rn)) that is
+// the reference's summation order, so MODE 0 / 1 are bit-identical to
+// k_fp_bins and to initErrorSinogam; MODE 2 / 3 accumulate in FP64 in the same
+// order (a product of two FP32 values is exact in FP64, so the sums equal
+// k_fp_bins' bit for bit).  A bin that a record's column does not reach (A = 0)
+// is passed over, so no value of that column touches it.  VEC: a z-line's four
+// rows are one 16-byte load (one detector row per slice, N_z a multiple of 4).
+//
+// What bounds it: L1, which returns 64-128 bytes of z-line a cycle, and in
+// FP64 the conversions to it (16 lanes a cycle; A is converted by integer
+// operations instead, being positive and normal).  Per bin, a warp over the 64
+// rows loaded 2.14 z-lines a (column, view), here 1.57; a CTA takes the same
+// bins of CSR_VIEWS views that follow each other in angle (T.order), whose
+// rays cross the same columns at the same time, so most z-lines are L1 hits
+// (eight bins of one view before).  Latency: with records read as they are
+// needed the pairs alone were no faster (9.3 ms).  512^2 x 64, 1024 views: e = y -
+// A x - d 9.6 -> 6.3 ms, FP64 cost 12.8 -> 8.0 ms; 256^2 x 32, 512 views 1.46 ->
+// 0.53 ms.
+// (s0, s1) += (x0, x1) a, product and sum each rounded, two rows per
+// instruction.  The product is a multiply-add of -0, which leaves it as it is
+// (neg0 is an argument so that nothing knows its value): a packed multiply
+// followed by a packed add comes out of the assembler as one multiply-add with
+// one rounding, whatever rounding the two ask for.
+__device__ __forceinline__ void mul_add2(float &s0, float &s1, float x0, float x1, float a, float neg0) {
+  asm("{\n\t.reg .b64 x, a, s, z;\n\t"
+      "mov.b64 x, {%2, %3};\n\tmov.b64 a, {%4, %4};\n\tmov.b64 s, {%0, %1};\n\tmov.b64 z, {%5, %5};\n\t"
+      "fma.rn.f32x2 x, x, a, z;\n\tadd.rn.f32x2 s, s, x;\n\tmov.b64 {%0, %1}, s;\n\t}"
+      : "+f"(s0), "+f"(s1)
+      : "f"(x0), "f"(x1), "f"(a), "f"(neg0));
+}
+
+#define CSR_WARPS 8  // consecutive views of a CTA, one per warp
+// resident CTAs the FP32 registers are cut for (3 and 5: 6.8 and 6.7 ms)
+#define CSR_CTAS 4
+template <int MODE, typename ACC, int LT, bool VEC>
+__global__ void __launch_bounds__(CSR_WARPS * 32, MODE < 2 ? CSR_CTAS : 3) k_fp_csr(DevGeo G, FpArgs F, CsrView T) {
+  constexpr int PW = 32 / LT;  // pairs per warp
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % LT;
+  const int ov = blockIdx.x * CSR_WARPS + warp, np2 = (G.N_r + 1) / 2, pair = blockIdx.y * PW + lane / LT;
+  if (ov >= G.N_p) return;  // whole warp; no block-wide barrier follows
+  const int p = T.order[ov];
+  const int t0 = blockIdx.z * (4 * LT) + 4 * sub;  // this lane's first row
+  const int nt = min(4, G.N_t - t0);               // rows it has (may be none)
   const float *xf = F.x + (size_t)F.fov[p] * G.N_y * G.N_x * G.N_z;
-  const float *xla = xf + (t0 + ta) / G.zovl, *xlb = xf + (t0 + tb) / G.zovl;
-  const long long e0 = T.ptr[(size_t)p * G.N_r + r], e1 = T.ptr[(size_t)p * G.N_r + r + 1];
-  ACC acc_a = (ACC)0, acc_b = (ACC)0;
-  auto add = [&](float xa, float xb, float a) {
-    if (MODE <= 1) {
-      acc_a = __fadd_rn(acc_a, __fmul_rn(xa, a));
-      acc_b = __fadd_rn(acc_b, __fmul_rn(xb, a));
+  const float *xl = xf + (VEC ? (nt > 0 ? t0 : 0) : 0);
+  int zr[4];
+#pragma unroll
+  for (int c = 0; c < 4; c++) zr[c] = c < nt ? (t0 + c) / G.zovl : 0;
+  long long i = 0, e1 = 0;
+  if (pair < np2) {  // (lanes without rows load records too)
+    i = T.ptr[(size_t)p * np2 + pair];
+    e1 = T.ptr[(size_t)p * np2 + pair + 1];
+  }
+  ACC acc0[4], acc1[4];
+#pragma unroll
+  for (int c = 0; c < 4; c++) acc0[c] = acc1[c] = (ACC)0;
+  auto load = [&](int off) {
+    if (VEC) return __ldg(reinterpret_cast<const float4 *>(xl + off));
+    return make_float4(__ldg(xl + off + zr[0]), __ldg(xl + off + zr[1]), __ldg(xl + off + zr[2]), __ldg(xl + off + zr[3]));
+  };
+  auto add1 = [&](ACC (&acc)[4], const ACC (&x)[4], float a) {
+    if constexpr (MODE <= 1) {
+      mul_add2(acc[0], acc[1], x[0], x[1], a, F.neg0);
+      mul_add2(acc[2], acc[3], x[2], x[3], a, F.neg0);
     } else {
-      acc_a += (ACC)xa * (ACC)a;
-      acc_b += (ACC)xb * (ACC)a;
+      const uint32_t u = __float_as_uint(a);  // FP64 form of a positive normal: a shift and a bias
+      const double ad = __hiloint2double((int)((u >> 3) + 0x38000000u), (int)(u << 29));
+#pragma unroll
+      for (int c = 0; c < 4; c++) acc[c] += x[c] * ad;
     }
   };
-  auto load = [&](int off, float &xa, float &xb) {
-    if (PAIR) {
-      const float2 v = va ? __ldg(reinterpret_cast<const float2 *>(xla + off)) : make_float2(0.f, 0.f);
-      xa = v.x;
-      xb = v.y;
-    } else {
-      xa = va ? __ldg(xla + off) : 0.f;
-      xb = vb ? __ldg(xlb + off) : 0.f;
+  auto add = [&](const float4 v, float a0, float a1) {
+    const ACC x[4] = {(ACC)v.x, (ACC)v.y, (ACC)v.z, (ACC)v.w};
+    if (a0 != 0.f) add1(acc0, x, a0);
+    if (a1 != 0.f) add1(acc1, x, a1);
+  };
+  // Sixteen records of each pair at a time: its lanes load them in one coalesced
+  // run while the sixteen before are added, and read them back from shared
+  // memory; z-lines are loaded four records ahead.  (Records past the row's
+  // end: A = 0 at column 0.)
+  constexpr int RC = 16, RL = RC / LT;  // records a lane loads
+  __shared__ __align__(16) int4 recs[CSR_WARPS][2][PW][RC + 1];
+  const int len = (int)(e1 - i), most = __reduce_max_sync(0xffffffffu, len);
+  int4 nx[RL];
+  auto fetch = [&](int r0) {
+#pragma unroll
+    for (int m = 0; m < RL; m++) {
+      const int r = r0 + sub + m * LT;
+      nx[m] = r < len ? __ldcs(T.ent + i + r) : make_int4(0, 0, 0, 0);
     }
   };
-  long long i = e0;
-  if (i < e1 && (i & 1)) {  // to a 16-byte boundary of the entry array
-    const int2 en = __ldg(T.ent + i);
-    float xa, xb;
-    load(en.x, xa, xb);
-    add(xa, xb, __int_as_float(en.y));
-    i++;
-  }
-  for (; i + 8 <= e1; i += 8) {
-    const int4 *q = reinterpret_cast<const int4 *>(T.ent + i);
-    int4 qv[4];
+  fetch(0);
+  for (int r0 = 0, buf = 0; r0 < most; r0 += RC, buf ^= 1) {
+    int4 *R = recs[warp][buf][lane / LT];
 #pragma unroll
-    for (int u = 0; u < 4; u++) qv[u] = __ldg(q + u);
-    float xa[8], xb[8];
+    for (int m = 0; m < RL; m++) R[sub + m * LT] = nx[m];
+    __syncwarp();  // (the other buffer was read before the last one's barrier)
+    fetch(r0 + RC);
+    float4 v[4];
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      load(qv[u].x, xa[2 * u], xb[2 * u]);
-      load(qv[u].z, xa[2 * u + 1], xb[2 * u + 1]);
+    for (int u = 0; u < 4; u++) v[u] = load(R[u].x);
+#pragma unroll
+    for (int g = 0; g < RC; g += 4) {
+      float4 vn[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (g + 4 < RC) vn[u] = load(R[g + 4 + u].x);
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        add(v[u], __int_as_float(R[g + u].y), __int_as_float(R[g + u].z));
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) v[u] = vn[u];
     }
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      add(xa[2 * u], xb[2 * u], __int_as_float(qv[u].y));
-      add(xa[2 * u + 1], xb[2 * u + 1], __int_as_float(qv[u].w));
-    }
-  }
-  for (; i < e1; i++) {
-    const int2 en = __ldg(T.ent + i);
-    float xa, xb;
-    load(en.x, xa, xb);
-    add(xa, xb, __int_as_float(en.y));
   }
   double cacc = 0.0;
+  if (pair < np2) {
 #pragma unroll
-  for (int h = 0; h < 2; h++) {
-    const int t = h ? tb : ta;
-    if (!FULL && t >= nt) continue;
-    const ACC sacc = h ? acc_b : acc_a;
-    const size_t o = ((size_t)p * G.N_r + r) * G.N_t + t0 + t;
-    const size_t od = (size_t)r * G.N_t + t0 + t;
-    if (MODE == 0) {
-      F.out[o] = (float)sacc;
-    } else if (MODE == 1) {
-      F.out[o] = __fsub_rn(__fsub_rn(F.y[o], (float)sacc), F.d[od]);
-    } else {
-      // A * delta_t: the system matrix of the voxel update (XT_VoxUpdate.c:27, 67)
-      const double e64 = (double)F.y[o] - (double)G.delta_t * (double)sacc - (double)F.d[od];
-      if (MODE == 2) F.out[o] = (float)e64;
-      const double sw = e64 * sqrt((double)F.w[o]);
-      if (fabs(sw) < (double)F.T)
-        cacc += sw * sw;
-      else
-        cacc += 2.0 * (double)F.delta * (double)F.T * fabs(sw) + (double)F.T * (double)F.T * (1.0 - 2.0 * (double)F.delta);
+    for (int h = 0; h < 2; h++) {
+      const int r = 2 * pair + h;
+      if (r >= G.N_r) continue;
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        if (c >= nt) continue;
+        const ACC sacc = h ? acc1[c] : acc0[c];
+        const size_t o = ((size_t)p * G.N_r + r) * G.N_t + t0 + c;
+        const size_t od = (size_t)r * G.N_t + t0 + c;
+        if (MODE == 0) {
+          F.out[o] = (float)sacc;
+        } else if (MODE == 1) {
+          F.out[o] = __fsub_rn(__fsub_rn(F.y[o], (float)sacc), F.d[od]);
+        } else {
+          // A * delta_t: the system matrix of the voxel update (XT_VoxUpdate.c:27, 67)
+          const double e64 = (double)F.y[o] - (double)G.delta_t * (double)sacc - (double)F.d[od];
+          if (MODE == 2) F.out[o] = (float)e64;
+          const double sw = e64 * sqrt((double)F.w[o]);
+          if (fabs(sw) < (double)F.T)
+            cacc += sw * sw;
+          else
+            cacc += 2.0 * (double)F.delta * (double)F.T * fabs(sw) + (double)F.T * (double)F.T * (1.0 - 2.0 * (double)F.delta);
+        }
+      }
     }
   }
   if (MODE >= 2) {
+    __syncwarp();
     for (int off = 16; off > 0; off >>= 1) cacc += __shfl_xor_sync(0xffffffffu, cacc, off);
-    if (lane == 0) atomicAdd(&F.cost_slots[(blockIdx.x * 7 + r + blockIdx.z) % 64], cacc);
+    if (lane == 0) atomicAdd(&F.cost_slots[(blockIdx.x * 7 + blockIdx.y + warp + blockIdx.z) % 64], cacc);
   }
 }
 
-template <bool PAIR, bool FULL>
+template <int LT, bool VEC>
 static void launch_fp_csr_t(const DevGeo &G, const FpArgs &F, const CsrView &T, int mode, cudaStream_t st) {
-  dim3 grid((unsigned)G.N_p, (unsigned)((G.N_r + CSR_WARPS - 1) / CSR_WARPS), (unsigned)((G.N_t + 63) / 64));
+  const int np2 = (G.N_r + 1) / 2, pw = 32 / LT;
+  const dim3 grid((unsigned)((G.N_p + CSR_WARPS - 1) / CSR_WARPS), (unsigned)((np2 + pw - 1) / pw),
+                  (unsigned)((G.N_t + 4 * LT - 1) / (4 * LT)));
   switch (mode) {
-    case 0: k_fp_csr<0, float, PAIR, FULL><<<grid, CSR_WARPS * 32, 0, st>>>(G, F, T); break;
-    case 1: k_fp_csr<1, float, PAIR, FULL><<<grid, CSR_WARPS * 32, 0, st>>>(G, F, T); break;
-    case 2: k_fp_csr<2, double, PAIR, FULL><<<grid, CSR_WARPS * 32, 0, st>>>(G, F, T); break;
-    default: k_fp_csr<3, double, PAIR, FULL><<<grid, CSR_WARPS * 32, 0, st>>>(G, F, T); break;
+    case 0: k_fp_csr<0, float, LT, VEC><<<grid, CSR_WARPS * 32, 0, st>>>(G, F, T); break;
+    case 1: k_fp_csr<1, float, LT, VEC><<<grid, CSR_WARPS * 32, 0, st>>>(G, F, T); break;
+    case 2: k_fp_csr<2, double, LT, VEC><<<grid, CSR_WARPS * 32, 0, st>>>(G, F, T); break;
+    default: k_fp_csr<3, double, LT, VEC><<<grid, CSR_WARPS * 32, 0, st>>>(G, F, T); break;
   }
 }
 
 cudaError_t launch_fp_csr(const DevGeo &G, const FpArgs &F, const CsrView &T, int mode, cudaStream_t st) {
-  // paired rows need one detector row per slice, an even row count (so a
-  // chunk never ends inside a pair) and 8-byte aligned z-lines
-  if (G.zovl == 1 && G.N_t % 2 == 0 && G.N_z % 2 == 0) {
-    if (G.N_t % 64 == 0)
-      launch_fp_csr_t<true, true>(G, F, T, mode, st);
-    else
-      launch_fp_csr_t<true, false>(G, F, T, mode, st);
-  } else {
-    launch_fp_csr_t<false, false>(G, F, T, mode, st);
-  }
+  // one 16-byte load for four rows where rows and slices are the same and
+  // z-lines keep 16-byte alignment; lanes per pair: as many as the rows fill
+  const bool vec = G.zovl == 1 && G.N_z % 4 == 0;
+  if (G.N_t <= 16)
+    vec ? launch_fp_csr_t<4, true>(G, F, T, mode, st) : launch_fp_csr_t<4, false>(G, F, T, mode, st);
+  else if (G.N_t <= 32)
+    vec ? launch_fp_csr_t<8, true>(G, F, T, mode, st) : launch_fp_csr_t<8, false>(G, F, T, mode, st);
+  else
+    vec ? launch_fp_csr_t<16, true>(G, F, T, mode, st) : launch_fp_csr_t<16, false>(G, F, T, mode, st);
   return cudaGetLastError();
 }
 
