@@ -89,9 +89,16 @@ constexpr int TILE_AHEAD = 2;      // stages a loader has in flight before it wa
 // box a chunk (2340 rows of 32 bytes for TZ 4) the copies took 3.4 cycles a
 // row and set the time, 1.86 ms; 80 -> 32 4.21 -> 2.85 ms, 48 -> 48 at half the
 // resolution 496 -> 414 us.
-template <int EPI, int TZ>
+//
+// CAT: the input is the concatenation of a 2x nearest upsampling (the first ca
+// channels, read from the coarse volume `up`) and `in` (the others); it is
+// never formed.  At 512^2 x 64 forming it took 0.85 ms for the 80-channel
+// level and 1.02 ms in all; read in place the 80 -> 32 convolution takes 2.86
+// ms against 2.85.
+template <int EPI, int TZ, bool CAT>
 __global__ void __launch_bounds__(288, 1)
-    k_conv_tile(const __nv_bfloat16 *__restrict__ in, ConvShape s, const __nv_bfloat16 *__restrict__ wp,
+    k_conv_tile(const __nv_bfloat16 *__restrict__ in, const __nv_bfloat16 *__restrict__ up, int ca, ConvShape s,
+                const __nv_bfloat16 *__restrict__ wp,
                 const float *__restrict__ bias, void *out, int nstage, int *err) {
   using D = TileDims<TZ>;
   constexpr int TZS = D::TZS;
@@ -153,13 +160,16 @@ __global__ void __launch_bounds__(288, 1)
     // and destination offsets are worked out once (done per stage they were
     // the kernel's bound), and which copies lie on the tile's edges.
     constexpr int NE = (TXS * TZS * 2 + TILE_LOADERS - 1) / TILE_LOADERS;
-    int off[NE];
+    const int cs = CAT ? s.cin - ca : s.cin;  // channels of `in`
+    int off[NE], upo[CAT ? NE : 1];
     uint32_t dst[NE], have = 0, on_x0 = 0, on_x1 = 0, on_z0 = 0, on_z1 = 0, on_h1 = 0;
 #pragma unroll
     for (int e = 0; e < NE; e++) {
       const int i = lt + e * TILE_LOADERS;
       const int xx = i / (TZS * 2), rem = i - xx * (TZS * 2), zz = rem >> 1, h = rem & 1, r = zz * TXS + xx;
-      off[e] = (xx * s.Z + zz) * s.cin + 8 * h;
+      off[e] = (xx * s.Z + zz) * cs + 8 * h;
+      // (x0 and z0 are even: voxel x0 - 1 + xx lies in coarse voxel x0 / 2 + floor((xx - 1) / 2))
+      if (CAT) upo[e] = (((xx - 1) >> 1) * (s.Z >> 1) + ((zz - 1) >> 1)) * ca + 8 * h;
       dst[e] = (uint32_t)r * 32u + (uint32_t)((h ^ ((r >> 2) & 1)) << 4);
       if (xx < TXS) have |= 1u << e;
       if (xx == 0) on_x0 |= 1u << e;
@@ -183,8 +193,8 @@ __global__ void __launch_bounds__(288, 1)
       if (x0 + TX == s.X) inside &= ~on_x1;
       if (z0 == 0) inside &= ~on_z0;
       if (z0 + TZ == s.Z) inside &= ~on_z1;
-      const __nv_bfloat16 *row = in + (((long long)b * s.Y + y - 1) * s.X + x0 - 1) * s.Z * s.cin + (z0 - 1) * s.cin;
-      const long long ystep = (long long)s.X * s.Z * s.cin;
+      const __nv_bfloat16 *row = in + (((long long)b * s.Y + y - 1) * s.X + x0 - 1) * s.Z * cs + (z0 - 1) * cs - (CAT ? ca : 0);
+      const long long ystep = (long long)s.X * s.Z * cs;
       int c = 0, dyi = 0;
       for (int k = 0; k < nq; k++) {
         if (!mbar_wait(&empty[st], ph, lim) || bad) {
@@ -199,12 +209,15 @@ __global__ void __launch_bounds__(288, 1)
         const int y2 = y + dyi - 1;
         uint32_t m = y2 >= 0 && y2 < s.Y ? inside : 0u;
         if (16 * c + 8 >= s.cin) m &= ~on_h1;  // a half chunk
-        const __nv_bfloat16 *src = row + dyi * ystep + 16 * c;
+        const bool coarse = CAT && 16 * c < ca;
+        const __nv_bfloat16 *src =
+            coarse ? up + (((long long)b * (s.Y >> 1) + (y2 >> 1)) * (s.X >> 1) + (x0 >> 1)) * (s.Z >> 1) * ca + (z0 >> 1) * ca + 16 * c
+                   : row + dyi * ystep + 16 * c;
         const uint32_t sa = smem_u32(a);
 #pragma unroll
         for (int e = 0; e < NE; e++) {
           const bool v = (m >> e) & 1u;
-          const __nv_bfloat16 *g = v ? src + off[e] : in;
+          const __nv_bfloat16 *g = v ? src + (CAT && coarse ? upo[CAT ? e : 0] : off[e]) : in;
           if (e + 1 < NE || ((have >> e) & 1u))
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sa + dst[e]), "l"(g), "r"(v ? 16 : 0)
                          : "memory");
@@ -616,18 +629,24 @@ cudaError_t conv_tile_pack(int cin, int n, int kpad, int sign, const __nv_bfloat
 }
 
 cudaError_t conv_forward_tile(const ConvShape &s, const __nv_bfloat16 *in, const __nv_bfloat16 *wp, const float *bias,
-                              void *out, int epi, int sign, int *err, cudaStream_t st) {
+                              void *out, int epi, int sign, int *err, cudaStream_t st, const __nv_bfloat16 *up, int ca) {
   if (!conv_tile_supported(s) || (epi == 0 && !bias) || epi < 0 || epi > 2 || (sign != 1 && sign != -1) ||
       (reinterpret_cast<uintptr_t>(in) & 15))
     return cudaErrorNotSupported;
+  if (up && (epi != 0 || ca < 16 || ca % 16 || s.cin <= ca || s.cin % 16 || s.Y % 2 || s.X % 2 || s.Z % 2 ||
+             (reinterpret_cast<uintptr_t>(up) & 15)))
+    return cudaErrorNotSupported;
   const int tz = tile_tz(s);
-  typedef void (*K)(const __nv_bfloat16 *, ConvShape, const __nv_bfloat16 *, const float *, void *, int, int *);
+  typedef void (*K)(const __nv_bfloat16 *, const __nv_bfloat16 *, int, ConvShape, const __nv_bfloat16 *, const float *,
+                    void *, int, int *);
   K k;
   // the sign lives in the packed weights
-  if (tz == 4)
-    k = epi == 0 ? k_conv_tile<0, 4> : epi == 1 ? k_conv_tile<1, 4> : k_conv_tile<2, 4>;
+  if (up)
+    k = tz == 4 ? k_conv_tile<0, 4, true> : k_conv_tile<0, 2, true>;
+  else if (tz == 4)
+    k = epi == 0 ? k_conv_tile<0, 4, false> : epi == 1 ? k_conv_tile<1, 4, false> : k_conv_tile<2, 4, false>;
   else
-    k = epi == 0 ? k_conv_tile<0, 2> : epi == 1 ? k_conv_tile<1, 2> : k_conv_tile<2, 2>;
+    k = epi == 0 ? k_conv_tile<0, 2, false> : epi == 1 ? k_conv_tile<1, 2, false> : k_conv_tile<2, 2, false>;
   const size_t stage =
       (size_t)(tz == 4 ? TileDims<4>::A_STAGE : TileDims<2>::A_STAGE) + (b_stage_bytes(s.n) + 1023) / 1024 * 1024;
   const int nstage = (int)std::min<size_t>(TILE_STAGES, (size_t)220 * 1024 / stage);
@@ -642,7 +661,7 @@ cudaError_t conv_forward_tile(const ConvShape &s, const __nv_bfloat16 *in, const
   }
   const long long ntiles = (long long)(s.X / TX) * (s.Z / tz) * s.nb * s.Y;
   const unsigned grid = (unsigned)std::min<long long>(ntiles, sms);  // one CTA per SM (shared memory)
-  k<<<grid, 288, smem, st>>>(in, s, wp, bias, out, nstage, err);
+  k<<<grid, 288, smem, st>>>(in, up, ca, s, wp, bias, out, nstage, err);
   return cudaGetLastError();
 }
 

@@ -149,9 +149,6 @@ int ensure_buffers(xtc_net *n, int nb, int Y, int X, int Z, bool training) {
   NCK(n->p0.ensure(v1 * 32 * sizeof(bf16)));
   NCK(n->p1.ensure(v2 * 48 * sizeof(bf16)));
   NCK(n->p2.ensure(v3 * 64 * sizeof(bf16)));
-  NCK(n->u2.ensure(v2 * 160 * sizeof(bf16)));
-  NCK(n->u1.ensure(v1 * 112 * sizeof(bf16)));
-  NCK(n->u0.ensure(v0 * 80 * sizeof(bf16)));
   if (training) {
     NCK(n->g32.ensure(gmax * sizeof(float)));
     NCK(n->gtmp.ensure(gmax * sizeof(float)));
@@ -191,6 +188,25 @@ int conv(xtc_net *n, int li, const bf16 *in, int lvl, bf16 *out) {
   return 0;
 }
 
+// conv li of the concatenation of a's 2x upsampling (ca channels) and skip: read
+// in place where the tile kernel takes the shape, else (or where training needs
+// it later) formed in cat
+int conv_cat(xtc_net *n, int li, const bf16 *a, int ca, const bf16 *skip, int cb, int lvl, Buf &cat, bf16 *out, bool keep) {
+  const Layer &l = n->L[li];
+  xtc::ConvShape s{n->nb, n->Y >> lvl, n->X >> lvl, n->Z >> lvl, l.cin, l.cout, l.kpad};
+  if (!keep && l.Wp && xtc::conv_tile_supported(s)) {
+    const cudaError_t e = xtc::conv_forward_tile(s, skip, l.Wp, n->P + l.off_b, out, 0, 1, n->d_err, n->st, a, ca);
+    if (e != cudaErrorNotSupported) {
+      NCK(e);
+      return 0;
+    }
+    cudaGetLastError();
+  }
+  NCK(cat.ensure((size_t)s.nb * s.Y * s.X * s.Z * l.cin * sizeof(bf16)));
+  xtc::up_concat(n->nb, s.Y, s.X, s.Z, ca, cb, a, skip, cat.as<bf16>(), n->st);
+  return conv(n, li, cat.as<bf16>(), lvl, out);
+}
+
 int forward(xtc_net *n, const float *fbp, const float *icd, float *out, const float *target) {
   const int nb = n->nb, Y = n->Y, X = n->X, Z = n->Z;
   const long long v0 = (long long)nb * Y * X * Z;
@@ -215,14 +231,12 @@ int forward(xtc_net *n, const float *fbp, const float *icd, float *out, const fl
   xtc::avgpool(nb, Y / 4, X / 4, Z / 4, 64, A[5], n->p2.as<bf16>(), st);
   if ((rc = conv(n, 6, n->p2.as<bf16>(), 3, A[6]))) return rc;
   if ((rc = conv(n, 7, A[6], 3, A[7]))) return rc;
-  xtc::up_concat(nb, Y / 4, X / 4, Z / 4, 96, 64, A[7], A[5], n->u2.as<bf16>(), st);
-  if ((rc = conv(n, 8, n->u2.as<bf16>(), 2, A[8]))) return rc;
+  const bool keep = target != nullptr;
+  if ((rc = conv_cat(n, 8, A[7], 96, A[5], 64, 2, n->u2, A[8], keep))) return rc;
   if ((rc = conv(n, 9, A[8], 2, A[9]))) return rc;
-  xtc::up_concat(nb, Y / 2, X / 2, Z / 2, 64, 48, A[9], A[3], n->u1.as<bf16>(), st);
-  if ((rc = conv(n, 10, n->u1.as<bf16>(), 1, A[10]))) return rc;
+  if ((rc = conv_cat(n, 10, A[9], 64, A[3], 48, 1, n->u1, A[10], keep))) return rc;
   if ((rc = conv(n, 11, A[10], 1, A[11]))) return rc;
-  xtc::up_concat(nb, Y, X, Z, 48, 32, A[11], A[1], n->u0.as<bf16>(), st);
-  if ((rc = conv(n, 12, n->u0.as<bf16>(), 0, A[12]))) return rc;
+  if ((rc = conv_cat(n, 12, A[11], 48, A[1], 32, 0, n->u0, A[12], keep))) return rc;
   if ((rc = conv(n, 13, A[12], 0, A[13]))) return rc;
   if (target) {
     NCK(cudaMemsetAsync(n->d_loss, 0, sizeof(double), st));

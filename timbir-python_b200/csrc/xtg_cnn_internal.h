@@ -20,14 +20,17 @@ cudaError_t conv_first_pack(int n, int cin, int kpad, const __nv_bfloat16 *w, __
 cudaError_t conv_first(int nb, int Y, int X, int Z, const float *a, const float *b, float scale,
                        const __nv_bfloat16 *w64, const float *bias, int n, __nv_bfloat16 *out, int *err,
                        cudaStream_t st);
-// the TMA-staged tile kernel (cnn_conv_tile.cu): X a multiple of 128, Z even,
+// the staged tile kernel (cnn_conv_tile.cu): X a multiple of 128, Z even,
 // n <= 64; weights pre-packed by conv_tile_pack into conv_tile_wp_elems values
 bool conv_tile_supported(const ConvShape &s);
 size_t conv_tile_wp_elems(int cin, int n);
 cudaError_t conv_tile_pack(int cin, int n, int kpad, int sign, const __nv_bfloat16 *w, __nv_bfloat16 *wp,
                            cudaStream_t st);
+// with `up`, channels [0, ca) are the 2x nearest upsampling of that coarse
+// volume (ca channels) and `in` holds the other cin - ca (epi 0)
 cudaError_t conv_forward_tile(const ConvShape &s, const __nv_bfloat16 *in, const __nv_bfloat16 *wp, const float *bias,
-                              void *out, int epi, int sign, int *err, cudaStream_t st);
+                              void *out, int epi, int sign, int *err, cudaStream_t st, const __nv_bfloat16 *up = nullptr,
+                              int ca = 0);
 // TMA boxes of 128 voxels per tap (cnn_conv_box.cu): any volume, cin and n
 // multiples of 16; weights pre-packed by conv_box_pack into
 // conv_box_wp_elems values (the sign stays an argument)
