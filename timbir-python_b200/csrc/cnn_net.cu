@@ -68,7 +68,6 @@ struct xtc_net {
   Layer L[kLayers];
   size_t n_params = 0, off_hw = 0, off_hb = 0;
   float *P = nullptr, *G = nullptr, *M = nullptr, *V = nullptr;  // parameters, gradients, Adam moments
-  float *graw = nullptr;  // raw weight gradient of the input layer (cin padded)
   double *d_loss = nullptr;
   int *d_err = nullptr;
   int step = 0;
@@ -252,21 +251,19 @@ int forward(xtc_net *n, const float *fbp, const float *icd, float *out, const fl
 // backward of conv li with post-ReLU gradient dpost (FP32, rows of ld floats,
 // the layer's channels from off on; plus the pooling's, `pooled`, where the
 // layer was pooled too) and post-activation `post`; writes the input gradient
-// (FP32) to din when din != nullptr
+// (FP32) to din when din != nullptr.  The first layer has no `in` but the two
+// input volumes.
 int conv_back(xtc_net *n, int li, const float *dpost, const bf16 *post, const bf16 *in, int lvl, float *din, int ld = 0,
-              int off = 0, const float *pooled = nullptr) {
+              int off = 0, const float *pooled = nullptr, const float *fbp = nullptr, const float *icd = nullptr) {
   const Layer &l = n->L[li];
   bf16 *dpre = n->gpre.as<bf16>();
   xtc::relu_back(n->nb, n->Y >> lvl, n->X >> lvl, n->Z >> lvl, l.cout, dpost, ld ? ld : l.cout, off, pooled, post, dpre,
                  n->G + l.off_b, n->st);
   xtc::ConvShape s{n->nb, n->Y >> lvl, n->X >> lvl, n->Z >> lvl, l.cin, l.cout, l.kpad};
-  if (l.cin == l.cin_real) {
+  if (!in)
+    NCK(xtc::wgrad_first(n->nb, n->Y, n->X, n->Z, fbp, icd, kScale, dpre, n->G + l.off_w, n->d_err, n->st));
+  else
     NCK(xtc::conv_wgrad(s, in, dpre, n->G + l.off_w, n->d_err, n->st));
-  } else {
-    NCK(cudaMemsetAsync(n->graw, 0, sizeof(float) * 27 * l.cin * l.cout, n->st));
-    NCK(xtc::conv_wgrad(s, in, dpre, n->graw, n->d_err, n->st));
-    xtc::fold_wgrad(l.cin_real, l.cin, l.cout, n->graw, n->G + l.off_w, n->st);
-  }
   if (din) {
     // the input gradient: the same convolution with transposed weights and
     // negated offsets, on the tile kernel where the shape allows
@@ -292,7 +289,7 @@ int conv_back(xtc_net *n, int li, const float *dpost, const bf16 *post, const bf
   return 0;
 }
 
-int backward(xtc_net *n) {
+int backward(xtc_net *n, const float *fbp, const float *icd) {
   const int nb = n->nb, Y = n->Y, X = n->X, Z = n->Z;
   cudaStream_t st = n->st;
   bf16 *A[kLayers];
@@ -319,7 +316,7 @@ int backward(xtc_net *n) {
   if ((rc = conv_back(n, 3, u1, A[3], A[2], 1, g, 112, 64, t))) return rc;         // g = d A2
   if ((rc = conv_back(n, 2, g, A[2], n->p0.as<bf16>(), 1, t))) return rc;          // t = d p0
   if ((rc = conv_back(n, 1, u0, A[1], A[0], 0, g, 80, 48, t))) return rc;          // g = d A0
-  if ((rc = conv_back(n, 0, g, A[0], n->in0.as<bf16>(), 0, nullptr))) return rc;
+  if ((rc = conv_back(n, 0, g, A[0], nullptr, 0, nullptr, 0, 0, nullptr, fbp, icd))) return rc;
   NCK(cudaGetLastError());
   return 0;
 }
@@ -373,7 +370,6 @@ int xtc_net_create(uint64_t seed, xtc_net **out) {
   A((void **)&n->G, off * 4);
   A((void **)&n->M, off * 4);
   A((void **)&n->V, off * 4);
-  A((void **)&n->graw, (size_t)27 * 8 * 32 * 4);
   A((void **)&n->d_loss, 8);
   A((void **)&n->d_err, 4);
   for (int i = 0; i < kLayers; i++) {
@@ -401,7 +397,7 @@ int xtc_net_create(uint64_t seed, xtc_net **out) {
 
 void xtc_net_destroy(xtc_net *n) {
   if (!n) return;
-  for (float *p : {n->P, n->G, n->M, n->V, n->graw})
+  for (float *p : {n->P, n->G, n->M, n->V})
     if (p) cudaFree(p);
   if (n->d_loss) cudaFree(n->d_loss);
   if (n->d_err) cudaFree(n->d_err);
@@ -503,7 +499,7 @@ int xtc_net_backward(xtc_net *n, const float *fbp, const float *icd, const float
   if (!n->packed && (rc = pack_all(n))) return rc;
   NCK(cudaMemsetAsync(n->G, 0, n->n_params * 4, n->st));
   if ((rc = forward(n, fbp, icd, nullptr, target))) return rc;
-  if ((rc = backward(n))) return rc;
+  if ((rc = backward(n, fbp, icd))) return rc;
   if (loss) NCK(cudaMemcpyAsync(loss, n->d_loss, sizeof(double), cudaMemcpyDeviceToHost, n->st));
   return check_err(n);
 }

@@ -324,18 +324,6 @@ __global__ void k_pack_weights(int cin_real, int cin, int cout, int kpad, int kp
   }
 }
 
-// the weight gradient rows of a padded input layer ([(tap*cin + ci)][cout],
-// cin padded) folded to the master layout ([(tap*cin_real + ci)][cout])
-__global__ void k_fold_wgrad(int cin_real, int cin, int cout, const float *g, float *out) {
-  const long long n = 27LL * cin_real * cout;
-  GRID_STRIDE(i, n) {
-    const int co = (int)(i % cout);
-    const long long r = i / cout;
-    const int tap = (int)(r / cin_real), ci = (int)(r % cin_real);
-    out[i] = g[((size_t)tap * cin + ci) * cout + co];
-  }
-}
-
 // Adam (Kingma & Ba 2015) with bias correction
 __global__ void k_adam(long long n, float *p, const float *g, float *m, float *v, float lr, float b1, float b2,
                        float eps, float c1, float c2) {
@@ -423,9 +411,6 @@ void head_train(long long nv, const __nv_bfloat16 *h, const float *w, const floa
 void pack_weights(int cin_real, int cin, int cout, int kpad, int kpad_t, const float *P, __nv_bfloat16 *W,
                   __nv_bfloat16 *Wt, cudaStream_t st) {
   k_pack_weights<<<blocks((long long)cout * kpad), 256, 0, st>>>(cin_real, cin, cout, kpad, kpad_t, P, W, Wt);
-}
-void fold_wgrad(int cin_real, int cin, int cout, const float *g, float *out, cudaStream_t st) {
-  k_fold_wgrad<<<blocks(27LL * cin_real * cout), 256, 0, st>>>(cin_real, cin, cout, g, out);
 }
 void adam(long long n, float *p, const float *g, float *m, float *v, float lr, float b1, float b2, float eps, int t,
           cudaStream_t st) {

@@ -145,6 +145,19 @@ __device__ __forceinline__ void tmem_st16_zero(uint32_t taddr) {
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// 16 BF16 values (or 8 FP32 values) to global memory: one 32-byte store, a whole
+// sector, where p is 32-byte aligned; two 16-byte ones otherwise
+__device__ __forceinline__ void store32(void *p, const int4 &a, const int4 &b) {
+  if ((reinterpret_cast<uintptr_t>(p) & 31) == 0) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
+                 "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
+  } else {
+    reinterpret_cast<int4 *>(p)[0] = a;
+    reinterpret_cast<int4 *>(p)[1] = b;
+  }
+}
+
 // TMEM columns to allocate for N accumulator columns (power of two, >= 32)
 __host__ __device__ constexpr uint32_t tmem_cols(int n) {
   return n <= 32 ? 32u : n <= 64 ? 64u : n <= 128 ? 128u : 256u;

@@ -20,6 +20,9 @@ cudaError_t conv_first_pack(int n, int cin, int kpad, const __nv_bfloat16 *w, __
 cudaError_t conv_first(int nb, int Y, int X, int Z, const float *a, const float *b, float scale,
                        const __nv_bfloat16 *w64, const float *bias, int n, __nv_bfloat16 *out, int *err,
                        cudaStream_t st);
+// its weight gradient (32 output channels), added to dw [2 tap + channel][32]
+cudaError_t wgrad_first(int nb, int Y, int X, int Z, const float *a, const float *b, float scale,
+                        const __nv_bfloat16 *dout, float *dw, int *err, cudaStream_t st);
 // the staged tile kernel (cnn_conv_tile.cu): X a multiple of 128, Z even,
 // n <= 64; weights pre-packed by conv_tile_pack into conv_tile_wp_elems values
 bool conv_tile_supported(const ConvShape &s);
@@ -68,7 +71,6 @@ void head_train(long long nv, const __nv_bfloat16 *h, const float *w, const floa
                 const float *target, double *loss, float *dh, float *dw, float *db, cudaStream_t st);
 void pack_weights(int cin_real, int cin, int cout, int kpad, int kpad_t, const float *P, __nv_bfloat16 *W,
                   __nv_bfloat16 *Wt, cudaStream_t st);
-void fold_wgrad(int cin_real, int cin, int cout, const float *g, float *out, cudaStream_t st);
 void adam(long long n, float *p, const float *g, float *m, float *v, float lr, float b1, float b2, float eps, int t,
           cudaStream_t st);
 void crop(int np, const float *const *src, const int4 *org, int Y, int X, int Z, int py, int px, int pz, float *dst,
