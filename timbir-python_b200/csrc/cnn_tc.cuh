@@ -81,6 +81,27 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity, long 
   return false;
 }
 
+// The warp that issues MMAs runs as a whole and lets one elected lane issue: with
+// its waits' outcomes and its warp number known to be the same in every lane,
+// descriptors and counters stay in uniform registers, from which tcgen05.mma takes
+// its operands.  Under `if (lane == 0)` an issue cost about 200 cycles, the same for
+// N = 16 and 256: the halo convolution 32 -> 80 of 1048576 voxels took 573 us, 325
+// with this.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(p));
+  return p != 0;
+}
+// bounded wait of a whole warp
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *mbar, uint32_t parity, long long limit) {
+  return __all_sync(0xffffffffu, mbar_wait(mbar, parity, limit));
+}
+
 // the single arrival of a transaction barrier, announcing `bytes` to come
 __device__ __forceinline__ void mbar_expect_tx(uint64_t *mbar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(mbar)), "r"(bytes) : "memory");
