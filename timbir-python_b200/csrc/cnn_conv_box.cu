@@ -147,14 +147,13 @@ __device__ __forceinline__ void tap_of(int t, int &dy, int &dx, int &dz) {
 template <int EPI>
 __device__ __forceinline__ void drain(bool in, size_t vox, int N, uint32_t acc, const float *__restrict__ bias, void *out) {
   for (int n0 = 0; n0 < N; n0 += 16) {
-    float v[16];
+    __align__(16) float v[16];
     tmem_ld16(acc + (uint32_t)n0, v);
     if (in) {
       if (EPI == 2) {
         float *o = reinterpret_cast<float *>(out) + vox * N + n0;
-#pragma unroll
-        for (int i = 0; i < 16; i += 4)
-          *reinterpret_cast<float4 *>(o + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+        store32(o, *reinterpret_cast<const int4 *>(v), *reinterpret_cast<const int4 *>(v + 4));
+        store32(o + 8, *reinterpret_cast<const int4 *>(v + 8), *reinterpret_cast<const int4 *>(v + 12));
       } else {
         __align__(16) __nv_bfloat16 h[16];
 #pragma unroll
@@ -164,8 +163,7 @@ __device__ __forceinline__ void drain(bool in, size_t vox, int N, uint32_t acc, 
           h[i] = __float2bfloat16_rn(f);
         }
         __nv_bfloat16 *o = reinterpret_cast<__nv_bfloat16 *>(out) + vox * N + n0;
-        *reinterpret_cast<int4 *>(o) = *reinterpret_cast<const int4 *>(h);
-        *reinterpret_cast<int4 *>(o + 8) = *reinterpret_cast<const int4 *>(h + 8);
+        store32(o, *reinterpret_cast<const int4 *>(h), *reinterpret_cast<const int4 *>(h + 8));
       }
     }
     __syncwarp();

@@ -93,8 +93,14 @@ constexpr int TILE_AHEAD = 2;      // stages a loader has in flight before it wa
 // CAT: the input is the concatenation of a 2x nearest upsampling (the first ca
 // channels, read from the coarse volume `up`) and `in` (the others); it is
 // never formed.  At 512^2 x 64 forming it took 0.85 ms for the 80-channel
-// level and 1.02 ms in all; read in place the 80 -> 32 convolution takes 2.86
-// ms against 2.85.
+// level and 1.02 ms in all; read in place the 80 -> 32 convolution takes the
+// same time.
+//
+// With the MMAs issued from a warp-uniform loop and whole sectors stored 32 -> 32
+// takes 1.23 ms (1.27 before), 80 -> 32 2.55 (2.86), 48 -> 48 at half the
+// resolution 0.36 (0.41).  Alone the copies, the MMAs (about 65 cycles each, near
+// what reading A's 4 KB from shared memory takes) and the epilogue need 0.9, 0.85
+// and 0.6 ms of the 1.23.
 template <int EPI, int TZ, bool CAT>
 __global__ void __launch_bounds__(288, 1)
     k_conv_tile(const __nv_bfloat16 *__restrict__ in, const __nv_bfloat16 *__restrict__ up, int ca, ConvShape s,
@@ -108,7 +114,7 @@ __global__ void __launch_bounds__(288, 1)
   __shared__ uint64_t full[TILE_STAGES], empty[TILE_STAGES], acc_full[2], acc_empty[2], done;
   __shared__ uint32_t tbase;
   __shared__ volatile int bad;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int nchunk = (s.cin + 15) >> 4;
   const int XT = s.X / TX, ZT = s.Z / TZ;
   const int ntiles = XT * ZT * s.nb * s.Y;
@@ -247,29 +253,30 @@ __global__ void __launch_bounds__(288, 1)
     // the weights issued last land before the shared memory is released
     for (int i = q > nstage ? q - nstage : 0; i < q; i++) mbar_wait(&full[i % nstage], (uint32_t)(i / nstage) & 1u, lim);
   } else if (warp == 4) {
-    if (lane == 0 && mine > 0) {
-      const uint32_t idesc[3] = {idesc_bf16(N, 0, 0), idesc_bf16(2 * N, 0, 0), idesc_bf16(3 * N, 0, 0)};
-      bool ok = true;
-      int st = 0;
-      uint32_t ph = 0;
-      for (int tl = 0; tl < mine && ok; tl++) {
-        const int ab = tl & 1;
-        if (!mbar_wait(&acc_empty[ab], (uint32_t)(((tl >> 1) & 1) ^ 1), lim)) {
+    const uint32_t idesc[3] = {idesc_bf16(N, 0, 0), idesc_bf16(2 * N, 0, 0), idesc_bf16(3 * N, 0, 0)};
+    const bool lead = elect_one();
+    bool ok = true;
+    int st = 0;
+    uint32_t ph = 0;
+    for (int tl = 0; tl < mine && ok; tl++) {
+      const int ab = tl & 1;
+      if (!mbar_wait_warp(&acc_empty[ab], (uint32_t)(((tl >> 1) & 1) ^ 1), lim)) {
+        ok = false;
+        break;
+      }
+      const uint32_t acc = tmem + (uint32_t)(ab * TZ * N);
+      for (int k = 0; k < nq; k++) {
+        if (!mbar_wait_warp(&full[st], ph, lim)) {
           ok = false;
           break;
         }
-        const uint32_t acc = tmem + (uint32_t)(ab * TZ * N);
-        for (int k = 0; k < nq; k++) {
-          if (!mbar_wait(&full[st], ph, lim) || bad) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          // descriptors advance in 16-byte units: an A row by 2; a (dy, dx)
-          // B block (2 halves x 3 dz x N rows x 16 bytes) by 6N, one dz block by N
-          const uint32_t a0 = smem_u32(sm + (size_t)st * STAGE);
-          const uint64_t da0 = sdesc_sw32(a0);
-          uint64_t db = sdesc(a0 + D::A_STAGE, (uint32_t)N * 48, 128);
+        tc_fence_after();
+        // descriptors advance in 16-byte units: an A row by 2; a (dy, dx)
+        // B block (2 halves x 3 dz x N rows x 16 bytes) by 6N, one dz block by N
+        const uint32_t a0 = smem_u32(sm) + (uint32_t)st * STAGE;
+        const uint64_t da0 = sdesc_sw32(a0);
+        uint64_t db = sdesc(a0 + D::A_STAGE, (uint32_t)N * 48, 128);
+        if (lead) {
 #pragma unroll
           for (int dxi = 0; dxi < 3; dxi++) {
 #pragma unroll
@@ -284,21 +291,23 @@ __global__ void __launch_bounds__(288, 1)
             db += (uint64_t)(6 * N);
           }
           mma_commit(&empty[st]);
-          if (++st == nstage) {
-            st = 0;
-            ph ^= 1u;
-          }
         }
-        if (ok) mma_commit(&acc_full[ab]);
+        __syncwarp();
+        if (++st == nstage) {
+          st = 0;
+          ph ^= 1u;
+        }
       }
-      if (!ok) {
-        atomicExch(err, 1);
-        bad = 1;
-      }
-      mma_commit(&done);
-      mbar_wait(&done, 0, lim);  // every MMA issued above has completed
+      if (ok && lead) mma_commit(&acc_full[ab]);
+      ok = __all_sync(0xffffffffu, ok && !bad);
     }
+    if (!ok && lead) {
+      atomicExch(err, 1);
+      bad = 1;
+    }
+    if (lead) mma_commit(&done);
     __syncwarp();
+    mbar_wait(&done, 0, lim);  // every MMA issued above has completed
   } else {
     // epilogue: warp w drains accumulator rows (x) 32w .. 32w + 31
     for (int tl = 0; tl < mine; tl++) {
@@ -315,13 +324,12 @@ __global__ void __launch_bounds__(288, 1)
       for (int zo = 0; zo < TZ; zo++) {
         const size_t vox = (((size_t)b * s.Y + y) * s.X + x0 + warp * 32 + lane) * s.Z + z0 + zo;
         for (int n0 = 0; n0 < N; n0 += 16) {
-          float v[16];
+          __align__(16) float v[16];
           tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((ab * TZ + zo) * N + n0), v);
           if (EPI == 2) {
             float *o = reinterpret_cast<float *>(out) + vox * N + n0;
-#pragma unroll
-            for (int q = 0; q < 16; q += 4)
-              *reinterpret_cast<float4 *>(o + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+            store32(o, *reinterpret_cast<const int4 *>(v), *reinterpret_cast<const int4 *>(v + 4));
+            store32(o + 8, *reinterpret_cast<const int4 *>(v + 8), *reinterpret_cast<const int4 *>(v + 12));
           } else {
             __align__(16) __nv_bfloat16 h[16];
 #pragma unroll
@@ -331,8 +339,7 @@ __global__ void __launch_bounds__(288, 1)
               h[q] = __float2bfloat16_rn(t);
             }
             __nv_bfloat16 *o = reinterpret_cast<__nv_bfloat16 *>(out) + vox * N + n0;
-            *reinterpret_cast<int4 *>(o) = *reinterpret_cast<const int4 *>(h);
-            *reinterpret_cast<int4 *>(o + 8) = *reinterpret_cast<const int4 *>(h + 8);
+            store32(o, *reinterpret_cast<const int4 *>(h), *reinterpret_cast<const int4 *>(h + 8));
           }
         }
       }
@@ -427,7 +434,7 @@ __global__ void __launch_bounds__(160, 1)
   __shared__ uint64_t full[2], empty[2], acc_full;
   __shared__ uint32_t tbase;
   __shared__ volatile int bad;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int nchunk = s.cin >> 4;
   const int cpg = nchunk < WG_CPG ? nchunk : WG_CPG;
   const uint32_t STAGE = wg_stage(cpg);
@@ -469,72 +476,74 @@ __global__ void __launch_bounds__(160, 1)
     b = t / s.Y;
   };
   if (warp == 4) {
-    if (lane == 0) {
-      bool ok = true;
-      if (mine > 0) {
-        const uint32_t idesc = idesc_bf16(WG_N, 1, 1);
-        int issued[2] = {0, 0}, landed[2] = {0, 0};
-        auto load = [&](int q) {
-          const int st = q & 1;
-          int x0, z0, y, b;
-          tile_of(q, x0, z0, y, b);
-          uint8_t *g = sm + st * STAGE;
+    const bool lead = elect_one();
+    bool ok = true;
+    if (mine > 0) {
+      const uint32_t idesc = idesc_bf16(WG_N, 1, 1);
+      int issued = 0, landed = 0;  // tiles whose copies were issued, have landed
+      auto load = [&](int q) {
+        const int st = q & 1;
+        int x0, z0, y, b;
+        tile_of(q, x0, z0, y, b);
+        uint8_t *g = sm + (size_t)st * STAGE;
+        if (lead) {
           mbar_expect_tx(&full[st], 6 * WG_DB + (uint32_t)nck * WG_XB);
           // box j = dy + 1 holds dY row y0 - dy (zero fill outside)
           for (int j = 0; j < 3; j++)
             for (int h = 0; h < 2; h++) tma_load_5d(g + (j * 2 + h) * WG_DB, &tdy, 16 * h, x0, z0, y + 1 - j, b, &full[st]);
           for (int c = 0; c < nck; c++)
             tma_load_5d(g + WG_A + c * WG_XS, &tin, 16 * (c0 + c), x0 - 1, z0 - 1, y, b, &full[st]);
-          issued[st]++;
-        };
-        load(0);
-        if (mine > 1) load(1);
-        for (int q = 0; q < mine && ok; q++) {
-          const int st = q & 1;
-          if (!mbar_wait(&full[st], (uint32_t)(q >> 1) & 1u, lim)) {
+        }
+        __syncwarp();
+        issued++;
+      };
+      load(0);
+      if (mine > 1) load(1);
+      for (int q = 0; q < mine && ok; q++) {
+        const int st = q & 1;
+        if (!mbar_wait_warp(&full[st], (uint32_t)(q >> 1) & 1u, lim)) {
+          ok = false;
+          break;
+        }
+        landed++;
+        tc_fence_after();
+        const uint32_t g = smem_u32(sm) + (uint32_t)st * STAGE;
+        const uint64_t da = sdesc_mn_sw32(g, WG_DB);
+        if (lead) {
+          for (int c = 0; c < nck; c++) {
+            const uint64_t db = sdesc_mn_sw32(g + WG_A + (uint32_t)c * WG_XS, TXS * 32);
+            const uint32_t acc = tmem + (uint32_t)(c * 3 * WG_N);
+#pragma unroll
+            for (int q3 = 0; q3 < 3; q3++)  // dx = q3 - 1
+#pragma unroll
+              for (int zo = 0; zo < WG_TZ; zo++)
+#pragma unroll
+                for (int ks = 0; ks < TX / 16; ks++)
+                  mma_bf16(acc + (uint32_t)(q3 * WG_N), da + (uint64_t)(2 * (zo * TX + ks * 16)),
+                           db + (uint64_t)(2 * (zo * TXS + ks * 16 + q3)), idesc, 1u);
+          }
+          mma_commit(&empty[st]);
+        }
+        __syncwarp();
+        if (q >= 1 && q + 1 < mine) {
+          // tile q + 1 reuses the stage of tile q - 1 once its MMAs are done
+          if (!mbar_wait_warp(&empty[(q - 1) & 1], (uint32_t)((q - 1) >> 1) & 1u, lim)) {
             ok = false;
             break;
           }
-          landed[st]++;
-          tc_fence_after();
-          const uint32_t g = smem_u32(sm + st * STAGE);
-          for (int c = 0; c < nck; c++) {
-            for (int q3 = 0; q3 < 3; q3++) {  // dx = q3 - 1
-              const uint32_t acc = tmem + (uint32_t)((c * 3 + q3) * WG_N);
-#pragma unroll
-              for (int zo = 0; zo < WG_TZ; zo++) {
-#pragma unroll
-                for (int ks = 0; ks < TX / 16; ks++) {
-                  const uint64_t da = sdesc_mn_sw32(g + (uint32_t)(zo * TX + ks * 16) * 32, WG_DB);
-                  const uint64_t db = sdesc_mn_sw32(g + WG_A + (uint32_t)c * WG_XS + (uint32_t)(zo * TXS + ks * 16 + q3) * 32,
-                                                    TXS * 32);
-                  mma_bf16(acc, da, db, idesc, 1u);
-                }
-              }
-            }
-          }
-          mma_commit(&empty[st]);
-          if (q >= 1 && q + 1 < mine) {
-            // tile q + 1 reuses the stage of tile q - 1 once its MMAs are done
-            if (!mbar_wait(&empty[(q - 1) & 1], (uint32_t)((q - 1) >> 1) & 1u, lim)) {
-              ok = false;
-              break;
-            }
-            load(q + 1);
-          }
-        }
-        if (!ok) {
-          // let the copies already issued land before the shared memory is released
-          for (int st = 0; st < 2; st++)
-            for (; landed[st] < issued[st]; landed[st]++) mbar_wait(&full[st], (uint32_t)landed[st] & 1u, lim);
+          load(q + 1);
         }
       }
-      if (!ok) {
-        atomicExch(err, 1);
-        bad = 1;
-      }
-      mma_commit(&acc_full);  // arrives once every MMA issued above has completed
+      // after a wait that gave up, let the copies already issued land before the
+      // shared memory is released
+      if (!ok)
+        for (; landed < issued; landed++) mbar_wait(&full[landed & 1], (uint32_t)(landed >> 1) & 1u, lim);
     }
+    if (!ok && lead) {
+      atomicExch(err, 1);
+      bad = 1;
+    }
+    if (lead) mma_commit(&acc_full);  // arrives once every MMA issued above has completed
     __syncwarp();
   } else {
     const bool ready = mbar_wait(&acc_full, 0, lim);
