@@ -325,66 +325,87 @@ __global__ void __launch_bounds__(CONV_THREADS) k_wgrad_tc(ConvShape s, const __
 // image, FP32 [nb][Y][X][Z], times scale), so K = 27 taps x 2 = 54, padded to 64:
 // one MMA stage whose A rows (voxel x 64, k = 2 tap + channel) are built from
 // the FP32 volumes, the input packing fused in.  A tile is 128 voxels of one
-// y-row, ZT z x 128 / ZT x (Z is a multiple of ZT); its halo is read once into
+// y-row, ZT z x 128 / ZT x (the network's Z is a multiple of 8); its halo lies in
 // shared memory as pairs of BF16, and a thread puts its row together from 27
-// words of it.
+// words of it.  A CTA goes along y, so each tile brings one new halo row.
 struct FirstTile {
-  int zt, xt, nzt, nxt, ntiles;
+  int zt, nzt, nxt, ntiles;  // tiles in the order y, z, x, batch
 };
 static FirstTile first_tile(int nb, int Y, int X, int Z) {
   FirstTile t;
-  t.zt = Z % 32 == 0 ? 32 : Z % 16 == 0 ? 16 : Z % 8 == 0 ? 8 : 1;
-  t.xt = 128 / t.zt;
+  t.zt = Z % 32 == 0 ? 32 : Z % 16 == 0 ? 16 : 8;
   t.nzt = Z / t.zt;
-  t.nxt = (X + t.xt - 1) / t.xt;
+  t.nxt = (X + 128 / t.zt - 1) / (128 / t.zt);
   t.ntiles = nb * Y * t.nxt * t.nzt;
   return t;
 }
-constexpr int FIRST_HALO = 3 * 130 * 3;  // words of the largest halo, 3 (xt + 2) (zt + 2) for zt = 1
 
-struct FirstPos {
-  int b, y, x0, z0;
-};
-__device__ __forceinline__ FirstPos first_pos(const FirstTile &t, int Y, int i) {
-  FirstPos p;
-  p.z0 = (i % t.nzt) * t.zt;
-  i /= t.nzt;
-  p.x0 = (i % t.nxt) * t.xt;
-  i /= t.nxt;
-  p.y = i % Y;
-  p.b = i / Y;
-  return p;
-}
-// the tile's halo -> halo[(dy + 1)][x - x0 + 1][z - z0 + 1], zero outside the volume
-__device__ __forceinline__ void first_halo(const FirstTile &t, const FirstPos &p, int Y, int X, int Z,
-                                           const float *__restrict__ fa, const float *__restrict__ fb, float scale,
-                                           uint32_t *halo) {
-  const int zs = t.zt + 2, xs = t.xt + 2, n = 3 * xs * zs;
-  for (int i = threadIdx.x; i < n; i += CONV_THREADS) {
-    const int zz = i % zs, r = i / zs, xx = r % xs, yy = r / xs;
-    const int y2 = p.y + yy - 1, x2 = p.x0 + xx - 1, z2 = p.z0 + zz - 1;
-    __nv_bfloat162 h = __floats2bfloat162_rn(0.f, 0.f);
-    if (y2 >= 0 && y2 < Y && x2 >= 0 && x2 < X && z2 >= 0 && z2 < Z) {
-      const size_t o = (((size_t)p.b * Y + y2) * X + x2) * Z + z2;
-      h = __floats2bfloat162_rn(__ldg(fa + o) * scale, __ldg(fb + o) * scale);
+// The halo of a column of tiles along y: three rows (XT + 2) x (ZT + 2) of pairs in
+// shared memory, the next tile's new row read ahead into registers.
+template <int ZT>
+struct FirstRows {
+  static constexpr int XT = 128 / ZT, XS = XT + 2, ZS = ZT + 2, NW = XS * ZS, NE = (NW + CONV_THREADS - 1) / CONV_THREADS;
+  const float *fa, *fb;  // of the column's batch
+  int off[NE], Y, XZ, x, z;
+  uint32_t in;
+  float ra[NE], rb[NE];
+
+  // column `col` of t; x and z are this thread's voxel
+  __device__ __forceinline__ void column(const FirstTile &t, int col, int Y_, int X, int Z, const float *fa_, const float *fb_) {
+    const int z0 = col % t.nzt * ZT, q = col / t.nzt, x0 = q % t.nxt * XT, b = q / t.nxt;
+    Y = Y_;
+    XZ = X * Z;
+    fa = fa_ + (size_t)b * Y * XZ;
+    fb = fb_ + (size_t)b * Y * XZ;
+    x = x0 + (int)threadIdx.x / ZT;
+    z = z0 + (int)threadIdx.x % ZT;
+    in = 0;
+#pragma unroll
+    for (int e = 0; e < NE; e++) {
+      const int i = threadIdx.x + e * CONV_THREADS, xx = x0 + i / ZS - 1, zz = z0 + i % ZS - 1;
+      const bool ok = i < NW && xx >= 0 && xx < X && zz >= 0 && zz < Z;
+      off[e] = ok ? xx * Z + zz : 0;
+      if (ok) in |= 1u << e;
     }
-    halo[i] = *reinterpret_cast<const uint32_t *>(&h);
   }
-}
-// this thread's A row: word t = tap t's two channels
-__device__ __forceinline__ void first_row(const FirstTile &t, const uint32_t *halo, uint32_t (&row)[32]) {
-  const int zs = t.zt + 2, xs = t.xt + 2;
-  const uint32_t *c = halo + (threadIdx.x / t.zt) * zs + threadIdx.x % t.zt;
+  __device__ __forceinline__ void fetch(int y) {
+    const uint32_t m = y >= 0 && y < Y ? in : 0u;
+    const size_t o = (size_t)(m ? y : 0) * XZ;
 #pragma unroll
-  for (int k = 0; k < 27; k++) row[k] = c[((k / 9) * xs + (k / 3) % 3) * zs + k % 3];
+    for (int e = 0; e < NE; e++) {
+      const bool v = (m >> e) & 1u;
+      ra[e] = v ? __ldg(fa + o + off[e]) : 0.f;
+      rb[e] = v ? __ldg(fb + o + off[e]) : 0.f;
+    }
+  }
+  __device__ __forceinline__ void put(uint32_t *row, float scale) const {
 #pragma unroll
-  for (int k = 27; k < 32; k++) row[k] = 0u;
-}
+    for (int e = 0; e < NE; e++) {
+      const __nv_bfloat162 h = __floats2bfloat162_rn(ra[e] * scale, rb[e] * scale);
+      const int i = threadIdx.x + e * CONV_THREADS;
+      if (i < NW) row[i] = *reinterpret_cast<const uint32_t *>(&h);
+    }
+  }
+  // this thread's A row: word k = tap k's two channels; s0: slot of row y - 1
+  __device__ __forceinline__ void build(const uint32_t *halo, int s0, uint32_t (&row)[32]) const {
+    const uint32_t *c = halo + (threadIdx.x / ZT) * ZS + threadIdx.x % ZT;
+#pragma unroll
+    for (int dy = 0; dy < 3; dy++) {
+      const int sl = s0 + dy < 3 ? s0 + dy : s0 + dy - 3;
+#pragma unroll
+      for (int k = 0; k < 9; k++) row[dy * 9 + k] = c[sl * NW + (k / 3) * ZS + k % 3];
+    }
+#pragma unroll
+    for (int k = 27; k < 32; k++) row[k] = 0u;
+  }
+};
 
 // w64: [n][64] BF16, k = 2 tap + channel.  Output: ReLU(acc + bias) in BF16
 // [voxel][n].  Persistent CTAs keep the weights and the TMEM columns over their
-// tiles.  With every row's 54 values loaded from L1 with its own bounds tests
-// 512^2 x 64 took 1.36 ms, now 0.74 ms (0.19 ms for the bytes).
+// run of tiles.  With every row's 54 values loaded from L1 with its own bounds
+// tests 512^2 x 64 took 1.36 ms, with the halo read anew for each tile 0.74, now
+// 0.40 ms (0.19 for the bytes).
+template <int ZT>
 __global__ void __launch_bounds__(CONV_THREADS) k_conv_first(FirstTile t, int Y, int X, int Z, const float *__restrict__ fa,
                                                              const float *__restrict__ fb, float scale,
                                                              const __nv_bfloat16 *__restrict__ w64,
@@ -393,7 +414,7 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv_first(FirstTile t, int Y,
   extern __shared__ __align__(128) uint8_t sm[];
   uint8_t *sA = sm;                 // [8][128][16 B]
   uint8_t *sB = sm + 128 * 64 * 2;  // [8][N][16 B]
-  __shared__ uint32_t halo[FIRST_HALO];
+  __shared__ uint32_t halo[3 * FirstRows<ZT>::NW];
   __shared__ float sbias[256];
   __shared__ uint64_t mbar;
   __shared__ uint32_t tbase;
@@ -413,15 +434,27 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv_first(FirstTile t, int Y,
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tbase;
+  FirstRows<ZT> f;
   uint32_t ph = 0;
+  int s0 = 0;  // slot of the tile's first halo row
+  const int i0 = (int)((long long)t.ntiles * blockIdx.x / gridDim.x), i1 = (int)((long long)t.ntiles * (blockIdx.x + 1) / gridDim.x);
+  int y = i0 % Y, col = i0 / Y;
   bool ok = true;
-  for (int i = blockIdx.x; i < t.ntiles && ok; i += gridDim.x, ph ^= 1u) {
-    const FirstPos p = first_pos(t, Y, i);
-    first_halo(t, p, Y, X, Z, fa, fb, scale, halo);
+  for (int i = i0; i < i1 && ok; i++, ph ^= 1u) {
+    if (i == i0 || y == 0) {
+      f.column(t, col, Y, X, Z, fa, fb);
+      s0 = 0;
+      for (int r = 0; r < 3; r++) {
+        f.fetch(y + r - 1);
+        f.put(halo + r * f.NW, scale);
+      }
+    } else {
+      f.put(halo + (s0 == 0 ? 2 : s0 - 1) * f.NW, scale);
+    }
     __syncthreads();
     {
       __align__(16) uint32_t row[32];
-      first_row(t, halo, row);
+      f.build(halo, s0, row);
 #pragma unroll
       for (int c = 0; c < 8; c++)
         *reinterpret_cast<int4 *>(sA + c * (128 * 16) + tid * 16) = *reinterpret_cast<const int4 *>(row + 4 * c);
@@ -438,20 +471,25 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv_first(FirstTile t, int Y,
                  ks > 0 ? 1u : 0u);
       mma_commit(&mbar);
     }
+    if (y + 1 < Y) f.fetch(y + 2);
     ok = wait_stage(&mbar, ph, err);
     tc_fence_after();
     if (ok) {
-      const int x = p.x0 + tid / t.zt, z = p.z0 + tid % t.zt;
-      const size_t v0 = (((size_t)p.b * Y + p.y) * X + x) * Z + z;
+      const size_t v0 = ((size_t)(col / t.nzt / t.nxt) * Y + y) * f.XZ + (size_t)f.x * Z + f.z;
       for (int n0 = 0; n0 < N; n0 += 16) {
         float v[16];
         tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)n0, v);
         __align__(16) __nv_bfloat16 h[16];
 #pragma unroll
         for (int q = 0; q < 16; q++) h[q] = __float2bfloat16_rn(fmaxf(v[q] + sbias[n0 + q], 0.f));
-        if (x < X) store32(out + v0 * N + n0, *reinterpret_cast<const int4 *>(h), *reinterpret_cast<const int4 *>(h + 8));
+        if (f.x < X) store32(out + v0 * N + n0, *reinterpret_cast<const int4 *>(h), *reinterpret_cast<const int4 *>(h + 8));
         __syncwarp();
       }
+    }
+    s0 = s0 == 2 ? 0 : s0 + 1;
+    if (++y == Y) {
+      y = 0;
+      col++;
     }
   }
   tc_fence_before();
@@ -468,14 +506,15 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv_first(FirstTile t, int Y,
 // MMA's upper 64 rows read other voxels and are discarded), 64-byte rows of
 // dout, swizzled like TMA would.  The accumulator stays in TMEM over a CTA's
 // tiles.  As a gather over the packed 8-channel input it took 437 us for 8 x 32 x
-// 128 x 32 voxels, now 119 us.
+// 128 x 32 voxels, with the halo read anew for each tile 119, now 102.
+template <int ZT>
 __global__ void __launch_bounds__(CONV_THREADS) k_wgrad_first(FirstTile t, int Y, int X, int Z, const float *__restrict__ fa,
                                                               const float *__restrict__ fb, float scale,
                                                               const __nv_bfloat16 *__restrict__ dout, float *dw, int *err) {
   extern __shared__ __align__(1024) uint8_t sm_raw[];
   uint8_t *sA = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);  // [128][128 B]
   uint8_t *sB = sA + 128 * 128;                                           // [128][64 B]
-  __shared__ uint32_t halo[FIRST_HALO];
+  __shared__ uint32_t halo[3 * FirstRows<ZT>::NW];
   __shared__ uint64_t mbar;
   __shared__ uint32_t tbase;
   const int tid = threadIdx.x, warp = tid >> 5;
@@ -488,20 +527,37 @@ __global__ void __launch_bounds__(CONV_THREADS) k_wgrad_first(FirstTile t, int Y
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tbase;
+  FirstRows<ZT> f;
   uint32_t ph = 0;
+  int s0 = 0;
+  const int i0 = (int)((long long)t.ntiles * blockIdx.x / gridDim.x), i1 = (int)((long long)t.ntiles * (blockIdx.x + 1) / gridDim.x);
+  int y = i0 % Y, col = i0 / Y;
   bool ok = true, any = false;
-  for (int i = blockIdx.x; i < t.ntiles; i += gridDim.x) {
-    const FirstPos p = first_pos(t, Y, i);
-    first_halo(t, p, Y, X, Z, fa, fb, scale, halo);  // (the tile before has built its rows)
-    const int x = p.x0 + tid / t.zt, z = p.z0 + tid % t.zt;
-    const size_t v = (((size_t)p.b * Y + p.y) * X + x) * Z + z;
+  for (int i = i0; i < i1; i++) {
+    if (i == i0 || y == 0) {
+      f.column(t, col, Y, X, Z, fa, fb);
+      s0 = 0;
+      for (int r = 0; r < 3; r++) {
+        f.fetch(y + r - 1);
+        f.put(halo + r * f.NW, scale);
+      }
+    } else {
+      f.put(halo + (s0 == 0 ? 2 : s0 - 1) * f.NW, scale);
+    }
+    const size_t v = ((size_t)(col / t.nzt / t.nxt) * Y + y) * f.XZ + (size_t)f.x * Z + f.z;
     int4 g[4];
 #pragma unroll
     for (int u = 0; u < 4; u++)
-      g[u] = x < X ? __ldg(reinterpret_cast<const int4 *>(dout + v * 32) + u) : make_int4(0, 0, 0, 0);
+      g[u] = f.x < X ? __ldg(reinterpret_cast<const int4 *>(dout + v * 32) + u) : make_int4(0, 0, 0, 0);
     __syncthreads();
     __align__(16) uint32_t row[32];
-    first_row(t, halo, row);
+    f.build(halo, s0, row);
+    if (y + 1 < Y) f.fetch(y + 2);
+    s0 = s0 == 2 ? 0 : s0 + 1;
+    if (++y == Y) {
+      y = 0;
+      col++;
+    }
     if (any) {  // the tile before has been multiplied
       ok = wait_stage(&mbar, ph, err);
       if (!ok) break;
@@ -629,25 +685,28 @@ cudaError_t conv_first_pack(int n, int cin, int kpad, const __nv_bfloat16 *w, __
 cudaError_t conv_first(int nb, int Y, int X, int Z, const float *a, const float *b, float scale,
                        const __nv_bfloat16 *w64, const float *bias, int n, __nv_bfloat16 *out, int *err,
                        cudaStream_t st) {
-  if (n % 16 || n < 16 || n > 256 || (long long)nb * Y * X * Z / 8 >= (1ll << 31)) return cudaErrorInvalidValue;
+  if (n % 16 || n < 16 || n > 256 || Z % 8 || (long long)nb * Y * X * Z / 8 >= (1ll << 31))
+    return cudaErrorInvalidValue;
   const FirstTile t = first_tile(nb, Y, X, Z);
   size_t smem = (size_t)128 * 64 * 2 + (size_t)n * 64 * 2;
   // no more CTAs on an SM than its 512 TMEM columns hold
   const size_t fit = 512 / tmem_cols(n), floor_bytes = 228 * 1024 / (fit + 1) + 1024;
   if (smem < floor_bytes) smem = floor_bytes;
-  cudaError_t e =
-      cudaFuncSetAttribute((const void *)k_conv_first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const auto k = t.zt == 32 ? k_conv_first<32> : t.zt == 16 ? k_conv_first<16> : k_conv_first<8>;
+  cudaError_t e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const unsigned grid = (unsigned)std::min(t.ntiles, 148 * 8);
-  k_conv_first<<<grid, CONV_THREADS, smem, st>>>(t, Y, X, Z, a, b, scale, w64, bias, n, out, err);
+  k<<<grid, CONV_THREADS, smem, st>>>(t, Y, X, Z, a, b, scale, w64, bias, n, out, err);
   return cudaGetLastError();
 }
 
 cudaError_t wgrad_first(int nb, int Y, int X, int Z, const float *a, const float *b, float scale,
                         const __nv_bfloat16 *dout, float *dw, int *err, cudaStream_t st) {
   const FirstTile t = first_tile(nb, Y, X, Z);
+  if (Z % 8) return cudaErrorInvalidValue;
   const size_t smem = 1024 + 128 * 128 + 128 * 64;
-  k_wgrad_first<<<(unsigned)std::min(t.ntiles, 148 * 6), CONV_THREADS, smem, st>>>(t, Y, X, Z, a, b, scale, dout, dw, err);
+  const auto k = t.zt == 32 ? k_wgrad_first<32> : t.zt == 16 ? k_wgrad_first<16> : k_wgrad_first<8>;
+  k<<<(unsigned)std::min(t.ntiles, 148 * 6), CONV_THREADS, smem, st>>>(t, Y, X, Z, a, b, scale, dout, dw, err);
   return cudaGetLastError();
 }
 
