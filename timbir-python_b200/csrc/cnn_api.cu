@@ -89,8 +89,9 @@ int xtc_conv3d_path(const void *in, const void *w, const float *bias, void *out,
       if ((e = cudaMalloc(&wp, need)) != cudaSuccess) return fail(e, "xtc_conv3d");
       wp_bytes = need;
     }
-    e = tile ? xtc::conv_tile_pack(cin, cout, kpad, sign, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)wp, 0)
-             : xtc::conv_box_pack(cin, cout, kpad, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)wp, 0);
+    const xtc::PackJob job{tile ? xtc::PACK_TILE : xtc::PACK_BOX, cin, cout, kpad, sign, (const __nv_bfloat16 *)w,
+                           (__nv_bfloat16 *)wp};
+    e = xtc::pack_kernel_weights(&job, 1, 0);
     if (e == cudaSuccess && box)
       e = xtc::conv_forward_box(s, (const __nv_bfloat16 *)in, (const __nv_bfloat16 *)wp, bias, out, epi, sign, g_err, 0);
     else if (e == cudaSuccess)

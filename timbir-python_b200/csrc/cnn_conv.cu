@@ -608,15 +608,6 @@ __global__ void __launch_bounds__(CONV_THREADS) k_wgrad_first(FirstTile t, int Y
   }
 }
 
-// [n][kpad] with k = tap * cin + ci (ci < 2 real) -> [n][64] with k = 2 tap + ci
-__global__ void k_pack_first(int n, int cin, int kpad, const __nv_bfloat16 *__restrict__ w,
-                             __nv_bfloat16 *__restrict__ w64) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n * 64) return;
-  const int nn = i / 64, k = i % 64;
-  w64[i] = k < 54 ? w[(size_t)nn * kpad + (k / 2) * cin + (k % 2)] : __float2bfloat16_rn(0.f);
-}
-
 // Dynamic shared memory per CTA: the two operand stages, raised where needed
 // so that no more CTAs fit on an SM (228 KB) than its 512 TMEM columns hold.
 static size_t conv_smem(int n) {
@@ -675,12 +666,6 @@ cudaError_t conv_wgrad(const ConvShape &s, const __nv_bfloat16 *in, const __nv_b
 }  // namespace xtc
 
 namespace xtc {
-
-cudaError_t conv_first_pack(int n, int cin, int kpad, const __nv_bfloat16 *w, __nv_bfloat16 *w64, cudaStream_t st) {
-  if (cin < 2) return cudaErrorInvalidValue;
-  k_pack_first<<<(n * 64 + 255) / 256, 256, 0, st>>>(n, cin, kpad, w, w64);
-  return cudaGetLastError();
-}
 
 cudaError_t conv_first(int nb, int Y, int X, int Z, const float *a, const float *b, float scale,
                        const __nv_bfloat16 *w64, const float *bias, int n, __nv_bfloat16 *out, int *err,

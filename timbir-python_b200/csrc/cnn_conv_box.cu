@@ -101,15 +101,6 @@ __device__ __forceinline__ void halo_origin(const Halo &H, int t, int &z0, int &
   b = t / H.Y;
 }
 
-// channels per TMA row
-int box_ch(int cin) { return (cin + 63) / 64 * 64 <= (cin + 31) / 32 * 32 ? 64 : 32; }
-
-// 16-byte unit u of row r in the swizzle of CH-channel rows (as TMA writes it)
-template <int CH>
-__host__ __device__ constexpr int swz(int r, int u) {
-  return CH == 64 ? u ^ (r & 7) : u ^ ((r >> 1) & 3);
-}
-
 // K-major operand: rows of CH channels, 8-row groups CH * 16 bytes apart
 template <int CH>
 __device__ __forceinline__ uint64_t desc_k(uint32_t saddr) {
@@ -324,21 +315,6 @@ __global__ void __launch_bounds__(192) k_conv_box(const __grid_constant__ CUtens
   if (warp == 0) {
     tc_fence_after();
     tmem_free(tmem, cols);
-  }
-}
-
-// K-major W[n][kpad] (k = tap * cin + ci) -> rows of CH channels per (tap,
-// chunk, n), 16-byte units swizzled, zero past cin
-template <int CH>
-__global__ void k_pack_box_w(int cin, int n, int kpad, const __nv_bfloat16 *__restrict__ w, __nv_bfloat16 *__restrict__ wp) {
-  const int nchunk = (cin + CH - 1) / CH;
-  const long long total = 27ll * nchunk * n * CH;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int e = (int)(i % 8), u = (int)(i / 8 % (CH / 8));
-    const long long row = i / CH;  // (tap * nchunk + c) * n + nn
-    const int nn = (int)(row % n), tc = (int)(row / n), c = tc % nchunk, t = tc / nchunk;
-    const int ci = c * CH + swz<CH>(nn, u) * 8 + e;
-    wp[i] = ci < cin ? w[(size_t)nn * kpad + (size_t)t * cin + ci] : __float2bfloat16_rn(0.f);
   }
 }
 
@@ -928,15 +904,6 @@ bool conv_box_supported(const ConvShape &s) {
 size_t conv_box_wp_elems(int cin, int n) {
   const int ch = box_ch(cin);
   return (size_t)27 * ((cin + ch - 1) / ch) * n * ch;
-}
-
-cudaError_t conv_box_pack(int cin, int n, int kpad, const __nv_bfloat16 *w, __nv_bfloat16 *wp, cudaStream_t st) {
-  const unsigned grid = (unsigned)std::min<size_t>((conv_box_wp_elems(cin, n) + 255) / 256, 4096);
-  if (box_ch(cin) == 64)
-    k_pack_box_w<64><<<grid, 256, 0, st>>>(cin, n, kpad, w, wp);
-  else
-    k_pack_box_w<32><<<grid, 256, 0, st>>>(cin, n, kpad, w, wp);
-  return cudaGetLastError();
 }
 
 cudaError_t conv_forward_box(const ConvShape &s, const __nv_bfloat16 *in, const __nv_bfloat16 *wp, const float *bias,

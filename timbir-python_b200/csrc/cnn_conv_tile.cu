@@ -360,32 +360,6 @@ __global__ void __launch_bounds__(288, 1)
   }
 }
 
-// K-major W[n][kpad] (k = tap * cin + ci, tap = (dy+1)*9 + (dx+1)*3 + (dz+1))
-// -> Wp[chunk][(ey+1)*3 + (ex+1)][half][dzi][n][8], ci = 16 chunk + 8 half + e,
-// effective offsets (ey, ex, ez = 1 - dzi) = sign x (dy, dx, dz)
-__global__ void k_pack_tile_w(int cin, int n, int kpad, int sign, const __nv_bfloat16 *__restrict__ w,
-                              __nv_bfloat16 *__restrict__ wp) {
-  const long long total = (long long)((cin + 15) / 16) * 27 * 2 * n * 8;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    long long r = i;
-    const int e = (int)(r % 8);
-    r /= 8;
-    const int nn = (int)(r % n);
-    r /= n;
-    const int dzi = (int)(r % 3);
-    r /= 3;
-    const int h = (int)(r % 2);
-    r /= 2;
-    const int g = (int)(r % 9);
-    const int c = (int)(r / 9);
-    const int ci = 16 * c + 8 * h + e;
-    const int dy = sign * (g / 3 - 1), dx = sign * (g % 3 - 1), dz = sign * (1 - dzi);
-    const int t = (dy + 1) * 9 + (dx + 1) * 3 + (dz + 1);
-    wp[i] = ci < cin ? w[(size_t)nn * kpad + (size_t)t * cin + ci] : __float2bfloat16_rn(0.f);
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Weight gradient on staged tiles (cout = 32, cin a multiple of 16, X a
 // multiple of 128, Z even):
@@ -628,14 +602,6 @@ bool conv_tile_supported(const ConvShape &s) {
 }
 
 size_t conv_tile_wp_elems(int cin, int n) { return (size_t)((cin + 15) / 16) * 27 * 2 * n * 8; }
-
-cudaError_t conv_tile_pack(int cin, int n, int kpad, int sign, const __nv_bfloat16 *w, __nv_bfloat16 *wp,
-                           cudaStream_t st) {
-  const long long total = (long long)conv_tile_wp_elems(cin, n);
-  const unsigned grid = (unsigned)std::min<long long>((total + 255) / 256, 4096);
-  k_pack_tile_w<<<grid, 256, 0, st>>>(cin, n, kpad, sign, w, wp);
-  return cudaGetLastError();
-}
 
 cudaError_t conv_forward_tile(const ConvShape &s, const __nv_bfloat16 *in, const __nv_bfloat16 *wp, const float *bias,
                               void *out, int epi, int sign, int *err, cudaStream_t st, const __nv_bfloat16 *up, int ca) {

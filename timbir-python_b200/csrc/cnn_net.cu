@@ -107,16 +107,20 @@ double gauss(uint64_t &s) {  // Box-Muller
 }
 
 int pack_all(xtc_net *n) {
+  xtc::PackLayer layers[kLayers];
+  xtc::PackJob jobs[4 * kLayers + 1];
+  int nj = 0;
   for (int i = 0; i < kLayers; i++) {
     Layer &l = n->L[i];
-    xtc::pack_weights(l.cin_real, l.cin, l.cout, l.kpad, l.kpad_t, n->P + l.off_w, l.W, i ? l.Wt : nullptr, n->st);
-    if (l.Wp) NCK(xtc::conv_tile_pack(l.cin, l.cout, l.kpad, 1, l.W, l.Wp, n->st));
-    if (l.Wtp) NCK(xtc::conv_tile_pack(l.cout, l.cin, l.kpad_t, -1, l.Wt, l.Wtp, n->st));
-    if (l.Wb) NCK(xtc::conv_box_pack(l.cin, l.cout, l.kpad, l.W, l.Wb, n->st));
-    if (l.Wtb) NCK(xtc::conv_box_pack(l.cout, l.cin, l.kpad_t, l.Wt, l.Wtb, n->st));
-    if (l.W64) NCK(xtc::conv_first_pack(l.cout, l.cin, l.kpad, l.W, l.W64, n->st));
+    layers[i] = {l.cin_real, l.cin, l.cout, l.kpad, l.kpad_t, n->P + l.off_w, l.W, i ? l.Wt : nullptr};
+    if (l.Wp) jobs[nj++] = {xtc::PACK_TILE, l.cin, l.cout, l.kpad, 1, l.W, l.Wp};
+    if (l.Wtp) jobs[nj++] = {xtc::PACK_TILE, l.cout, l.cin, l.kpad_t, -1, l.Wt, l.Wtp};
+    if (l.Wb) jobs[nj++] = {xtc::PACK_BOX, l.cin, l.cout, l.kpad, 1, l.W, l.Wb};
+    if (l.Wtb) jobs[nj++] = {xtc::PACK_BOX, l.cout, l.cin, l.kpad_t, 1, l.Wt, l.Wtb};
+    if (l.W64) jobs[nj++] = {xtc::PACK_FIRST, l.cin, l.cout, l.kpad, 1, l.W, l.W64};
   }
-  NCK(cudaGetLastError());
+  xtc::pack_weights(layers, kLayers, n->st);
+  NCK(xtc::pack_kernel_weights(jobs, nj, n->st));
   n->packed = true;
   return 0;
 }

@@ -16,7 +16,6 @@ struct ConvShape {
 cudaError_t conv_forward(const ConvShape &s, const __nv_bfloat16 *in, const __nv_bfloat16 *w, const float *bias,
                          void *out, int epi, int sign, int *err, cudaStream_t st);
 // the first layer (2 FP32 input channels, the input packing fused in): w64 [n][64], k = 2 tap + channel
-cudaError_t conv_first_pack(int n, int cin, int kpad, const __nv_bfloat16 *w, __nv_bfloat16 *w64, cudaStream_t st);
 cudaError_t conv_first(int nb, int Y, int X, int Z, const float *a, const float *b, float scale,
                        const __nv_bfloat16 *w64, const float *bias, int n, __nv_bfloat16 *out, int *err,
                        cudaStream_t st);
@@ -24,22 +23,19 @@ cudaError_t conv_first(int nb, int Y, int X, int Z, const float *a, const float 
 cudaError_t wgrad_first(int nb, int Y, int X, int Z, const float *a, const float *b, float scale,
                         const __nv_bfloat16 *dout, float *dw, int *err, cudaStream_t st);
 // the staged tile kernel (cnn_conv_tile.cu): X a multiple of 128, Z even,
-// n <= 64; weights pre-packed by conv_tile_pack into conv_tile_wp_elems values
+// n <= 64; weights pre-packed (PACK_TILE) into conv_tile_wp_elems values
 bool conv_tile_supported(const ConvShape &s);
 size_t conv_tile_wp_elems(int cin, int n);
-cudaError_t conv_tile_pack(int cin, int n, int kpad, int sign, const __nv_bfloat16 *w, __nv_bfloat16 *wp,
-                           cudaStream_t st);
 // with `up`, channels [0, ca) are the 2x nearest upsampling of that coarse
 // volume (ca channels) and `in` holds the other cin - ca (epi 0)
 cudaError_t conv_forward_tile(const ConvShape &s, const __nv_bfloat16 *in, const __nv_bfloat16 *wp, const float *bias,
                               void *out, int epi, int sign, int *err, cudaStream_t st, const __nv_bfloat16 *up = nullptr,
                               int ca = 0);
 // TMA boxes of 128 voxels per tap (cnn_conv_box.cu): any volume, cin and n
-// multiples of 16; weights pre-packed by conv_box_pack into
+// multiples of 16; weights pre-packed (PACK_BOX) into
 // conv_box_wp_elems values (the sign stays an argument)
 bool conv_box_supported(const ConvShape &s);
 size_t conv_box_wp_elems(int cin, int n);
-cudaError_t conv_box_pack(int cin, int n, int kpad, const __nv_bfloat16 *w, __nv_bfloat16 *wp, cudaStream_t st);
 cudaError_t conv_forward_box(const ConvShape &s, const __nv_bfloat16 *in, const __nv_bfloat16 *wp, const float *bias,
                              void *out, int epi, int sign, int *err, cudaStream_t st);
 bool wgrad_box_supported(const ConvShape &s);
@@ -69,8 +65,25 @@ void head(long long nv, int C, const __nv_bfloat16 *h, const float *w, const flo
           float *y, cudaStream_t st);
 void head_train(long long nv, const __nv_bfloat16 *h, const float *w, const float *bias, const float *base, float scale,
                 const float *target, double *loss, float *dh, float *dw, float *db, cudaStream_t st);
-void pack_weights(int cin_real, int cin, int cout, int kpad, int kpad_t, const float *P, __nv_bfloat16 *W,
-                  __nv_bfloat16 *Wt, cudaStream_t st);
+// master weights of a layer -> its K-major BF16 rows, and the transposed ones (wt may be null)
+struct PackLayer {
+  int cin_real, cin, cout, kpad, kpad_t;
+  const float *p;
+  __nv_bfloat16 *w, *wt;
+};
+void pack_weights(const PackLayer *layers, int count, cudaStream_t st);  // 16 layers at most
+// K-major rows w[n][kpad] -> the order a kernel reads: the tile kernel's (with
+// the taps' sign), the box and halo kernels', or the first layer's [n][64]
+enum PackKind { PACK_TILE, PACK_BOX, PACK_FIRST };
+struct PackJob {
+  int kind, cin, n, kpad, sign;
+  const __nv_bfloat16 *w;
+  __nv_bfloat16 *wp;
+};
+cudaError_t pack_kernel_weights(const PackJob *jobs, int count, cudaStream_t st);  // 64 jobs at most
+// channels per TMA row of the box kernels, and where 16-byte unit u of such a row r lies in its swizzle
+__host__ __device__ constexpr int box_ch(int cin) { return (cin + 63) / 64 * 64 <= (cin + 31) / 32 * 32 ? 64 : 32; }
+__host__ __device__ constexpr int box_swizzle(int ch, int r, int u) { return ch == 64 ? u ^ (r & 7) : u ^ ((r >> 1) & 3); }
 void adam(long long n, float *p, const float *g, float *m, float *v, float lr, float b1, float b2, float eps, int t,
           cudaStream_t st);
 void crop(int np, const float *const *src, const int4 *org, int Y, int X, int Z, int py, int px, int pz, float *dst,
