@@ -28,3 +28,22 @@ def test_concatenation_in_place(shape):
     assert torch.max(torch.abs(out.cpu() - ry)) <= 2e-2 * float(corr.max() - corr.min())
     assert loss == pytest.approx(rloss, rel=2e-2)
     net.close()
+
+
+def test_head_beside_and_inside_the_last_convolution():
+    """The fused head needs 16-byte aligned volumes; a volume that is not gets the
+    separate head, with the same sums in the same order."""
+    shape = (1, 8, 128, 24)
+    net = xtg.WarmNet(seed=3)
+    net.set_params(random_params(net, 4))
+    fbp, icd, _ = volumes(shape, 9)
+    n = fbp.numel()
+    outs = []
+    for off_out, off_icd in ((0, 0), (1, 0), (0, 3)):
+        out = torch.empty(n + 8, device="cuda")[off_out:off_out + n]
+        base = torch.empty(n + 8, device="cuda")[off_icd:off_icd + n]
+        base.copy_(icd.reshape(-1))
+        net.forward(fbp.cuda(), base, out, shape)
+        outs.append(out.cpu())
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    net.close()

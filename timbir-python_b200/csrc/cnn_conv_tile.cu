@@ -71,7 +71,8 @@ __device__ __forceinline__ uint64_t sdesc_sw32(uint32_t saddr) {
 // a stage's weights: nine taps of 16 channels
 __host__ __device__ constexpr uint32_t b_stage_bytes(int n) { return 9u * (uint32_t)n * 32u; }
 
-constexpr int TILE_LOADERS = 128;  // threads of warps 5-8
+constexpr int TILE_LOADERS = 128;  // threads of warps 5-8 (eight warps: no faster over a whole pass)
+constexpr int TILE_THREADS = 160 + TILE_LOADERS;
 constexpr int TILE_STAGES = 6;     // at most; as many as shared memory holds
 constexpr int TILE_AHEAD = 2;      // stages a loader has in flight before it waits for the oldest
 
@@ -79,8 +80,8 @@ constexpr int TILE_AHEAD = 2;      // stages a loader has in flight before it wa
 // A stage is one (16-channel chunk, dy): the staged y-row y + dy and its nine
 // taps' weights.  Warps 5-8 copy it in with 16-byte asynchronous copies (a row
 // is two of them; zero filled outside the volume), several stages ahead, and
-// publish it to the tensor core's proxy once it has landed; warp 4 (one
-// thread) issues the MMAs; the accumulators alternate between two TMEM
+// publish it to the tensor core's proxy once it has landed; warp 4 issues the
+// MMAs; the accumulators alternate between two TMEM
 // buffers, so warps 0-3 (TMEM lanes 32w .. 32w + 31) drain tile i while tile
 // i + 1 is computed.
 //
@@ -96,16 +97,20 @@ constexpr int TILE_AHEAD = 2;      // stages a loader has in flight before it wa
 // level and 1.02 ms in all; read in place the 80 -> 32 convolution takes the
 // same time.
 //
+// EPI 3 (inference's last layer): the 1x1 head on the rounded outputs, added in
+// the order of k_head, in place of storing them (k_head took 0.21 ms at 512^2 x 64,
+// the stores it read about as much).
+//
 // With the MMAs issued from a warp-uniform loop and whole sectors stored 32 -> 32
 // takes 1.23 ms (1.27 before), 80 -> 32 2.55 (2.86), 48 -> 48 at half the
 // resolution 0.36 (0.41).  Alone the copies, the MMAs (about 65 cycles each, near
 // what reading A's 4 KB from shared memory takes) and the epilogue need 0.9, 0.85
 // and 0.6 ms of the 1.23.
 template <int EPI, int TZ, bool CAT>
-__global__ void __launch_bounds__(288, 1)
+__global__ void __launch_bounds__(TILE_THREADS, 1)
     k_conv_tile(const __nv_bfloat16 *__restrict__ in, const __nv_bfloat16 *__restrict__ up, int ca, ConvShape s,
                 const __nv_bfloat16 *__restrict__ wp,
-                const float *__restrict__ bias, void *out, int nstage, int *err) {
+                const float *__restrict__ bias, void *out, TileHead hd, int nstage, int *err) {
   using D = TileDims<TZ>;
   constexpr int TZS = D::TZS;
   extern __shared__ __align__(1024) uint8_t sm[];
@@ -114,6 +119,7 @@ __global__ void __launch_bounds__(288, 1)
   __shared__ uint64_t full[TILE_STAGES], empty[TILE_STAGES], acc_full[2], acc_empty[2], done;
   __shared__ uint32_t tbase;
   __shared__ volatile int bad;
+  __shared__ __align__(16) float sbias[64], shead[64];
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int nchunk = (s.cin + 15) >> 4;
   const int XT = s.X / TX, ZT = s.Z / TZ;
@@ -134,6 +140,8 @@ __global__ void __launch_bounds__(288, 1)
     mbar_init_fence();
     bad = 0;
   }
+  if ((EPI == 0 || EPI == 3) && tid < N) sbias[tid] = bias[tid];
+  if (EPI == 3 && tid < N) shead[tid] = hd.w[tid];
   if (warp == 0) tmem_alloc(&tbase, acc_cols);
   tc_fence_before();
   __syncthreads();
@@ -321,8 +329,12 @@ __global__ void __launch_bounds__(288, 1)
       tc_fence_after();
       int x0, z0, y, b;
       tile_of(tl, x0, z0, y, b);
+      const size_t vox0 = (((size_t)b * s.Y + y) * s.X + x0 + warp * 32 + lane) * s.Z + z0;
+      __align__(16) float yv[TZ];  // EPI 3: the head's outputs
+#pragma unroll
       for (int zo = 0; zo < TZ; zo++) {
-        const size_t vox = (((size_t)b * s.Y + y) * s.X + x0 + warp * 32 + lane) * s.Z + z0 + zo;
+        const size_t vox = vox0 + zo;
+        float acc = EPI == 3 ? hd.b[0] : 0.f;
         for (int n0 = 0; n0 < N; n0 += 16) {
           __align__(16) float v[16];
           tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((ab * TZ + zo) * N + n0), v);
@@ -335,13 +347,24 @@ __global__ void __launch_bounds__(288, 1)
 #pragma unroll
             for (int q = 0; q < 16; q++) {
               float t = v[q];
-              if (EPI == 0) t = fmaxf(t + bias[n0 + q], 0.f);
+              if (EPI != 1) t = fmaxf(t + sbias[n0 + q], 0.f);
               h[q] = __float2bfloat16_rn(t);
             }
-            __nv_bfloat16 *o = reinterpret_cast<__nv_bfloat16 *>(out) + vox * N + n0;
-            store32(o, *reinterpret_cast<const int4 *>(h), *reinterpret_cast<const int4 *>(h + 8));
+            if (EPI == 3) {
+#pragma unroll
+              for (int q = 0; q < 16; q++) acc += __bfloat162float(h[q]) * shead[n0 + q];
+            } else {
+              __nv_bfloat16 *o = reinterpret_cast<__nv_bfloat16 *>(out) + vox * N + n0;
+              store32(o, *reinterpret_cast<const int4 *>(h), *reinterpret_cast<const int4 *>(h + 8));
+            }
           }
         }
+        if (EPI == 3) yv[zo] = acc / hd.scale;
+      }
+      if (EPI == 3) {  // (TZ 4)
+        float *o = reinterpret_cast<float *>(out) + vox0;
+        const float4 p = *reinterpret_cast<const float4 *>(hd.base + vox0);
+        *reinterpret_cast<float4 *>(o) = make_float4(p.x + yv[0], p.y + yv[1], p.z + yv[TZ - 2], p.w + yv[TZ - 1]);
       }
       // the buffer starts the CTA's next tile at zero
       for (int col = 0; col < TZ * N; col += 16)
@@ -604,20 +627,25 @@ bool conv_tile_supported(const ConvShape &s) {
 size_t conv_tile_wp_elems(int cin, int n) { return (size_t)((cin + 15) / 16) * 27 * 2 * n * 8; }
 
 cudaError_t conv_forward_tile(const ConvShape &s, const __nv_bfloat16 *in, const __nv_bfloat16 *wp, const float *bias,
-                              void *out, int epi, int sign, int *err, cudaStream_t st, const __nv_bfloat16 *up, int ca) {
-  if (!conv_tile_supported(s) || (epi == 0 && !bias) || epi < 0 || epi > 2 || (sign != 1 && sign != -1) ||
+                              void *out, int epi, int sign, int *err, cudaStream_t st, const __nv_bfloat16 *up, int ca,
+                              const TileHead &hd) {
+  if (!conv_tile_supported(s) || (epi % 3 == 0 && !bias) || epi < 0 || epi > 3 || (sign != 1 && sign != -1) ||
       (reinterpret_cast<uintptr_t>(in) & 15))
     return cudaErrorNotSupported;
   if (up && (epi != 0 || ca < 16 || ca % 16 || s.cin <= ca || s.cin % 16 || s.Y % 2 || s.X % 2 || s.Z % 2 ||
              (reinterpret_cast<uintptr_t>(up) & 15)))
     return cudaErrorNotSupported;
+  if (epi == 3 && (up || !hd.w || tile_tz(s) != 4 || ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(hd.base)) & 15)))
+    return cudaErrorNotSupported;
   const int tz = tile_tz(s);
   typedef void (*K)(const __nv_bfloat16 *, const __nv_bfloat16 *, int, ConvShape, const __nv_bfloat16 *, const float *,
-                    void *, int, int *);
+                    void *, TileHead, int, int *);
   K k;
   // the sign lives in the packed weights
   if (up)
     k = tz == 4 ? k_conv_tile<0, 4, true> : k_conv_tile<0, 2, true>;
+  else if (epi == 3)
+    k = k_conv_tile<3, 4, false>;
   else if (tz == 4)
     k = epi == 0 ? k_conv_tile<0, 4, false> : epi == 1 ? k_conv_tile<1, 4, false> : k_conv_tile<2, 4, false>;
   else
@@ -636,7 +664,7 @@ cudaError_t conv_forward_tile(const ConvShape &s, const __nv_bfloat16 *in, const
   }
   const long long ntiles = (long long)(s.X / TX) * (s.Z / tz) * s.nb * s.Y;
   const unsigned grid = (unsigned)std::min<long long>(ntiles, sms);  // one CTA per SM (shared memory)
-  k<<<grid, 288, smem, st>>>(in, up, ca, s, wp, bias, out, nstage, err);
+  k<<<grid, TILE_THREADS, smem, st>>>(in, up, ca, s, wp, bias, out, hd, nstage, err);
   return cudaGetLastError();
 }
 

@@ -142,10 +142,10 @@ int ensure_buffers(xtc_net *n, int nb, int Y, int X, int Z, bool training) {
   if (n->nb == nb && n->Y == Y && n->X == X && n->Z == Z && (n->grads || !training)) return 0;
   const size_t v0 = (size_t)nb * Y * X * Z, v1 = v0 / 8, v2 = v1 / 8, v3 = v2 / 8;
   const size_t lv[kLayers] = {v0, v0, v1, v1, v2, v2, v3, v3, v2, v2, v1, v1, v0, v0};
-  NCK(n->in0.ensure(v0 * 8 * sizeof(bf16)));
+  if (training) NCK(n->in0.ensure(v0 * 8 * sizeof(bf16)));
   size_t gmax = 0;
   for (int i = 0; i < kLayers; i++) {
-    NCK(n->a[i].ensure(lv[i] * n->L[i].cout * sizeof(bf16)));
+    if (i < 13 || training) NCK(n->a[i].ensure(lv[i] * n->L[i].cout * sizeof(bf16)));  // (forward: where it is stored)
     if (i != 8 && i != 10 && i != 12) gmax = std::max(gmax, lv[i] * (size_t)n->L[i].cin);  // (those go to gcat)
     gmax = std::max(gmax, lv[i] * (size_t)n->L[i].cout);
   }
@@ -217,7 +217,7 @@ int forward(xtc_net *n, const float *fbp, const float *icd, float *out, const fl
   bf16 *A[kLayers];
   for (int i = 0; i < kLayers; i++) A[i] = n->a[i].as<bf16>();
   int rc;
-  if (target) {  // training keeps the packed input for the first layer's weight gradient
+  if (target) {  // training's first layer sums over the packed input, in the general kernels' order
     xtc::pack_input(v0, fbp, icd, kScale, n->in0.as<bf16>(), st);
     if ((rc = conv(n, 0, n->in0.as<bf16>(), 0, A[0]))) return rc;
   } else {
@@ -240,6 +240,22 @@ int forward(xtc_net *n, const float *fbp, const float *icd, float *out, const fl
   if ((rc = conv_cat(n, 10, A[9], 64, A[3], 48, 1, n->u1, A[10], keep))) return rc;
   if ((rc = conv(n, 11, A[10], 1, A[11]))) return rc;
   if ((rc = conv_cat(n, 12, A[11], 48, A[1], 32, 0, n->u0, A[12], keep))) return rc;
+  if (!target) {
+    // the last layer and the head in one kernel where the tile kernel takes the shape
+    const Layer &l = n->L[13];
+    const xtc::ConvShape s{nb, Y, X, Z, l.cin, l.cout, l.kpad};
+    if (l.Wp && xtc::conv_tile_supported(s)) {
+      const cudaError_t e = xtc::conv_forward_tile(s, A[12], l.Wp, n->P + l.off_b, out, 3, 1, n->d_err, st, nullptr, 0,
+                                                   {n->P + n->off_hw, n->P + n->off_hb, icd, kScale});
+      if (e != cudaErrorNotSupported) {
+        NCK(e);
+        return 0;
+      }
+      cudaGetLastError();
+    }
+    NCK(n->a[13].ensure((size_t)v0 * l.cout * sizeof(bf16)));
+    A[13] = n->a[13].as<bf16>();
+  }
   if ((rc = conv(n, 13, A[12], 0, A[13]))) return rc;
   if (target) {
     NCK(cudaMemsetAsync(n->d_loss, 0, sizeof(double), st));

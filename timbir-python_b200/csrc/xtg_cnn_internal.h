@@ -26,11 +26,16 @@ cudaError_t wgrad_first(int nb, int Y, int X, int Z, const float *a, const float
 // n <= 64; weights pre-packed (PACK_TILE) into conv_tile_wp_elems values
 bool conv_tile_supported(const ConvShape &s);
 size_t conv_tile_wp_elems(int cin, int n);
+// (epi 3: the output head on relu(acc + bias) in BF16, out = base + (h . w + b) / scale in FP32)
+struct TileHead {
+  const float *w = nullptr, *b = nullptr, *base = nullptr;
+  float scale = 1.f;
+};
 // with `up`, channels [0, ca) are the 2x nearest upsampling of that coarse
 // volume (ca channels) and `in` holds the other cin - ca (epi 0)
 cudaError_t conv_forward_tile(const ConvShape &s, const __nv_bfloat16 *in, const __nv_bfloat16 *wp, const float *bias,
                               void *out, int epi, int sign, int *err, cudaStream_t st, const __nv_bfloat16 *up = nullptr,
-                              int ca = 0);
+                              int ca = 0, const TileHead &hd = TileHead{});
 // TMA boxes of 128 voxels per tap (cnn_conv_box.cu): any volume, cin and n
 // multiples of 16; weights pre-packed (PACK_BOX) into
 // conv_box_wp_elems values (the sign stays an argument)
