@@ -333,45 +333,62 @@ __device__ __forceinline__ void mul_add2(float &s0, float &s1, float x0, float x
 #define CSR_WARPS 8  // consecutive views of a CTA, one per warp
 // resident CTAs the FP32 registers are cut for (3 and 5: 6.8 and 6.7 ms)
 #define CSR_CTAS 4
-template <int MODE, typename ACC, int LT, bool VEC>
+template <int MODE, typename ACC, int LT, int R, bool VEC>
 __global__ void __launch_bounds__(CSR_WARPS * 32, MODE < 2 ? CSR_CTAS : 3) k_fp_csr(DevGeo G, FpArgs F, CsrView T) {
   constexpr int PW = 32 / LT;  // pairs per warp
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % LT;
   const int ov = blockIdx.x * CSR_WARPS + warp, np2 = (G.N_r + 1) / 2, pair = blockIdx.y * PW + lane / LT;
   if (ov >= G.N_p) return;  // whole warp; no block-wide barrier follows
   const int p = T.order[ov];
-  const int t0 = blockIdx.z * (4 * LT) + 4 * sub;  // this lane's first row
-  const int nt = min(4, G.N_t - t0);               // rows it has (may be none)
+  const int t0 = blockIdx.z * (R * LT) + R * sub;  // this lane's first row
+  const int nt = min(R, G.N_t - t0);               // rows it has (may be none)
   const float *xf = F.x + (size_t)F.fov[p] * G.N_y * G.N_x * G.N_z;
   const float *xl = xf + (VEC ? (nt > 0 ? t0 : 0) : 0);
-  int zr[4];
+  int zr[R];
 #pragma unroll
-  for (int c = 0; c < 4; c++) zr[c] = c < nt ? (t0 + c) / G.zovl : 0;
+  for (int c = 0; c < R; c++) zr[c] = c < nt ? (t0 + c) / G.zovl : 0;
   long long i = 0, e1 = 0;
   if (pair < np2) {  // (lanes without rows load records too)
     i = T.ptr[(size_t)p * np2 + pair];
     e1 = T.ptr[(size_t)p * np2 + pair + 1];
   }
-  ACC acc0[4], acc1[4];
+  ACC acc0[R], acc1[R];
 #pragma unroll
-  for (int c = 0; c < 4; c++) acc0[c] = acc1[c] = (ACC)0;
-  auto load = [&](int off) {
-    if (VEC) return __ldg(reinterpret_cast<const float4 *>(xl + off));
-    return make_float4(__ldg(xl + off + zr[0]), __ldg(xl + off + zr[1]), __ldg(xl + off + zr[2]), __ldg(xl + off + zr[3]));
+  for (int c = 0; c < R; c++) acc0[c] = acc1[c] = (ACC)0;
+  struct Rows {
+    float x[R];
   };
-  auto add1 = [&](ACC (&acc)[4], const ACC (&x)[4], float a) {
-    if constexpr (MODE <= 1) {
-      mul_add2(acc[0], acc[1], x[0], x[1], a, F.neg0);
-      mul_add2(acc[2], acc[3], x[2], x[3], a, F.neg0);
+  auto load = [&](int off) {
+    Rows v;
+    if constexpr (VEC) {
+      const float4 q = __ldg(reinterpret_cast<const float4 *>(xl + off));
+      v.x[0] = q.x;
+      v.x[R / 4] = q.y;
+      v.x[R / 2] = q.z;
+      v.x[R - 1] = q.w;
+    } else {
+#pragma unroll
+      for (int c = 0; c < R; c++) v.x[c] = __ldg(xl + off + zr[c]);
+    }
+    return v;
+  };
+  auto add1 = [&](ACC (&acc)[R], const ACC (&x)[R], float a) {
+    if constexpr (MODE <= 1 && R == 1) {
+      acc[0] = __fadd_rn(acc[0], __fmul_rn(x[0], a));
+    } else if constexpr (MODE <= 1) {
+#pragma unroll
+      for (int c = 0; c + 1 < R; c += 2) mul_add2(acc[c], acc[c + 1], x[c], x[c + 1], a, F.neg0);
     } else {
       const uint32_t u = __float_as_uint(a);  // FP64 form of a positive normal: a shift and a bias
       const double ad = __hiloint2double((int)((u >> 3) + 0x38000000u), (int)(u << 29));
 #pragma unroll
-      for (int c = 0; c < 4; c++) acc[c] += x[c] * ad;
+      for (int c = 0; c < R; c++) acc[c] += x[c] * ad;
     }
   };
-  auto add = [&](const float4 v, float a0, float a1) {
-    const ACC x[4] = {(ACC)v.x, (ACC)v.y, (ACC)v.z, (ACC)v.w};
+  auto add = [&](const Rows &v, float a0, float a1) {
+    ACC x[R];
+#pragma unroll
+    for (int c = 0; c < R; c++) x[c] = (ACC)v.x[c];
     if (a0 != 0.f) add1(acc0, x, a0);
     if (a1 != 0.f) add1(acc1, x, a1);
   };
@@ -379,7 +396,7 @@ __global__ void __launch_bounds__(CSR_WARPS * 32, MODE < 2 ? CSR_CTAS : 3) k_fp_
   // run while the sixteen before are added, and read them back from shared
   // memory; z-lines are loaded four records ahead.  (Records past the row's
   // end: A = 0 at column 0.)
-  constexpr int RC = 16, RL = RC / LT;  // records a lane loads
+  constexpr int RC = 16, RL = (RC + LT - 1) / LT;  // records a lane loads
   __shared__ __align__(16) int4 recs[CSR_WARPS][2][PW][RC + 1];
   const int len = (int)(e1 - i), most = __reduce_max_sync(0xffffffffu, len);
   int4 nx[RL];
@@ -387,28 +404,29 @@ __global__ void __launch_bounds__(CSR_WARPS * 32, MODE < 2 ? CSR_CTAS : 3) k_fp_
 #pragma unroll
     for (int m = 0; m < RL; m++) {
       const int r = r0 + sub + m * LT;
-      nx[m] = r < len ? __ldcs(T.ent + i + r) : make_int4(0, 0, 0, 0);
+      nx[m] = r < len && (LT <= RC || sub < RC) ? __ldcs(T.ent + i + r) : make_int4(0, 0, 0, 0);
     }
   };
   fetch(0);
   for (int r0 = 0, buf = 0; r0 < most; r0 += RC, buf ^= 1) {
-    int4 *R = recs[warp][buf][lane / LT];
+    int4 *rec = recs[warp][buf][lane / LT];
 #pragma unroll
-    for (int m = 0; m < RL; m++) R[sub + m * LT] = nx[m];
+    for (int m = 0; m < RL; m++)
+      if (LT <= RC || sub < RC) rec[sub + m * LT] = nx[m];
     __syncwarp();  // (the other buffer was read before the last one's barrier)
     fetch(r0 + RC);
-    float4 v[4];
+    Rows v[4];
 #pragma unroll
-    for (int u = 0; u < 4; u++) v[u] = load(R[u].x);
+    for (int u = 0; u < 4; u++) v[u] = load(rec[u].x);
 #pragma unroll
     for (int g = 0; g < RC; g += 4) {
-      float4 vn[4];
+      Rows vn[4];
 #pragma unroll
       for (int u = 0; u < 4; u++)
-        if (g + 4 < RC) vn[u] = load(R[g + 4 + u].x);
+        if (g + 4 < RC) vn[u] = load(rec[g + 4 + u].x);
 #pragma unroll
       for (int u = 0; u < 4; u++) {
-        add(v[u], __int_as_float(R[g + u].y), __int_as_float(R[g + u].z));
+        add(v[u], __int_as_float(rec[g + u].y), __int_as_float(rec[g + u].z));
       }
 #pragma unroll
       for (int u = 0; u < 4; u++) v[u] = vn[u];
@@ -421,7 +439,7 @@ __global__ void __launch_bounds__(CSR_WARPS * 32, MODE < 2 ? CSR_CTAS : 3) k_fp_
       const int r = 2 * pair + h;
       if (r >= G.N_r) continue;
 #pragma unroll
-      for (int c = 0; c < 4; c++) {
+      for (int c = 0; c < R; c++) {
         if (c >= nt) continue;
         const ACC sacc = h ? acc1[c] : acc0[c];
         const size_t o = ((size_t)p * G.N_r + r) * G.N_t + t0 + c;
@@ -450,16 +468,16 @@ __global__ void __launch_bounds__(CSR_WARPS * 32, MODE < 2 ? CSR_CTAS : 3) k_fp_
   }
 }
 
-template <int LT, bool VEC>
+template <int LT, int R, bool VEC>
 static void launch_fp_csr_t(const DevGeo &G, const FpArgs &F, const CsrView &T, int mode, cudaStream_t st) {
   const int np2 = (G.N_r + 1) / 2, pw = 32 / LT;
   const dim3 grid((unsigned)((G.N_p + CSR_WARPS - 1) / CSR_WARPS), (unsigned)((np2 + pw - 1) / pw),
-                  (unsigned)((G.N_t + 4 * LT - 1) / (4 * LT)));
+                  (unsigned)((G.N_t + R * LT - 1) / (R * LT)));
   switch (mode) {
-    case 0: k_fp_csr<0, float, LT, VEC><<<grid, CSR_WARPS * 32, 0, st>>>(G, F, T); break;
-    case 1: k_fp_csr<1, float, LT, VEC><<<grid, CSR_WARPS * 32, 0, st>>>(G, F, T); break;
-    case 2: k_fp_csr<2, double, LT, VEC><<<grid, CSR_WARPS * 32, 0, st>>>(G, F, T); break;
-    default: k_fp_csr<3, double, LT, VEC><<<grid, CSR_WARPS * 32, 0, st>>>(G, F, T); break;
+    case 0: k_fp_csr<0, float, LT, R, VEC><<<grid, CSR_WARPS * 32, 0, st>>>(G, F, T); break;
+    case 1: k_fp_csr<1, float, LT, R, VEC><<<grid, CSR_WARPS * 32, 0, st>>>(G, F, T); break;
+    case 2: k_fp_csr<2, double, LT, R, VEC><<<grid, CSR_WARPS * 32, 0, st>>>(G, F, T); break;
+    default: k_fp_csr<3, double, LT, R, VEC><<<grid, CSR_WARPS * 32, 0, st>>>(G, F, T); break;
   }
 }
 
@@ -467,12 +485,31 @@ cudaError_t launch_fp_csr(const DevGeo &G, const FpArgs &F, const CsrView &T, in
   // one 16-byte load for four rows where rows and slices are the same and
   // z-lines keep 16-byte alignment; lanes per pair: as many as the rows fill
   const bool vec = G.zovl == 1 && G.N_z % 4 == 0;
-  if (G.N_t <= 16)
-    vec ? launch_fp_csr_t<4, true>(G, F, T, mode, st) : launch_fp_csr_t<4, false>(G, F, T, mode, st);
-  else if (G.N_t <= 32)
-    vec ? launch_fp_csr_t<8, true>(G, F, T, mode, st) : launch_fp_csr_t<8, false>(G, F, T, mode, st);
-  else
-    vec ? launch_fp_csr_t<16, true>(G, F, T, mode, st) : launch_fp_csr_t<16, false>(G, F, T, mode, st);
+  // Else fewer rows a lane and more lanes a pair, where loads and conversions
+  // row by row are what a warp waits for.  One row up to 16 (FP64 cost, four rows
+  // a lane against one: 100^2 x 5, 128 views 214 -> 118 us; 400^2 x 13, 600 views 3.64
+  // -> 2.09 ms; FP32 FBP start there 3.56 -> 3.18), two in FP64 above that, in
+  // tiles of 64 rows where they leave no more empty than tiles of 32 (256^2 x 31,
+  // 512 views: four rows 1.73 ms, one 1.36, two 1.13; 300^2 x 62, 300 views 2.67, 2.35,
+  // 1.90).  In FP32 four rows stay the faster there (300^2 x 62: 2.84 against 3.12).
+  if (!vec && (mode >= 2 || G.N_t <= 16)) {
+    if (G.N_t <= 4)
+      launch_fp_csr_t<4, 1, false>(G, F, T, mode, st);
+    else if (G.N_t <= 8)
+      launch_fp_csr_t<8, 1, false>(G, F, T, mode, st);
+    else if (G.N_t <= 16)
+      launch_fp_csr_t<16, 1, false>(G, F, T, mode, st);
+    else if ((G.N_t + 63) / 64 * 2 == (G.N_t + 31) / 32)
+      launch_fp_csr_t<32, 2, false>(G, F, T, mode, st);
+    else
+      launch_fp_csr_t<16, 2, false>(G, F, T, mode, st);
+  } else if (G.N_t <= 16) {
+    vec ? launch_fp_csr_t<4, 4, true>(G, F, T, mode, st) : launch_fp_csr_t<4, 4, false>(G, F, T, mode, st);
+  } else if (G.N_t <= 32) {
+    vec ? launch_fp_csr_t<8, 4, true>(G, F, T, mode, st) : launch_fp_csr_t<8, 4, false>(G, F, T, mode, st);
+  } else {
+    vec ? launch_fp_csr_t<16, 4, true>(G, F, T, mode, st) : launch_fp_csr_t<16, 4, false>(G, F, T, mode, st);
+  }
   return cudaGetLastError();
 }
 
