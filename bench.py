@@ -293,8 +293,7 @@ def kernel_timings(args, reps=5):
         "map_cost_fp64": (ctx.cost, 8.0 * ns + 8.0 * entries + 4.0 * nvox, "k_fp_csr<3>, k_prior_cost64"),
         "map_cost_running": (ctx.cost_running, 8.0 * ns + 4.0 * nvox, "k_running_cost64, k_prior_cost64"),
         "zinger_refresh": (lambda: ctx.zinger_refresh(want_mask=False), 8.0 * ns, "k_zinger_refresh"),
-        "nhicd_select": (lambda: ctx.nhicd_select(usn), 4.0 * nmag * 6, "k_vsc_filter, k_rs_hist, k_rs_pick, "
-                                                                         "k_nhicd_compact"),
+        "nhicd_select": (lambda: ctx.nhicd_select(usn), 4.0 * nmag * 6, "k_vsc_filter, k_nhicd_pick"),
     }
     out = {"workload": workload_name(w), "sinogram_entries": ns, "voxels": nvox, "table_entries": entries,
            "peak_gbs": peak, "peak_kind": peak_kind_note(kind), "calls": {}}

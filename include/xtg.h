@@ -99,8 +99,8 @@ int xtg_set_options(xtg_ctx *ctx, int32_t a_mode, int32_t order, int32_t max_col
 /* Forward projector.  Both give the same values (bit-identical in FP32, the
  * reference's summation order; FP64 sums otherwise):
  *   XTG_PROJ_AUTO:   at the first projection the context builds a bin-major
- *                    A table (rows (view, bin), entries in the reference's
- *                    (row, column) order; 8 B per entry) when it fits in free
+ *                    A table (rows (view, two bins), records in the reference's
+ *                    (row, column) order; 16 B each) when it fits in free
  *                    device memory next to the ICD column table and 2 GiB to
  *                    spare, and projects from it; else as XTG_PROJ_GATHER.
  *   XTG_PROJ_GATHER: A evaluated on the fly for each (view, 32 bins), no
