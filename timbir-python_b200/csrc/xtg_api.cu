@@ -68,6 +68,8 @@ struct IterBlock {
 #define ITER_CLEAR offsetof(IterBlock, err)
 // parallel ICD: at most 1 in XTG_CONC_DIV of the columns updated at once
 #define XTG_CONC_DIV 32
+// short items of a launch per CTA in flight
+#define XTG_CONC_ITEMS 8
 // ICD footprint loads keep w in L2 (like e) when e and w together take at
 // most XTG_W_KEEP_BYTES; larger sinograms evict w first
 #ifndef XTG_W_KEEP
@@ -2005,6 +2007,17 @@ static int run_columns(xtg_ctx *c, int iter, const int4 *items, int lo, int n, c
     // items of this launch; a selection keeps about one column in
     // XT_NHICD_CHUNKS, half of them in each half-pass
     const long long nexp = (n_dev ? (long long)g.N_time * g.nzb * (c->n_masked / XT_NHICD_CHUNKS) / 2 : n) * (long long)nsub;
+    // ... and no more than 1024 threads an SM's worth of CTAs cut for the item
+    // length, one in XTG_CONC_ITEMS of a launch's short items: more of them in
+    // flight were faster still but moved an iteration's update percentage
+    // (136^2 x 56, 115 views +1.4 %; 140^2 x 32, 4 frames of 70 views +3.6 %; runs
+    // differ by 0.1-0.2 %).
+    const int unit = vec == 4 && amode && zmax * g.zovl <= 16 ? 64 : vec == 4 && amode && vcap <= 1024 ? 128 : 256;
+    cols = std::min(cols, c->sm_count * (1024 / unit));
+    // (items of few rows, or of long runs, bear twice as many: 128^2 x 4 1.43 -> 1.17
+    // ms, half-lines of 256^2 x 32 with 512 views 9.4 -> 8.7 ms a step, no shift)
+    const int per = unit == 64 && (zmax * g.zovl <= 8 || vcap > 1024) ? XTG_CONC_ITEMS / 2 : XTG_CONC_ITEMS;
+    if (unit < 256) cols = std::min(cols, (int)std::max((nexp + per - 1) / per, 1ll));
     if (!n_dev) cols = std::min(cols, (int)std::max(nexp, 1ll));
     nt = icd_threads(vec, amode, 0, zmax, g.zovl, vcap, cols, c->sm_count);
     grid = std::min(cols, c->sm_count * icd_occupancy(vec, amode, 0, as, vcap, zmax, g.zovl, nt));
