@@ -2019,8 +2019,8 @@ static int run_columns(xtg_ctx *c, int iter, const int4 *items, int lo, int n, c
     const int per = unit == 64 && (zmax * g.zovl <= 8 || vcap > 1024) ? XTG_CONC_ITEMS / 2 : XTG_CONC_ITEMS;
     if (unit < 256) cols = std::min(cols, (int)std::max((nexp + per - 1) / per, 1ll));
     if (!n_dev) cols = std::min(cols, (int)std::max(nexp, 1ll));
-    nt = icd_threads(vec, amode, 0, zmax, g.zovl, vcap, cols, c->sm_count);
-    grid = std::min(cols, c->sm_count * icd_occupancy(vec, amode, 0, as, vcap, zmax, g.zovl, nt));
+    nt = icd_threads(vec, amode, 0, as, zmax, g.zovl, vcap, cols, c->sm_count);
+    grid = std::min(cols, c->sm_count * std::max(1, icd_occupancy(vec, amode, 0, as, vcap, zmax, g.zovl, nt)));
     // a batch per atomic only where every CTA gets several of them: eight at a
     // time left 205 of 512 CTAs with all of a 128^2 x 4 launch's items (69 us
     // a launch against 38)

@@ -784,17 +784,21 @@ cudaError_t launch_magmap_zero(const DevGeo &G, const IcdArgs &A, int grid, cuda
 }
 
 // Threads per CTA for items of zmax slices, at most `cols` of them in flight
-// on `sms` SMs.  Table modes, parallel schedule; otherwise XTG_THREADS.
-int icd_threads(int vec, int amode, int seq, int zmax, int zovl, int vmax, int cols, int sms) {
+// on `sms` SMs.  Table modes, parallel schedule; otherwise XTG_THREADS.  A larger
+// CTA keeps more partial sums beside the column run (2 rows a warp), so sizes
+// past what an SM's shared memory holds are not taken.
+int icd_threads(int vec, int amode, int seq, int as, int zmax, int zovl, int vmax, int cols, int sms) {
   if (amode == 0 || seq) return XTG_THREADS;
   int tlp = 1;
   while (tlp * vec < zmax * zovl) tlp *= 2;
   const long long groups = (long long)tlp * vmax;
+  auto fits = [&](int n) { return icd_occupancy(vec, amode, 0, as, vmax, zmax, zovl, n) > 0; };
   int nt = XTG_NT_MIN;
   // long items
-  while (nt < XTG_THREADS && groups > (long long)nt * XTG_GROUPS_LONG) nt *= 2;
+  while (nt < XTG_THREADS && groups > (long long)nt * XTG_GROUPS_LONG && fits(2 * nt)) nt *= 2;
   // too few columns in flight to fill the SMs' 1024 threads each
-  while (nt < XTG_NT_MAX && (long long)cols * nt * 4 < (long long)sms * 1024 * XTG_FILL4 && groups > (long long)nt * XTG_GROUPS_PER_THREAD)
+  while (nt < XTG_NT_MAX && (long long)cols * nt * 4 < (long long)sms * 1024 * XTG_FILL4 &&
+         groups > (long long)nt * XTG_GROUPS_PER_THREAD && fits(2 * nt))
     nt *= 2;
   return nt;
 }
@@ -811,6 +815,7 @@ cudaError_t launch_icd(const DevGeo &G, const IcdArgs &A, int vec, int amode, in
   return cudaGetLastError();
 }
 
+// CTAs of nt threads on an SM; 0 where one alone does not fit
 int icd_occupancy(int vec, int amode, int seq, int as, int vmax, int zmax, int zovl, int nt) {
   const size_t smem = icd_smem_bytes(vmax, zmax, zovl, as, amode, vec, nt);
   IcdKernel k = icd_kernel(vec, amode, seq, as, nt);
@@ -823,16 +828,18 @@ int icd_occupancy(int vec, int amode, int seq, int as, int vmax, int zmax, int z
   static std::mutex mu;
   static std::vector<Entry> seen;
   int dev = 0, nb = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   std::lock_guard<std::mutex> lk(mu);
   for (const Entry &q : seen)
     if (q.fn == (const void *)k && q.smem == smem && q.dev == dev) return q.nb;
   if (full_smem((const void *)k) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void *)k, nt, smem) != cudaSuccess)
-    return 1;
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void *)k, nt, smem) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
   if (seen.size() >= 1024) seen.clear();
-  seen.push_back(Entry{(const void *)k, smem, dev, nb > 0 ? nb : 1});
-  return seen.back().nb;
+  seen.push_back(Entry{(const void *)k, smem, dev, nb});
+  return nb;
 }
 
 // Once per kernel and device: as much dynamic shared memory as the device
