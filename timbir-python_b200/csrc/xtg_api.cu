@@ -66,10 +66,6 @@ struct IterBlock {
   int err;                          // not cleared with the rest
 };
 #define ITER_CLEAR offsetof(IterBlock, err)
-// parallel ICD: at most 1 in XTG_CONC_DIV of the columns updated at once
-#define XTG_CONC_DIV 32
-// short items of a launch per CTA in flight
-#define XTG_CONC_ITEMS 8
 // ICD footprint loads keep w in L2 (like e) when e and w together take at
 // most XTG_W_KEEP_BYTES; larger sinograms evict w first
 #ifndef XTG_W_KEEP
@@ -1990,41 +1986,18 @@ static int run_columns(xtg_ctx *c, int iter, const int4 *items, int lo, int n, c
     CK(launch_magmap_zero(c->G, A, c->sm_count * 4, c->st));
     c->launches++;
   }
-  int grid, nt = XTG_THREADS;
+  int grid = 1, nt = XTG_THREADS;
   A.grab = 1;
-  if (seq) {
-    grid = 1;
-  } else {
-    // Columns updated at the same time read each other's stale error
-    // sinogram; near neighbours share most of their footprint, so too many
-    // of them at once overshoot (Jacobi-like) and the cost stops falling.
-    // At most 1 in XTG_CONC_DIV of the grid's columns is in flight: on a
-    // 32^2-column grid 64 and more at once left the cost oscillating 20-50 %
-    // above the converged value, 32 did not; grids of 256^2 columns and up
-    // keep every resident CTA busy.
-    int cols = std::max(8, (int)(((long long)g.N_time * c->n_masked) / XTG_CONC_DIV));
-    if (c->max_columns > 0) cols = std::min(cols, c->max_columns);
+  if (!seq) {
+    const IcdFlight fl = icd_flight(vec, amode, as, vcap, zmax, g.zovl, (long long)g.N_time * c->n_masked, c->sm_count);
     // items of this launch; a selection keeps about one column in
     // XT_NHICD_CHUNKS, half of them in each half-pass
     const long long nexp = (n_dev ? (long long)g.N_time * g.nzb * (c->n_masked / XT_NHICD_CHUNKS) / 2 : n) * (long long)nsub;
-    // ... and no more than 1024 threads an SM's worth of CTAs cut for the item
-    // length, one in XTG_CONC_ITEMS of a launch's short items: more of them in
-    // flight were faster still but moved an iteration's update percentage
-    // (136^2 x 56, 115 views +1.4 %; 140^2 x 32, 4 frames of 70 views +3.6 %; runs
-    // differ by 0.1-0.2 %).
-    const int unit = vec == 4 && amode && zmax * g.zovl <= 16 ? 64 : vec == 4 && amode && vcap <= 1024 ? 128 : 256;
-    cols = std::min(cols, c->sm_count * (1024 / unit));
-    // (items of few rows, or of long runs, bear twice as many: 128^2 x 4 1.43 -> 1.17
-    // ms, half-lines of 256^2 x 32 with 512 views 9.4 -> 8.7 ms a step, no shift)
-    const int per = unit == 64 && (zmax * g.zovl <= 8 || vcap > 1024) ? XTG_CONC_ITEMS / 2 : XTG_CONC_ITEMS;
-    if (unit < 256) cols = std::min(cols, (int)std::max((nexp + per - 1) / per, 1ll));
-    if (!n_dev) cols = std::min(cols, (int)std::max(nexp, 1ll));
-    nt = icd_threads(vec, amode, 0, as, zmax, g.zovl, vcap, cols, c->sm_count);
-    grid = std::min(cols, c->sm_count * std::max(1, icd_occupancy(vec, amode, 0, as, vcap, zmax, g.zovl, nt)));
-    // a batch per atomic only where every CTA gets several of them: eight at a
-    // time left 205 of 512 CTAs with all of a 128^2 x 4 launch's items (69 us
-    // a launch against 38)
-    if (nt < XTG_THREADS) A.grab = (int)std::max(1ll, std::min(8ll, nexp / (4ll * grid)));
+    A.grab = fl.batch;
+    grid = fl.cols;
+    if (c->max_columns > 0) grid = std::min(grid, c->max_columns);
+    if (!n_dev) grid = std::min(grid, (int)std::max(nexp, 1ll));
+    nt = icd_threads(vec, amode, as, zmax, g.zovl, vcap, (int)std::min<long long>(grid, (nexp + fl.batch - 1) / fl.batch), c->sm_count);
   }
   if (slot < 0) CK(cudaMemsetAsync(A.counter, 0, 4, c->st));  // an iteration clears its launches' counters together
   CK(launch_icd(c->G, A, vec, amode, seq, as, vcap, zmax, grid, nt, c->st));

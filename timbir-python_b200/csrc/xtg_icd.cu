@@ -28,6 +28,7 @@
 // (Source_Code_4D_Fast/XT_VoxUpdate.c:11-254), CE_FunctionalSubstitution
 // (XT_ICD_update.c:130-179); the z-line batching follows updateVoxels_AttTomo
 // (XT_VoxUpdate.c:266-586).
+#include <algorithm>
 #include <mutex>
 #include <utility>
 #include <vector>
@@ -40,20 +41,11 @@ namespace xtg {
 // footprint entry) are dealt to the CTA's threads, so small items want small
 // CTAs (the fixed work of an item -- neighbourhood, A staging, barriers, the
 // surrogate step -- then overlaps over more items at once) and long items, or
-// few columns in flight, want large ones.  icd_threads picks the size per
-// launch from these three, all measured:
-// XTG_GROUPS_LONG: row groups per thread above which an item counts as long.
-// 24 / 48 / 96: 256^2 x 32, 512 views, a scan step 12.6 / 11.6 / 11.3 ms (17.8
-// with 64 threads for every item of at most 16 rows); 108^2 x 85 x 8 frames
-// 9.8 / 8.5 / 8.5 ms; 260^2 x 4, 602 views 6.75 / 6.75 / 6.94 ms.
-#define XTG_GROUPS_LONG 48
-// XTG_GROUPS_PER_THREAD: below it a larger CTA no longer helps to fill the
-// SMs.  2 / 4 / 8: 128^2 x 4, 180 views 3.15 / 2.69 / 2.61 ms an iteration.
+// few columns in flight, want large ones.  icd_threads takes the largest size
+// that keeps the columns in flight resident, down to
+// XTG_GROUPS_PER_THREAD row groups a thread, below which a larger CTA no
+// longer helps to fill the SMs.
 #define XTG_GROUPS_PER_THREAD 8
-// XTG_FILL4: quarters of the SMs' threads that the columns in flight must
-// leave idle before larger CTAs are taken.  2 / 3 / 4: the 128^2 x 16 coarse
-// stage of a 256^2 x 32 start 166 / 166 / 180 ms (319 with 64 threads).
-#define XTG_FILL4 3
 #define XTG_NT_MIN 64
 #define XTG_NT_MAX 1024
 
@@ -783,22 +775,60 @@ cudaError_t launch_magmap_zero(const DevGeo &G, const IcdArgs &A, int grid, cuda
   return cudaGetLastError();
 }
 
-// Threads per CTA for items of zmax slices, at most `cols` of them in flight
-// on `sms` SMs.  Table modes, parallel schedule; otherwise XTG_THREADS.  A larger
-// CTA keeps more partial sums beside the column run (2 rows a warp), so sizes
-// past what an SM's shared memory holds are not taken.
-int icd_threads(int vec, int amode, int seq, int as, int zmax, int zovl, int vmax, int cols, int sms) {
-  if (amode == 0 || seq) return XTG_THREADS;
+// Columns in flight: CTAs of a launch, and the items each takes at a time.
+//
+// Columns updated at the same time read each other's stale error sinogram, so
+// how many there are, and in which groups, is part of an iteration's result.
+// Near neighbours share most of their footprint: too many of them at once
+// overshoot (Jacobi-like) and the cost stops falling -- on a 32^2-column grid 64
+// and more at once left the cost oscillating 20-50 % above the converged value,
+// 32 did not.  The schedule that sets the iterations' course is one column in
+// 32, no more than are resident in CTAs of 64 threads for items of at most 16
+// rows, 128 for runs of at most 1024 entries, 256 otherwise, the first two eight
+// items at a time (so an eighth of a launch's items are in flight).  Items that
+// spend less of their time outside [first read of e, last write of e] are staler
+// at the same number: with it this kernel moves an iteration's update percentage
+// by up to 3.3 times what runs differ by, with twice as many by 5 to 9 times
+// (64^2 x 8, 4 frames of 48 views, iteration 8: 0.168 -> 0.173 %).  Hence, where
+// the fixed work weighs (shift in units of the run-to-run spread, which is 0.05 to
+// 0.3 % of the percentage, without -> with):
+//   one column in 33 for single-row and long items read from a table (128^2 x 9
+//     +1.0 -> +0.8), one in 36 for short ones
+//   an eighth fewer than are resident for short items with runs of at most 512
+//     entries (256^2 x 16 x 16 frames +1.7 -> +0.7), and for the others where that is
+//     more than one column in 256 (180^2 x 27 +2.1 -> +0.6)
+//   for such runs ten items at a time in the 128-thread class and nine in the
+//     64-thread one above 1536 rows x entries (140^2 x 32, 4 frames +2.6 -> +0.4;
+//     96^2 x 32, 8 frames +3.3 -> +0.4; 96^2 x 16, 4 frames +1.4 -> 0.0)
+// 114 volumes of 64^2 to 512^2, 3 to 80 rows, 1 to 16 frames lie between -1.5 and
+// +1.8 with it (one of 8 frames with A computed here +2.7), half of them within
+// 0.4.  It costs time: 80^2 x 8, 500 views 1.4 ms an iteration with twice the
+// columns, 2.5 so; 256^2 x 32, 512 views 7.7 and 10.0; 128^2 x 4 1.1 and 1.4.
+IcdFlight icd_flight(int vec, int amode, int as, int vmax, int zmax, int zovl, long long columns, int sms) {
+  const int rows = zmax * zovl;
+  const int unit = vec != 4 || amode == 0 ? XTG_THREADS : rows <= 16 ? 64 : vmax <= 1024 ? 128 : XTG_THREADS;
+  // shared memory of such a CTA: run, 128 partial sums twice a warp, neighbourhood
+  const size_t smem = (size_t)vmax * (amode == 0 ? 8 + 4 * as : 8) + (size_t)unit * 32 + (size_t)rows * 8 + (size_t)zmax * 48 + 1280;
+  long long resident = (long long)sms * std::max(1, std::min(1024 / unit, (int)(228 * 1024 / smem)));
+  if (amode && (unit < XTG_THREADS ? vmax <= 512 : resident * 256 > columns)) resident -= resident / 8;
+  IcdFlight f;
+  f.cols = (int)std::min(resident, std::max(8ll, columns / (amode == 0 ? 32 : unit == XTG_THREADS ? 33 : 36)));
+  f.batch = unit == XTG_THREADS ? 1 : vmax > 512 ? 8 : unit == 128 ? 10 : rows * vmax > 1536 ? 9 : 8;
+  return f;
+}
+
+// Threads per CTA for items of zmax slices, `cols` of them in flight on `sms`
+// SMs.  Table modes, parallel schedule; otherwise XTG_THREADS.  A larger CTA
+// keeps more partial sums beside the column run (2 rows a warp), so sizes past
+// what an SM's shared memory holds are not taken either.
+int icd_threads(int vec, int amode, int as, int zmax, int zovl, int vmax, int cols, int sms) {
+  if (amode == 0) return XTG_THREADS;
   int tlp = 1;
   while (tlp * vec < zmax * zovl) tlp *= 2;
   const long long groups = (long long)tlp * vmax;
-  auto fits = [&](int n) { return icd_occupancy(vec, amode, 0, as, vmax, zmax, zovl, n) > 0; };
   int nt = XTG_NT_MIN;
-  // long items
-  while (nt < XTG_THREADS && groups > (long long)nt * XTG_GROUPS_LONG && fits(2 * nt)) nt *= 2;
-  // too few columns in flight to fill the SMs' 1024 threads each
-  while (nt < XTG_NT_MAX && (long long)cols * nt * 4 < (long long)sms * 1024 * XTG_FILL4 &&
-         groups > (long long)nt * XTG_GROUPS_PER_THREAD && fits(2 * nt))
+  while (nt < XTG_NT_MAX && groups > (long long)nt * XTG_GROUPS_PER_THREAD &&
+         (long long)sms * icd_occupancy(vec, amode, 0, as, vmax, zmax, zovl, 2 * nt) >= std::max(cols, 1))
     nt *= 2;
   return nt;
 }

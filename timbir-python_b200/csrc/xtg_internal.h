@@ -98,7 +98,11 @@ cudaError_t launch_magmap_zero(const DevGeo &G, const IcdArgs &A, int grid, cuda
 cudaError_t launch_icd(const DevGeo &G, const IcdArgs &A, int vec, int amode, int seq, int as, int vmax, int zmax,
                        int grid, int nt, cudaStream_t st);
 cudaError_t full_smem(const void *fn);
-int icd_threads(int vec, int amode, int seq, int as, int zmax, int zovl, int vmax, int cols, int sms);
+struct IcdFlight {
+  int cols, batch;
+};
+IcdFlight icd_flight(int vec, int amode, int as, int vmax, int zmax, int zovl, long long columns, int sms);
+int icd_threads(int vec, int amode, int as, int zmax, int zovl, int vmax, int cols, int sms);
 int icd_occupancy(int vec, int amode, int seq, int as, int vmax, int zmax, int zovl, int nt);
 
 }  // namespace xtg
