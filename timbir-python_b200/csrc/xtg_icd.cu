@@ -114,13 +114,15 @@ struct ItemMeta {
 // sigma_q times the surrogate coefficient rho'(d) / d of the qGGMRF prior with
 // q = 2 (CE_QGGMRF, XT_ICD_update.c:79-125): with t = |d|^(2-p) / sigma_qp it is
 // (2 - (2-p) t / (c+t)) / (c+t) = (2c + p t) / (c+t)^2, one reciprocal; t comes
-// from the special-function unit's log2 and 2^x (lq = log2 sigma_qp).  The step
-// size only needs a few digits, the fixed point of the iteration is unchanged.
+// from the special-function unit's log2 and 2^x (lq = log2 sigma_qp).  The log2 of a
+// subnormal d, flushed to -inf, is taken as that of the smallest one: with p = 2
+// (e2p = 0) its product would be NaN.  The step size only needs a few digits, the
+// fixed point of the iteration is unchanged.
 __device__ __forceinline__ float qcoef(float d, float c, float lq, float e2p, float p) {
   const float ad = fabsf(d);
   float l, t;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(ad));
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(e2p, l, -lq)));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(e2p, fmaxf(l, -149.f), -lq)));
   t = ad == 0.f ? 0.f : t;
   const float r = __fdividef(1.0f, c + t);
   return fmaf(p, t, 2.0f * c) * r * r;
