@@ -350,6 +350,7 @@ __constant__ float c_vsc[25] = {0.0064f, 0.0432f, 0.0800f, 0.0432f, 0.0064f, 0.0
                                 0.0432f, 0.0800f, 0.5400f, 1.0000f, 0.5400f, 0.0800f, 0.0432f, 0.2916f, 0.5400f,
                                 0.2916f, 0.0432f, 0.0064f, 0.0432f, 0.0800f, 0.0432f, 0.0064f};
 
+// (plain loads: k_nhicd_pick clears entries of the map it has filtered)
 __device__ __forceinline__ float vsc_value(const float *m, int ny, int nx, int j, int k) {
   float f = 0.f;
   if (j >= 2 && j + 2 < ny && k >= 2 && k + 2 < nx) {
@@ -357,7 +358,7 @@ __device__ __forceinline__ float vsc_value(const float *m, int ny, int nx, int j
 #pragma unroll
     for (int p = 0; p < 5; p++)
 #pragma unroll
-      for (int s = 0; s < 5; s++) f = __fadd_rn(f, __fmul_rn(c_vsc[p * 5 + s], __ldg(c + (size_t)p * nx + s)));
+      for (int s = 0; s < 5; s++) f = __fadd_rn(f, __fmul_rn(c_vsc[p * 5 + s], c[(size_t)p * nx + s]));
     return f;
   }
   for (int p = -2; p <= 2; p++)
