@@ -148,6 +148,22 @@ __global__ void __launch_bounds__(256, 2) k_backproject(DevGeo G, const float *_
   const int V = view_num[fr], vs = view_start[fr];
   // vsplit warps share the rows of warp group wg, each every vsplit-th view
   const int wg = warp / vsplit, wv = warp - wg * vsplit;
+  // a tile outside the object-support disk is 0 (512^2 x 64, 1024 views, a whole
+  // start: disk of half the width 12.2 ms, of a quarter 8.7; 13.3 when every tile was
+  // summed)
+  bool used = false;
+  for (int i = tid; i < NS * BP_C; i += 256) {
+    const int j = j0 + i / BP_C, k = k0 + i % BP_C;
+    used = used || (j < G.N_y && k < G.N_x && col_rank[(size_t)j * G.N_x + k] >= 0);
+  }
+  if (!__syncthreads_or(used)) {  // uniform over the CTA
+    const int nz = min(TZ, G.N_z - z0);
+    for (int i = tid; i < NS * BP_C * TZ; i += 256) {
+      const int zz = i % TZ, j = j0 + i / (TZ * BP_C), k = k0 + i / TZ % BP_C;
+      if (zz < nz && j < G.N_y && k < G.N_x) x[(((size_t)fr * G.N_y + j) * G.N_x + k) * G.N_z + z0 + zz] = 0.f;
+    }
+    return;
+  }
   // the lane's own strip and slices
   const int sl = lane / LT, tl = lane % LT;
   // the entries it computes: column lane % 16 of strips 2 m + lane / 16
