@@ -100,9 +100,11 @@ int xtg_set_options(xtg_ctx *ctx, int32_t a_mode, int32_t order, int32_t max_col
  * reference's summation order; FP64 sums otherwise):
  *   XTG_PROJ_AUTO:   at the first projection the context builds a bin-major
  *                    A table (rows (view, two bins), records in the reference's
- *                    (row, column) order; 16 B each) when it fits in free
- *                    device memory next to the ICD column table and 2 GiB to
- *                    spare, and projects from it; else as XTG_PROJ_GATHER.
+ *                    (row, column) order; 12 B each) when 8 B per A entry fit
+ *                    in free device memory next to the ICD column table and
+ *                    2 GiB to spare, and projects from it (where the records,
+ *                    about a tenth larger, do not fit, for as many views as
+ *                    do); else as XTG_PROJ_GATHER.
  *   XTG_PROJ_GATHER: A evaluated on the fly for each (view, 32 bins), no
  *                    table.
  * xtg_get_projector reports XTG_PROJ_TABLE once the table is in use (or

@@ -90,7 +90,7 @@ struct xtg_ctx {
   float *d_hr = nullptr, *d_cos = nullptr, *d_sin = nullptr, *d_ax = nullptr, *d_filt = nullptr, *d_tmp = nullptr;
   float *d_num = nullptr, *d_den = nullptr, *d_thr = nullptr, *d_var = nullptr;
   int *d_view_idx = nullptr, *d_view_start = nullptr, *d_view_num = nullptr, *d_fov = nullptr;
-  int *d_vord = nullptr;  // views by frame, then angle
+  int *d_vord = nullptr;  // device copy of vord
   int *d_mcols = nullptr, *d_rank = nullptr;
   IterBlock *d_it = nullptr, *h_it = nullptr;  // device, pinned host copy
   int phase = 0;  // whose statistics the ICD launches add to
@@ -105,11 +105,14 @@ struct xtg_ctx {
   float *d_tval32 = nullptr, *d_tscale = nullptr;
   __half *d_tval16 = nullptr;
   int table_mode = 0;  // 0 none, XTG_A_FP16 or XTG_A_TABLE32 when built
-  // bin-major A table of the projector (rows (view, bin)); csr_state 0 = not
+  // bin-major A table of the projector (rows (view, two bins)); csr_state 0 = not
   // tried yet, 1 = built, -1 = not used (does not fit, or the gather projector
-  // was requested)
-  long long *d_cptr = nullptr;
-  int4 *d_cent = nullptr;
+  // was requested); csr_views: how many views of `vord` it covers
+  long long *d_cptr = nullptr;  // the allocation: row starts, then A at both bins, then offsets
+  int *d_coff = nullptr;
+  float2 *d_cval = nullptr;
+  std::vector<int> vord;  // views by frame, then angle
+  int csr_views = 0;
   int csr_state = 0, projector = XTG_PROJ_AUTO;
   long long csr_nnz = 0;   // A entries of the table
   size_t csr_bytes = 0;
@@ -847,55 +850,84 @@ static cudaError_t ensure_csr(xtg_ctx *c) {
   if (c->projector == XTG_PROJ_GATHER) return cudaSuccess;
   // entries hold a z-line's element offset within its frame as an int32
   if ((size_t)c->g.N_y * c->g.N_x * c->g.N_z >= ((size_t)1 << 31)) return cudaSuccess;
-  const size_t rows = (size_t)c->g.N_p * ((c->g.N_r + 1) / 2);
-  int *d_cnt = nullptr;  // records per row, then (8-byte aligned) the entry count
+  const size_t nv = (size_t)c->g.N_p, np2 = ((size_t)c->g.N_r + 1) / 2, rows = nv * np2;
+  int *d_cnt = nullptr;  // records per row, then (8-byte aligned) the entries per view
   const size_t ent_at = (rows + 1) / 2 * 2;
-  if (cudaMalloc(&d_cnt, ent_at * 4 + 8) != cudaSuccess) {
+  if (cudaMalloc(&d_cnt, ent_at * 4 + nv * 8) != cudaSuccess) {
     cudaGetLastError();
     return cudaSuccess;
   }
   CsrBuildArgs B;
   memset(&B, 0, sizeof(B));
   B.hr = c->d_hr; B.cosv = c->d_cos; B.sinv = c->d_sin; B.win_margin = fp_win_margin(c); B.count = d_cnt;
+  B.order = c->d_vord; B.nviews = c->g.N_p;
   B.entries = reinterpret_cast<unsigned long long *>(d_cnt + ent_at);
-  cudaError_t e = cudaMemsetAsync(B.entries, 0, 8, c->st);
+  cudaError_t e = cudaMemsetAsync(B.entries, 0, nv * 8, c->st);
   if (e == cudaSuccess) e = launch_csr_build(c->G, B, 0, c->span, c->st);
   std::vector<int> cnt(rows);
-  unsigned long long entries = 0;
+  std::vector<unsigned long long> entries(nv);
   if (e == cudaSuccess) e = cudaMemcpyAsync(cnt.data(), d_cnt, rows * 4, cudaMemcpyDeviceToHost, c->st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&entries, B.entries, 8, cudaMemcpyDeviceToHost, c->st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(entries.data(), B.entries, nv * 8, cudaMemcpyDeviceToHost, c->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
   cudaFree(d_cnt);
   c->launches++;
   if (e != cudaSuccess) return e;
-  std::vector<long long> ptr(rows + 1, 0);
-  for (size_t i = 0; i < rows; i++) ptr[i + 1] = ptr[i] + cnt[i];
-  const long long nrec = ptr[rows];
+  unsigned long long total = 0;
+  for (unsigned long long n : entries) total += n;
   size_t fr = 0, tot = 0;
   if ((e = cudaMemGetInfo(&fr, &tot)) != cudaSuccess) return e;
   // the column table, if one is still to be built, has at most as many entries
-  const size_t pending = (c->a_mode != XTG_A_FP32 && c->table_mode == 0) ? (size_t)entries * 8 : 0;
-  const size_t need = (size_t)nrec * 16 + (rows + 1) * 8;
-  if (need + pending + ((size_t)2 << 30) > fr) return cudaSuccess;
-  if (cudaMalloc(&c->d_cptr, (rows + 1) * 8) != cudaSuccess || cudaMalloc(&c->d_cent, (size_t)nrec * 16 + 16) != cudaSuccess) {
+  const size_t pending = (c->a_mode != XTG_A_FP32 && c->table_mode == 0) ? (size_t)total * 8 : 0;
+  const size_t taken = pending + ((size_t)2 << 30), room = fr > taken ? fr - taken : 0;
+  // Records name two bins (12 bytes, 1.57 of them for 2.14 entries), so a table of
+  // all views takes a tenth more than entries of one bin (8 bytes) did.  Where those
+  // would fit and the records do not, the views that fit in the entries' bytes are
+  // entered, and the others left to k_fp_bins: at 512^2 x 64 no table takes six times
+  // as long as a full one.
+  const size_t single = (size_t)total * 8 + (nv * c->g.N_r + 1) * 8;
+  if (single > room) return cudaSuccess;
+  std::vector<long long> vrec(nv, 0);
+  size_t need = (rows + 4) * 8;
+  for (size_t p = 0; p < nv; p++) {
+    for (size_t i = 0; i < np2; i++) vrec[p] += cnt[p * np2 + i] = (cnt[p * np2 + i] + 3) / 4 * 4;
+    need += (size_t)vrec[p] * 12;
+  }
+  int in = c->g.N_p;
+  if (need > room) {
+    size_t used = (rows + 4) * 8;
+    for (in = 0; in < c->g.N_p && used + (size_t)vrec[c->vord[in]] * 12 <= single; in++) used += (size_t)vrec[c->vord[in]] * 12;
+    if (in == 0) return cudaSuccess;
+    need = used;
+    for (int i = in; i < c->g.N_p; i++) {
+      const size_t p = (size_t)c->vord[i];
+      std::fill(cnt.begin() + p * np2, cnt.begin() + (p + 1) * np2, 0);
+      total -= entries[p];
+    }
+  }
+  std::vector<long long> ptr(rows + 1, 0);
+  for (size_t i = 0; i < rows; i++) ptr[i + 1] = ptr[i] + cnt[i];
+  const size_t head = (rows + 1 + 3) / 4 * 32;  // (records start 32-byte aligned)
+  if (cudaMalloc(&c->d_cptr, head + (size_t)ptr[rows] * 12) != cudaSuccess) {
     cudaGetLastError();
-    cudaFree(c->d_cptr);
-    cudaFree(c->d_cent);
     c->d_cptr = nullptr;
-    c->d_cent = nullptr;
     return cudaSuccess;
   }
-  c->csr_bytes = need + 16;
+  c->d_cval = reinterpret_cast<float2 *>(reinterpret_cast<char *>(c->d_cptr) + head);
+  c->d_coff = reinterpret_cast<int *>(c->d_cval + ptr[rows]);
+  c->csr_bytes = need;
   c->dev_bytes += c->csr_bytes;
   if ((e = cudaMemcpyAsync(c->d_cptr, ptr.data(), (rows + 1) * 8, cudaMemcpyHostToDevice, c->st)) != cudaSuccess)
     return e;
   B.count = nullptr;
+  B.nviews = in;
   B.ptr = c->d_cptr;
-  B.ent = c->d_cent;
+  B.off = c->d_coff;
+  B.val = c->d_cval;
   if ((e = launch_csr_build(c->G, B, 1, c->span, c->st)) != cudaSuccess) return e;
   if ((e = cudaStreamSynchronize(c->st)) != cudaSuccess) return e;
   c->launches++;
-  c->csr_nnz = (long long)entries;
+  c->csr_nnz = (long long)total;
+  c->csr_views = in;
   c->csr_state = 1;
   return cudaSuccess;
 }
@@ -909,13 +941,15 @@ static cudaError_t launch_fp(xtg_ctx *c, float *out, double *slots) {
   F.fov = c->d_fov; F.out = out; F.cost_slots = slots; F.T = c->g.T; F.delta = c->g.delta;
   F.win_margin = fp_win_margin(c);
   F.neg0 = -0.0f;
+  F.order = nullptr;
+  F.nviews = c->g.N_p;
   c->launches++;
   if (c->csr_state == 1) {
-    CsrView T;
-    T.ptr = c->d_cptr;
-    T.ent = c->d_cent;
-    T.order = c->d_vord;
-    return xtg::launch_fp_csr(c->G, F, T, MODE, c->st);
+    const CsrView T{c->d_cptr, c->d_coff, c->d_cval, c->d_vord, c->csr_views};
+    if ((e = xtg::launch_fp_csr(c->G, F, T, MODE, c->st)) != cudaSuccess || c->csr_views == c->g.N_p) return e;
+    F.order = c->d_vord + c->csr_views;
+    F.nviews = c->g.N_p - c->csr_views;
+    c->launches++;
   }
   return xtg::launch_fp(c->G, F, MODE, c->span, c->st);
 }
@@ -932,7 +966,7 @@ void xtg_destroy(xtg_ctx *c) {
                   c->d_filt, c->d_tmp, c->d_num, c->d_den, c->d_thr, c->d_var, c->d_view_idx, c->d_view_start,
                   c->d_view_num, c->d_fov, c->d_vord, c->d_mcols, c->d_rank, c->d_it, c->d_kth,
                   c->d_items, c->d_nh, c->d_red, c->d_cnt, c->d_tstart, c->d_toff, c->d_tval32,
-                  c->d_tscale, c->d_tval16, c->d_cptr, c->d_cent};
+                  c->d_tscale, c->d_tval16, c->d_cptr};
   if (c->dl_pending && c->ev_dl) cudaEventSynchronize(c->ev_dl);
   for (void *p : ptrs)
     if (p) cudaFree(p);
@@ -1063,7 +1097,8 @@ int xtg_create(const xt_params *prm, const double *times, const double *angles, 
   CK(cudaMemcpy(c->d_view_start, c->v.view_start, (size_t)g.N_time * 4, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(c->d_view_num, c->v.view_num, (size_t)g.N_time * 4, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(c->d_fov, c->v.frame_of_view, (size_t)g.N_p * 4, cudaMemcpyHostToDevice));
-  std::vector<int> ord((size_t)g.N_p);
+  std::vector<int> &ord = c->vord;
+  ord.resize((size_t)g.N_p);
   std::iota(ord.begin(), ord.end(), 0);
   std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) {
     if (c->v.frame_of_view[a] != c->v.frame_of_view[b]) return c->v.frame_of_view[a] < c->v.frame_of_view[b];
@@ -1825,10 +1860,8 @@ int xtg_set_projector(xtg_ctx *c, int32_t kind) {
   }
   if (kind != c->projector) {
     cudaFree(c->d_cptr);
-    cudaFree(c->d_cent);
-    if (c->csr_state == 1) c->dev_bytes -= c->csr_bytes;
     c->d_cptr = nullptr;
-    c->d_cent = nullptr;
+    if (c->csr_state == 1) c->dev_bytes -= c->csr_bytes;
     c->csr_state = 0;
     c->csr_nnz = 0;
     c->projector = kind;

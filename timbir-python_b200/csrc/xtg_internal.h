@@ -56,21 +56,29 @@ struct FpArgs {
   float delta;
   double win_margin;
   float neg0;          // -0
+  const int *order;    // the views to project, or null: all
+  int nviews;
 };
 
-// bin-major A table: row (view p, bins 2 i and 2 i + 1) = records [ptr[p np2 + i], ptr[p np2 + i + 1]), np2 = ceil(N_r / 2)
+// bin-major A table: row (view p, bins 2 i and 2 i + 1) = records [ptr[p np2 + i], ptr[p np2 + i + 1]), np2 = ceil(N_r / 2),
+// padded to a multiple of 4 records
 struct CsrBuildArgs {
   const float *hr, *cosv, *sinv;
   double win_margin;
+  const int *order;             // the views to enter
+  int nviews;
   int *count;                   // build pass 0: records per row
-  unsigned long long *entries;  // ... and A entries in all
+  unsigned long long *entries;  // ... and A entries per view
   const long long *ptr;         // build pass 1: row starts
-  int4 *ent;                    // {(j * N_x + k) * N_z, bits of its A at either bin (without delta_t), 0} per record
+  int *off;                     // per record: (j * N_x + k) * N_z
+  float2 *val;                  // ... and its A at either bin (without delta_t)
 };
 struct CsrView {
   const long long *ptr;
-  const int4 *ent;
-  const int *order;  // views by frame, then angle
+  const int *off;
+  const float2 *val;
+  const int *order;  // views by frame, then angle: the first nviews of them have rows
+  int nviews;
 };
 
 struct TableArgs {

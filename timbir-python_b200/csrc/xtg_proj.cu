@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(FP_WARPS * 32) k_fp_bins(DevGeo G, FpArgs F) {
   ACC *acc = reinterpret_cast<ACC *>(fp_sm) + (size_t)warp * 32 * 64;  // [32 bins][64 rows]
   // the A entries of the warp's 32 candidate columns, [lane][NS]
   float *vsm = reinterpret_cast<float *>(fp_sm + (size_t)FP_WARPS * 32 * 64 * sizeof(ACC)) + (size_t)warp * 32 * NS;
-  const int p = blockIdx.x;
+  const int p = F.order ? F.order[blockIdx.x] : (int)blockIdx.x;
   const int rb = (blockIdx.y * FP_WARPS + warp) * 32;
   const int t0 = blockIdx.z * 64, nt = min(64, G.N_t - t0);
   if (rb >= G.N_r) return;  // whole warp; no block-wide barrier follows
@@ -185,7 +185,8 @@ template <int MODE, typename ACC>
 static cudaError_t launch_fp_t(const DevGeo &G, const FpArgs &F, int ns, cudaStream_t st) {
   const int nsv = ns <= 3 ? 3 : ns <= 4 ? 4 : 12;
   const size_t smem = (size_t)FP_WARPS * 32 * 64 * sizeof(ACC) + (size_t)FP_WARPS * 32 * nsv * sizeof(float);
-  dim3 grid((unsigned)G.N_p, (unsigned)((G.N_r + FP_WARPS * 32 - 1) / (FP_WARPS * 32)), (unsigned)((G.N_t + 63) / 64));
+  dim3 grid((unsigned)(F.order ? F.nviews : G.N_p), (unsigned)((G.N_r + FP_WARPS * 32 - 1) / (FP_WARPS * 32)),
+            (unsigned)((G.N_t + 63) / 64));
   typedef void (*K)(DevGeo, FpArgs);
   K k = ns <= 3 ? k_fp_bins<MODE, ACC, 3> : ns <= 4 ? k_fp_bins<MODE, ACC, 4> : k_fp_bins<MODE, ACC, 12>;
   cudaError_t e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -221,7 +222,7 @@ __global__ void __launch_bounds__(FP_WARPS * 32) k_csr_build(DevGeo G, CsrBuildA
   extern __shared__ __align__(16) unsigned char cb_sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float *vsm = reinterpret_cast<float *>(cb_sm) + (size_t)warp * 32 * NS;
-  const int p = blockIdx.x;
+  const int p = B.order[blockIdx.x];
   const int rb = (blockIdx.y * FP_WARPS + warp) * 32;
   if (rb >= G.N_r) return;  // whole warp; no block-wide barrier follows
   const float cp = B.cosv[p], sp = B.sinv[p];
@@ -263,19 +264,26 @@ __global__ void __launch_bounds__(FP_WARPS * 32) k_csr_build(DevGeo G, CsrBuildA
         const float a1 = __shfl_down_sync(0xffffffffu, a, 1);
         ent += a != 0.f;
         if (head && (a != 0.f || a1 != 0.f)) {
-          if (FILL)
-            B.ent[cur++] = make_int4((j * G.N_x + kb + l) * G.N_z, __float_as_int(a), __float_as_int(a1), 0);
-          else
+          if (FILL) {
+            B.off[cur] = (j * G.N_x + kb + l) * G.N_z;
+            B.val[cur++] = make_float2(a, a1);
+          } else {
             cnt++;
+          }
         }
       }
       __syncwarp();  // the staged entries are rewritten by the next round
     }
   }
+  if (FILL && head)
+    for (; cur < B.ptr[row + 1]; cur++) {  // up to a multiple of 4 records: A = 0 at column 0
+      B.off[cur] = 0;
+      B.val[cur] = make_float2(0.f, 0.f);
+    }
   if (!FILL) {
     if (head) B.count[row] = cnt;
     for (int off = 16; off > 0; off >>= 1) ent += __shfl_xor_sync(0xffffffffu, ent, off);
-    if (lane == 0) atomicAdd(B.entries, (unsigned long long)ent);
+    if (lane == 0) atomicAdd(&B.entries[p], (unsigned long long)ent);
   }
 }
 
@@ -283,7 +291,7 @@ template <int FILL>
 static cudaError_t launch_csr_build_t(const DevGeo &G, const CsrBuildArgs &B, int ns, cudaStream_t st) {
   const int nsv = ns <= 3 ? 3 : ns <= 4 ? 4 : 12;
   const size_t smem = (size_t)FP_WARPS * 32 * nsv * sizeof(float);
-  dim3 grid((unsigned)G.N_p, (unsigned)((G.N_r + FP_WARPS * 32 - 1) / (FP_WARPS * 32)));
+  dim3 grid((unsigned)B.nviews, (unsigned)((G.N_r + FP_WARPS * 32 - 1) / (FP_WARPS * 32)));
   if (ns <= 3)
     k_csr_build<FILL, 3><<<grid, FP_WARPS * 32, smem, st>>>(G, B);
   else if (ns <= 4)
@@ -311,7 +319,7 @@ cudaError_t launch_csr_build(const DevGeo &G, const CsrBuildArgs &B, int fill, i
 // FP64 the conversions to it (16 lanes a cycle; A is converted by integer
 // operations instead, being positive and normal).  Per bin, a warp over the 64
 // rows loaded 2.14 z-lines a (column, view), here 1.57; a CTA takes the same
-// bins of CSR_VIEWS views that follow each other in angle (T.order), whose
+// bins of CSR_WARPS views that follow each other in angle (T.order), whose
 // rays cross the same columns at the same time, so most z-lines are L1 hits
 // (eight bins of one view before).  Latency: with records read as they are
 // needed the pairs alone were no faster (9.3 ms).  512^2 x 64, 1024 views: e = y -
@@ -338,7 +346,7 @@ __global__ void __launch_bounds__(CSR_WARPS * 32, MODE < 2 ? CSR_CTAS : 3) k_fp_
   constexpr int PW = 32 / LT;  // pairs per warp
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % LT;
   const int ov = blockIdx.x * CSR_WARPS + warp, np2 = (G.N_r + 1) / 2, pair = blockIdx.y * PW + lane / LT;
-  if (ov >= G.N_p) return;  // whole warp; no block-wide barrier follows
+  if (ov >= T.nviews) return;  // whole warp; no block-wide barrier follows
   const int p = T.order[ov];
   const int t0 = blockIdx.z * (R * LT) + R * sub;  // this lane's first row
   const int nt = min(R, G.N_t - t0);               // rows it has (may be none)
@@ -395,16 +403,37 @@ __global__ void __launch_bounds__(CSR_WARPS * 32, MODE < 2 ? CSR_CTAS : 3) k_fp_
   // Sixteen records of each pair at a time: its lanes load them in one coalesced
   // run while the sixteen before are added, and read them back from shared
   // memory; z-lines are loaded four records ahead.  (Records past the row's
-  // end: A = 0 at column 0.)
+  // end: A = 0 at column 0.)  Offsets and values lie in arrays of their own, 12
+  // bytes a record, a row at a multiple of four records: with four a lane they are
+  // one 16-byte and one 32-byte load (16-byte records {offset, two values, 0} against
+  // that: 256^2 x 16 x 8 frames 0.44 -> 0.41 ms, 512^2 x 8 2.71 -> 2.51, 512^2 x 64 6.33 ->
+  // 6.30; 200^2 x 5 0.227 -> 0.243).
   constexpr int RC = 16, RL = (RC + LT - 1) / LT;  // records a lane loads
   __shared__ __align__(16) int4 recs[CSR_WARPS][2][PW][RC + 1];
   const int len = (int)(e1 - i), most = __reduce_max_sync(0xffffffffu, len);
-  int4 nx[RL];
+  int nxo[RL];
+  float2 nxv[RL];
   auto fetch = [&](int r0) {
+    if constexpr (RL == 4) {  // four in a row
+      const int r = r0 + sub * RL;
+      int4 q = make_int4(0, 0, 0, 0);
+      float2 a = make_float2(0.f, 0.f), b = a, c = a, d = a;
+      if (r < len) {
+        q = __ldcs(reinterpret_cast<const int4 *>(T.off + i + r));
+        asm volatile("ld.global.cs.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=f"(a.x), "=f"(a.y), "=f"(b.x), "=f"(b.y), "=f"(c.x), "=f"(c.y), "=f"(d.x), "=f"(d.y)
+                     : "l"(T.val + i + r));
+      }
+      nxo[0] = q.x; nxo[RL / 4] = q.y; nxo[RL / 2] = q.z; nxo[RL - 1] = q.w;
+      nxv[0] = a; nxv[RL / 4] = b; nxv[RL / 2] = c; nxv[RL - 1] = d;
+    } else {
 #pragma unroll
-    for (int m = 0; m < RL; m++) {
-      const int r = r0 + sub + m * LT;
-      nx[m] = r < len && (LT <= RC || sub < RC) ? __ldcs(T.ent + i + r) : make_int4(0, 0, 0, 0);
+      for (int m = 0; m < RL; m++) {
+        const int r = r0 + sub + m * LT;
+        const bool in = r < len && (LT <= RC || sub < RC);
+        nxo[m] = in ? __ldcs(T.off + i + r) : 0;
+        nxv[m] = in ? __ldcs(T.val + i + r) : make_float2(0.f, 0.f);
+      }
     }
   };
   fetch(0);
@@ -412,7 +441,7 @@ __global__ void __launch_bounds__(CSR_WARPS * 32, MODE < 2 ? CSR_CTAS : 3) k_fp_
     int4 *rec = recs[warp][buf][lane / LT];
 #pragma unroll
     for (int m = 0; m < RL; m++)
-      if (LT <= RC || sub < RC) rec[sub + m * LT] = nx[m];
+      if (LT <= RC || sub < RC) rec[RL == 4 ? sub * RL + m : sub + m * LT] = make_int4(nxo[m], __float_as_int(nxv[m].x), __float_as_int(nxv[m].y), 0);
     __syncwarp();  // (the other buffer was read before the last one's barrier)
     fetch(r0 + RC);
     Rows v[4];
@@ -471,7 +500,7 @@ __global__ void __launch_bounds__(CSR_WARPS * 32, MODE < 2 ? CSR_CTAS : 3) k_fp_
 template <int LT, int R, bool VEC>
 static void launch_fp_csr_t(const DevGeo &G, const FpArgs &F, const CsrView &T, int mode, cudaStream_t st) {
   const int np2 = (G.N_r + 1) / 2, pw = 32 / LT;
-  const dim3 grid((unsigned)((G.N_p + CSR_WARPS - 1) / CSR_WARPS), (unsigned)((np2 + pw - 1) / pw),
+  const dim3 grid((unsigned)((T.nviews + CSR_WARPS - 1) / CSR_WARPS), (unsigned)((np2 + pw - 1) / pw),
                   (unsigned)((G.N_t + R * LT - 1) / (R * LT)));
   switch (mode) {
     case 0: k_fp_csr<0, float, LT, R, VEC><<<grid, CSR_WARPS * 32, 0, st>>>(G, F, T); break;
