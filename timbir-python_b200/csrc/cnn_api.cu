@@ -5,11 +5,20 @@
 #include "../../include/xtg.h"
 #include "../../include/xtg_cnn.h"
 #include "xtg_cnn_internal.h"
+#include "xtg_per_device.h"
 
 void xtg_set_error_text(const char *msg);  // xtg_api.cu
 
 namespace {
-int *g_err = nullptr;  // device flag: a bounded wait in a tensor-core kernel gave up
+struct CudaApi {
+  typedef cudaError_t Error;
+  static constexpr Error ok = cudaSuccess;
+  static Error device(int *d) { return cudaGetDevice(d); }
+  static Error allocate(void **p, size_t n) { return cudaMalloc(p, n); }
+  static void release(void *p) { cudaFree(p); }
+};
+std::mutex g_mu;                        // of the two below
+xtg::PerDevice<CudaApi> g_flags, g_packed;  // error flag; packed weights
 
 int fail(cudaError_t e, const char *what) {
   char b[256];
@@ -18,12 +27,12 @@ int fail(cudaError_t e, const char *what) {
   return XTG_E_CUDA;
 }
 
-int check_err_flag(const char *what) {
+int check_err_flag(const char *what, int *flag) {
   int h = 0;
-  cudaError_t e = cudaMemcpy(&h, g_err, sizeof(int), cudaMemcpyDeviceToHost);
+  cudaError_t e = cudaMemcpy(&h, flag, sizeof(int), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return fail(e, what);
   if (h) {
-    cudaMemset(g_err, 0, sizeof(int));
+    cudaMemset(flag, 0, sizeof(int));
     char b[256];
     snprintf(b, sizeof b, "%s: tensor-core pipeline wait timed out", what);
     xtg_set_error_text(b);
@@ -32,11 +41,14 @@ int check_err_flag(const char *what) {
   return 0;
 }
 
-int ensure_err() {
-  if (g_err) return 0;
-  cudaError_t e = cudaMalloc(&g_err, sizeof(int));
-  if (e != cudaSuccess) return fail(e, "xtc: error flag");
-  e = cudaMemset(g_err, 0, sizeof(int));
+// the current device's flag: a bounded wait in a tensor-core kernel gave up
+int ensure_err(int **flag) {
+  std::lock_guard<std::mutex> lk(g_mu);
+  void *p = nullptr;
+  bool fresh = false;
+  cudaError_t e = g_flags.get(sizeof(int), &p, &fresh);
+  if (e == cudaSuccess && fresh) e = cudaMemset(p, 0, sizeof(int));
+  *flag = static_cast<int *>(p);
   return e == cudaSuccess ? 0 : fail(e, "xtc: error flag");
 }
 }  // namespace
@@ -48,12 +60,13 @@ int xtc_wait_selftest(int32_t arrive, int64_t polls) {
     xtg_set_error_text("xtc_wait_selftest: polls must be positive");
     return XTG_E_ARG;
   }
-  int rc = ensure_err();
+  int *err = nullptr;
+  int rc = ensure_err(&err);
   if (rc) return rc;
-  cudaError_t e = xtc::wait_selftest(arrive != 0, (long long)polls, g_err, 0);
+  cudaError_t e = xtc::wait_selftest(arrive != 0, (long long)polls, err, 0);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return fail(e, "xtc_wait_selftest");
-  return check_err_flag("xtc_wait_selftest");
+  return check_err_flag("xtc_wait_selftest", err);
 }
 
 int xtc_conv3d_path(const void *in, const void *w, const float *bias, void *out, int32_t nb, int32_t Y, int32_t X,
@@ -63,7 +76,8 @@ int xtc_conv3d_path(const void *in, const void *w, const float *bias, void *out,
     xtg_set_error_text("xtc_conv3d: bad argument");
     return XTG_E_ARG;
   }
-  int rc = ensure_err();
+  int *err = nullptr;
+  int rc = ensure_err(&err);
   if (rc) return rc;
   xtc::ConvShape s{nb, Y, X, Z, cin, cout, kpad};
   const bool tile = path != XTC_CONV_GATHER && xtc::conv_tile_supported(s);
@@ -72,42 +86,35 @@ int xtc_conv3d_path(const void *in, const void *w, const float *bias, void *out,
     return XTG_E_ARG;
   }
   const bool box = path == XTC_CONV_AUTO && !tile && kpad % 64 == 0 && kpad >= 27 * cin && xtc::conv_box_supported(s);
-  cudaError_t e;
-  static std::mutex mu;
-  std::unique_lock<std::mutex> lk(mu, std::defer_lock);
+  cudaError_t e = cudaErrorNotSupported;
+  std::unique_lock<std::mutex> lk(g_mu, std::defer_lock);
+  void *wp = nullptr;
   if (tile || box) {
-    // the packed weights, in a buffer kept for later calls: one call at a time
-    // (each ends synchronised)
+    // the packed weights, in a buffer of the device kept for later calls: one call
+    // at a time (each ends synchronised)
     lk.lock();
-    static void *wp = nullptr;
-    static size_t wp_bytes = 0;
-    const size_t need = (tile ? xtc::conv_tile_wp_elems(cin, cout) : xtc::conv_box_wp_elems(cin, cout)) * 2;
-    if (need > wp_bytes) {
-      if (wp) cudaFree(wp);
-      wp = nullptr;
-      wp_bytes = 0;
-      if ((e = cudaMalloc(&wp, need)) != cudaSuccess) return fail(e, "xtc_conv3d");
-      wp_bytes = need;
-    }
+    e = g_packed.get((tile ? xtc::conv_tile_wp_elems(cin, cout) : xtc::conv_box_wp_elems(cin, cout)) * 2, &wp);
+    if (e != cudaSuccess && tile) return fail(e, "xtc_conv3d");
+    if (e != cudaSuccess) e = cudaErrorNotSupported;  // the gather kernel needs none
+  }
+  if (wp) {
     const xtc::PackJob job{tile ? xtc::PACK_TILE : xtc::PACK_BOX, cin, cout, kpad, sign, (const __nv_bfloat16 *)w,
                            (__nv_bfloat16 *)wp};
     e = xtc::pack_kernel_weights(&job, 1, 0);
     if (e == cudaSuccess && box)
-      e = xtc::conv_forward_box(s, (const __nv_bfloat16 *)in, (const __nv_bfloat16 *)wp, bias, out, epi, sign, g_err, 0);
+      e = xtc::conv_forward_box(s, (const __nv_bfloat16 *)in, (const __nv_bfloat16 *)wp, bias, out, epi, sign, err, 0);
     else if (e == cudaSuccess)
       e = xtc::conv_forward_tile(s, (const __nv_bfloat16 *)in, (const __nv_bfloat16 *)wp, bias, out, epi, sign,
-                                 g_err, 0);
-  } else {
-    e = cudaErrorNotSupported;
+                                 err, 0);
   }
   if (e == cudaErrorNotSupported && !tile) {
     cudaGetLastError();
-    e = xtc::conv_forward(s, (const __nv_bfloat16 *)in, (const __nv_bfloat16 *)w, bias, out, epi, sign, g_err, 0);
+    e = xtc::conv_forward(s, (const __nv_bfloat16 *)in, (const __nv_bfloat16 *)w, bias, out, epi, sign, err, 0);
   }
   if (e != cudaSuccess) return fail(e, "xtc_conv3d");
   e = cudaStreamSynchronize(0);
   if (e != cudaSuccess) return fail(e, "xtc_conv3d");
-  return check_err_flag("xtc_conv3d");
+  return check_err_flag("xtc_conv3d", err);
 }
 
 int xtc_conv3d(const void *in, const void *w, const float *bias, void *out, int32_t nb, int32_t Y, int32_t X,
@@ -126,18 +133,19 @@ int xtc_conv3d_wgrad_path(const void *in, const void *dout, float *dw, int32_t n
     xtg_set_error_text("xtc_conv3d_wgrad: bad argument");
     return XTG_E_ARG;
   }
-  int rc = ensure_err();
+  int *err = nullptr;
+  int rc = ensure_err(&err);
   if (rc) return rc;
   xtc::ConvShape s{nb, Y, X, Z, cin, cout, 0};
   if (path == XTC_CONV_TILE && !xtc::wgrad_tile_supported(s)) {
     xtg_set_error_text("xtc_conv3d_wgrad: shape not supported by the tile kernel");
     return XTG_E_ARG;
   }
-  cudaError_t e = xtc::conv_wgrad(s, (const __nv_bfloat16 *)in, (const __nv_bfloat16 *)dout, dw, g_err, 0, path);
+  cudaError_t e = xtc::conv_wgrad(s, (const __nv_bfloat16 *)in, (const __nv_bfloat16 *)dout, dw, err, 0, path);
   if (e != cudaSuccess) return fail(e, "xtc_conv3d_wgrad");
   e = cudaStreamSynchronize(0);
   if (e != cudaSuccess) return fail(e, "xtc_conv3d_wgrad");
-  return check_err_flag("xtc_conv3d_wgrad");
+  return check_err_flag("xtc_conv3d_wgrad", err);
 }
 
 }  // extern "C"
