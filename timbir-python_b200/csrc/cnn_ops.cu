@@ -197,11 +197,6 @@ __global__ void __launch_bounds__(192) k_relu_back(unsigned nv, int C8, const fl
   for (int c = threadIdx.x; c < 8 * C8; c += blockDim.x) atomicAdd(&dbias[c], sb[c]);
 }
 
-// BF16 -> FP32 conversion (input gradients of the convolutions are produced in FP32 directly)
-__global__ void k_to_f32(long long n, const __nv_bfloat16 *a, float *b) {
-  GRID_STRIDE(i, n) b[i] = __bfloat162float(a[i]);
-}
-
 // 1x1 head: y[v] = base[v] + (sum_c h[v][c] w[c] + bias) / scale
 __global__ void k_head(long long nv, int C, const __nv_bfloat16 *h, const float *w, const float *bias,
                        const float *base, float scale, float *y) {
@@ -447,9 +442,6 @@ void relu_back(int nb, int Y, int X, int Z, int C, const float *dpost, int ld, i
   k_relu_back<<<grid, (unsigned)(vpb * c8), C * sizeof(float), st>>>(nv, c8, dpost, ld, off,
                                                                      reinterpret_cast<const int4 *>(post),
                                                                      reinterpret_cast<int4 *>(dpre), dbias, pooled, Y, X, Z);
-}
-void to_f32(long long n, const __nv_bfloat16 *a, float *b, cudaStream_t st) {
-  k_to_f32<<<blocks(n), 256, 0, st>>>(n, a, b);
 }
 void head(long long nv, int C, const __nv_bfloat16 *h, const float *w, const float *bias, const float *base, float scale,
           float *y, cudaStream_t st) {

@@ -56,9 +56,10 @@ void xtg_set_error_text(const char *msg) { snprintf(g_err, sizeof g_err, "%s", m
 // What an iteration's kernels count, in one block: cleared by one memset when
 // the iteration starts and read by one copy when it ends (with the error flag,
 // which outlives it).  The host copy is not page-locked: locking it took 1.4 to 2.6
-// ms of a context's creation and 0.5 of its end, for 7 us an iteration.  Statistics have three phases, since the
-// reference's vox_mag covers the last chunk's random pass alone
-// (XT_ICD_update.c:798): launches before it, it, launches after it.
+// ms of a context's creation and 0.5 of its end, for 7 us an iteration.
+// Statistics have three phases, since the reference's vox_mag covers the last
+// chunk's random pass alone (XT_ICD_update.c:798): launches before it, it, launches
+// after it.
 struct IterBlock {
   double absx[3][NSLOT];            // sum |x| over updated voxels
   unsigned long long cnt[3][4];     // voxel updates, zero skipped, items
@@ -613,8 +614,10 @@ __global__ void __launch_bounds__(SEL_THREADS) k_nhicd_pick(SelArgs S, SelRanks 
   cluster_barrier();  // no CTA leaves while its histogram may be read
 }
 
-// nseg segments of ny x nx values; returns the launches made through *launches
-static cudaError_t nhicd_pick(SelArgs S, const SelRanks *R, int nseg, int sms, float *filt, cudaStream_t st, int *launches) {
+// nseg segments of ny x nx values; returns the launches made through *launches.
+// filt: the filtered maps, where they are formed in memory (`keep`: always)
+static cudaError_t nhicd_pick(SelArgs S, const SelRanks *R, int nseg, int sms, float *filt, bool keep, cudaStream_t st,
+                              int *launches) {
   const size_t seglen = (size_t)S.ny * S.nx;
   // CTAs per segment: enough to share the work, no more than the GPU holds
   // twice, but chunks that fit in shared memory where eight can do that
@@ -625,7 +628,7 @@ static cudaError_t nhicd_pick(SelArgs S, const SelRanks *R, int nseg, int sms, f
   // the GPU idle and chunks are long, all of it filters sooner (16 maps of
   // 256^2: 57 us here, 47 with the filter kernel; 32 of them: 53 and 61 an
   // iteration chunk; 4 of 128^2 30 either way)
-  const int fill = S.chunk <= (nseg * nc >= sms ? 8192 : 2048) ? 2 : S.chunk <= 49152 ? 1 : 0;
+  const int fill = !keep && S.chunk <= (nseg * nc >= sms ? 8192 : 2048) ? 2 : S.chunk <= 49152 ? 1 : 0;
   *launches = 1;
   if (fill < 2) {
     const size_t n = (size_t)nseg * seglen;
@@ -2069,7 +2072,7 @@ static int nhicd_select_device(xtg_ctx *c, int *cnt) {
   S.list1 = c->d_nh + S.cap0;
   S.cnt = cnt;
   int nl = 0;
-  CK(nhicd_pick(S, nullptr, g.N_time * g.nzb, c->sm_count, c->d_filt, c->st, &nl));
+  CK(nhicd_pick(S, nullptr, g.N_time * g.nzb, c->sm_count, c->d_filt, false, c->st, &nl));
   c->launches += nl;
   return 0;
 }
@@ -2462,9 +2465,6 @@ int xtg_nhicd_select(xtg_ctx *c, const int32_t *usn, int32_t *nnum, int32_t *xse
       return XTG_E_ARG;
     }
   CK(cudaMemcpyAsync(c->d_kth, kth.data(), nseg * 4, cudaMemcpyHostToDevice, c->st));
-  const unsigned grid = std::min<unsigned>(blocks_for(c->nmag, 256), (unsigned)c->sm_count * 8);
-  k_vsc_filter<<<grid, 256, 0, c->st>>>(nseg, g.N_y, g.N_x, c->d_mag, c->d_filt);
-  CK(cudaGetLastError());
   SelArgs S;
   memset(&S, 0, sizeof(S));
   S.map = c->d_mag;
@@ -2473,8 +2473,8 @@ int xtg_nhicd_select(xtg_ctx *c, const int32_t *usn, int32_t *nnum, int32_t *xse
   S.kth_dev = c->d_kth;
   S.thr = c->d_thr;
   int nl = 0;
-  CK(nhicd_pick(S, nullptr, nseg, c->sm_count, c->d_filt, c->st, &nl));
-  c->launches += 1 + nl;
+  CK(nhicd_pick(S, nullptr, nseg, c->sm_count, c->d_filt, true, c->st, &nl));
+  c->launches += nl;
   std::vector<float> th(nseg), f(c->nmag);
   CK(cudaMemcpyAsync(th.data(), c->d_thr, nseg * 4, cudaMemcpyDeviceToHost, c->st));
   CK(cudaMemcpyAsync(f.data(), c->d_filt, c->nmag * 4, cudaMemcpyDeviceToHost, c->st));
@@ -2572,6 +2572,6 @@ extern "C" int xtg_nhicd_threshold_noalloc(const float *magmap, int32_t nmaps, i
   S.thr = thresholds;
   S.sel = select;
   int nl = 0;
-  CK(nhicd_pick(S, &r, nmaps, 148, filt, st, &nl));
+  CK(nhicd_pick(S, &r, nmaps, 148, filt, false, st, &nl));
   return 0;
 }

@@ -65,7 +65,6 @@ void up_back(int nb, int Y, int X, int Z, int Ca, int Cb, const float *dout, flo
 // dpost: rows of ld floats, the C channels from off on; pooled (or null): gradient of the 2x pooling of the same layer
 void relu_back(int nb, int Y, int X, int Z, int C, const float *dpost, int ld, int off, const float *pooled,
                const __nv_bfloat16 *post, __nv_bfloat16 *dpre, float *dbias, cudaStream_t st);
-void to_f32(long long n, const __nv_bfloat16 *a, float *b, cudaStream_t st);
 void head(long long nv, int C, const __nv_bfloat16 *h, const float *w, const float *bias, const float *base, float scale,
           float *y, cudaStream_t st);
 void head_train(long long nv, const __nv_bfloat16 *h, const float *w, const float *bias, const float *base, float scale,

@@ -77,12 +77,6 @@ __device__ __forceinline__ float4 ld_w(const float *p, bool keep) {
 // Asynchronous global -> shared copies (no registers held while in flight);
 // cp_wait_all completes the calling thread's copies and makes them visible to it.
 __device__ __forceinline__ uint32_t icd_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void cp_async16(void *s, const void *g) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(icd_smem(s)), "l"(g) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void *s, const void *g) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(icd_smem(s)), "l"(g) : "memory");
-}
 __device__ __forceinline__ void cp_async4(void *s, const void *g) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(icd_smem(s)), "l"(g) : "memory");
 }
