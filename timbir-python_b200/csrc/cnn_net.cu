@@ -140,6 +140,7 @@ int check_err(xtc_net *n) {
 // activation buffers for a batch shape, and gradient buffers for training
 int ensure_buffers(xtc_net *n, int nb, int Y, int X, int Z, bool training) {
   if (n->nb == nb && n->Y == Y && n->X == X && n->Z == Z && (n->grads || !training)) return 0;
+  n->nb = 0;  // no shape's buffers, until all of them are there
   const size_t v0 = (size_t)nb * Y * X * Z, v1 = v0 / 8, v2 = v1 / 8, v3 = v2 / 8;
   const size_t lv[kLayers] = {v0, v0, v1, v1, v2, v2, v3, v3, v2, v2, v1, v1, v0, v0};
   if (training) NCK(n->in0.ensure(v0 * 8 * sizeof(bf16)));
