@@ -789,24 +789,26 @@ cudaError_t launch_magmap_zero(const DevGeo &G, const IcdArgs &A, int grid, cuda
 // the fixed work weighs (shift in units of the run-to-run spread, which is 0.05 to
 // 0.3 % of the percentage, without -> with):
 //   one column in 33 for single-row and long items read from a table (128^2 x 9
-//     +1.0 -> +0.8), one in 36 for short ones
+//     +1.0 -> +0.3), one in 36 for short ones
 //   an eighth fewer than are resident for short items with runs of at most 512
-//     entries (256^2 x 16 x 16 frames +1.7 -> +0.7), and for the others where that is
-//     more than one column in 256 (180^2 x 27 +2.1 -> +0.6)
+//     entries (256^2 x 16 x 16 frames +1.7 -> +0.7) and for long ones where that is more
+//     than one column in 256; three sixteenths fewer for single rows above one in 320
+//     (180^2 x 27 +2.1 -> -0.1, 148^2 x 12 +1.8 -> +0.1)
 //   for such runs ten items at a time in the 128-thread class and nine in the
 //     64-thread one above 1536 rows x entries (140^2 x 32, 4 frames +2.6 -> +0.4;
 //     96^2 x 32, 8 frames +3.3 -> +0.4; 96^2 x 16, 4 frames +1.4 -> 0.0)
-// 114 volumes of 64^2 to 512^2, 3 to 80 rows, 1 to 16 frames lie between -1.5 and
+// 114 volumes of 64^2 to 512^2, 3 to 80 rows, 1 to 16 frames lie between -2.2 and
 // +1.8 with it (one of 8 frames with A computed here +2.7), half of them within
 // 0.4.  It costs time: 80^2 x 8, 500 views 1.4 ms an iteration with twice the
-// columns, 2.5 so; 256^2 x 32, 512 views 7.7 and 10.0; 128^2 x 4 1.1 and 1.4.
+// columns, 2.5 so; 256^2 x 32, 512 views 7.7 and 10.0; 128^2 x 4 1.1 and 1.5.
 IcdFlight icd_flight(int vec, int amode, int as, int vmax, int zmax, int zovl, long long columns, int sms) {
   const int rows = zmax * zovl;
   const int unit = vec != 4 || amode == 0 ? XTG_THREADS : rows <= 16 ? 64 : vmax <= 1024 ? 128 : XTG_THREADS;
   // shared memory of such a CTA: run, 128 partial sums twice a warp, neighbourhood
   const size_t smem = (size_t)vmax * (amode == 0 ? 8 + 4 * as : 8) + (size_t)unit * 32 + (size_t)rows * 8 + (size_t)zmax * 48 + 1280;
   long long resident = (long long)sms * std::max(1, std::min(1024 / unit, (int)(228 * 1024 / smem)));
-  if (amode && (unit < XTG_THREADS ? vmax <= 512 : resident * 256 > columns)) resident -= resident / 8;
+  if (amode && vec == 4 && (unit < XTG_THREADS ? vmax <= 512 : resident * 256 > columns)) resident -= resident / 8;
+  if (amode && vec != 4 && resident * 320 > columns) resident -= resident * 3 / 16;
   IcdFlight f;
   f.cols = (int)std::min(resident, std::max(8ll, columns / (amode == 0 ? 32 : unit == XTG_THREADS ? 33 : 36)));
   f.batch = unit == XTG_THREADS ? 1 : vmax > 512 ? 8 : unit == 128 ? 10 : rows * vmax > 1536 ? 9 : 8;
