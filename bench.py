@@ -226,14 +226,19 @@ def network_roofline(ctx, net, coarse_iters, reps=3):
             "frac": flops / ms / 1e9 / peak, "peak_kind": kind, "bound": "tensor"}
 
 
+# bytes of the bin-major A table per A entry: records of two bins, 12 bytes each, 1.57
+# of them for 2.14 entries at voxels one bin wide
+TABLE_BYTES = 12 * 1.57 / 2.14
+
+
 def projector_timing(ctx, reps=3):
     """Forward-projection calls on the resident (zero) object, each through
     the C ABI (which synchronises its stream): e = y - Ax - d in FP32 (the
     reference's order) and the FP64 resync, with the bin-major A table (the
     default where it fits) and with the table-free gather.  Algorithmic HBM
     bytes of one table launch: y read + e written (+ w read for the resync's
-    cost) + 8 B per table entry; the object (a z-line per entry) is re-read
-    from L2 and L1."""
+    cost) + the table (TABLE_BYTES an entry); the object (a z-line per record)
+    is re-read from L2 and L1."""
     import torch
     out = {}
     for kind, key in ((xtg.XTG_PROJ_GATHER, "gather"), (xtg.XTG_PROJ_AUTO, "table")):
@@ -252,7 +257,7 @@ def projector_timing(ctx, reps=3):
             if used == xtg.XTG_PROJ_TABLE:
                 ns = int(np.prod(ctx.sino_shape))
                 peak, _ = peaks()
-                alg = {"init_error_ms": 8.0 * ns + 8.0 * entries, "resync_fp64_ms": 12.0 * ns + 8.0 * entries}
+                alg = {"init_error_ms": 8.0 * ns + TABLE_BYTES * entries, "resync_fp64_ms": 12.0 * ns + TABLE_BYTES * entries}
                 r["table_entries"] = entries
                 r["hbm_gbs_alg"] = {k: alg[k] / (r[k] / 1e3) / 1e9 for k in alg}
                 r["frac_of_measured_hbm"] = {k: alg[k] / (r[k] / 1e3) / 1e9 / peak for k in alg}
@@ -267,7 +272,7 @@ def kernel_timings(args, reps=5):
     the call (the call synchronises the library's stream; the mean of `reps`
     calls), with the algorithmic HBM bytes of one call and their rate against
     the measured copy bandwidth.  Bytes: sinogram arrays 4 B per entry each
-    (e, w, y read; e written), the bin-major A table 8 B per entry, the
+    (e, w, y read; e written), the bin-major A table TABLE_BYTES per entry, the
     object 4 B per voxel (its neighbours come from L1/L2), the NHICD maps
     4 B per value per pass.  The ncu summaries in profiles/ capture the same
     command."""
@@ -288,9 +293,9 @@ def kernel_timings(args, reps=5):
     peak, kind = peaks()
     calls = {
         # name: (call, algorithmic bytes, kernels)
-        "init_error_sino": (ctx.init_error_sino, 8.0 * ns + 8.0 * entries, "k_fp_csr<1>"),
-        "resync_fp64": (ctx.resync_fp64, 12.0 * ns + 8.0 * entries + 4.0 * nvox, "k_fp_csr<2>, k_prior_cost64"),
-        "map_cost_fp64": (ctx.cost, 8.0 * ns + 8.0 * entries + 4.0 * nvox, "k_fp_csr<3>, k_prior_cost64"),
+        "init_error_sino": (ctx.init_error_sino, 8.0 * ns + TABLE_BYTES * entries, "k_fp_csr<1>"),
+        "resync_fp64": (ctx.resync_fp64, 12.0 * ns + TABLE_BYTES * entries + 4.0 * nvox, "k_fp_csr<2>, k_prior_cost64"),
+        "map_cost_fp64": (ctx.cost, 8.0 * ns + TABLE_BYTES * entries + 4.0 * nvox, "k_fp_csr<3>, k_prior_cost64"),
         "map_cost_running": (ctx.cost_running, 8.0 * ns + 4.0 * nvox, "k_running_cost64, k_prior_cost64"),
         "zinger_refresh": (lambda: ctx.zinger_refresh(want_mask=False), 8.0 * ns, "k_zinger_refresh"),
         "nhicd_select": (lambda: ctx.nhicd_select(usn), 4.0 * nmag * 6, "k_vsc_filter, k_nhicd_pick"),

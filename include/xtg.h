@@ -296,8 +296,8 @@ int xtg_update_variance(xtg_ctx *ctx);
  * Work is queued on `stream` (a cudaStream_t, NULL = default stream) and is
  * complete when that stream is.
  * Scratch is one fixed array inside the library, XTG_NOALLOC_MAX_ELEMS floats
- * (4 MiB) plus XTG_NOALLOC_MAX_MAPS ints, held on every GPU that loads the
- * library until the process exits; larger inputs are rejected with XTG_E_ARG.
+ * (4 MiB), held on every GPU that loads the library until the process exits;
+ * larger inputs are rejected with XTG_E_ARG.
  * The first call on a device resolves the array's device address
  * (cudaGetSymbolAddress), so make that first call before any stream capture.
  * All calls share the array: calls that overlap on the GPU (other streams,
@@ -317,7 +317,9 @@ int64_t xtg_device_bytes(const xtg_ctx *ctx);
 int64_t xtg_launch_count(const xtg_ctx *ctx);
 /* Device time (ms) of the ICD column kernel in the last xtg_icd_iteration /
  * xtg_update_columns call, the random-pass column work items it processed and
- * the number of ICD kernel launches it issued. */
+ * the number of ICD kernel launches it issued.  In the parallel schedule of an
+ * iteration, launches with nothing queued between them (a chunk's two half-passes
+ * and the next chunk's) are timed as one run, the gaps between them included. */
 int xtg_last_kernel_time(const xtg_ctx *ctx, float *ms, int64_t *items, int64_t *launches);
 
 #ifdef __cplusplus

@@ -29,11 +29,12 @@ int xtc_conv3d(const void *in, const void *w, const float *bias, void *out, int3
                int32_t Z, int32_t cin, int32_t cout, int32_t kpad, int32_t epi, int32_t sign);
 
 /* xtc_conv3d with the kernel chosen: XTC_CONV_AUTO (what xtc_conv3d does), XTC_CONV_GATHER (operands
- * gathered per K stage by the CTA's threads) or XTC_CONV_TILE (input tile staged once by TMA, every tap
- * a shifted view of it; X a multiple of 128, Z even, cout <= 64, else XTG_E_ARG).  AUTO uses the tile
- * kernel wherever it applies, else, with cin a multiple of 16, boxes of 128 voxels staged by TMA per tap
- * (the gather kernel's sums in its order).  The packed weights go to one buffer the library keeps; calls
- * that use it take turns. */
+ * gathered per K stage by the CTA's threads) or XTC_CONV_TILE (a tile's input halo staged a y-row at a
+ * time by loader warps, every tap a shifted view of it; X a multiple of 128, Z even, cout <= 64, else
+ * XTG_E_ARG).  AUTO uses the tile kernel wherever it applies, else, with cin and cout multiples of 16,
+ * halo tiles of 8 z x 16 x voxels staged by TMA once for nine taps, or boxes of 128 voxels per tap where
+ * the planes are too small for those (both the gather kernel's sums in its order).  The packed weights go
+ * to a buffer that the library keeps per device; calls that use it take turns. */
 enum { XTC_CONV_AUTO = 0, XTC_CONV_GATHER = 1, XTC_CONV_TILE = 2 };
 int xtc_conv3d_path(const void *in, const void *w, const float *bias, void *out, int32_t nb, int32_t Y, int32_t X,
                     int32_t Z, int32_t cin, int32_t cout, int32_t kpad, int32_t epi, int32_t sign, int32_t path);
@@ -46,8 +47,8 @@ int xtc_conv3d_wgrad(const void *in, const void *dout, float *dw, int32_t nb, in
  * (operands gathered and transposed per K stage by the CTA's threads) or XTC_CONV_TILE (dout and the input
  * halo staged by TMA per tile of 128 x 2 voxels, the three dy taps stacked along M and the three dz taps
  * along N of each MMA; cout 32, cin a multiple of 16, X a multiple of 128, Z even, else XTG_E_ARG).  AUTO
- * uses the tile kernel wherever it applies, else, with cin a multiple of 16 and cout up to 96, boxes of 128
- * voxels staged by TMA per tap. */
+ * uses the tile kernel wherever it applies, else, with cin a multiple of 16 and cout up to 96, halo tiles
+ * or boxes of 128 voxels staged by TMA, as above. */
 int xtc_conv3d_wgrad_path(const void *in, const void *dout, float *dw, int32_t nb, int32_t Y, int32_t X, int32_t Z,
                           int32_t cin, int32_t cout, int32_t path);
 

@@ -327,9 +327,9 @@ cudaError_t launch_csr_build(const DevGeo &G, const CsrBuildArgs &B, int fill, i
 // 0.53 ms.
 // (s0, s1) += (x0, x1) a, product and sum each rounded, two rows per
 // instruction.  The product is a multiply-add of -0, which leaves it as it is
-// (neg0 is an argument so that nothing knows its value): a packed multiply
-// followed by a packed add comes out of the assembler as one multiply-add with
-// one rounding, whatever rounding the two ask for.
+// (neg0 is an argument so that nothing knows its value): with a packed multiply
+// and a packed add the sums had one rounding a term and not the reference's bits,
+// as k_fp_bins shows them.
 __device__ __forceinline__ void mul_add2(float &s0, float &s1, float x0, float x1, float a, float neg0) {
   asm("{\n\t.reg .b64 x, a, s, z;\n\t"
       "mov.b64 x, {%2, %3};\n\tmov.b64 a, {%4, %4};\n\tmov.b64 s, {%0, %1};\n\tmov.b64 z, {%5, %5};\n\t"
